@@ -181,6 +181,9 @@ _SIGNATURES["sm100"]["ti_attention_prefill_pair_bf16"] = [
 _SIGNATURES["sm100"]["ti_attention_prefill_tc_bf16"] = [
     c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
     c_float, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p]
+_SIGNATURES["f32"] = {
+    "ti_gemm_f32_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+}
 PREFILL_TILE = 256        # most query rows per CTA of the prefill attention kernels (two tiles of 128)
 PAIR_MIN_CTAS = 148       # fewer CTAs than this of the two-tile kernel: its tiles run as halves, one a CTA
 KEY_SPLIT_MAX_CTAS = 148  # at most half as many CTAs of the one-tile kernel: the keys are shared out over CTAs as well
@@ -258,6 +261,19 @@ def _tensor_core_ok(x: torch.Tensor, w: torch.Tensor, *others) -> bool:
     if x.dtype != torch.bfloat16 or x.shape[1] % 8:
         return False
     return all(t is None or t.data_ptr() % 16 == 0 for t in (x, w) + others)
+
+
+F32_FEW_ROWS = 8          # up to so many rows a float32 product streams its weights past the rows of x held in registers
+F32_MIN_K = 256           # below, the general kernel's few steps are as quick, and its sums have one order for any number of rows
+
+
+def _float32_product(out, x, w, bias, residual, m, n, k, gated) -> bool:
+    """Runs a float32 product on the kernel made for its size, if there is one; False: the general kernel is to run it.
+    The weights are read 16 bytes at a time: whole rows of them, on 16-byte boundaries."""
+    if x.dtype != torch.float32 or k % 4 or k < F32_MIN_K or not 1 <= m <= F32_FEW_ROWS or (x.data_ptr() | w.data_ptr()) % 16:
+        return False
+    _run("f32", "ti_gemm_f32_few", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), m, n, k, gated, _stream())
+    return True
 
 
 def _fn(lib_name: str, name: str):
@@ -496,6 +512,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
              m, n, k, 0, int(out_float32), ws.data_ptr(), ws.numel(), counters.data_ptr(), counters.numel(),
              kernel_status(x.device).data_ptr(), _stream())
         return (out, None) if wants_link else out
+    if _float32_product(out, x, w, bias, residual, m, n, k, 0):
+        return (out, None) if wants_link else out
     _run("core", "ti_gemm_simt", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual),
          m, n, k, 0, int(out_float32 and x.dtype != torch.float32), _dtype_code(x), _stream())
     return (out, None) if wants_link else out
@@ -535,6 +553,8 @@ def gated_linear(x: torch.Tensor, w_gate_up: torch.Tensor, *, link: Optional[Nor
         _run("sm100", "ti_gemm_bf16", out.data_ptr(), x.data_ptr(), w_gate_up.data_ptr(), _ptr(bias), None,
              m, inter, k, act, 0, ws.data_ptr(), ws.numel(), counters.data_ptr(), counters.numel(),
              kernel_status(x.device).data_ptr(), _stream())
+        return out
+    if _float32_product(out, x, w_gate_up, bias, None, m, inter, k, act):
         return out
     _run("core", "ti_gemm_simt", out.data_ptr(), x.data_ptr(), w_gate_up.data_ptr(), _ptr(bias), None,
          m, inter, k, act, 0, _dtype_code(x), _stream())
