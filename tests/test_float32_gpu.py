@@ -1,11 +1,17 @@
 """Kernels of the 32-bit path on the GPU against 64-bit references, with bounds that follow from the number of roundings."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
-from test_kernels_gpu import ops, rnd  # noqa: F401  (the fixture)
+from test_kernels_gpu import ops, fill_cache, paged_setup, rnd  # noqa: F401  (the fixture and the paged caches)
 
 pytestmark = pytest.mark.gpu
 EPS = 2.0 ** -24
+
+
+def dev():
+    return torch.device("cuda:0")
 
 
 def gated(z, act):
@@ -44,3 +50,69 @@ def test_product_of_few_rows_does_not_depend_on_the_rows(ops):
     whole = ops.linear(x, w)
     for m in (1, 2, 3, 4, 6):
         assert torch.equal(ops.linear(x[:m].contiguous(), w), whole[:m])
+
+
+ATTENTION = [
+    # hq, hkv, d, page, window, [(context, q_len)]
+    (16, 8, 128, 64, None, [(333, 333), (1025, 1), (1, 1), (64, 1), (257, 1)]),
+    (4, 4, 64, 16, None, [(130, 130), (129, 1), (200, 2), (2300, 1)]),
+    (12, 4, 128, 48, 40, [(300, 44), (65, 1), (64, 1), (700, 301)]),
+    (32, 1, 64, 64, -50, [(149, 99), (150, 1), (151, 1), (333, 17)]),
+    (6, 1, 128, 5, None, [(91, 1), (64, 64), (65, 64)]),
+]
+
+
+@pytest.mark.parametrize("hq,hkv,d,page,window,work", ATTENTION)
+def test_attention(ops, hq, hkv, d, page, window, work):
+    lens = [c for c, _ in work]
+    bt, kv = paged_setup(torch.float32, lens, hq, hkv, d, page, seed=1)
+    ks, vs = fill_cache(kv, bt, lens, hkv, d, page, torch.float32)
+    q_lens, starts = [n for _, n in work], [c - n for c, n in work]
+    rows, tiles, pairs = ops.plan_attention(q_lens, starts)
+    step = SimpleNamespace(decode_rows=torch.tensor(rows or [0], dtype=torch.int32, device=dev()), num_decode=len(rows),
+                           prefill_tiles=torch.tensor(tiles or [0], dtype=torch.int32, device=dev()),
+                           num_prefill_tiles=len(tiles) // 4, num_pair_tiles=pairs, max_context=max(lens))
+    pos = torch.tensor([p for c, n in work for p in range(c - n, c)], dtype=torch.int32, device=dev())
+    seq = torch.tensor([i for i, (c, n) in enumerate(work) for _ in range(n)], dtype=torch.int32, device=dev())
+    q = rnd(pos.shape[0], hq, d, dtype=torch.float32, seed=7)
+    status = torch.zeros(1, dtype=torch.int32, device=dev())
+    mask = dict(window=window) if (window or 0) >= 0 else dict(chunk=-window)
+    out = ops.paged_attention(q, kv, positions=pos, token_seq=seq, block_table=bt, scale=d ** -0.5, step=step, status=status,
+                              **mask)
+    assert int(status.item()) == 0
+    got, row = out.view(-1, hq, d).double(), 0
+    for i, (c, n) in enumerate(work):
+        k, v = (x[i].double().repeat_interleave(hq // hkv, dim=1) for x in (ks, vs))
+        p, j = torch.arange(c - n, c, device=dev())[:, None], torch.arange(c, device=dev())[None]
+        lo = torch.zeros_like(p) if not window else p - window + 1 if window > 0 else p - p % -window
+        z = torch.einsum("nhd,lhd->hnl", q[row:row + n].double(), k) * d ** -0.5
+        a = torch.softmax(z.masked_fill((j > p) | (j < lo), float("-inf")), dim=-1)
+        want = torch.einsum("hnl,lhd->nhd", a, v)
+        # a score is off by at most d roundings of sum |q||k| (some 0.7 d^1/2 here), a probability by that factor, and the
+        # sums over the keys, of at most |v| = 5, by c / 8 roundings
+        assert (got[row:row + n] - want).abs().max() <= EPS * 5 * (2 * d + c / 8 + 16)
+        row += n
+
+
+def test_attention_reports_a_key_without_a_page_and_keeps_rows_apart(ops):
+    """A missing page is reported and its keys are left out; infinities of a later token of the portion do not reach the
+    tokens before it."""
+    hq, hkv, d, page = 4, 2, 64, 16
+    bt, kv = paged_setup(torch.float32, [40, 40], hq, hkv, d, page, seed=1)
+    fill_cache(kv, bt, [40, 40], hkv, d, page, torch.float32)
+    q = rnd(21, hq, d, dtype=torch.float32, seed=3)
+    rows, tiles, pairs = ops.plan_attention([20, 1], [20, 39])
+    step = SimpleNamespace(decode_rows=torch.tensor(rows, dtype=torch.int32, device=dev()), num_decode=1,
+                           prefill_tiles=torch.tensor(tiles, dtype=torch.int32, device=dev()), num_prefill_tiles=1,
+                           num_pair_tiles=pairs, max_context=40)
+    args = dict(positions=torch.tensor(list(range(20, 40)) + [39], dtype=torch.int32, device=dev()),
+                token_seq=torch.tensor([0] * 20 + [1], dtype=torch.int32, device=dev()), scale=0.125, step=step)
+    status = torch.zeros(1, dtype=torch.int32, device=dev())
+    want = ops.paged_attention(q, kv, block_table=bt, status=status, **args)
+    assert int(status.item()) == 0
+    kv[:, int(bt[0, 38 // page]), :, 38 % page] = float("inf")
+    got = ops.paged_attention(q, kv, block_table=bt, status=status, **args)
+    assert torch.equal(got[:18], want[:18]) and torch.equal(got[20], want[20]) and not torch.isfinite(got[18:20]).all()
+    bt[1, 0] = -1
+    got = ops.paged_attention(q, kv, block_table=bt, status=status, **args)
+    assert int(status.item()) == 2 and torch.isfinite(got[20]).all() and torch.equal(got[:18], want[:18])

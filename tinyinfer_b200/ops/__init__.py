@@ -183,6 +183,8 @@ _SIGNATURES["sm100"]["ti_attention_prefill_tc_bf16"] = [
     c_float, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p]
 _SIGNATURES["f32"] = {
     "ti_gemm_f32_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "ti_attention_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
+                         c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
 }
 PREFILL_TILE = 256        # most query rows per CTA of the prefill attention kernels (two tiles of 128)
 PAIR_MIN_CTAS = 148       # fewer CTAs than this of the two-tile kernel: its tiles run as halves, one a CTA
@@ -671,6 +673,14 @@ def attention_tensor_cores_ok(q: torch.Tensor, kv_cache: torch.Tensor, maps: int
             and (page in (16, 32) or page % 64 == 0))
 
 
+def attention_float32_ok(q: torch.Tensor, kv_cache: torch.Tensor) -> bool:
+    """The float32 attention kernels take head sizes 64 and 128 and up to 32 query heads per kv head."""
+    _, hq, d = q.shape
+    hkv = kv_cache.shape[2]
+    return (q.dtype == torch.float32 and d in (64, 128) and hq % hkv == 0 and hq // hkv <= 32
+            and (q.data_ptr() | kv_cache.data_ptr()) % 16 == 0)
+
+
 _generic_warned = set()
 
 
@@ -797,6 +807,12 @@ def paged_attention(q: torch.Tensor, kv_cache: torch.Tensor, *, positions: torch
                                   scale=scale, sink=sink, window=window, chunk=chunk, out_scale=out_scale, status=status,
                                   head_sinks=head_sinks, gate=gate, gate_offset=gate_offset, softcap=softcap,
                                   keep_first=keep_first, feature_gate=feature_gate, difference=difference)
+        if step is not None and attention_float32_ok(q, kv_cache):      # without the step's split nothing is read back for it
+            _run("f32", "ti_attention_f32", out.data_ptr(), q.data_ptr(), kv_cache.data_ptr(), positions.data_ptr(),
+                 token_seq.data_ptr(), step.decode_rows.data_ptr(), step.num_decode, step.prefill_tiles.data_ptr(),
+                 step.num_prefill_tiles, min(t, PREFILL_TILE), block_table.data_ptr(), block_table.shape[1], hq, hkv, d,
+                 page_size, num_pages, float(scale), mask, _ptr(status), _stream())
+            return out
         _run("core", "ti_attention_generic", out.data_ptr(), q.data_ptr(), kv_cache.data_ptr(),
              positions.data_ptr(), token_seq.data_ptr(), block_table.data_ptr(), block_table.shape[1],
              t, hq, hkv, d, page_size, num_pages, float(scale), mask, _ptr(status),

@@ -36,8 +36,8 @@ LIBRARIES: Dict[str, dict] = {
     "core": dict(sources=["runtime.cu", "elementwise.cu", "rope_append.cu",
                           "attention_generic.cu", "gemm_simt.cu", "sampling.cu"],
                  headers=["common.cuh"], link=[]),
-    # the 32-bit path at the sizes it is used at: products
-    "f32": dict(sources=["runtime.cu", "gemm_f32_few.cu"], headers=["common.cuh"], link=[]),
+    # the 32-bit path at the sizes it is used at: products and attention
+    "f32": dict(sources=["runtime.cu", "gemm_f32_few.cu", "attention_f32.cu"], headers=["common.cuh"], link=[]),
     # parts of designs with a cached latent, gated recurrences and routed experts around a float32 stream
     "latent": dict(sources=["runtime.cu", "stream.cu", "gemm_batched.cu", "latent_attention.cu",
                             "latent_attention_mma.cu", "recurrent.cu"],
