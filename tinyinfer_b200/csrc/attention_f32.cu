@@ -10,8 +10,8 @@
 // Portions of prompts: a block takes 32 query rows, which are the query heads of one kv head for 32 / G neighbouring tokens,
 // over tiles of 64 keys: keys and values come in by cp.async, the values' copy runs under the scores. 256 threads make 2 x 4
 // scores and 2 x (D / 16) outputs each. Bound by shared-memory reads beside the multiply-adds.
-// A layer of 16 over 8 heads of 128: 333 prompt tokens 0.8 ms with a block a (token, head) -> 0.28 ms or less (as seen with
-// its wait for the kernel ahead).
+// A layer of 16 over 8 heads of 128: 333 prompt tokens 0.8 ms with a block a (token, head) -> 53 us; 4 tokens behind 1,024 keys
+// 32 us with the queries in registers and one block an SM -> 13 us with them in shared memory and two.
 #include "common.cuh"
 #include <cooperative_groups.h>
 #include <type_traits>
@@ -39,11 +39,13 @@ __device__ __forceinline__ long long key_row(const AfArgs& a, const int* table, 
 constexpr int DEC_CTAS = 8, DEC_WARPS = 8;
 
 template <int D, int GT>
-__global__ void __cluster_dims__(DEC_CTAS, 1, 1) __launch_bounds__(DEC_WARPS * 32) decode_f32_kernel(const AfArgs a) {
+__global__ void __cluster_dims__(DEC_CTAS, 1, 1) __launch_bounds__(DEC_WARPS * 32, GT <= 2 ? 2 : 1) decode_f32_kernel(const AfArgs a) {
     constexpr int E4 = D / 32;                   // float4s of a head that a lane holds
     constexpr int U = 2;                         // keys of a lane group asked for together
-    __shared__ float wm[DEC_WARPS][GT], wl[DEC_WARPS][GT], wacc[DEC_WARPS][GT][D];
+    __shared__ float wm[DEC_WARPS][GT], wl[DEC_WARPS][GT];
+    __shared__ __align__(16) float wacc[DEC_WARPS][GT][D];
     __shared__ float cm[GT], cl[GT], cacc[GT][D];
+    __shared__ __align__(16) float qs[GT][D];        // read anew for every key: registers for it would cost the second block of an SM
     ti_grid_launch_dependents();
     ti_grid_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7, grp = lane >> 3;
@@ -56,14 +58,12 @@ __global__ void __cluster_dims__(DEC_CTAS, 1, 1) __launch_bounds__(DEC_WARPS * 3
     const int share = ((pos + 1 - lo + DEC_CTAS - 1) / DEC_CTAS + 31) & ~31;
     const int begin = lo + (int)blockIdx.x * share, end = min(pos + 1, begin + share);
 
-    float4 q[GT][E4];
+    for (int i = threadIdx.x; i < GT * D; i += DEC_WARPS * 32)
+        qs[i / D][i % D] = a.q[((size_t)t * a.hq + kvh * G + min(g0 + i / D, G - 1)) * D + i % D];
+    __syncthreads();
     float acc[GT][4 * E4], m[GT], l[GT];
 #pragma unroll
     for (int g = 0; g < GT; ++g) {
-        const int h = kvh * G + min(g0 + g, G - 1);
-        const float4* src = reinterpret_cast<const float4*>(a.q + ((size_t)t * a.hq + h) * D);
-#pragma unroll
-        for (int i = 0; i < E4; ++i) q[g][i] = src[sub + 8 * i];
 #pragma unroll
         for (int i = 0; i < 4 * E4; ++i) acc[g][i] = 0.f;
         m[g] = -INFINITY;
@@ -89,17 +89,21 @@ __global__ void __cluster_dims__(DEC_CTAS, 1, 1) __launch_bounds__(DEC_WARPS * 3
         }
 #pragma unroll
         for (int g = 0; g < GT; ++g) {
-            float s[U], top = m[g];
+            float s[U] = {}, top = m[g];
+#pragma unroll
+            for (int i = 0; i < E4; ++i) {
+                const float4 q = *reinterpret_cast<const float4*>(&qs[g][4 * (sub + 8 * i)]);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    s[u] = fmaf(q.x, kf[u][i].x, s[u]);
+                    s[u] = fmaf(q.y, kf[u][i].y, s[u]);
+                    s[u] = fmaf(q.z, kf[u][i].z, s[u]);
+                    s[u] = fmaf(q.w, kf[u][i].w, s[u]);
+                }
+            }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                float dot = 0.f;
-#pragma unroll
-                for (int i = 0; i < E4; ++i) {
-                    dot = fmaf(q[g][i].x, kf[u][i].x, dot);
-                    dot = fmaf(q[g][i].y, kf[u][i].y, dot);
-                    dot = fmaf(q[g][i].z, kf[u][i].z, dot);
-                    dot = fmaf(q[g][i].w, kf[u][i].w, dot);
-                }
+                float dot = s[u];
 #pragma unroll
                 for (int o = 4; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
                 s[u] = there[u] ? dot * a.scale : -INFINITY;
