@@ -52,6 +52,52 @@ def test_product_of_few_rows_does_not_depend_on_the_rows(ops):
         assert torch.equal(ops.linear(x[:m].contiguous(), w), whole[:m])
 
 
+@pytest.mark.parametrize("m,n,k", [(9, 2, 256), (16, 130, 260), (17, 514, 2048), (48, 96, 6148), (64, 4096, 1024), (127, 64, 320),
+                                   (128, 1000, 2048), (129, 130, 516), (333, 2048, 6144), (300, 12000, 256), (1000, 388, 1100)])
+def test_product_on_the_tensor_cores(ops, m, n, k):
+    # what is cut off of 16 products at a time, in runs of 64 that are added up: fewer roundings than k / 16
+    check_product(ops, m, n, k, k / 16 + 8)
+
+
+def test_split_products_back_to_back(ops):
+    """Products that start while the one before still runs (their weights are on their way long before x is there)."""
+    x, w = rnd(333, 6144, dtype=torch.float32, seed=1), rnd(2048, 6144, dtype=torch.float32, seed=2)
+    outs = [ops.linear(x, w) for _ in range(12)]
+    want = x.double() @ w.double().T
+    assert ((outs[0] - want).norm() / want.norm()).item() < 1e-6
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+
+
+def test_split_product_is_no_less_exact_than_multiply_adds(ops):
+    """Sizes of the 1.7B model against 64 bits, beside the general kernel's sums in k order."""
+    for m, n, k, std in ((333, 2048, 6144, 1.0), (37, 4096, 2048, 0.02), (200, 6144, 2048, 30.0)):
+        x, w = rnd(m, k, dtype=torch.float32, seed=1), rnd(n, k, dtype=torch.float32, seed=2, std=std)
+        want = x.double() @ w.double().T
+        plain = torch.empty((m, n), dtype=torch.float32, device=dev())
+        ops._run("core", "ti_gemm_simt", plain.data_ptr(), x.data_ptr(), w.data_ptr(), None, None, m, n, k, 0, 0, 0, ops._stream())
+        errors = [((y - want).norm() / want.norm()).item() for y in (ops.linear(x, w), plain)]
+        assert errors[0] <= errors[1], errors
+
+
+def test_split_product_takes_infinite_and_tiny_operands_as_multiply_adds_do(ops):
+    m, n, k = 40, 200, 512
+    x, w = rnd(m, k, dtype=torch.float32, seed=1), rnd(n, k, dtype=torch.float32, seed=2)
+    x[3, 7], x[5, 9], w[11, 100], x[20], x[21] = float("inf"), float("nan"), -float("inf"), 0.0, 1e-30
+    w[12] = 3.4e38                                     # rounds to infinity in bfloat16
+    x[22] = 0.0
+    x[22, 0] = 0.5
+    want = (x.double() @ w.double().T)
+    got = ops.linear(x, w)
+    judged = torch.ones_like(want, dtype=torch.bool)
+    judged[:, 12] = False                              # products that overflow on the way, in any order of the sums ...
+    judged[20:23, 12] = True                           # ... but for these rows
+    assert torch.equal(torch.isnan(got)[judged], torch.isnan(want)[judged])
+    assert torch.equal(torch.isinf(got)[judged], torch.isinf(want)[judged])
+    fine = judged & torch.isfinite(want)
+    mass = x.double().abs() @ w.double().abs().T
+    assert ((got - want).abs()[fine] <= EPS * (k / 16 + 8) * mass[fine]).all()
+
+
 ATTENTION = [
     # hq, hkv, d, page, window, [(context, q_len)]
     (16, 8, 128, 64, None, [(333, 333), (1025, 1), (1, 1), (64, 1), (257, 1)]),

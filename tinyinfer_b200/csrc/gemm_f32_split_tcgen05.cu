@@ -4,41 +4,50 @@
 // the multiplier; what is left out is below 2^-25 |a b|, half of what one float32 rounding of the product may cost.
 //
 // The sums decide the precision. The tensor core cuts bits off when it adds to its accumulator, always towards zero, so a
-// long run in one accumulator would drift. Here a run is CHUNK = 2 k blocks of 64, the small parts of a block before the
-// large ones; then the accumulator is added, rounded to nearest, to float32 registers and starts again from zero.
+// long run in one accumulator would drift. Here a run is CHUNK = 2 k blocks of 32, the small parts of a block before the
+// large ones; then the accumulator is added, rounded to nearest, to float32 registers and starts again from zero. Against 64
+// bits, at K = 2048 and 6144: 3.3e-7 of the result's norm, where multiply-adds in k order have 8.1e-7 and 1.4e-6.
 //
 //   weights on the 128 accumulator lanes (gated form: 64 gate rows and the 64 up rows of the same outputs), up to 128 tokens
 //   on the columns; a cluster of S CTAs cuts the k range of a tile where the tiles alone would leave SMs idle, and adds its
 //   parts up in a fixed order through distributed shared memory, each CTA finishing a share of the tokens.
-//   warps 8..15   read the float32 weights (32 bytes a lane, a k block ahead in registers), split them, and write three
-//                 swizzled bfloat16 planes into the stage
-//   warp 16       TMA: the three planes of x, which a small kernel has laid out before ([3][M][Kp])
-//   warp 17       one thread issues the MMAs, 24 of 128 x BN x 16 a k block
+//   warp 16       TMA: the float32 weights, several k blocks ahead
+//   warps 8..13   in pairs, a k block each: take it into registers, split it, write three swizzled bfloat16 planes. (All
+//                 on one block at a time waited for one another's latencies: 0.9 us a block whatever the number of tokens.)
+//   warp 14       TMA: the three planes of x, which a small kernel has laid out before ([3][M][Kp])
+//   warp 15       one thread issues the MMAs, 12 of 128 x BN x 16 a k block
 //   warps 0..7    drain finished chunks into their registers, at the end into shared memory
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
 // multiply-adds in k order, so that such operands give what they give in float32.
-// MEASURED
+// Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 118 us (142 TFLOP/s), by 2,048 x 6,144
+// 799 -> 78 us; 9 rows 306 -> 51 us; 256 x 256 weights, the smallest that come here, 20 -> 5.5 us.
 #include "sm100_ptx.cuh"
+#include <algorithm>
+#include <array>
 #include <cooperative_groups.h>
 
 namespace {
 
-constexpr int BK = 64;                           // bf16 elements of a 128-byte swizzled row
+constexpr int BK = 32;                           // bf16 elements of a 64-byte swizzled row
 constexpr int CHUNK = 2;                         // k blocks a run of the accumulator
 constexpr int MAX_BN = 128;
-constexpr int PLANE_A = 128 * BK * 2;            // 16 KB
-constexpr int MAX_STAGES = 4;
-constexpr int DRAIN_WARPS = 8, SPLIT_WARPS = 8;
-constexpr int NUM_THREADS = (DRAIN_WARPS + SPLIT_WARPS + 2) * 32;
-constexpr int SMEM_BYTES = 227 * 1024;
-constexpr int STAGE_ROOM = SMEM_BYTES - 1024 - 256;          // alignment slack, barriers
+constexpr int PLANE_A = 128 * BK * 2;            // 8 KB
+constexpr int SLOT = 128 * BK * 4;               // float32 weights of a k block
+constexpr int A_STAGES = 3;                      // planes of the weights: stage s belongs to the splitting pair s
+constexpr int MAX_B_STAGES = 6;                  // planes of x: a copy takes about a microsecond to come
+constexpr int MAX_SLOTS = 6;                     // fetched weights; a multiple of A_STAGES, so that a slot too is one pair's: it
+                                                 // sees every phase of the barriers it waits on
+constexpr int DRAIN_WARPS = 8, SPLIT_WARPS = 6, PAIR = SPLIT_WARPS / A_STAGES;
+constexpr int X_WARP = DRAIN_WARPS + SPLIT_WARPS, MMA_WARP = X_WARP + 1, W_WARP = X_WARP + 2;
+constexpr int NUM_THREADS = (W_WARP + 1) * 32;
+constexpr int SMEM_BYTES = 226 * 1024;           // beside the barriers, of 227 KB
 
 struct SplitParams {
     float* out;
     const float *x, *w, *bias, *residual;
     int M, N, K, gated;                          // gated: 0 no, 1 silu, 2 the tanh form of gelu; then w has 2N rows
-    int bn, stages;
+    int bn, b_stages, slots;
     int* status;
 };
 
@@ -76,24 +85,34 @@ __global__ void __launch_bounds__(256) split_rows_kernel(__nv_bfloat16* planes, 
     *reinterpret_cast<uint2*>(planes + 2 * total + i) = p3;
 }
 
+// Shared-memory operand descriptor: K-major tile of rows x 32 bf16, 64-byte swizzle; groups of 8 rows 512 bytes apart.
+__device__ __forceinline__ uint64_t make_sw64_desc(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
+
 __device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
     float v = 0.f;
     for (int k = 0; k < K; ++k) v = fmaf(x[k], w[k], v);
     return v;
 }
 
-__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const SplitParams p) {
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const SplitParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    __shared__ uint64_t bars[2 * MAX_STAGES + 4];
+    __shared__ uint64_t bars[2 * (A_STAGES + MAX_B_STAGES + MAX_SLOTS) + 4];
     __shared__ uint32_t tmem_base_sh;
     __shared__ int abort_sh;
     volatile int* abort_flag = &abort_sh;
     const uint32_t bar0 = smem_u32(bars);
-    auto full_bar = [&](int s) { return bar0 + 8u * s; };
-    auto empty_bar = [&](int s) { return bar0 + 8u * (MAX_STAGES + s); };
-    auto acc_full_bar = [&](int a) { return bar0 + 8u * (2 * MAX_STAGES + a); };
-    auto acc_empty_bar = [&](int a) { return bar0 + 8u * (2 * MAX_STAGES + 2 + a); };
+    auto acc_full_bar = [&](int a) { return bar0 + 8u * a; };
+    auto acc_empty_bar = [&](int a) { return bar0 + 8u * (2 + a); };
+    auto a_full_bar = [&](int s) { return bar0 + 8u * (4 + s); };
+    auto a_empty_bar = [&](int s) { return bar0 + 8u * (4 + A_STAGES + s); };
+    auto b_full_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + s); };
+    auto b_empty_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + MAX_B_STAGES + s); };
+    auto w_full_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + 2 * MAX_B_STAGES + s); };
+    auto w_empty_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + 2 * MAX_B_STAGES + MAX_SLOTS + s); };
 
     ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -103,15 +122,19 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
     const int num_kb = (p.K + BK - 1) / BK;
     const int kb0 = num_kb * part / splits, kb1 = num_kb * (part + 1) / splits;      // at least one each: splits <= num_kb
     const int blocks = kb1 - kb0, chunks = (blocks + CHUNK - 1) / CHUNK;
-    const int plane_b = p.bn * BK * 2, stage_bytes = 3 * (PLANE_A + plane_b);
+    const int plane_b = p.bn * BK * 2;
+    uint8_t* b_ring = smem + A_STAGES * 3 * PLANE_A;
+    uint8_t* slot_ring = b_ring + p.b_stages * 3 * plane_b;
 
     if (threadIdx.x == 0) {
         abort_sh = 0;
-        for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full_bar(s), 1 + SPLIT_WARPS); mbar_init(empty_bar(s), 1); }
+        for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full_bar(s), PAIR); mbar_init(a_empty_bar(s), 1); }
+        for (int s = 0; s < MAX_SLOTS; ++s) { mbar_init(w_full_bar(s), 1); mbar_init(w_empty_bar(s), PAIR); }
+        for (int s = 0; s < MAX_B_STAGES; ++s) { mbar_init(b_full_bar(s), 1); mbar_init(b_empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(acc_full_bar(a), 1); mbar_init(acc_empty_bar(a), DRAIN_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == DRAIN_WARPS + SPLIT_WARPS + 1) tmem_alloc(&tmem_base_sh, 2 * MAX_BN);
+    if (warp == MMA_WARP) tmem_alloc(&tmem_base_sh, 2 * MAX_BN);
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
@@ -123,11 +146,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
         const int group = warp & 3, half = warp >> 2;        // the 32 lanes this warp may read; its part of the columns
         const int units = p.bn / 16, unit0 = half ? (units + 1) / 2 : 0, count = half ? units / 2 : (units + 1) / 2;
         float acc[4][16] = {};
-        bool ok = true;
-        for (int c = 0; c < chunks && ok; ++c) {
+        for (int c = 0; c < chunks; ++c) {
             const int a = c & 1;
             // the whole warp goes on or leaves: what follows is for all 32 lanes
-            if (!__all_sync(0xffffffffu, mbar_wait(acc_full_bar(a), (c >> 1) & 1u, abort_flag, p.status, 81))) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(acc_full_bar(a), (c >> 1) & 1u, abort_flag, p.status, 81))) break;
             tmem_fence_after();
             const uint32_t t = tmem_base + a * MAX_BN + unit0 * 16 + ((uint32_t)(group * 32) << 16);
 #pragma unroll
@@ -143,7 +165,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty_bar(a));
         }
-        ti_grid_wait();                                      // this CTA's outputs are written behind the kernels ahead
         // the last chunk's barrier says that every MMA has read its stage: shared memory is free
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -152,57 +173,49 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
                 for (int i = 0; i < 16; ++i) sums[((unit0 + u) * 16 + i) * 128 + group * 32 + lane] = acc[u][i];
             }
         }
-    } else if (warp < DRAIN_WARPS + SPLIT_WARPS) {
+    } else if (warp < X_WARP) {
         // ------------------------------------------------------------ weights: float32 -> three planes
-        const int t = (int)threadIdx.x - DRAIN_WARPS * 32;
-        const int c = t & 7, row0 = t >> 3;                  // 8 lanes a row of 64 floats, 32 rows at a time
-        const float* src[4];
-        bool there[4];
+        const int s = (warp - DRAIN_WARPS) / PAIR;           // this pair's stage; it takes k blocks s, s + A_STAGES, ...
+        const int t = ((int)threadIdx.x - DRAIN_WARPS * 32) % (PAIR * 32);
+        constexpr int ROWS = PAIR * 8, STEPS = 128 / ROWS;   // 4 lanes a row of 32 floats
+        const int c = t & 3, row0 = t >> 2;
+        uint8_t* a = smem + s * (3 * PLANE_A);
+        int slot = s;
+        uint32_t slot_phase = 0, phase = 0;
+        for (int i = s; i < blocks; i += A_STAGES, phase ^= 1u) {
+            if (!__all_sync(0xffffffffu, mbar_wait(w_full_bar(slot), slot_phase, abort_flag, p.status, 87))) break;
+            const uint8_t* d = slot_ring + slot * SLOT;      // rows of 128 bytes, 128-byte swizzle
+            float4 v[STEPS][2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = row0 + 32 * i;
-            const int o = n0 + (p.gated ? r & 63 : r);
-            there[i] = o < p.N;
-            src[i] = p.w + (size_t)(there[i] ? (p.gated && r >= 64 ? p.N + o : o) : 0) * p.K;
-        }
-        auto load = [&](int kb, float4 (&v)[4][2]) {
-            const int k = kb * BK + c * 8;
+            for (int j = 0; j < STEPS; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-                    v[i][h] = there[i] && kb < kb1 && k + 4 * h < p.K ? __ldg(reinterpret_cast<const float4*>(src[i] + k + 4 * h))
-                                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
-        };
-        float4 cur[4][2], nxt[4][2];
-        load(kb0, cur);
-        int s = 0;
-        uint32_t phase = 0;
-        for (int kb = kb0; kb < kb1; ++kb) {
-            load(kb + 1, nxt);
-            if (!__all_sync(0xffffffffu, mbar_wait(empty_bar(s), phase ^ 1u, abort_flag, p.status, 82))) break;
-            uint8_t* a = smem + s * stage_bytes;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = row0 + 32 * i;
-                uint4 q1, q2, q3;
-                split2(cur[i][0].x, cur[i][0].y, q1.x, q2.x, q3.x);
-                split2(cur[i][0].z, cur[i][0].w, q1.y, q2.y, q3.y);
-                split2(cur[i][1].x, cur[i][1].y, q1.z, q2.z, q3.z);
-                split2(cur[i][1].z, cur[i][1].w, q1.w, q2.w, q3.w);
-                uint8_t* d = a + r * 128 + ((c ^ (r & 7)) << 4);
-                *reinterpret_cast<uint4*>(d) = q1;
-                *reinterpret_cast<uint4*>(d + PLANE_A) = q2;
-                *reinterpret_cast<uint4*>(d + 2 * PLANE_A) = q3;
-            }
+                for (int h = 0; h < 2; ++h) {
+                    const int r = row0 + ROWS * j;
+                    v[j][h] = *reinterpret_cast<const float4*>(d + r * 128 + (((2 * c + h) ^ (r & 7)) << 4));
+                }
+            // the copy that refills the slot is the async proxy's: without this fence the loads above may be put off past it
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(full_bar(s));
+            if (lane == 0) mbar_arrive(w_empty_bar(slot));
+            if ((slot += A_STAGES) >= p.slots) { slot = s; slot_phase ^= 1u; }
+            if (!__all_sync(0xffffffffu, mbar_wait(a_empty_bar(s), phase ^ 1u, abort_flag, p.status, 82))) break;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { cur[i][0] = nxt[i][0]; cur[i][1] = nxt[i][1]; }
-            if (++s == p.stages) { s = 0; phase ^= 1u; }
+            for (int j = 0; j < STEPS; ++j) {
+                const int r = row0 + ROWS * j;
+                uint4 q[3];
+                split2(v[j][0].x, v[j][0].y, q[0].x, q[1].x, q[2].x);
+                split2(v[j][0].z, v[j][0].w, q[0].y, q[1].y, q[2].y);
+                split2(v[j][1].x, v[j][1].y, q[0].z, q[1].z, q[2].z);
+                split2(v[j][1].z, v[j][1].w, q[0].w, q[1].w, q[2].w);
+#pragma unroll
+                for (int plane = 0; plane < 3; ++plane)
+                    *reinterpret_cast<uint4*>(a + plane * PLANE_A + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = q[plane];
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the MMAs read what was written
+            __syncwarp();
+            if (lane == 0) mbar_arrive(a_full_bar(s));
         }
-    } else if (warp == DRAIN_WARPS + SPLIT_WARPS) {
+    } else if (warp == X_WARP) {
         // ------------------------------------------------------------ TMA: the planes of x
         if (lane == 0) {
             ti_grid_wait();
@@ -210,14 +223,34 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
             uint32_t phase = 0;
             bool ok = true;
             for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(empty_bar(s), phase ^ 1u, abort_flag, p.status, 83)) { ok = false; break; }
-                mbar_expect_tx(full_bar(s), 3 * plane_b);
-                const uint32_t b = smem_u32(smem + s * stage_bytes) + 3 * PLANE_A;
+                if (!mbar_wait(b_empty_bar(s), phase ^ 1u, abort_flag, p.status, 83)) { ok = false; break; }
+                mbar_expect_tx(b_full_bar(s), 3 * plane_b);
+                const uint32_t b = smem_u32(b_ring) + s * 3 * plane_b;
                 // rows past M of a plane are the next plane's, or zeros: columns that nothing reads
-                for (int q = 0; q < 3; ++q) tma_load_2d(b + q * plane_b, &map_x, full_bar(s), kb * BK, q * p.M + m0);
-                if (++s == p.stages) { s = 0; phase ^= 1u; }
+                for (int q = 0; q < 3; ++q) tma_load_2d(b + q * plane_b, &map_x, b_full_bar(s), kb * BK, q * p.M + m0);
+                if (++s == p.b_stages) { s = 0; phase ^= 1u; }
             }
             if (!ok) {       // give the copies still in flight time to land before shared memory is given up
+                const unsigned long long t0 = global_ns();
+                while (global_ns() - t0 < 1000000ull) {}
+            }
+        }
+    } else if (warp == W_WARP) {
+        // ------------------------------------------------------------ TMA: the weights, which no earlier kernel writes
+        if (lane == 0) {
+            int slot = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                if (!mbar_wait(w_empty_bar(slot), phase ^ 1u, abort_flag, p.status, 88)) { ok = false; break; }
+                mbar_expect_tx(w_full_bar(slot), SLOT);
+                const uint32_t d = smem_u32(slot_ring) + slot * SLOT;
+                // rows past N are the other half's, or zeros: outputs that nothing stores
+                tma_load_2d(d, &map_w, w_full_bar(slot), kb * BK, n0);
+                tma_load_2d(d + SLOT / 2, &map_w, w_full_bar(slot), kb * BK, p.gated ? p.N + n0 : n0 + 64);
+                if (++slot == p.slots) { slot = 0; phase ^= 1u; }
+            }
+            if (!ok) {
                 const unsigned long long t0 = global_ns();
                 while (global_ns() - t0 < 1000000ull) {}
             }
@@ -225,8 +258,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
     } else if (lane == 0) {
         // ------------------------------------------------------------ MMA issuer
         const uint32_t idesc = make_idesc(128, p.bn);
-        int s = 0, kb = 0;
-        uint32_t phase = 0;
+        int sa = 0, sb = 0, kb = 0;
+        uint32_t phase_a = 0, phase_b = 0;
         bool ok = true;
         for (int c = 0; c < chunks && ok; ++c) {
             const int a = c & 1;
@@ -235,14 +268,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
             const uint32_t d = tmem_base + a * MAX_BN;
             uint32_t accumulate = 0;
             for (int j = 0; j < CHUNK && kb < blocks; ++j, ++kb) {
-                if (!mbar_wait(full_bar(s), phase, abort_flag, p.status, 85)) { ok = false; break; }
+                if (!mbar_wait(b_full_bar(sb), phase_b, abort_flag, p.status, 85) ||
+                    !mbar_wait(a_full_bar(sa), phase_a, abort_flag, p.status, 86)) { ok = false; break; }
                 tmem_fence_after();
-                const uint32_t addr = smem_u32(smem + s * stage_bytes);
+                const uint32_t addr = smem_u32(smem) + sa * (3 * PLANE_A), addr_b = smem_u32(b_ring) + sb * 3 * plane_b;
                 uint64_t A[3], B[3];
 #pragma unroll
                 for (int q = 0; q < 3; ++q) {
-                    A[q] = make_sw128_desc(addr + q * PLANE_A);
-                    B[q] = make_sw128_desc(addr + 3 * PLANE_A + q * plane_b);
+                    A[q] = make_sw64_desc(addr + q * PLANE_A);
+                    B[q] = make_sw64_desc(addr_b + q * plane_b);
                 }
                 auto products = [&](int qa, int qb) {
 #pragma unroll
@@ -254,8 +288,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
                 products(1, 1); products(0, 2); products(2, 0);          // the small ones first
                 products(0, 1); products(1, 0);
                 products(0, 0);
-                umma_commit(empty_bar(s));
-                if (++s == p.stages) { s = 0; phase ^= 1u; }
+                umma_commit(a_empty_bar(sa));
+                umma_commit(b_empty_bar(sb));
+                if (++sa == A_STAGES) { sa = 0; phase_a ^= 1u; }
+                if (++sb == p.b_stages) { sb = 0; phase_b ^= 1u; }
             }
             if (ok) umma_commit(acc_full_bar(a));
         }
@@ -269,47 +305,90 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_split_kernel(const __
     else __syncthreads();
     const int c0 = p.bn * part / splits, c1 = p.bn * (part + 1) / splits;
     if (!*abort_flag) {
-        ti_grid_wait();
-        for (int i = threadIdx.x; i < (c1 - c0) * outs; i += NUM_THREADS) {
-            const int col = c0 + i / outs, o = i % outs, m = m0 + col, n = n0 + o;
+        ti_grid_wait();                                      // out and residual belong to the kernels ahead until now
+        const int quads = outs / 4;                          // four neighbouring outputs a thread
+        for (int i = threadIdx.x; i < (c1 - c0) * quads; i += NUM_THREADS) {
+            const int col = c0 + i / quads, o = i % quads * 4, m = m0 + col, n = n0 + o;
             if (m >= p.M || n >= p.N) continue;
-            auto total = [&](int row, int w_row) {
-                float v = 0.f;
-                for (int r = 0; r < splits; ++r) v += *cluster.map_shared_rank(sums + col * 128 + row, r);
-                return isfinite(v) ? v : plain_dot(p.x + (size_t)m * p.K, p.w + (size_t)w_row * p.K, p.K);
-            };
-            float v = total(o, n);
-            if (p.bias) v += p.bias[n];
-            if (p.gated) {
-                float up = total(64 + o, p.N + n);
-                if (p.bias) up += p.bias[p.N + n];
-                if (p.gated == 1) v = v / (1.f + expf(-v));
-                else v = 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-                v *= up;
-            } else if (p.residual) {
-                v += p.residual[(size_t)m * p.N + n];
+            float total[2][4] = {};
+            const int kinds = p.gated ? 2 : 1;
+            for (int g = 0; g < kinds; ++g) {
+                float4 f[8];
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                    if (r < splits) f[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums + col * 128 + o + 64 * g, r));
+#pragma unroll
+                for (int r = 0; r < 8; ++r)
+                    if (r < splits) {
+                        total[g][0] += f[r].x; total[g][1] += f[r].y; total[g][2] += f[r].z; total[g][3] += f[r].w;
+                    }
             }
-            p.out[(size_t)m * p.N + n] = v;
+            float res[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (n + e >= p.N) { res[e] = 0.f; continue; }
+                auto finite = [&](float v, int w_row) {
+                    return isfinite(v) ? v : plain_dot(p.x + (size_t)m * p.K, p.w + (size_t)w_row * p.K, p.K);
+                };
+                float v = finite(total[0][e], n + e);
+                if (p.bias) v += p.bias[n + e];
+                if (p.gated) {
+                    float up = finite(total[1][e], p.N + n + e);
+                    if (p.bias) up += p.bias[p.N + n + e];
+                    if (p.gated == 1) v = v / (1.f + expf(-v));
+                    else v = 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
+                    v *= up;
+                } else if (p.residual) {
+                    v += p.residual[(size_t)m * p.N + n + e];
+                }
+                res[e] = v;
+            }
+            float* dst = p.out + (size_t)m * p.N + n;
+            if (p.N % 4 == 0 && ((uintptr_t)p.out & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(res[0], res[1], res[2], res[3]);
+            else
+                for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = res[e];
         }
     }
     tmem_fence_before();
     if (splits > 1) cluster.sync();                          // nobody leaves while its sums may be read
     else __syncthreads();
-    if (warp == DRAIN_WARPS + SPLIT_WARPS + 1) {
+    if (warp == MMA_WARP) {
         tmem_fence_after();
         tmem_dealloc(tmem_base, 2 * MAX_BN);
     }
 }
 
+// How many clusters of s CTAs the device holds at a time (a cluster lies within one GPC, so some sizes leave SMs unused).
+int resident_clusters(int s) {
+    static const std::array<int, 9> counts = [] {
+        std::array<int, 9> n{};
+        for (int c = 1; c <= 8; ++c) {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(c);
+            cfg.blockDim = NUM_THREADS;
+            cfg.dynamicSmemBytes = SMEM_BYTES;
+            cudaLaunchAttribute attr;
+            attr.id = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x = c;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs = &attr;
+            cfg.numAttrs = 1;
+            int got = 0;
+            n[c] = cudaOccupancyMaxActiveClusters(&got, gemm_f32_split_kernel, &cfg) == cudaSuccess && got > 0 ? got : std::max(1, ti_sm_count() / (2 * c));
+        }
+        cudaGetLastError();
+        return n;
+    }();
+    return counts[s];
+}
 // How many CTAs share a tile's k range: the count with the least time, in k blocks and with some for the start and the end
-// of a CTA, over the waves it makes. A cluster lies within a GPC of 18 SMs at most, so some counts leave SMs unused.
+// of a CTA, over the waves it makes.
 int choose_splits(int tiles, int num_kb) {
     int best = 1;
     double least = 1e30;
     for (int s = 1; s <= 8 && s <= num_kb; ++s) {
-        const int sms = s <= 2 ? ti_sm_count() / s * s : 18 / s * s * 8;
-        const int waves = (tiles * s + sms - 1) / sms;
-        const double cost = waves * ((double)((num_kb + s - 1) / s) + 4.0);
+        const int waves = (tiles + resident_clusters(s) - 1) / resident_clusters(s);
+        const double cost = waves * ((double)((num_kb + s - 1) / s) + 12.0);
         if (cost < least * 0.999) { least = cost; best = s; }
     }
     return best;
@@ -324,23 +403,39 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
     TI_REQUIRE(M >= 1 && N > 0 && K > 0 && K % 4 == 0, "gemm_f32_split: bad sizes M=%d N=%d K=%d", M, N, K);
     TI_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)planes) % 16 == 0, "gemm_f32_split: operands must lie on 16-byte boundaries");
     TI_REQUIRE(!(gated && residual), "gemm: the gated form takes no residual");
-    const int Kp = (K + BK - 1) / BK * BK;
-    SplitParams p{out, x, w, bias, residual, M, N, K, gated, 0, 0, status};
+    const int Kp = (K + 63) / 64 * 64;
+    SplitParams p{out, x, w, bias, residual, M, N, K, gated, 0, 0, 0, status};
     const int row_tiles = (M + MAX_BN - 1) / MAX_BN;
     p.bn = ((M + row_tiles - 1) / row_tiles + 15) / 16 * 16;
     const int outs = gated ? 64 : 128, col_tiles = (N + outs - 1) / outs;
     TI_REQUIRE(row_tiles <= 65535 && col_tiles <= 65535, "gemm_f32_split: too many tiles");
-    const int stage_bytes = 3 * (PLANE_A + p.bn * BK * 2);
-    p.stages = STAGE_ROOM / stage_bytes < MAX_STAGES ? STAGE_ROOM / stage_bytes : MAX_STAGES;
-    CUtensorMap map;
-    if (!ti_get_bf16_map(planes, 3ll * M, Kp, p.bn, &map)) return -1;
+    // shared memory: the weights' planes, then for many columns as many copies of x as leave room for three slots, for few
+    // columns (where the weights' way from HBM is what a step waits for) as many slots as there are
+    const int b_bytes = 3 * p.bn * BK * 2, room = SMEM_BYTES - 1024 - A_STAGES * 3 * PLANE_A;
+    p.b_stages = std::min(MAX_B_STAGES, (room - 3 * SLOT) / b_bytes);       // at least three
+    p.slots = std::min(MAX_SLOTS, (room - p.b_stages * b_bytes) / SLOT / A_STAGES * A_STAGES);
+    static_assert(A_STAGES * 3 * PLANE_A + 3 * 3 * MAX_BN * BK * 2 + 3 * SLOT <= SMEM_BYTES - 1024, "128 columns: three copies, three slots");
+    static_assert(MAX_SLOTS % A_STAGES == 0 && A_STAGES == 3, "three slots at least, a whole number a pair");
+    TiEncodeTiledFn encode = ti_encode_tiled_fn();
+    TI_REQUIRE(encode, "cuTensorMapEncodeTiled is not available from this driver");
+    CUtensorMap map, map_w;
+    const cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)M * 3}, strides[1] = {(cuuint64_t)Kp * 2};
+    const cuuint32_t box[2] = {BK, (cuuint32_t)p.bn}, elem[2] = {1, 1};
+    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, planes, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                              CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    const cuuint64_t w_dims[2] = {(cuuint64_t)K, (cuuint64_t)N * (gated ? 2 : 1)}, w_strides[1] = {(cuuint64_t)K * 4};
+    const cuuint32_t w_box[2] = {BK, 64};
+    const CUresult rw = encode(&map_w, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(w), w_dims, w_strides, w_box, elem,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    TI_REQUIRE(r == CUDA_SUCCESS && rw == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d, %d) for M=%d N=%d K=%d", (int)r, (int)rw, M, N, K);
     static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     TI_REQUIRE(set == cudaSuccess, "gemm_f32_split: %s", cudaGetErrorString(set));
+    const int splits = choose_splits(row_tiles * col_tiles, (K + BK - 1) / BK);
     const long long quads = (long long)M * Kp / 4;
     ti_launch(split_rows_kernel, dim3((unsigned)((quads + 255) / 256)), 256, 0, stream, (__nv_bfloat16*)planes, x, M, K, Kp);
     TI_CHECK_LAUNCH("gemm_f32_split rows");
     cudaLaunchConfig_t cfg = {};
-    const int splits = choose_splits(row_tiles * col_tiles, (K + BK - 1) / BK);
     cfg.gridDim = dim3(splits, row_tiles, col_tiles);
     cfg.blockDim = NUM_THREADS;
     cfg.dynamicSmemBytes = SMEM_BYTES;
@@ -353,7 +448,7 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ti_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, gemm_f32_split_kernel, map, p);
+    cudaLaunchKernelEx(&cfg, gemm_f32_split_kernel, map, map_w, p);
     TI_CHECK_LAUNCH("gemm_f32_split");
     return 0;
 }

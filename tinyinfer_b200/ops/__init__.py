@@ -183,6 +183,7 @@ _SIGNATURES["sm100"]["ti_attention_prefill_tc_bf16"] = [
     c_float, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p]
 _SIGNATURES["f32"] = {
     "ti_gemm_f32_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+    "ti_gemm_f32_split": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "ti_attention_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                          c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
 }
@@ -272,9 +273,15 @@ F32_MIN_K = 256           # below, the general kernel's few steps are as quick, 
 def _float32_product(out, x, w, bias, residual, m, n, k, gated) -> bool:
     """Runs a float32 product on the kernel made for its size, if there is one; False: the general kernel is to run it.
     The weights are read 16 bytes at a time: whole rows of them, on 16-byte boundaries."""
-    if x.dtype != torch.float32 or k % 4 or k < F32_MIN_K or not 1 <= m <= F32_FEW_ROWS or (x.data_ptr() | w.data_ptr()) % 16:
+    if x.dtype != torch.float32 or k % 4 or k < F32_MIN_K or m < 1 or (x.data_ptr() | w.data_ptr()) % 16:
         return False
-    _run("f32", "ti_gemm_f32_few", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), m, n, k, gated, _stream())
+    if m <= F32_FEW_ROWS:
+        _run("f32", "ti_gemm_f32_few", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), m, n, k, gated,
+             _stream())
+    else:
+        planes = torch.empty((3, m, -(-k // 64) * 64), dtype=torch.bfloat16, device=x.device)
+        _run("f32", "ti_gemm_f32_split", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), planes.data_ptr(),
+             m, n, k, gated, kernel_status(x.device).data_ptr(), _stream())
     return True
 
 

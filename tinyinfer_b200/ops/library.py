@@ -4,7 +4,7 @@ Each library is a plain shared object with ``extern "C"`` launchers, compiled by
 first use and kept in ``tinyinfer_b200/csrc/_build`` (or, if the checkout is read-only, in a
 per-user folder under the system's temporary directory). The file name carries a hash of the
 sources and flags, so an edited kernel is rebuilt and a stale object is never loaded. A library
-is only built when something asks for it: a 32-bit run never compiles the tensor-core kernels, and a model
+is only built when something asks for it: a 32-bit run never compiles the bfloat16 tensor-core kernels, and a model
 builds only the libraries its own parts call.
 
 There is no fallback: if ``nvcc`` or the build fails, loading raises.
@@ -37,7 +37,8 @@ LIBRARIES: Dict[str, dict] = {
                           "attention_generic.cu", "gemm_simt.cu", "sampling.cu"],
                  headers=["common.cuh"], link=[]),
     # the 32-bit path at the sizes it is used at: products and attention
-    "f32": dict(sources=["runtime.cu", "gemm_f32_few.cu", "attention_f32.cu"], headers=["common.cuh"], link=[]),
+    "f32": dict(sources=["runtime.cu", "sm100_host.cu", "gemm_f32_few.cu", "gemm_f32_split_tcgen05.cu", "attention_f32.cu"],
+                headers=["common.cuh", "sm100_ptx.cuh"], link=[]),
     # parts of designs with a cached latent, gated recurrences and routed experts around a float32 stream
     "latent": dict(sources=["runtime.cu", "stream.cu", "gemm_batched.cu", "latent_attention.cu",
                             "latent_attention_mma.cu", "recurrent.cu"],
