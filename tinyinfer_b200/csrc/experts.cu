@@ -8,9 +8,8 @@
 //              (token, choice) its rank among them. The last experts of the router may be identity experts, whose
 //              output is the token's row itself: they have no weights, the plan gives them no tiles, and `combine`
 //              adds weight * row for them
-//   plan     : one block: where every expert's rows start in the sorted order, and the list of row tiles
-//              [expert, first row, rows] that the grouped product walks
-//   place    : slot of every (token, choice) in the sorted order and the token of every slot
+//   place    : where every expert's rows start in the sorted order, the list of row tiles [expert, first row, rows] that the
+//              grouped product walks, the slot of every (token, choice) in the sorted order and the token of every slot
 //   route by table : no router. A row of a table names the experts of a token id, so the routing of every such layer is known
 //              from the step's token ids alone: one launch makes it for all layers at once, a block a layer (count, plan and
 //              place in shared memory), before the first layer runs
@@ -33,52 +32,89 @@
 constexpr int EX_MAX_TOP = 16;
 
 // ------------------------------------------------------------------ route
-// One block per token: its warps share out the experts' logits (16-byte loads of the router's rows where they are
-// aligned), then the first warp holds the scores of up to 32 * EX_PER_LANE experts, a lane apiece, and chooses.
+// A block's 16 warps make the logits of TOK tokens, four experts at a time in a warp, a lane L neighbouring features at a time
+// (16-byte loads of the router's rows where the tokens' rows are float32 and everything is aligned; else one by one), then a
+// warp a token holds the scores of up to 32 * EX_PER_LANE experts, a lane apiece, and chooses.
+// Bound by the router's rows from L2 in a step of many tokens: a block a token read 256 KB of them (64 experts of 2048) for
+// each of 2,048 tokens; TOK = 8 reads them an eighth as often, the tokens' rows are in shared memory and every piece of them
+// that is read meets four experts. For few tokens a block a token spreads the work widest. The sums' order is L's alone.
+// 2,048 tokens, 64 experts of 2048: 99 -> 36 us (float32 rows), 112 -> 60 us (bfloat16 rows, 2,000 tokens); 8 tokens 16 -> 8.7 us
+// (the choices drew their ranks one after the other) and 29 -> 27 us.
 constexpr int EX_PER_LANE = 8;
 constexpr int EX_ROUTE_THREADS = 512;
+constexpr int EX_AT_ONCE = 4;                    // experts a warp multiplies a piece of a token's row with
 
-template <typename T, typename XT>
+template <int L> __device__ __forceinline__ void ex_load(float* f, const float* x) {
+    if constexpr (L == 1) f[0] = x[0];
+    else
+#pragma unroll
+        for (int i = 0; i < L / 4; ++i) reinterpret_cast<float4*>(f)[i] = reinterpret_cast<const float4*>(x)[i];
+}
+template <int L> __device__ __forceinline__ void ex_load(float* f, const __nv_bfloat16* x) {
+    if constexpr (L == 1) f[0] = __bfloat162float(x[0]);
+    else {
+        static_assert(L == 8, "16 bytes");
+        const uint4 u = *reinterpret_cast<const uint4*>(x);
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { const float2 v = __bfloat1622float2(h[i]); f[2 * i] = v.x; f[2 * i + 1] = v.y; }
+    }
+}
+
+// RANKED: every (token, choice) also draws its rank among its expert's, and the experts' counts are kept.
+template <typename T, typename XT, int TOK, int L, bool RANKED>
 __global__ void __launch_bounds__(EX_ROUTE_THREADS) moe_route_kernel(
     int* __restrict__ chosen, float* __restrict__ weight, int* __restrict__ rank, int* __restrict__ counts,
     const XT* __restrict__ x32, const T* __restrict__ w_router, int num_tokens, int hidden, int experts, int top,
     float weight_eps, const float* __restrict__ correction, int renorm, int scoring, int groups, int keep, float weight_scale) {
-    __shared__ float logits[32 * EX_PER_LANE];
-    __shared__ int group_kept[32 * EX_PER_LANE];
+    extern __shared__ float4 rows4[];                // TOK > 1: the tokens' rows in float32
+    __shared__ float logits_sh[TOK][32 * EX_PER_LANE];
+    __shared__ int kept_sh[TOK][32 * EX_PER_LANE];
     ti_grid_launch_dependents();
     ti_grid_wait();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x;
-    const XT* x = x32 + (size_t)t * hidden;
-    constexpr int VEC = 16 / sizeof(T);
-    const bool aligned = sizeof(XT) == 4 && hidden % VEC == 0 && ((uintptr_t)w_router & 15) == 0 && ((uintptr_t)x32 & 15) == 0;
-    for (int e = warp; e < experts; e += EX_ROUTE_THREADS / 32) {
-        const T* w = w_router + (size_t)e * hidden;
-        float dot = 0.f;
-        if (aligned) {
-            const uint4* w4 = reinterpret_cast<const uint4*>(w);
-#pragma unroll 4
-            for (int v = lane; v < hidden / VEC; v += 32) {
-                const uint4 q = w4[v];
-                const T* we = reinterpret_cast<const T*>(&q);
-                const float4* xp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + (size_t)v * VEC);
+    const int t0 = blockIdx.x * TOK;
+    float* rows = reinterpret_cast<float*>(rows4);
+    if constexpr (TOK > 1) {
+        constexpr int P = sizeof(XT) == 4 ? 4 : 8;   // 16 bytes
+        for (int i = threadIdx.x * P; i < TOK * hidden; i += EX_ROUTE_THREADS * P)
+            ex_load<P>(rows + i, x32 + (size_t)min(t0 + i / hidden, num_tokens - 1) * hidden + i % hidden);
+        __syncthreads();
+    }
+    for (int e0 = warp * EX_AT_ONCE; e0 < experts; e0 += EX_ROUTE_THREADS / 32 * EX_AT_ONCE) {
+        float dot[EX_AT_ONCE][TOK] = {};
+        const T* w[EX_AT_ONCE];
 #pragma unroll
-                for (int i = 0; i < VEC / 4; ++i) {
-                    const float4 f = xp[i];
-                    dot = fmaf(f.x, to_f32(we[4 * i]), dot);
-                    dot = fmaf(f.y, to_f32(we[4 * i + 1]), dot);
-                    dot = fmaf(f.z, to_f32(we[4 * i + 2]), dot);
-                    dot = fmaf(f.w, to_f32(we[4 * i + 3]), dot);
-                }
+        for (int j = 0; j < EX_AT_ONCE; ++j) w[j] = w_router + (size_t)min(e0 + j, experts - 1) * hidden;
+#pragma unroll (L > 1 ? (TOK > 1 ? 1 : 2) : (TOK > 1 ? 2 : 8))
+        for (int v = lane * L; v < hidden; v += 32 * L) {
+            float we[EX_AT_ONCE][L];
+#pragma unroll
+            for (int j = 0; j < EX_AT_ONCE; ++j) ex_load<L>(we[j], w[j] + v);
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) {
+                float f[L];
+                if constexpr (TOK > 1) ex_load<L>(f, rows + t * hidden + v);
+                else ex_load<L>(f, x32 + (size_t)t0 * hidden + v);
+#pragma unroll
+                for (int j = 0; j < EX_AT_ONCE; ++j)
+#pragma unroll
+                    for (int i = 0; i < L; ++i) dot[j][t] = fmaf(f[i], we[j][i], dot[j][t]);
             }
-        } else {
-            for (int i = lane; i < hidden; i += 32) dot = fmaf(to_f32(x[i]), to_f32(w[i]), dot);
         }
-        dot = warp_sum(dot);
-        if (lane == 0) logits[e] = dot;
+#pragma unroll
+        for (int j = 0; j < EX_AT_ONCE; ++j)
+#pragma unroll
+            for (int t = 0; t < TOK; ++t) {
+                const float z = warp_sum(dot[j][t]);
+                if (lane == 0 && e0 + j < experts) logits_sh[t][e0 + j] = z;
+            }
     }
     __syncthreads();
-    if (warp != 0) return;
+    const int t = t0 + warp;                           // warp w chooses for token w of the block
+    if (warp >= TOK || t >= num_tokens) return;
+    float* logits = logits_sh[warp];
+    int* group_kept = kept_sh[warp];
     float z[EX_PER_LANE];                              // lane holds experts lane, lane + 32, ...
 #pragma unroll
     for (int k = 0; k < EX_PER_LANE; ++k) z[k] = (k * 32 + lane < experts) ? logits[k * 32 + lane] : -INFINITY;
@@ -144,9 +180,8 @@ __global__ void __launch_bounds__(EX_ROUTE_THREADS) moe_route_kernel(
             if (e < experts && !group_kept[e / per_group]) c[k] = -INFINITY;
         }
     }
-    float best[EX_MAX_TOP];
-    int who[EX_MAX_TOP];
-    float total = 0.f;
+    float mine = 0.f, total = 0.f;                     // lane ch keeps choice ch
+    int who = 0;
     for (int ch = 0; ch < top; ++ch) {
         float v = -INFINITY, sv = 0.f;
         int idx = 0x7fffffff;
@@ -160,65 +195,100 @@ __global__ void __launch_bounds__(EX_ROUTE_THREADS) moe_route_kernel(
             const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
             if (ov > v || (ov == v && oi < idx)) { v = ov; sv = os; idx = oi; }
         }
-        best[ch] = sv;
-        who[ch] = idx;
+        if (lane == ch) { mine = sv; who = idx < experts ? idx : 0; }       // no number left to choose by (NaN): any expert
         total += sv;
 #pragma unroll
         for (int k = 0; k < EX_PER_LANE; ++k)
             if (idx == k * 32 + lane) c[k] = -INFINITY;
     }
-    if (lane == 0) {
+    if (lane < top) {
         const float norm = (renorm ? 1.f / (total + weight_eps) : 1.f) * weight_scale;
-        for (int ch = 0; ch < top; ++ch) {
-            chosen[(size_t)t * top + ch] = who[ch];
-            weight[(size_t)t * top + ch] = best[ch] * norm;
-            rank[(size_t)t * top + ch] = atomicAdd(counts + who[ch], 1);
-        }
+        chosen[(size_t)t * top + lane] = who;
+        weight[(size_t)t * top + lane] = mine * norm;
+        if constexpr (RANKED) rank[(size_t)t * top + lane] = atomicAdd(counts + who, 1);
     }
 }
 
-// ------------------------------------------------------------------ plan
-// counts[e] -> starts[e] (exclusive sums, starts[experts] = all rows) and tiles [expert, first row, rows] of the
-// first real_experts experts (the others have no weights to multiply by); num_tiles[0] = how many. One block;
-// experts and tiles are few.
-__global__ void moe_plan_kernel(int* __restrict__ starts, int* __restrict__ tiles, int* __restrict__ num_tiles,
-                                const int* __restrict__ counts, int experts, int real_experts, int tile_rows, int max_tiles) {
-    ti_grid_launch_dependents();
-    ti_grid_wait();
-    if (threadIdx.x != 0) return;
-    int row = 0, n = 0;
-    for (int e = 0; e < experts; ++e) {
-        starts[e] = row;
-        const int c = counts[e];
-        for (int r = 0; r < c && n < max_tiles && e < real_experts; r += tile_rows) {      // identity experts: rows, no tiles
-            tiles[3 * n] = e;
-            tiles[3 * n + 1] = row + r;
-            tiles[3 * n + 2] = min(tile_rows, c - r);
-            ++n;
-        }
-        row += c;
-    }
-    starts[experts] = row;
-    num_tiles[0] = n;
-}
+// ------------------------------------------------------------------ plan and place
+// counts[e] -> where every expert's rows start (exclusive sums) and the tiles [expert, first row, rows] of the first
+// real_experts experts (the others have no weights to multiply by); num_tiles[0] = how many; then the slot of every (token,
+// choice) and the token of every slot. Every block scans the counts itself (a warp, 32 experts at a time); block 0 writes the
+// tiles. A single thread that walked the counts took 7 to 10 us, and the places were another 2 us and a launch; now 2.4 to 3.6 us.
+// ALONE: one block does it all for a step of few choices: it counts in shared memory, so the router draws no ranks and nobody
+// clears the counts beforehand.
+constexpr int EX_PLACE_THREADS = 256;
+constexpr int EX_ALONE_MAX = 2048;                 // (token, choice) pairs of a step that one block places
 
-__global__ void moe_place_kernel(int* __restrict__ slot_of, int* __restrict__ token_of, const int* __restrict__ chosen,
-                                 const int* __restrict__ rank, const int* __restrict__ starts, int n, int top,
-                                 float* __restrict__ slot_weight, const float* __restrict__ weight) {
+template <bool ALONE>
+__global__ void __launch_bounds__(EX_PLACE_THREADS) moe_place_kernel(
+    int* __restrict__ starts, int* __restrict__ tiles, int* __restrict__ num_tiles, int* __restrict__ counts,
+    int* __restrict__ slot_of, int* __restrict__ token_of, const int* __restrict__ chosen, const int* __restrict__ rank, int n,
+    int top, int experts, int real_experts, int tile_rows, int max_tiles, float* __restrict__ slot_weight,
+    const float* __restrict__ weight) {
+    __shared__ int count_sh[32 * EX_PER_LANE], start_sh[32 * EX_PER_LANE], tile_sh[32 * EX_PER_LANE];
     ti_grid_launch_dependents();
     ti_grid_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int slot = starts[chosen[i]] + rank[i];
-    slot_of[i] = slot;
-    token_of[slot] = i / top;
-    if (slot_weight) slot_weight[slot] = weight[i];        // the weights in expert order, for whoever works on sorted rows
+    const int tid = threadIdx.x, lane = tid & 31;
+    for (int e = tid; e < experts; e += EX_PLACE_THREADS) count_sh[e] = ALONE ? 0 : counts[e];
+    __syncthreads();
+    int mine[ALONE ? EX_ALONE_MAX / EX_PLACE_THREADS : 1];      // this thread's ranks
+    if constexpr (ALONE) {
+#pragma unroll
+        for (int k = 0; k < EX_ALONE_MAX / EX_PLACE_THREADS; ++k) {
+            const int i = tid + k * EX_PLACE_THREADS;
+            if (i < n) mine[k] = atomicAdd(&count_sh[chosen[i]], 1);
+        }
+        __syncthreads();
+    }
+    if (tid < 32) {
+        int rows = 0, tls = 0;
+        for (int e0 = 0; e0 < experts; e0 += 32) {
+            const int e = e0 + lane, c = e < experts ? count_sh[e] : 0;
+            const int k = e < real_experts ? (c + tile_rows - 1) / tile_rows : 0;      // identity experts: rows, no tiles
+            int ci = c, ki = k;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int cv = __shfl_up_sync(0xffffffffu, ci, o), kv = __shfl_up_sync(0xffffffffu, ki, o);
+                if (lane >= o) { ci += cv; ki += kv; }
+            }
+            if (e < experts) { start_sh[e] = rows + ci - c; tile_sh[e] = tls + ki - k; }
+            rows += __shfl_sync(0xffffffffu, ci, 31);
+            tls += __shfl_sync(0xffffffffu, ki, 31);
+        }
+        if (blockIdx.x == 0 && lane == 0) {
+            num_tiles[0] = min(tls, max_tiles);
+            starts[experts] = rows;
+        }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {
+        for (int e = tid; e < experts; e += EX_PLACE_THREADS) {
+            const int c = count_sh[e];
+            starts[e] = start_sh[e];
+            if (ALONE) counts[e] = c;
+            if (e >= real_experts) continue;
+            for (int r = 0, k = tile_sh[e]; r < c && k < max_tiles; r += tile_rows, ++k) {
+                tiles[3 * k] = e;
+                tiles[3 * k + 1] = start_sh[e] + r;
+                tiles[3 * k + 2] = min(tile_rows, c - r);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < (ALONE ? EX_ALONE_MAX / EX_PLACE_THREADS : 1); ++k) {
+        const int i = ALONE ? tid + k * EX_PLACE_THREADS : blockIdx.x * EX_PLACE_THREADS + tid;
+        if (i >= n) continue;
+        const int slot = start_sh[chosen[i]] + (ALONE ? mine[k] : rank[i]);
+        slot_of[i] = slot;
+        token_of[slot] = i / top;
+        if (slot_weight) slot_weight[slot] = weight[i];    // the weights in expert order, for whoever works on sorted rows
+    }
 }
 
 // scoring 0: softmax over the experts; 1: the sigmoid of each logit.
 // slot_weight (float32 [tokens * top], or null): also receives every (token, choice)'s weight at its row in expert order.
 // groups > 1: only experts of the keep_groups best groups can be chosen; weight_scale: a factor on every weight.
-// counts (experts ints) must be zero on entry; the launcher clears them. x_dtype: of the tokens' rows (float32, or
+// counts (experts ints): the tokens of every expert; rank (tokens * top ints) is scratch. x_dtype: of the tokens' rows (float32, or
 // the compute dtype of a sublayer's input); correction: float32 [experts] or null; renorm: the weights are divided by
 // their sum; real_experts: how many of the router's outputs are experts with weights (the rest: identity experts).
 TI_API int ti_moe_route(int* chosen, float* weight, int* rank, int* counts, int* starts, int* tiles, int* num_tiles,
@@ -236,24 +306,57 @@ TI_API int ti_moe_route(int* chosen, float* weight, int* rank, int* counts, int*
     TI_REQUIRE(real_experts >= 0 && real_experts <= experts, "moe_route: %d of %d experts have weights", real_experts, experts);
     TI_REQUIRE(x_dtype == TI_F32 || x_dtype == dtype, "moe_route: the rows are float32 or of the router's dtype");
     if (num_tokens == 0) return 0;
-    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * experts, stream);
-    TI_REQUIRE(e == cudaSuccess, "moe_route: %s", cudaGetErrorString(e));
-    const int blocks = num_tokens;
+    const int n = num_tokens * top;
+    const bool alone = n <= EX_ALONE_MAX;
+    if (!alone) {
+        const cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(int) * experts, stream);
+        TI_REQUIRE(e == cudaSuccess, "moe_route: %s", cudaGetErrorString(e));
+    }
+    const int esize = dtype == TI_F32 ? 4 : 2;
+    const bool on16 = ((uintptr_t)w_router & 15) == 0 && ((uintptr_t)x & 15) == 0;
+    const bool vec = on16 && x_dtype == TI_F32 && hidden % (16 / esize) == 0;
+    // eight tokens a block once that still leaves a block for every SM (and their rows fit beside another block's)
+    const bool many = on16 && hidden % 8 == 0 && num_tokens >= 8 * 148 && hidden <= 3072;
     typedef __nv_bfloat16 B;
-#define EX_ROUTE(T, XT) ti_launch(moe_route_kernel<T, XT>, blocks, EX_ROUTE_THREADS, 0, stream, chosen, weight, rank, counts, \
-                                  (const XT*)x, (const T*)w_router, num_tokens, hidden, experts, top, weight_eps, correction, renorm, scoring, groups, keep_groups, weight_scale)
-    if (dtype == TI_F32) EX_ROUTE(float, float);
-    else if (dtype == TI_BF16 && x_dtype == TI_F32) EX_ROUTE(B, float);
-    else if (dtype == TI_BF16) EX_ROUTE(B, B);
+#define EX_ROUTE(T, XT, TOK, L, RANKED)                                                                                            \
+    do {                                                                                                                           \
+        const size_t smem = TOK > 1 ? (size_t)TOK * hidden * 4 : 0;                                                                \
+        if (smem > 24 * 1024) {                                                                                                    \
+            const cudaError_t e = cudaFuncSetAttribute(moe_route_kernel<T, XT, TOK, L, RANKED>,                                    \
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                    \
+            TI_REQUIRE(e == cudaSuccess, "moe_route: shared memory: %s", cudaGetErrorString(e));                                   \
+        }                                                                                                                          \
+        ti_launch(moe_route_kernel<T, XT, TOK, L, RANKED>, (num_tokens + TOK - 1) / TOK, EX_ROUTE_THREADS, smem, stream, chosen,   \
+                  weight, rank, counts, (const XT*)x, (const T*)w_router, num_tokens, hidden, experts, top, weight_eps, correction, \
+                  renorm, scoring, groups, keep_groups, weight_scale);                                                             \
+    } while (0)
+#define EX_ROUTE_RANKED(T, XT, TOK, L)                   \
+    do {                                                 \
+        if (alone) EX_ROUTE(T, XT, TOK, L, false);       \
+        else EX_ROUTE(T, XT, TOK, L, true);              \
+    } while (0)
+#define EX_ROUTE_SIZED(T, XT)                                                      \
+    do {                                                                           \
+        constexpr int WIDE = sizeof(XT) == 4 ? 16 / sizeof(T) : 1;                 \
+        if (many && vec) EX_ROUTE_RANKED(T, XT, 8, WIDE);                          \
+        else if (many) EX_ROUTE_RANKED(T, XT, 8, 1);                               \
+        else if (vec) EX_ROUTE_RANKED(T, XT, 1, WIDE);                             \
+        else EX_ROUTE_RANKED(T, XT, 1, 1);                                         \
+    } while (0)
+    if (dtype == TI_F32) EX_ROUTE_SIZED(float, float);
+    else if (dtype == TI_BF16 && x_dtype == TI_F32) EX_ROUTE_SIZED(B, float);
+    else if (dtype == TI_BF16) EX_ROUTE_SIZED(B, B);
     else TI_REQUIRE(false, "moe_route: unknown dtype %d", dtype);
+#undef EX_ROUTE_SIZED
+#undef EX_ROUTE_RANKED
 #undef EX_ROUTE
     TI_CHECK_LAUNCH("moe_route");
-    ti_launch(moe_plan_kernel, 1, 32, 0, stream, starts, tiles, num_tiles, (const int*)counts, experts, real_experts, tile_rows,
-              max_tiles);
-    TI_CHECK_LAUNCH("moe_plan");
-    const int n = num_tokens * top;
-    ti_launch(moe_place_kernel, (n + 127) / 128, 128, 0, stream, slot_of, token_of, (const int*)chosen, (const int*)rank,
-              (const int*)starts, n, top, slot_weight, (const float*)weight);
+#define EX_PLACE(ALONE, BLOCKS)                                                                                                  \
+    ti_launch(moe_place_kernel<ALONE>, BLOCKS, EX_PLACE_THREADS, 0, stream, starts, tiles, num_tiles, counts, slot_of, token_of, \
+              (const int*)chosen, (const int*)rank, n, top, experts, real_experts, tile_rows, max_tiles, slot_weight, (const float*)weight)
+    if (alone) EX_PLACE(true, 1);
+    else EX_PLACE(false, (n + EX_PLACE_THREADS - 1) / EX_PLACE_THREADS);
+#undef EX_PLACE
     TI_CHECK_LAUNCH("moe_place");
     return 0;
 }
