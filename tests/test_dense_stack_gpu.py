@@ -1,0 +1,73 @@
+"""A dense decoder's layers from one native call against the same layers part by part."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def make(dtype, heads, kv_heads, dim, hidden, inter, layers, page, tied=True):
+    from tinyinfer_b200.config import Qwen3Config
+    from tinyinfer_b200 import models  # noqa: F401
+    from tinyinfer_b200.config import lookup_architecture
+    from tinyinfer_b200.engine.runner import ModelRunner
+    cfg = dict(architectures=["Qwen3ForCausalLM"], vocab_size=515, hidden_size=hidden, num_hidden_layers=layers, num_attention_heads=heads,
+               num_key_value_heads=kv_heads, head_dim=dim, intermediate_size=inter, rms_norm_eps=1e-6, rope_theta=1e6,
+               tie_word_embeddings=tied, max_position_embeddings=4096)
+    arch = lookup_architecture("Qwen3ForCausalLM")
+    model = arch.model_factory(Qwen3Config.from_dict(cfg), dtype, torch.device("cuda:0"))
+    gen = torch.Generator(device="cuda:0").manual_seed(3)
+    tensors = {}
+    for name, ts in model.expected_tensors().items():
+        t = torch.randn(tuple(ts.shape), generator=gen, device="cuda:0")
+        tensors[name] = 1.0 + 0.1 * t if ts.role == "vector32" else (t * (1.0 if "embed" in name else 0.05)).to(dtype)
+    model.load_tensors(tensors)
+    return model, lambda graphs=False: ModelRunner(model, page_size=page, num_pages=900, max_requests=12, max_tokens_per_step=3000,
+                                                   max_model_len=2600, cuda_graphs=graphs)
+
+
+STEPS = [[(0, 37)], [(0, 1)], [(0, 1), (1, 300)], [(0, 1), (1, 1), (2, 64), (3, 65)], [(4, 2200)], [(4, 130), (0, 1), (5, 9)],
+         [(i, 1) for i in range(6)], [(4, 1), (6, 7)], [(i, 1) for i in range(7)] + [(7, 600)]]
+
+
+def run(runner, steps):
+    from tinyinfer_b200.engine.batch import StepEntry
+    gen = torch.Generator().manual_seed(5)
+    return [runner.step([StepEntry(r, torch.randint(0, 515, (n,), generator=gen).tolist(), [0, n - 1] if n > 1 else [0])
+                         for r, n in step]).clone() for step in steps]
+
+
+@pytest.mark.parametrize("dtype,heads,kv_heads,dim,hidden,inter,page", [
+    (torch.bfloat16, 4, 2, 64, 256, 384, 16), (torch.bfloat16, 8, 1, 128, 520, 1000, 64), (torch.float32, 4, 2, 128, 256, 320, 64),
+    (torch.float32, 6, 2, 64, 260, 328, 5)])
+def test_stack_equals_the_parts(dtype, heads, kv_heads, dim, hidden, inter, page):
+    from tinyinfer_b200 import ops
+    model, runner = make(dtype, heads, kv_heads, dim, hidden, inter, 3, page)
+    stack = model._stack
+    assert stack is not None
+    # the parts round where the stack does, but for products of at most 8 bfloat16 tokens (their sums' order) and float32 ones
+    model._stack = None
+    want = run(runner(), STEPS)
+    model._stack = stack
+    for graphs in (False, True):
+        got = run(runner(graphs), STEPS)
+        for g, w, step in zip(got, want, STEPS):
+            assert torch.isfinite(g).all()
+            error = ((g - w).norm() / w.norm()).item()
+            assert error <= (2e-2 if dtype == torch.bfloat16 else 1e-5), (step, error)
+    ops.check_kernel_status()
+
+
+def test_what_the_stack_does_not_take(monkeypatch):
+    """Sizes of other kernels run part by part."""
+    from tinyinfer_b200 import ops
+    called = []
+    real = ops.dense_stack
+    monkeypatch.setattr(ops, "dense_stack", lambda *a, **k: called.append(1) or real(*a, **k))
+    for dtype, heads, kv, dim, hidden, inter, page, taken in (
+            (torch.bfloat16, 4, 2, 32, 128, 256, 16, False), (torch.bfloat16, 4, 2, 64, 132, 256, 16, False),
+            (torch.bfloat16, 4, 2, 64, 128, 256, 8, False), (torch.bfloat16, 4, 2, 64, 128, 256, 16, True),
+            (torch.float32, 4, 2, 48, 128, 256, 16, False)):
+        _, runner = make(dtype, heads, kv, dim, hidden, inter, 2, page)
+        del called[:]
+        out = run(runner(), [[(0, 20)], [(0, 1)]])
+        assert bool(called) == taken and all(torch.isfinite(o).all() for o in out)

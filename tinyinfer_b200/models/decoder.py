@@ -16,6 +16,7 @@ import torch
 from .. import ops
 from ..config.specs import ModelSpec
 from ..parts.experts import TableRoutes
+from ..parts.stack import DenseStack
 from ..parts import CacheNeed, StateNeed, TensorSpec, build_block, build_norm
 
 
@@ -32,6 +33,7 @@ class DecoderModel:
         self.head: Optional[torch.Tensor] = None
         self.entry_weight: Optional[torch.Tensor] = None      # of the entries that project [x; embedding]
         self.table_routes: Optional[TableRoutes] = None       # feed-forwards whose routing depends on the token ids alone
+        self._stack = DenseStack.of(self.blocks, spec.execution)     # blocks that one native call can launch, or None
         self.step_vectors: Optional[torch.Tensor] = None      # float32 [rows, hidden]: what entries of the run order add
 
     # ------------------------------------------------------------------ tensors
@@ -131,6 +133,10 @@ class DecoderModel:
 
     def run_blocks(self, x: torch.Tensor, step) -> torch.Tensor:
         """The blocks in the order the spec lists, each on its cache entry."""
+        if self._stack is not None:
+            out = self._stack.run(x, step)
+            if out is not None:
+                return out
         link = None        # what a block's last product leaves for the next block's first norm (see parts.base)
         order = self.spec.execution
         for i, entry in enumerate(order):

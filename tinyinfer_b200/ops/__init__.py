@@ -10,6 +10,7 @@ norm weights, biases and logits are float32, indices are int32, and everything i
 """
 from __future__ import annotations
 
+import array
 import ctypes
 from typing import Optional
 
@@ -181,6 +182,10 @@ _SIGNATURES["sm100"]["ti_attention_prefill_pair_bf16"] = [
 _SIGNATURES["sm100"]["ti_attention_prefill_tc_bf16"] = [
     c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
     c_float, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p]
+_SIGNATURES["stack"] = {
+    "ti_dense_stack": [c_void_p], "ti_dense_stack_portion_floats": [c_void_p],
+    "ti_dense_stack_bytes": [c_int, c_int, c_int, c_int, c_int, c_int],
+}
 _SIGNATURES["f32"] = {
     "ti_gemm_f32_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
     "ti_gemm_f32_split": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
@@ -671,6 +676,15 @@ def plan_attention(q_lens, starts):
     return decode_rows, [x for t in pairs + singles for x in t], len(pairs)
 
 
+def attention_shape_ok(dtype: torch.dtype, hq: int, hkv: int, d: int, page: int) -> bool:
+    """Whether these sizes have attention kernels of their own: bfloat16 on the tensor cores, or the float32 ones."""
+    if d not in (64, 128) or hq % hkv:
+        return False
+    if dtype == torch.float32:
+        return hq // hkv <= 32
+    return dtype == torch.bfloat16 and hq // hkv <= 16 and (page in (16, 32) or page % 64 == 0)
+
+
 def attention_tensor_cores_ok(q: torch.Tensor, kv_cache: torch.Tensor, maps: int = 1) -> bool:
     """The tensor-core attention kernels take bfloat16, head sizes 64 and 128, up to 16 query heads (or, with two maps a
     head, 8) per kv head, and pages of 16, 32 or a multiple of 64 tokens."""
@@ -1113,6 +1127,90 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
          _ptr(sink), positions.data_ptr(), token_seq.data_ptr(), block_table.data_ptr(), block_table.shape[1], t, heads,
          rank, rot, cache.shape[3], cache.shape[1], float(scale), int(window or 0), splits, _ptr(status),
          _dtype_code(cache), _stream())
+    return out
+
+
+# ---------------------------------------------------------------------- a dense decoder's blocks in one call
+_STACK_LAUNCHERS = (("core", "ti_rmsnorm"), ("core", "ti_qk_norm_rope_append"), ("sm100", "ti_gemm_bf16"),
+                    ("sm100", "ti_gemm_bf16_linked"), ("sm100", "ti_attention_decode_bf16"), ("sm100", "ti_attention_prefill_tc_bf16"),
+                    ("sm100", "ti_attention_prefill_pair_bf16"), ("core", "ti_gemm_simt"), ("f32", "ti_gemm_f32_few"),
+                    ("f32", "ti_gemm_f32_split"), ("f32", "ti_attention_f32"))
+_STACK_LIBRARIES = {torch.bfloat16: ("core", "sm100"), torch.float32: ("core", "f32")}
+_stack_launchers = {}
+
+
+class _StackCall(ctypes.Structure):
+    _fields_ = ([(name, c_void_p) for _, name in _STACK_LAUNCHERS] + [(n, c_void_p) for n in ("layer", "x", "out", "workspace")]
+                + [("workspace_bytes", c_ll)] + [(n, c_void_p) for n in ("positions", "token_seq", "decode_rows", "tiles", "gemm_ws")]
+                + [("gemm_ws_floats", c_ll), ("counters", c_void_p), ("attn_scratch", c_void_p), ("attn_floats", c_ll)]
+                + [(n, c_void_p) for n in ("wait_status", "page_status", "stream")]
+                + [(n, c_int) for n in ("layers", "tokens", "hidden", "heads", "kv_heads", "head_dim", "inter", "act", "page_size",
+                                        "dtype", "num_decode", "num_tiles", "num_pairs", "max_context", "table_positions",
+                                        "interleaved", "rotary_dim", "num_counters", "link_max_tokens", "pair_min_ctas",
+                                        "split_max_ctas", "few_rows", "min_k", "tile_rows")]
+                + [(n, c_float) for n in ("eps1", "eps2", "qk_eps", "scale")] + [("failed", c_int)])
+
+
+def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: int, head_dim: int, inter: int, activation: str,
+                page_size: int, eps: tuple, scale: float, rotation: Optional[Rotation]) -> torch.Tensor:
+    """Runs the blocks of a dense pre-norm decoder on ``x`` [T, hidden] by one native call that makes every launch of
+    ``linear``, ``rmsnorm``, ``qk_norm_rope_append``, ``paged_attention`` and ``gated_linear`` that the parts would.
+    ``layers``: per layer, in the order they run, 18 integers (addresses, 0 for what a layer has not, and sizes): w_qkv, b_qkv,
+    w_o, b_o, q norm, k norm, inverse frequencies, table of cosines and sines, norm 1, norm 2, w_gate_up, w_down, cache, block
+    table, its width, pages, window, whether it writes its cache. ``eps``: of the first norm, the second, and of q and k. The
+    caller has seen to it that the attention kernels take the shapes (``attention_shape_ok``) and that rows, matrices and
+    caches start on 16-byte boundaries."""
+    global _plain_next
+    _check(x, "x", None, 2)
+    t, hidden = x.shape
+    code = _dtype_code(x)
+    addresses = _stack_launchers.get(x.dtype)
+    if addresses is None:
+        wanted = _STACK_LIBRARIES[x.dtype]
+        addresses = _stack_launchers[x.dtype] = [ctypes.cast(_fn(lib, name), c_void_p).value if lib in wanted else None
+                                                 for lib, name in _STACK_LAUNCHERS]
+    size = _fn("stack", "ti_dense_stack_bytes")
+    size.restype = c_ll
+    nbytes = size(t, hidden, heads * head_dim, kv_heads * head_dim, inter, code)
+    workspace = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    out = torch.empty_like(x)
+    rows = array.array("q", [v for row in layers for v in row])
+    call = _StackCall(*addresses)
+    call.layer, call.x, call.out = rows.buffer_info()[0], x.data_ptr(), out.data_ptr()
+    call.workspace, call.workspace_bytes = workspace.data_ptr(), nbytes
+    call.positions, call.token_seq = step.positions.data_ptr(), step.token_seq.data_ptr()
+    call.decode_rows, call.tiles = step.decode_rows.data_ptr(), step.prefill_tiles.data_ptr()
+    call.wait_status, call.page_status, call.stream = status_words(x.device).data_ptr(), _ptr(step.status), _stream()
+    call.layers, call.tokens, call.hidden, call.heads, call.kv_heads = len(layers), t, hidden, heads, kv_heads
+    call.head_dim, call.inter, call.act, call.page_size, call.dtype = head_dim, inter, GATED_ACTIVATIONS[activation], page_size, code
+    call.num_decode, call.num_tiles, call.num_pairs = step.num_decode, step.num_prefill_tiles, step.num_pair_tiles
+    call.max_context = int(step.max_context)
+    if rotation is not None:
+        call.table_positions = rotation.cos_sin.shape[0] if rotation.cos_sin is not None else 0
+        call.interleaved, call.rotary_dim = int(rotation.interleaved), rotation.rotary_dim
+    call.link_max_tokens, call.pair_min_ctas, call.split_max_ctas = NORM_LINK_MAX_TOKENS, PAIR_MIN_CTAS, KEY_SPLIT_MAX_CTAS
+    call.few_rows, call.min_k, call.tile_rows = F32_FEW_ROWS, F32_MIN_K, PREFILL_TILE
+    call.eps1, call.eps2, call.qk_eps = eps
+    call.scale = scale
+    if code == 1:
+        ws, counters = _gemm_scratch(x.device)
+        call.gemm_ws, call.gemm_ws_floats, call.counters, call.num_counters = ws.data_ptr(), ws.numel(), counters.data_ptr(), counters.numel()
+        portions = _fn("stack", "ti_dense_stack_portion_floats")
+        portions.restype = c_ll
+        floats = portions(ctypes.addressof(call))
+        if step.num_decode:
+            floats = max([floats] + [decode_scratch_floats(step.num_decode, heads, kv_heads, head_dim, int(step.max_context), w)
+                                     for w in {row[16] for row in layers}])
+        if floats:
+            scratch = _decode_scratch(x.device, floats)
+            call.attn_scratch, call.attn_floats = scratch.data_ptr(), scratch.numel()
+    if _plain_next:                              # the first launch is the core library's
+        library.load("core").ti_plain_next_launch()
+        _plain_next = False
+    rc = _fn("stack", "ti_dense_stack")(ctypes.addressof(call))
+    if rc != 0:
+        said = [library.load(n).ti_last_error().decode(errors="replace") for n in ("stack", ("core", "sm100", "f32")[call.failed])]
+        raise KernelError(f"dense_stack failed ({rc}): {said[0] or said[1]}")
     return out
 
 
