@@ -1,5 +1,9 @@
 // The grouped products of routed experts for steps that bring an expert many rows, on tcgen05: the plan's row tiles
-// hold 128 sorted rows of one expert (experts.cu), a work unit is a row tile x 128 of the expert's output features.
+// hold 128 sorted rows of one expert (experts.cu), a work unit is a row tile x BN of the expert's output features: 256 where
+// that leaves every SM two units, else 128. An SM gets about 64 bytes a cycle from L2; a 64-wide k block of a 128-wide unit
+// takes 32 KB for 256 cycles of MMAs, of a 256-wide one 48 KB for 512.
+// 12,000 rows over 64 experts: up and down 166 -> 151 us at 2,816 and 2,048 features (means), 127 -> 120 us at 1,408 and 2,048; what
+// bounds it then is L2, which hands out some 10 TB/s.
 // One CTA an SM walks the units; warp 0 copies operand tiles with TMA (the sorted activations [slots, K] and the
 // experts' weights as one matrix [experts * N, K], each through one tensor map, 64 k a stage, 128-byte swizzle),
 // warp 1 issues the MMAs (128 x 128 x 16, float32 accumulators in tensor memory, two of them so that the epilogue of
@@ -10,9 +14,12 @@
 #include "sm100_ptx.cuh"
 
 namespace {
-constexpr int GT_BM = 128, GT_BN = 128, GT_BK = 64, GT_UMMA_K = 16, GT_THREADS = 192, GT_STAGES = 5;
-constexpr int GT_STAGE_BYTES = (GT_BM + GT_BN) * GT_BK * 2;
-constexpr int GT_SMEM = GT_STAGES * GT_STAGE_BYTES + 1024 + 256;
+constexpr int GT_BM = 128, GT_BK = 64, GT_UMMA_K = 16, GT_THREADS = 192;
+template <int BN> struct GtShape {
+    static constexpr int STAGES = BN == 128 ? 5 : 4;
+    static constexpr int STAGE_BYTES = (GT_BM + BN) * GT_BK * 2;
+    static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+};
 
 struct GtParams {
     void* out;
@@ -22,8 +29,10 @@ struct GtParams {
     int* status;
 };
 
+template <int GT_BN>
 __global__ void __launch_bounds__(GT_THREADS, 1)
 moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const GtParams p) {
+    constexpr int GT_STAGES = GtShape<GT_BN>::STAGES, GT_STAGE_BYTES = GtShape<GT_BN>::STAGE_BYTES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(stages + GT_STAGES * GT_STAGE_BYTES);
@@ -165,7 +174,7 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
 
 // 1 if the tcgen05 form takes these operands: whole k blocks, rows on 16-byte boundaries, operands at least a box tall.
 TI_API int ti_moe_gemm_tcgen05_ok(int slots, int experts, int N, int K) {
-    return (K % GT_BK == 0 && slots >= GT_BM && (long long)experts * N >= GT_BN && N > 0) ? 1 : 0;
+    return (K % GT_BK == 0 && slots >= GT_BM && (long long)experts * N >= 128 && N > 0) ? 1 : 0;
 }
 TI_API int ti_moe_tcgen05_tile_rows() { return GT_BM; }
 
@@ -177,20 +186,21 @@ TI_API int ti_moe_gemm_tcgen05(void* out, const void* x, const void* w, const in
     TI_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)out & 15) == 0, "moe_gemm_tcgen05: operands must be 16-byte aligned");
     if (max_tiles <= 0) return 0;
     CUtensorMap map_x, map_w;
+    // the real number of row tiles is on the device; at least slots / 128
+    const bool wide = N >= 256 && (long long)(slots / GT_BM) * ((N + 255) / 256) >= 2 * ti_sm_count();
+    const int bn = wide ? 256 : 128;
     if (!ti_get_bf16_map(x, slots, K, GT_BM, &map_x)) return -1;
-    if (!ti_get_bf16_map(w, (long long)experts * N, K, GT_BN, &map_w)) return -1;
-    static bool configured = false;
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(moe_gemm_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM);
-        TI_REQUIRE(e == cudaSuccess, "moe_gemm_tcgen05: cannot get %d bytes of shared memory: %s", GT_SMEM, cudaGetErrorString(e));
-        configured = true;
-    }
+    if (!ti_get_bf16_map(w, (long long)experts * N, K, bn, &map_w)) return -1;
+    static const cudaError_t narrow_set = cudaFuncSetAttribute(moe_gemm_tcgen05_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtShape<128>::SMEM);
+    static const cudaError_t wide_set = cudaFuncSetAttribute(moe_gemm_tcgen05_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtShape<256>::SMEM);
+    TI_REQUIRE(narrow_set == cudaSuccess && wide_set == cudaSuccess, "moe_gemm_tcgen05: shared memory: %s", cudaGetErrorString(wide ? wide_set : narrow_set));
     GtParams p;
-    p.out = out; p.tiles = tiles; p.num_tiles = num_tiles; p.N = N; p.K = K; p.col_tiles = (N + GT_BN - 1) / GT_BN; p.up = up;
+    p.out = out; p.tiles = tiles; p.num_tiles = num_tiles; p.N = N; p.K = K; p.col_tiles = (N + bn - 1) / bn; p.up = up;
     p.status = status;
     const long long units = (long long)max_tiles * p.col_tiles;
     const int grid = (int)(units < ti_sm_count() ? units : ti_sm_count());
-    ti_launch(moe_gemm_tcgen05_kernel, grid, GT_THREADS, GT_SMEM, stream, map_x, map_w, p);
+    if (wide) ti_launch(moe_gemm_tcgen05_kernel<256>, grid, GT_THREADS, GtShape<256>::SMEM, stream, map_x, map_w, p);
+    else ti_launch(moe_gemm_tcgen05_kernel<128>, grid, GT_THREADS, GtShape<128>::SMEM, stream, map_x, map_w, p);
     TI_CHECK_LAUNCH("moe_gemm_tcgen05");
     return 0;
 }
