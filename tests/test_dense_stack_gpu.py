@@ -25,7 +25,7 @@ def make(dtype, heads, kv_heads, dim, hidden, inter, layers, page, tied=True):
                                                    max_model_len=2600, cuda_graphs=graphs)
 
 
-STEPS = [[(0, 37)], [(0, 1)], [(0, 1), (1, 300)], [(0, 1), (1, 1), (2, 64), (3, 65)], [(4, 2200)], [(4, 130), (0, 1), (5, 9)],
+STEPS = [[(0, 37)], [(8, 8)], [(9, 3)], [(0, 1)], [(0, 1), (1, 300)], [(0, 1), (1, 1), (2, 64), (3, 65)], [(4, 2200)], [(4, 130), (0, 1), (5, 9)],
          [(i, 1) for i in range(6)], [(4, 1), (6, 7)], [(i, 1) for i in range(7)] + [(7, 600)]]
 
 
