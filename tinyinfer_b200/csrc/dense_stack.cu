@@ -36,15 +36,16 @@ typedef int (*Attention32Fn)(float*, const float*, const float*, const int*, con
 
 struct TiStackCall {
     RmsnormFn rmsnorm; AppendFn append; GemmFn gemm; LinkedFn linked; DecodeFn decode; OneTileFn one_tile; TwoTileFn two_tile;
+    void (*plain_next)();                          // sm100's: the next launch waits for all that its stream waits for
     SimtFn simt; FewFn few; SplitFn split; Attention32Fn attention32;
     const TiStackLayer* layer;
     const void* x; void* out;                      // [T, hidden]: the embedding's output, the last block's
     void* workspace; long long workspace_bytes;
     const int *positions, *token_seq, *decode_rows, *tiles;
     float* gemm_ws; long long gemm_ws_floats; int* counters;
-    float* attn_scratch; long long attn_floats;
+    float* attn_scratch; long long attn_floats, decode_floats;
     int *wait_status, *page_status;
-    cudaStream_t stream;
+    cudaStream_t stream, side;
     int layers, tokens, hidden, heads, kv_heads, head_dim, inter, act, page_size, dtype;
     int num_decode, num_tiles, num_pairs, max_context;
     int table_positions, interleaved, rotary_dim, num_counters;
@@ -82,6 +83,25 @@ Buffers lay_out(char* base, int tokens, int hidden, int q_size, int kv_size, int
     b.bytes = at;
     return b;
 }
+
+// The two events of a call that runs on two streams. An event may be given up while work still waits for it.
+struct Fork {
+    bool on, open = false;
+    cudaStream_t main, side;
+    cudaEvent_t begin = nullptr, end = nullptr;
+    Fork(bool wanted, cudaStream_t main, cudaStream_t side) : on(wanted), main(main), side(side) {
+        if (on && (cudaEventCreateWithFlags(&begin, cudaEventDisableTiming) != cudaSuccess ||
+                   cudaEventCreateWithFlags(&end, cudaEventDisableTiming) != cudaSuccess)) on = false;      // one stream, then
+    }
+    ~Fork() {
+        if (open) {                                 // a launch was refused in between: nobody frees what the second stream uses
+            cudaEventRecord(end, side);
+            cudaStreamWaitEvent(main, end, 0);
+        }
+        if (begin) cudaEventDestroy(begin);
+        if (end) cudaEventDestroy(end);
+    }
+};
 
 // Floats of scratch that a one-tile attention launch over `count` tiles needs, and its split of the keys: with few query tiles
 // behind a long prefix the keys are shared out over CTAs too (at least 1,024 to a CTA), so that most SMs have one.
@@ -172,6 +192,7 @@ TI_API int ti_dense_stack(TiStackCall* call) {
         const int rc__ = fused(__VA_ARGS__);      \
         if (rc__) return rc__;                    \
     } while (0)
+    Fork fork(!f32 && !few && c.side != nullptr && c.num_decode > 0 && c.num_tiles > 0, c.stream, c.side);
     const void* x = c.x;
     for (int i = 0; i < c.layers; ++i) {
         const TiStackLayer& l = c.layer[i];
@@ -192,10 +213,22 @@ TI_API int ti_dense_stack(TiStackCall* call) {
                                        c.num_decode, c.tiles, c.num_tiles, std::min(T, c.tile_rows), l.block_table, mb, c.heads, c.kv_heads,
                                        c.head_dim, c.page_size, pages, c.scale, window, c.page_status, c.stream));
         } else {
+            // Portions beside decoded tokens: two sets of rows, two kernels that each leave half the machine idle. The decoded
+            // tokens' runs on the second stream, on scratch of its own, and the output projection waits for both: a portion of 512
+            // tokens beside 27 decoded ones over 28 layers, 4.67 -> 4.49 ms.
+            if (fork.on) {
+                TI_REQUIRE(cudaEventRecord(fork.begin, c.stream) == cudaSuccess && cudaStreamWaitEvent(c.side, fork.begin, 0) == cudaSuccess,
+                           "dense_stack: the second stream cannot wait for the first");
+                fork.open = true;
+                c.plain_next();
+            }
             if (c.num_decode)
-                STACK_RUN(1, c.decode(b.att, b.q, l.kv, c.attn_scratch, c.attn_floats, c.decode_rows, c.num_decode, c.positions, c.token_seq,
+                STACK_RUN(1, c.decode(b.att, b.q, l.kv, c.attn_scratch, c.decode_floats, c.decode_rows, c.num_decode, c.positions, c.token_seq,
                                       l.block_table, mb, c.heads, c.kv_heads, c.head_dim, c.page_size, pages, c.scale, window, c.max_context,
-                                      c.wait_status, c.stream));
+                                      c.wait_status, fork.on ? c.side : c.stream));
+            if (fork.on) TI_REQUIRE(cudaEventRecord(fork.end, c.side) == cudaSuccess, "dense_stack: the second stream takes no event");
+            float* portion_scratch = c.attn_scratch + (fork.on ? c.decode_floats : 0);
+            const long long portion_floats = c.attn_floats - (fork.on ? c.decode_floats : 0);
             for (int kind = 0; kind < 2; ++kind) {  // tiles of more than 128 rows, then the ends of portions
                 const int first = kind ? c.num_pairs : 0, count = kind ? c.num_tiles - c.num_pairs : c.num_pairs;
                 if (!count) continue;
@@ -206,10 +239,15 @@ TI_API int ti_dense_stack(TiStackCall* call) {
                 }
                 int splits, split_keys;
                 const long long need = one_tile_plan(c, count, !kind, splits, split_keys);
-                TI_REQUIRE(need <= c.attn_floats, "dense_stack: %lld floats of attention scratch, %lld are needed", c.attn_floats, need);
+                TI_REQUIRE(need <= portion_floats, "dense_stack: %lld floats of attention scratch, %lld are needed", portion_floats, need);
                 STACK_RUN(1, c.one_tile(b.att, b.q, l.kv, c.tiles + 4 * first, count, T, l.block_table, mb, c.heads, c.kv_heads, c.head_dim,
-                                        c.page_size, pages, c.scale, window, !kind, splits, split_keys, splits > 1 ? c.attn_scratch : nullptr,
-                                        splits > 1 ? c.attn_floats : 0, c.wait_status, c.stream));
+                                        c.page_size, pages, c.scale, window, !kind, splits, split_keys, splits > 1 ? portion_scratch : nullptr,
+                                        splits > 1 ? portion_floats : 0, c.wait_status, c.stream));
+            }
+            if (fork.on) {
+                TI_REQUIRE(cudaStreamWaitEvent(c.stream, fork.end, 0) == cudaSuccess, "dense_stack: the first stream cannot wait for the second");
+                fork.open = false;
+                c.plain_next();
             }
         }
         void* out = last ? c.out : (void*)b.x2;

@@ -182,6 +182,7 @@ _SIGNATURES["sm100"]["ti_attention_prefill_pair_bf16"] = [
 _SIGNATURES["sm100"]["ti_attention_prefill_tc_bf16"] = [
     c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
     c_float, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_void_p]
+_SIGNATURES["sm100"]["ti_plain_next_launch"] = []
 _SIGNATURES["stack"] = {
     "ti_dense_stack": [c_void_p], "ti_dense_stack_portion_floats": [c_void_p],
     "ti_dense_stack_bytes": [c_int, c_int, c_int, c_int, c_int, c_int],
@@ -329,6 +330,14 @@ _branch = 0               # 1 while a ``Beside`` is open: products then use scra
 _side_streams = {}
 
 
+def _side_stream(device) -> torch.cuda.Stream:
+    key = torch.device(device)
+    side = _side_streams.get(key)
+    if side is None:
+        side = _side_streams[key] = torch.cuda.Stream(key, priority=-1)
+    return side
+
+
 class Beside:
     """Two independent chains of kernels side by side: what is launched inside ``with Beside(device) as b:`` runs on a second
     stream behind everything launched so far; what is launched between its end and ``b.join()`` runs on the current stream
@@ -338,11 +347,7 @@ class Beside:
     CTAs wait for one another may run in one of the chains only: the other one's must come to an end by themselves."""
 
     def __init__(self, device):
-        key = torch.device(device)
-        side = _side_streams.get(key)
-        if side is None:
-            side = _side_streams[key] = torch.cuda.Stream(key, priority=-1)
-        self.side, self.main = side, torch.cuda.current_stream(key)
+        self.side, self.main = _side_stream(device), torch.cuda.current_stream(torch.device(device))
 
     def __enter__(self):
         global _branch, _plain_next
@@ -1136,7 +1141,7 @@ FUSED_NORM_LAYER_BYTES = 48 << 20      # ... if a layer's matrices are no larger
                                        # 101 MB 4 to 16 % slower (more than a wave of blocks a product)
 _STACK_LAUNCHERS = (("core", "ti_rmsnorm"), ("core", "ti_qk_norm_rope_append"), ("sm100", "ti_gemm_bf16"),
                     ("sm100", "ti_gemm_bf16_linked"), ("sm100", "ti_attention_decode_bf16"), ("sm100", "ti_attention_prefill_tc_bf16"),
-                    ("sm100", "ti_attention_prefill_pair_bf16"), ("core", "ti_gemm_simt"), ("f32", "ti_gemm_f32_few"),
+                    ("sm100", "ti_attention_prefill_pair_bf16"), ("sm100", "ti_plain_next_launch"), ("core", "ti_gemm_simt"), ("f32", "ti_gemm_f32_few"),
                     ("f32", "ti_gemm_f32_split"), ("f32", "ti_attention_f32"))
 _STACK_LIBRARIES = {torch.bfloat16: ("core", "sm100"), torch.float32: ("core", "f32")}
 _stack_launchers = {}
@@ -1145,8 +1150,8 @@ _stack_launchers = {}
 class _StackCall(ctypes.Structure):
     _fields_ = ([(name, c_void_p) for _, name in _STACK_LAUNCHERS] + [(n, c_void_p) for n in ("layer", "x", "out", "workspace")]
                 + [("workspace_bytes", c_ll)] + [(n, c_void_p) for n in ("positions", "token_seq", "decode_rows", "tiles", "gemm_ws")]
-                + [("gemm_ws_floats", c_ll), ("counters", c_void_p), ("attn_scratch", c_void_p), ("attn_floats", c_ll)]
-                + [(n, c_void_p) for n in ("wait_status", "page_status", "stream")]
+                + [("gemm_ws_floats", c_ll), ("counters", c_void_p), ("attn_scratch", c_void_p), ("attn_floats", c_ll), ("decode_floats", c_ll)]
+                + [(n, c_void_p) for n in ("wait_status", "page_status", "stream", "side")]
                 + [(n, c_int) for n in ("layers", "tokens", "hidden", "heads", "kv_heads", "head_dim", "inter", "act", "page_size",
                                         "dtype", "num_decode", "num_tiles", "num_pairs", "max_context", "table_positions",
                                         "interleaved", "rotary_dim", "num_counters", "link_max_tokens", "pair_min_ctas",
@@ -1205,8 +1210,12 @@ def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: in
         portions.restype = c_ll
         floats = portions(ctypes.addressof(call))
         if step.num_decode:
-            floats = max([floats] + [decode_scratch_floats(step.num_decode, heads, kv_heads, head_dim, int(step.max_context), w)
-                                     for w in {row[16] for row in layers}])
+            call.decode_floats = max(decode_scratch_floats(step.num_decode, heads, kv_heads, head_dim, int(step.max_context), w)
+                                     for w in {row[16] for row in layers})
+            if step.num_prefill_tiles and not _branch:       # both kinds of attention at a time, on scratch of their own
+                call.side = _side_stream(x.device).cuda_stream
+                floats += call.decode_floats
+            floats = max(floats, call.decode_floats)
         if floats:
             scratch = _decode_scratch(x.device, floats)
             call.attn_scratch, call.attn_floats = scratch.data_ptr(), scratch.numel()
