@@ -105,6 +105,8 @@ ATTENTION = [
     (12, 4, 128, 48, 40, [(300, 44), (65, 1), (64, 1), (700, 301)]),
     (32, 1, 64, 64, -50, [(149, 99), (150, 1), (151, 1), (333, 17)]),
     (6, 1, 128, 5, None, [(91, 1), (64, 64), (65, 64)]),
+    (16, 16, 64, 64, None, [(1300, 1300), (77, 70)]),             # enough rows for 32 a block
+    (20, 4, 128, 64, None, [(700, 700), (1200, 513), (300, 300)]),
 ]
 
 

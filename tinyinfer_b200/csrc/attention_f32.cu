@@ -7,10 +7,11 @@
 // running maximum, sum and output of its own; they meet by shuffles, then in shared memory, then across the cluster through
 // distributed shared memory, where every block finishes an eighth of the output. Bound by the keys' and values' way from HBM.
 //
-// Portions of prompts: a block takes 32 query rows, which are the query heads of one kv head for 32 / G neighbouring tokens,
-// over tiles of 64 keys: keys and values come in by cp.async, the values' copy runs under the scores. 256 threads make 2 x 4
-// scores and 2 x (D / 16) outputs each. Bound by shared-memory reads beside the multiply-adds.
-// A layer of 16 over 8 heads of 128: 333 prompt tokens 0.8 ms with a block a (token, head) -> 53 us; 4 tokens behind 1,024 keys
+// Portions of prompts: a block takes 16 or 32 query rows, which are the query heads of one kv head for neighbouring tokens,
+// over tiles of 64 keys: keys and values come in by cp.async, the values' copy runs under the scores. A thread makes 2 x 4
+// scores and 2 x (D / 16) outputs. Bound by shared-memory reads beside the multiply-adds.
+// A layer of 16 over 8 heads of 128: 333 prompt tokens 0.8 ms with a block a (token, head) -> 53 us with
+// 32 rows a block -> some 30 us with 16, the longest ranges first (a step of 28 layers 11.0 -> 10.4 ms); 4 tokens behind 1,024 keys
 // 32 us with the queries in registers and one block an SM -> 13 us with them in shared memory and two.
 #include "common.cuh"
 #include <cooperative_groups.h>
@@ -191,9 +192,9 @@ __global__ void __cluster_dims__(DEC_CTAS, 1, 1) __launch_bounds__(DEC_WARPS * 3
     cluster.sync();                              // nobody leaves while its shared memory may be read
 }
 
-constexpr int PR_ROWS = 32, PR_KEYS = 64, PR_THREADS = 256;
+constexpr int PR_KEYS = 64, PR_MAX_ROWS = 32;
 
-template <int D> constexpr int portion_smem() {
+template <int D, int PR_ROWS> constexpr int portion_smem() {
     return 4 * (PR_ROWS * (D + 4) + PR_KEYS * (D + 4) + PR_KEYS * D + PR_ROWS * (PR_KEYS + 4)) + 8 * PR_KEYS;
 }
 __device__ __forceinline__ void copy16(void* dst, const void* src, bool there) {
@@ -201,20 +202,21 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool there) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
 
-template <int D>
-__global__ void __launch_bounds__(PR_THREADS) portion_f32_kernel(const AfArgs a) {
+template <int D, int PR_ROWS>
+__global__ void __launch_bounds__(PR_ROWS * 8) portion_f32_kernel(const AfArgs a) {
+    constexpr int PR_THREADS = PR_ROWS * 8;
     extern __shared__ float4 smem4[];
-    float* qs = reinterpret_cast<float*>(smem4);             // [32][D + 4]: rows 16 bytes askew, so that 8 lanes meet 32 banks
+    float* qs = reinterpret_cast<float*>(smem4);             // [PR_ROWS][D + 4]: rows 16 bytes askew, so that 8 lanes meet 32 banks
     float* ks = qs + PR_ROWS * (D + 4);                      // [64][D + 4]
     float* vs = ks + PR_KEYS * (D + 4);                      // [64][D]
-    float* ps = vs + PR_KEYS * D;                            // [32][64 + 4]
+    float* ps = vs + PR_KEYS * D;                            // [PR_ROWS][64 + 4]
     long long* off = reinterpret_cast<long long*>(ps + PR_ROWS * (PR_KEYS + 4));
     ti_grid_launch_dependents();
     ti_grid_wait();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int kvh = blockIdx.x, G = a.hq / a.hkv, per = PR_ROWS / G;
     const int* tile = a.rows + 4 * blockIdx.z;
-    const int first = (int)blockIdx.y * per;                 // the block's first token within the tile
+    const int first = ((int)gridDim.y - 1 - (int)blockIdx.y) * per;    // the block's first token within the tile, the longest ranges first
     const int tokens = min(per, tile[2] - first);
     if (tokens <= 0) return;
     const int row0 = tile[1] + first, pos0 = tile[3] + first, last = pos0 + tokens - 1;
@@ -349,16 +351,12 @@ __global__ void __launch_bounds__(PR_THREADS) portion_f32_kernel(const AfArgs a)
     }
 }
 
-template <int D>
+template <int D, int PR_ROWS>
 int launch_portions(const AfArgs& a, int tiles, int tile_rows, cudaStream_t stream) {
-    static bool set = false;
-    if (!set) {
-        const cudaError_t e = cudaFuncSetAttribute(portion_f32_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, portion_smem<D>());
-        TI_REQUIRE(e == cudaSuccess, "attention_f32: %s", cudaGetErrorString(e));
-        set = true;
-    }
+    static const cudaError_t set = cudaFuncSetAttribute(portion_f32_kernel<D, PR_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, portion_smem<D, PR_ROWS>());
+    TI_REQUIRE(set == cudaSuccess, "attention_f32: %s", cudaGetErrorString(set));
     const int per = PR_ROWS / (a.hq / a.hkv);
-    ti_launch(portion_f32_kernel<D>, dim3(a.hkv, (tile_rows + per - 1) / per, tiles), PR_THREADS, portion_smem<D>(), stream, a);
+    ti_launch(portion_f32_kernel<D, PR_ROWS>, dim3(a.hkv, (tile_rows + per - 1) / per, tiles), PR_ROWS * 8, portion_smem<D, PR_ROWS>(), stream, a);
     return 0;
 }
 template <int D>
@@ -380,7 +378,7 @@ TI_API int ti_attention_f32(float* out, const float* q, const float* kv_cache, c
                             const int* block_table, int max_blocks, int hq, int hkv, int d, int page_size, int num_pages,
                             float scale, int window, int* status, cudaStream_t stream) {
     TI_REQUIRE(d == 64 || d == 128, "attention_f32: head_dim %d is neither 64 nor 128", d);
-    TI_REQUIRE(hq > 0 && hkv > 0 && hq % hkv == 0 && hq / hkv <= PR_ROWS, "attention_f32: %d query heads over %d kv heads", hq, hkv);
+    TI_REQUIRE(hq > 0 && hkv > 0 && hq % hkv == 0 && hq / hkv <= PR_MAX_ROWS, "attention_f32: %d query heads over %d kv heads", hq, hkv);
     TI_REQUIRE(page_size > 0 && num_decode >= 0 && num_tiles >= 0 && tile_rows > 0 && num_decode <= 65535 && num_tiles <= 65535 &&
                    tile_rows <= 65535, "attention_f32: bad sizes");
     TI_REQUIRE(((uintptr_t)out | (uintptr_t)q | (uintptr_t)kv_cache) % 16 == 0, "attention_f32: operands must lie on 16-byte boundaries");
@@ -394,7 +392,12 @@ TI_API int ti_attention_f32(float* out, const float* q, const float* kv_cache, c
     }
     if (num_tiles) {
         a.rows = tiles;
-        const int rc = d == 128 ? launch_portions<128>(a, num_tiles, tile_rows, stream) : launch_portions<64>(a, num_tiles, tile_rows, stream);
+        // 16 rows a block until blocks of 32 would fill the machine four times over: 333 tokens make 168 of those, and the step
+        // waits for the one with the most keys
+        const int G = hq / hkv;
+        const bool small = G <= 16 && (long long)num_tiles * tile_rows * G / 32 * hkv < 4 * 148;
+        const int rc = d == 128 ? (small ? launch_portions<128, 16>(a, num_tiles, tile_rows, stream) : launch_portions<128, 32>(a, num_tiles, tile_rows, stream))
+                                : (small ? launch_portions<64, 16>(a, num_tiles, tile_rows, stream) : launch_portions<64, 32>(a, num_tiles, tile_rows, stream));
         if (rc) return rc;
         TI_CHECK_LAUNCH("attention_f32 portions");
     }
