@@ -5,9 +5,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# 2,048 choices are the most one block places; 1,184 tokens the fewest that go eight a block
+# 1,024 choices are the most one block places; 1,184 tokens the fewest that go eight a block
 @pytest.mark.parametrize("tokens,experts,identity,top,hidden", [
-    (1, 3, 0, 1, 40), (512, 33, 2, 4, 64), (513, 64, 0, 4, 72), (1183, 40, 1, 2, 128), (1184, 256, 0, 2, 96), (1201, 70, 6, 6, 2048),
+    (1, 3, 0, 1, 40), (256, 33, 2, 4, 64), (257, 64, 0, 4, 72), (1183, 40, 1, 2, 128), (1184, 256, 0, 2, 96), (1201, 70, 6, 6, 2048),
     (2048, 5, 0, 1, 64)])
 @pytest.mark.parametrize("router,rows", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
 def test_routing(tokens, experts, identity, top, hidden, router, rows):
