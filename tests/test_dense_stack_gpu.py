@@ -71,3 +71,17 @@ def test_what_the_stack_does_not_take(monkeypatch):
         del called[:]
         out = run(runner(), [[(0, 20)], [(0, 1)]])
         assert bool(called) == taken and all(torch.isfinite(o).all() for o in out)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim", [(5, 1, 128), (3, 3, 64), (7, 1, 64), (12, 4, 128)])
+def test_portions_beside_decoded_tokens_behind_a_long_prefix(heads, kv_heads, dim):
+    """Odd numbers of heads and rows: where the portions' keys are shared out over CTAs, their partial results lie behind the
+    decoded tokens' on one scratch. The kernels are the parts', and so are the bits."""
+    from tinyinfer_b200 import ops
+    model, runner = make(torch.bfloat16, heads, kv_heads, dim, 64 * heads, 384, 2, 64)
+    steps = [[(0, 2300)], [(1, 40), (2, 33), (3, 21)], [(1, 1), (0, 40)], [(2, 1), (0, 60), (1, 1)], [(1, 1), (2, 1), (3, 1), (0, 130)]]
+    got = run(runner(), steps)
+    model._stack = None
+    want = run(runner(), steps)
+    assert all(torch.equal(g, w) and torch.isfinite(g).all() for g, w in zip(got, want))
+    ops.check_kernel_status()

@@ -486,6 +486,7 @@ TI_API int ti_attention_prefill_tc_sink_bf16(void* out, const void* q, const voi
                                scratch_floats >= ti_attention_prefill_scratch_floats(num_tiles, halves, splits, hq, d)),
                "attention_prefill_tc: a split of the keys needs shares of a multiple of %d keys and %lld floats of scratch",
                KT, ti_attention_prefill_scratch_floats(num_tiles, halves, splits, hq, d));
+    TI_REQUIRE(((uintptr_t)scratch & 15) == 0, "attention_prefill_tc: scratch must lie on a 16-byte boundary");
     TI_REQUIRE(d == 64 || d == 128, "attention_prefill_tc: head_dim %d is not 64 or 128", d);
     TI_REQUIRE(hq > 0 && hkv > 0 && hq % hkv == 0, "attention_prefill_tc: bad head counts");
     TI_REQUIRE(num_tiles <= 32767, "attention_prefill_tc: more than 32767 tiles in one step");

@@ -1210,8 +1210,9 @@ def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: in
         portions.restype = c_ll
         floats = portions(ctypes.addressof(call))
         if step.num_decode:
-            call.decode_floats = max(decode_scratch_floats(step.num_decode, heads, kv_heads, head_dim, int(step.max_context), w)
-                                     for w in {row[16] for row in layers})
+            need = max(decode_scratch_floats(step.num_decode, heads, kv_heads, head_dim, int(step.max_context), w)
+                       for w in {row[16] for row in layers})
+            call.decode_floats = -(-need // 64) * 64         # the portions' scratch begins behind it and is written 16 bytes at a time
             if step.num_prefill_tiles and not _branch:       # both kinds of attention at a time, on scratch of their own
                 call.side = _side_stream(x.device).cuda_stream
                 floats += call.decode_floats
