@@ -6,7 +6,6 @@
 // the launch costs. What is launched, on what and in which order is what the layers' parts would launch.
 // 37 tokens, 28 layers of hidden size 1024: 3.66 -> 1.30 ms a step, the outputs the same bit for bit.
 #include "common.cuh"
-#include "gemm_few_mma.cuh"
 #include <algorithm>
 
 struct TiStackLayer {
@@ -49,7 +48,7 @@ struct TiStackCall {
     int layers, tokens, hidden, heads, kv_heads, head_dim, inter, act, page_size, dtype;
     int num_decode, num_tiles, num_pairs, max_context;
     int table_positions, interleaved, rotary_dim, num_counters;
-    int link_max_tokens, pair_min_ctas, split_max_ctas, few_rows, min_k, tile_rows, fused_rows;
+    int link_max_tokens, pair_min_ctas, split_max_ctas, few_rows, min_k, tile_rows;
     float eps1, eps2, qk_eps, scale;
     int failed;                                    // out: which library's launcher failed (0 core, 1 sm100, 2 f32)
 };
@@ -177,32 +176,14 @@ TI_API int ti_dense_stack(TiStackCall* call) {
         const int rc__ = product(__VA_ARGS__);    \
         if (rc__) return rc__;                    \
     } while (0)
-    // a bfloat16 step of few tokens: every product with the norm before it in one kernel
-    const bool few = !f32 && T <= c.fused_rows;
-    auto fused = [&](void* out, const void* x, const void* w, const float* g, float eps, const float* bias, const void* residual, int n,
-                     int k, int gated) -> int {
-        typedef __nv_bfloat16 B;
-        const cudaError_t e = few::product(few::Args{(B*)out, (const B*)x, (const B*)w, (const B*)residual, g, bias, eps, T, n, k}, gated, c.stream);
-        TI_REQUIRE(e == cudaSuccess, "dense_stack: gemm_few: %s", cudaGetErrorString(e));
-        ti_count_launch();
-        return 0;
-    };
-#define STACK_FUSED(...)                          \
-    do {                                          \
-        const int rc__ = fused(__VA_ARGS__);      \
-        if (rc__) return rc__;                    \
-    } while (0)
-    Fork fork(!f32 && !few && c.side != nullptr && c.num_decode > 0 && c.num_tiles > 0, c.stream, c.side);
+    Fork fork(!f32 && c.side != nullptr && c.num_decode > 0 && c.num_tiles > 0, c.stream, c.side);
     const void* x = c.x;
     for (int i = 0; i < c.layers; ++i) {
         const TiStackLayer& l = c.layer[i];
         const bool last = i + 1 == c.layers;
-        if (few) STACK_FUSED(b.qkv, x, l.w_qkv, l.norm1, c.eps1, l.b_qkv, nullptr, qs + 2 * kvs, H, 0);
-        else {
-            const bool from_link = parts > 0;
-            if (!from_link) STACK_RUN(0, c.rmsnorm(b.h, x, l.norm1, nullptr, T, H, c.eps1, c.dtype, c.stream));
-            STACK_PRODUCT(b.qkv, b.h, l.w_qkv, l.b_qkv, nullptr, qs + 2 * kvs, H, 0, from_link, c.eps1, nullptr);
-        }
+        const bool from_link = parts > 0;
+        if (!from_link) STACK_RUN(0, c.rmsnorm(b.h, x, l.norm1, nullptr, T, H, c.eps1, c.dtype, c.stream));
+        STACK_PRODUCT(b.qkv, b.h, l.w_qkv, l.b_qkv, nullptr, qs + 2 * kvs, H, 0, from_link, c.eps1, nullptr);
         STACK_RUN(0, c.append(b.q, b.qkv, l.writes ? l.kv : nullptr, l.q_norm, l.k_norm, c.qk_eps, l.inv_freq, l.cos_sin, c.table_positions,
                               c.interleaved, c.rotary_dim, c.positions, c.token_seq, l.block_table, (int)l.max_blocks, T, c.heads,
                               c.kv_heads, c.head_dim, l.writes ? c.page_size : 1, l.writes ? (int)l.num_pages : 1, c.page_status, c.dtype,
@@ -251,13 +232,6 @@ TI_API int ti_dense_stack(TiStackCall* call) {
             }
         }
         void* out = last ? c.out : (void*)b.x2;
-        if (few) {
-            STACK_FUSED(b.x1, b.att, l.w_o, nullptr, 0.f, l.b_o, x, H, qs, 0);
-            STACK_FUSED(b.hid, b.x1, l.w_gate_up, l.norm2, c.eps2, nullptr, nullptr, c.inter, H, c.act);
-            STACK_FUSED(out, b.hid, l.w_down, nullptr, 0.f, nullptr, b.x1, H, c.inter, 0);
-            x = out;
-            continue;
-        }
         parts = 0;
         STACK_PRODUCT(b.x1, b.att, l.w_o, l.b_o, x, H, qs, 0, false, 0.f, links ? l.norm2 : nullptr);
         const bool mlp_link = parts > 0;
@@ -267,7 +241,6 @@ TI_API int ti_dense_stack(TiStackCall* call) {
         STACK_PRODUCT(out, b.hid, l.w_down, nullptr, b.x1, H, c.inter, 0, false, 0.f, links && !last ? c.layer[i + 1].norm1 : nullptr);
         x = out;
     }
-#undef STACK_FUSED
 #undef STACK_PRODUCT
 #undef STACK_RUN
     return 0;

@@ -1136,9 +1136,6 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
 
 
 # ---------------------------------------------------------------------- a dense decoder's blocks in one call
-FUSED_NORM_ROWS = 8                    # bfloat16 steps of so many tokens run each product with the norm before it in one kernel ...
-FUSED_NORM_LAYER_BYTES = 48 << 20      # ... if a layer's matrices are no larger: at 31 MB it is 8 to 12 % of the step faster, at
-                                       # 101 MB 4 to 16 % slower (more than a wave of blocks a product)
 _STACK_LAUNCHERS = (("core", "ti_rmsnorm"), ("core", "ti_qk_norm_rope_append"), ("sm100", "ti_gemm_bf16"),
                     ("sm100", "ti_gemm_bf16_linked"), ("sm100", "ti_attention_decode_bf16"), ("sm100", "ti_attention_prefill_tc_bf16"),
                     ("sm100", "ti_attention_prefill_pair_bf16"), ("sm100", "ti_plain_next_launch"), ("core", "ti_gemm_simt"), ("f32", "ti_gemm_f32_few"),
@@ -1155,15 +1152,14 @@ class _StackCall(ctypes.Structure):
                 + [(n, c_int) for n in ("layers", "tokens", "hidden", "heads", "kv_heads", "head_dim", "inter", "act", "page_size",
                                         "dtype", "num_decode", "num_tiles", "num_pairs", "max_context", "table_positions",
                                         "interleaved", "rotary_dim", "num_counters", "link_max_tokens", "pair_min_ctas",
-                                        "split_max_ctas", "few_rows", "min_k", "tile_rows", "fused_rows")]
+                                        "split_max_ctas", "few_rows", "min_k", "tile_rows")]
                 + [(n, c_float) for n in ("eps1", "eps2", "qk_eps", "scale")] + [("failed", c_int)])
 
 
 def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: int, head_dim: int, inter: int, activation: str,
                 page_size: int, eps: tuple, scale: float, rotation: Optional[Rotation]) -> torch.Tensor:
     """Runs the blocks of a dense pre-norm decoder on ``x`` [T, hidden] by one native call that makes every launch of
-    ``linear``, ``rmsnorm``, ``qk_norm_rope_append``, ``paged_attention`` and ``gated_linear`` that the parts would (bfloat16 steps of
-    few tokens through small layers: products that hold the norm before them).
+    ``linear``, ``rmsnorm``, ``qk_norm_rope_append``, ``paged_attention`` and ``gated_linear`` that the parts would.
     ``layers``: per layer, in the order they run, 18 integers (addresses, 0 for what a layer has not, and sizes): w_qkv, b_qkv,
     w_o, b_o, q norm, k norm, inverse frequencies, table of cosines and sines, norm 1, norm 2, w_gate_up, w_down, cache, block
     table, its width, pages, window, whether it writes its cache. ``eps``: of the first norm, the second, and of q and k. The
@@ -1180,8 +1176,6 @@ def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: in
                                                  for lib, name in _STACK_LAUNCHERS]
     size = _fn("stack", "ti_dense_stack_bytes")
     size.restype = c_ll
-    layer_bytes = 2 * hidden * ((2 * heads + 2 * kv_heads) * head_dim + 3 * inter)
-    fused = FUSED_NORM_ROWS if code == 1 and layer_bytes <= FUSED_NORM_LAYER_BYTES else 0
     nbytes = size(t, hidden, heads * head_dim, kv_heads * head_dim, inter, code)
     workspace = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     out = torch.empty_like(x)
@@ -1200,7 +1194,7 @@ def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: in
         call.table_positions = rotation.cos_sin.shape[0] if rotation.cos_sin is not None else 0
         call.interleaved, call.rotary_dim = int(rotation.interleaved), rotation.rotary_dim
     call.link_max_tokens, call.pair_min_ctas, call.split_max_ctas = NORM_LINK_MAX_TOKENS, PAIR_MIN_CTAS, KEY_SPLIT_MAX_CTAS
-    call.few_rows, call.min_k, call.tile_rows, call.fused_rows = F32_FEW_ROWS, F32_MIN_K, PREFILL_TILE, fused
+    call.few_rows, call.min_k, call.tile_rows = F32_FEW_ROWS, F32_MIN_K, PREFILL_TILE
     call.eps1, call.eps2, call.qk_eps = eps
     call.scale = scale
     if code == 1:
@@ -1220,8 +1214,8 @@ def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: in
         if floats:
             scratch = _decode_scratch(x.device, floats)
             call.attn_scratch, call.attn_floats = scratch.data_ptr(), scratch.numel()
-    if _plain_next:                              # the first launch is the core library's, or this one's own
-        library.load("stack" if t <= fused else "core").ti_plain_next_launch()
+    if _plain_next:                              # the first launch is the core library's
+        library.load("core").ti_plain_next_launch()
         _plain_next = False
     rc = _fn("stack", "ti_dense_stack")(ctypes.addressof(call))
     if rc != 0:

@@ -37,7 +37,7 @@ LIBRARIES: Dict[str, dict] = {
                           "attention_generic.cu", "gemm_simt.cu", "sampling.cu"],
                  headers=["common.cuh"], link=[]),
     # a dense decoder's layers launched from one call, through the other libraries' launchers
-    "stack": dict(sources=["runtime.cu", "dense_stack.cu"], headers=["common.cuh", "gemm_few_mma.cuh"], link=[]),
+    "stack": dict(sources=["runtime.cu", "dense_stack.cu"], headers=["common.cuh"], link=[]),
     # the 32-bit path at the sizes it is used at: products and attention
     "f32": dict(sources=["runtime.cu", "sm100_host.cu", "gemm_f32_few.cu", "gemm_f32_split_tcgen05.cu", "attention_f32.cu"],
                 headers=["common.cuh", "sm100_ptx.cuh"], link=[]),
