@@ -164,3 +164,52 @@ def test_attention_reports_a_key_without_a_page_and_keeps_rows_apart(ops):
     bt[1, 0] = -1
     got = ops.paged_attention(q, kv, block_table=bt, status=status, **args)
     assert int(status.item()) == 2 and torch.isfinite(got[20]).all() and torch.equal(got[:18], want[:18])
+
+
+@pytest.mark.parametrize("m,n,k,act", [(9, 514, 2048, None), (130, 259, 516, None), (333, 1000, 1028, None), (140, 130, 6144, "gelu_tanh"), (333, 6000, 512, "silu")])
+def test_split_product_makes_infinite_and_nan_outputs_again(ops, m, n, k, act):
+    """Outputs that are not finite in parts are the general kernel's bit for bit, whatever share of a tile they are, and the rest
+    of the tile keeps its precision; a product of NaN alone costs no more than a few of the general kernel's."""
+    rows = n * (2 if act else 1)
+    x, w, b = (rnd(*s, dtype=torch.float32, seed=i) for i, s in enumerate(((m, k), (rows, k), (rows,))))
+    x[1], x[m - 1, k - 1], x[m // 2, 3], w[rows - 2, 5] = float("nan"), float("inf"), -float("inf"), float("nan")
+    w[3] = 0.0
+    w[3, ::7] = 3.4e38                                  # rounds to infinity in bfloat16: finite outputs of rows that are small enough
+    x[4:6] *= 1e-9
+
+    def product(x):
+        return ops.gated_linear(x, w, activation=act, bias=b) if act else ops.linear(x, w, bias=b)
+
+    def plain(x):
+        out = torch.empty((m, n), dtype=torch.float32, device=dev())
+        ops._run("core", "ti_gemm_simt", out.data_ptr(), x.data_ptr(), w.data_ptr(), b.data_ptr(), None, m, n, k,
+                 ops.GATED_ACTIVATIONS[act] if act else 0, 0, 0, ops._stream())
+        return out
+    got, want = product(x), plain(x)
+    same = torch.zeros((m, n), dtype=torch.bool, device=dev())
+    same[[1, m // 2, m - 1]] = True                     # made again whole
+    same[:, (rows - 2) % n] = True
+    same[:, 3] = True
+    assert torch.equal(torch.isnan(got), torch.isnan(want))
+    fine = same & ~torch.isnan(want)
+    if not act:
+        assert torch.equal(got[fine], want[fine])
+    z = x.double() @ w.double().T + b
+    rest = ~same
+    exact = gated(z, act) if act else z
+    assert (got - exact)[rest].norm() <= 2e-6 * exact[rest].norm()
+
+    def best(run):
+        times = []
+        for _ in range(4):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            run()
+            end.record()
+            torch.cuda.synchronize()
+            times.append(begin.elapsed_time(end))
+        return min(times)
+    x[:] = float("nan")
+    assert torch.isnan(product(x)).all()
+    assert best(lambda: product(x)) <= 4 * best(lambda: plain(x)) + 0.1
+    ops.check_kernel_status()

@@ -19,7 +19,8 @@
 //   warps 0..7    drain finished chunks into their registers, at the end into shared memory
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
-// multiply-adds in k order, so that such operands give what they give in float32.
+// multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
+// again through shared memory (redo_plain), at about the cost of gemm_simt.cu.
 // Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 118 us (142 TFLOP/s), by 2,048 x 6,144
 // 799 -> 78 us; 9 rows 306 -> 51 us; 256 x 256 weights, the smallest that come here, 20 -> 5.5 us.
 #include "sm100_ptx.cuh"
@@ -90,14 +91,48 @@ __device__ __forceinline__ uint64_t make_sw64_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
 }
 
-__device__ __noinline__ float plain_dot(const float* x, const float* w, int K) {
-    float v = 0.f;
-    for (int k = 0; k < K; ++k) v = fmaf(x[k], w[k], v);
-    return v;
+// The CTA's share of the outputs by multiply-adds in k order, one accumulator an output: out[col][row] for `cols` tokens from
+// m on and the 128 rows of w that the tile has on its lanes. A thread has one row and every fourth token, operands come 16 k at a time
+// through shared memory.
+constexpr int REDO_K = 16, REDO_LD = REDO_K + 4, REDO_THREADS = 512;
+__device__ __noinline__ void redo_plain(float* out, float* ws, float* xs, const SplitParams& p, int m, int cols, int n0, int outs) {
+    const int row = threadIdx.x & 127, group = threadIdx.x >> 7;
+    float acc[MAX_BN / 4] = {};
+    for (int k0 = 0; k0 < p.K; k0 += REDO_K) {
+        __syncthreads();                                     // everyone is done with the piece before
+        for (int i = threadIdx.x; i < 2 * 128 * (REDO_K / 4); i += NUM_THREADS) {
+            const int r = i / (REDO_K / 4) & 127, k = k0 + i % (REDO_K / 4) * 4;
+            const bool weights = i < 128 * (REDO_K / 4);
+            const int w_row = (r < outs ? 0 : p.N) + min(n0 + r % outs, p.N - 1);
+            const float* src = weights ? p.w + (size_t)w_row * p.K : p.x + (size_t)min(m + r, p.M - 1) * p.K;
+            const float4 v = k < p.K ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+            *reinterpret_cast<float4*>((weights ? ws : xs) + r * REDO_LD + k - k0) = v;
+        }
+        __syncthreads();
+        if (threadIdx.x >= REDO_THREADS) continue;
+#pragma unroll 1
+        for (int k = 0; k < REDO_K; k += 4) {
+            const float4 w = *reinterpret_cast<const float4*>(ws + row * REDO_LD + k);
+#pragma unroll
+            for (int j = 0; j < MAX_BN / 4; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(xs + (group + 4 * j) * REDO_LD + k);
+                acc[j] = fmaf(x.x, w.x, acc[j]);
+                acc[j] = fmaf(x.y, w.y, acc[j]);
+                acc[j] = fmaf(x.z, w.z, acc[j]);
+                acc[j] = fmaf(x.w, w.w, acc[j]);
+            }
+        }
+    }
+    if (threadIdx.x < REDO_THREADS) {
+#pragma unroll
+        for (int j = 0; j < MAX_BN / 4; ++j)
+            if (group + 4 * j < cols) out[(group + 4 * j) * 128 + row] = acc[j];
+    }
+    __syncthreads();
 }
 
 __global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const SplitParams p) {
+gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ SplitParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t bars[2 * (A_STAGES + MAX_B_STAGES + MAX_SLOTS) + 4];
@@ -306,47 +341,60 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int c0 = p.bn * part / splits, c1 = p.bn * (part + 1) / splits;
     if (!*abort_flag) {
         ti_grid_wait();                                      // out and residual belong to the kernels ahead until now
-        const int quads = outs / 4;                          // four neighbouring outputs a thread
-        for (int i = threadIdx.x; i < (c1 - c0) * quads; i += NUM_THREADS) {
-            const int col = c0 + i / quads, o = i % quads * 4, m = m0 + col, n = n0 + o;
-            if (m >= p.M || n >= p.N) continue;
-            float total[2][4] = {};
-            const int kinds = p.gated ? 2 : 1;
-            for (int g = 0; g < kinds; ++g) {
-                float4 f[8];
+        const int quads = outs / 4, kinds = p.gated ? 2 : 1; // four neighbouring outputs a thread
+        float* again = sums + MAX_BN * 128;                  // [c1 - c0][128]: outputs made again, behind the sums
+        // first the outputs whose sums are finite; if there are others, these once they have been made again
+        for (bool redone = false;; redone = true) {
+            bool odd = false;
+            for (int i = threadIdx.x; i < (c1 - c0) * quads; i += NUM_THREADS) {
+                const int col = c0 + i / quads, o = i % quads * 4, m = m0 + col, n = n0 + o;
+                if (m >= p.M || n >= p.N) continue;
+                float total[2][4] = {};
+                bool finite = true;
+                for (int g = 0; g < kinds; ++g) {
+                    float4 f[8];
 #pragma unroll
-                for (int r = 0; r < 8; ++r)
-                    if (r < splits) f[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums + col * 128 + o + 64 * g, r));
+                    for (int r = 0; r < 8; ++r)
+                        if (r < splits) f[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums + col * 128 + o + 64 * g, r));
 #pragma unroll
-                for (int r = 0; r < 8; ++r)
-                    if (r < splits) {
-                        total[g][0] += f[r].x; total[g][1] += f[r].y; total[g][2] += f[r].z; total[g][3] += f[r].w;
+                    for (int r = 0; r < 8; ++r)
+                        if (r < splits) {
+                            total[g][0] += f[r].x; total[g][1] += f[r].y; total[g][2] += f[r].z; total[g][3] += f[r].w;
+                        }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (!isfinite(total[g][e]) && n + e < p.N) {
+                            finite = false;
+                            total[g][e] = again[(col - c0) * 128 + o + 64 * g + e];
+                        }
                     }
-            }
-            float res[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                if (n + e >= p.N) { res[e] = 0.f; continue; }
-                auto finite = [&](float v, int w_row) {
-                    return isfinite(v) ? v : plain_dot(p.x + (size_t)m * p.K, p.w + (size_t)w_row * p.K, p.K);
-                };
-                float v = finite(total[0][e], n + e);
-                if (p.bias) v += p.bias[n + e];
-                if (p.gated) {
-                    float up = finite(total[1][e], p.N + n + e);
-                    if (p.bias) up += p.bias[p.N + n + e];
-                    if (p.gated == 1) v = v / (1.f + expf(-v));
-                    else v = 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-                    v *= up;
-                } else if (p.residual) {
-                    v += p.residual[(size_t)m * p.N + n + e];
                 }
-                res[e] = v;
+                odd |= !finite;
+                if (finite == redone) continue;
+                float res[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (n + e >= p.N) { res[e] = 0.f; continue; }
+                    float v = total[0][e];
+                    if (p.bias) v += p.bias[n + e];
+                    if (p.gated) {
+                        float up = total[1][e];
+                        if (p.bias) up += p.bias[p.N + n + e];
+                        if (p.gated == 1) v = v / (1.f + expf(-v));
+                        else v = 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
+                        v *= up;
+                    } else if (p.residual) {
+                        v += p.residual[(size_t)m * p.N + n + e];
+                    }
+                    res[e] = v;
+                }
+                float* dst = p.out + (size_t)m * p.N + n;
+                if (p.N % 4 == 0 && ((uintptr_t)p.out & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(res[0], res[1], res[2], res[3]);
+                else
+                    for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = res[e];
             }
-            float* dst = p.out + (size_t)m * p.N + n;
-            if (p.N % 4 == 0 && ((uintptr_t)p.out & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(res[0], res[1], res[2], res[3]);
-            else
-                for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = res[e];
+            if (redone || !__syncthreads_or(odd)) break;
+            redo_plain(again, again + MAX_BN * 128, again + MAX_BN * 128 + 128 * REDO_LD, p, m0 + c0, c1 - c0, n0, outs);
         }
     }
     tmem_fence_before();
@@ -414,6 +462,7 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
     const int b_bytes = 3 * p.bn * BK * 2, room = SMEM_BYTES - 1024 - A_STAGES * 3 * PLANE_A;
     p.b_stages = std::min(MAX_B_STAGES, (room - 3 * SLOT) / b_bytes);       // at least three
     p.slots = std::min(MAX_SLOTS, (room - p.b_stages * b_bytes) / SLOT / A_STAGES * A_STAGES);
+    static_assert(4 * (2 * MAX_BN * 128 + 2 * 128 * REDO_LD) <= SMEM_BYTES - 1024, "the sums, the outputs made again and their operands");
     static_assert(A_STAGES * 3 * PLANE_A + 3 * 3 * MAX_BN * BK * 2 + 3 * SLOT <= SMEM_BYTES - 1024, "128 columns: three copies, three slots");
     static_assert(MAX_SLOTS % A_STAGES == 0 && A_STAGES == 3, "three slots at least, a whole number a pair");
     TiEncodeTiledFn encode = ti_encode_tiled_fn();
