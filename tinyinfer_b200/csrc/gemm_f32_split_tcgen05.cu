@@ -20,7 +20,7 @@
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
 // multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
-// again through shared memory (redo_plain), at about the cost of gemm_simt.cu.
+// again through shared memory (redo_plain): 333 rows of NaN by 12,288 x 2,048 weights 1.26 ms, where gemm_simt.cu takes 0.89.
 // Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 118 us (142 TFLOP/s), by 2,048 x 6,144
 // 799 -> 78 us; 9 rows 306 -> 51 us; 256 x 256 weights, the smallest that come here, 20 -> 5.5 us.
 #include "sm100_ptx.cuh"
@@ -92,36 +92,53 @@ __device__ __forceinline__ uint64_t make_sw64_desc(uint32_t smem_addr) {
 }
 
 // The CTA's share of the outputs by multiply-adds in k order, one accumulator an output: out[col][row] for `cols` tokens from
-// m on and the 128 rows of w that the tile has on its lanes. A thread has one row and every fourth token, operands come 16 k at a time
-// through shared memory.
-constexpr int REDO_K = 16, REDO_LD = REDO_K + 4, REDO_THREADS = 512;
-__device__ __noinline__ void redo_plain(float* out, float* ws, float* xs, const SplitParams& p, int m, int cols, int n0, int outs) {
+// m on and the 128 rows of w that the tile has on its lanes. A thread has one row and every fourth token; operands come 32 k at a
+// time, the next piece while this one is multiplied.
+constexpr int REDO_K = 32, REDO_LD = REDO_K + 4, REDO_THREADS = 512, REDO_PIECE = 2 * 128 * REDO_LD;
+__device__ __forceinline__ void redo_plain(float* out, float* pieces, const SplitParams& p, int m, int cols, int n0, int outs) {
     const int row = threadIdx.x & 127, group = threadIdx.x >> 7;
-    float acc[MAX_BN / 4] = {};
-    for (int k0 = 0; k0 < p.K; k0 += REDO_K) {
-        __syncthreads();                                     // everyone is done with the piece before
-        for (int i = threadIdx.x; i < 2 * 128 * (REDO_K / 4); i += NUM_THREADS) {
-            const int r = i / (REDO_K / 4) & 127, k = k0 + i % (REDO_K / 4) * 4;
-            const bool weights = i < 128 * (REDO_K / 4);
+    auto fetch = [&](int k0) {                               // 128 rows of w, then up to 128 of x
+        float* to = pieces + k0 / REDO_K % 2 * REDO_PIECE;
+        for (int i = threadIdx.x; i < (128 + cols) * (REDO_K / 4); i += NUM_THREADS) {
+            const int r = i / (REDO_K / 4), k = k0 + i % (REDO_K / 4) * 4;
             const int w_row = (r < outs ? 0 : p.N) + min(n0 + r % outs, p.N - 1);
-            const float* src = weights ? p.w + (size_t)w_row * p.K : p.x + (size_t)min(m + r, p.M - 1) * p.K;
-            const float4 v = k < p.K ? *reinterpret_cast<const float4*>(src + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-            *reinterpret_cast<float4*>((weights ? ws : xs) + r * REDO_LD + k - k0) = v;
+            const float* src = r < 128 ? p.w + (size_t)w_row * p.K : p.x + (size_t)min(m + r - 128, p.M - 1) * p.K;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(to + r * REDO_LD + k - k0)), "l"(src + min(k, p.K - 4)),
+                         "r"(k < p.K ? 16 : 0) : "memory");
         }
-        __syncthreads();
-        if (threadIdx.x >= REDO_THREADS) continue;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float acc[MAX_BN / 4] = {};
+    fetch(0);
+    for (int k0 = 0; k0 < p.K; k0 += REDO_K) {
+        if (k0 + REDO_K < p.K) {
+            fetch(k0 + REDO_K);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();                                     // the piece is there
+        const float* ws = pieces + k0 / REDO_K % 2 * REDO_PIECE + row * REDO_LD;
+        const float* xs = pieces + k0 / REDO_K % 2 * REDO_PIECE + (128 + group) * REDO_LD;
+        if (threadIdx.x < REDO_THREADS) {
 #pragma unroll 1
-        for (int k = 0; k < REDO_K; k += 4) {
-            const float4 w = *reinterpret_cast<const float4*>(ws + row * REDO_LD + k);
+            for (int k = 0; k < REDO_K; k += 4) {
+                const float4 w = *reinterpret_cast<const float4*>(ws + k);
 #pragma unroll
-            for (int j = 0; j < MAX_BN / 4; ++j) {
-                const float4 x = *reinterpret_cast<const float4*>(xs + (group + 4 * j) * REDO_LD + k);
-                acc[j] = fmaf(x.x, w.x, acc[j]);
-                acc[j] = fmaf(x.y, w.y, acc[j]);
-                acc[j] = fmaf(x.z, w.z, acc[j]);
-                acc[j] = fmaf(x.w, w.w, acc[j]);
+                for (int j0 = 0; j0 < MAX_BN / 4; j0 += 4) {
+                    if (4 * j0 >= cols) break;
+#pragma unroll
+                    for (int j = j0; j < j0 + 4; ++j) {      // rows past cols hold what they hold, and are not stored
+                        const float4 x = *reinterpret_cast<const float4*>(xs + 4 * j * REDO_LD + k);
+                        acc[j] = fmaf(x.x, w.x, acc[j]);
+                        acc[j] = fmaf(x.y, w.y, acc[j]);
+                        acc[j] = fmaf(x.z, w.z, acc[j]);
+                        acc[j] = fmaf(x.w, w.w, acc[j]);
+                    }
+                }
             }
         }
+        __syncthreads();                                     // everyone is done with the piece
     }
     if (threadIdx.x < REDO_THREADS) {
 #pragma unroll
@@ -394,7 +411,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = res[e];
             }
             if (redone || !__syncthreads_or(odd)) break;
-            redo_plain(again, again + MAX_BN * 128, again + MAX_BN * 128 + 128 * REDO_LD, p, m0 + c0, c1 - c0, n0, outs);
+            redo_plain(again, again + MAX_BN * 128, p, m0 + c0, c1 - c0, n0, outs);
         }
     }
     tmem_fence_before();
@@ -462,7 +479,7 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
     const int b_bytes = 3 * p.bn * BK * 2, room = SMEM_BYTES - 1024 - A_STAGES * 3 * PLANE_A;
     p.b_stages = std::min(MAX_B_STAGES, (room - 3 * SLOT) / b_bytes);       // at least three
     p.slots = std::min(MAX_SLOTS, (room - p.b_stages * b_bytes) / SLOT / A_STAGES * A_STAGES);
-    static_assert(4 * (2 * MAX_BN * 128 + 2 * 128 * REDO_LD) <= SMEM_BYTES - 1024, "the sums, the outputs made again and their operands");
+    static_assert(4 * (2 * MAX_BN * 128 + 2 * REDO_PIECE) <= SMEM_BYTES - 1024, "the sums, the outputs made again and their operands");
     static_assert(A_STAGES * 3 * PLANE_A + 3 * 3 * MAX_BN * BK * 2 + 3 * SLOT <= SMEM_BYTES - 1024, "128 columns: three copies, three slots");
     static_assert(MAX_SLOTS % A_STAGES == 0 && A_STAGES == 3, "three slots at least, a whole number a pair");
     TiEncodeTiledFn encode = ti_encode_tiled_fn();
