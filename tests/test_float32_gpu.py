@@ -166,6 +166,17 @@ def test_attention_reports_a_key_without_a_page_and_keeps_rows_apart(ops):
     assert int(status.item()) == 2 and torch.isfinite(got[20]).all() and torch.equal(got[:18], want[:18])
 
 
+@pytest.mark.parametrize("size", [1e-30, 1e-33, 1e-35, 1e-37, 1e-38, 1e-42, 1e30])
+def test_split_product_keeps_the_bits_of_small_operands(ops, size):
+    """Operands down to float32's subnormal numbers against large partners: as exact as multiply-adds. The sums are judged as
+    float32 holds the operands."""
+    for m, n, k in ((40, 200, 512), (150, 130, 2052)):
+        small, large = rnd(m, k, dtype=torch.float32, seed=1) * size, rnd(n, k, dtype=torch.float32, seed=2) * min(1e10, 1e36 / size)
+        for x, w in ((small, large), (large, small)):
+            want, mass = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+            assert ((ops.linear(x, w) - want).abs() <= EPS * (k / 16 + 8) * mass + 2.0 ** -149).all()
+
+
 @pytest.mark.parametrize("m,n,k,act", [(9, 514, 2048, None), (130, 259, 516, None), (333, 1000, 1028, None), (140, 130, 6144, "gelu_tanh"), (333, 6000, 512, "silu")])
 def test_split_product_makes_infinite_and_nan_outputs_again(ops, m, n, k, act):
     """Outputs that are not finite in parts are the general kernel's bit for bit, whatever share of a tile they are, and the rest
