@@ -79,6 +79,20 @@ def test_split_product_is_no_less_exact_than_multiply_adds(ops):
         assert errors[0] <= errors[1], errors
 
 
+@pytest.mark.parametrize("draw", ["normal", "positive"])
+@pytest.mark.parametrize("m,n,k", [(1500, 4096, 256), (1500, 4096, 320), (200, 512, 320), (1500, 4096, 384), (40, 512, 512), (333, 1024, 1024)])
+def test_product_of_a_short_row_is_no_less_exact_than_multiply_adds(ops, m, n, k, draw):
+    """Where k is short the general kernel's sums are few, and the split products must not be further off."""
+    x, w = rnd(m, k, dtype=torch.float32, seed=1), rnd(n, k, dtype=torch.float32, seed=2)
+    if draw == "positive":
+        x, w = x.abs(), w.abs()
+    want = x.double() @ w.double().T
+    plain = torch.empty((m, n), dtype=torch.float32, device=dev())
+    ops._run("core", "ti_gemm_simt", plain.data_ptr(), x.data_ptr(), w.data_ptr(), None, None, m, n, k, 0, 0, 0, ops._stream())
+    errors = [((y - want).norm() / want.norm()).item() for y in (ops.linear(x, w), plain)]
+    assert errors[0] <= errors[1], errors
+
+
 def test_split_product_takes_infinite_and_tiny_operands_as_multiply_adds_do(ops):
     m, n, k = 40, 200, 512
     x, w = rnd(m, k, dtype=torch.float32, seed=1), rnd(n, k, dtype=torch.float32, seed=2)

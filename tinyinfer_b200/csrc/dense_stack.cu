@@ -48,7 +48,7 @@ struct TiStackCall {
     int layers, tokens, hidden, heads, kv_heads, head_dim, inter, act, page_size, dtype;
     int num_decode, num_tiles, num_pairs, max_context;
     int table_positions, interleaved, rotary_dim, num_counters;
-    int link_max_tokens, pair_min_ctas, split_max_ctas, few_rows, min_k, tile_rows;
+    int link_max_tokens, pair_min_ctas, split_max_ctas, few_rows, min_k, split_min_k, tile_rows;
     float eps1, eps2, qk_eps, scale;
     int failed;                                    // out: which library's launcher failed (0 core, 1 sm100, 2 f32)
 };
@@ -150,7 +150,7 @@ TI_API int ti_dense_stack(TiStackCall* call) {
     auto product = [&](void* out, const void* x, const void* w, const float* bias, const void* residual, int n, int k, int gated,
                        bool scaled, float eps, const float* emit) -> int {
         if (f32) {
-            const bool fits = k % 4 == 0 && k >= c.min_k && ((uintptr_t)x | (uintptr_t)w) % 16 == 0;
+            const bool fits = k % 4 == 0 && k >= (T <= c.few_rows ? c.min_k : c.split_min_k) && ((uintptr_t)x | (uintptr_t)w) % 16 == 0;
             if (!fits) STACK_RUN(0, c.simt(out, x, w, bias, residual, T, n, k, gated, 0, c.dtype, c.stream));
             else if (T <= c.few_rows)
                 STACK_RUN(2, c.few((float*)out, (const float*)x, (const float*)w, bias, (const float*)residual, T, n, k, gated, c.stream));

@@ -11,7 +11,8 @@
 // The sums decide the precision. The tensor core cuts bits off when it adds to its accumulator, always towards zero, so a
 // long run in one accumulator would drift. Here a run is CHUNK = 2 k blocks of 32, the small parts of a block before the
 // large ones; then the accumulator is added, rounded to nearest, to float32 registers and starts again from zero. Against 64
-// bits, at K = 2048 and 6144: 3.3e-7 of the result's norm, where multiply-adds in k order have 8.1e-7 and 1.4e-6.
+// bits, at K = 320, 2048 and 6144: 3.2e-7, 3.3e-7 and 3.3e-7 of the result's norm, where multiply-adds in k order have 3.2e-7,
+// 8.1e-7 and 1.4e-6 (at 256 2.9e-7: shorter rows are the general kernel's).
 //
 //   weights on the 128 accumulator lanes (gated form: 64 gate rows and the 64 up rows of the same outputs), up to 128 tokens
 //   on the columns; a cluster of S CTAs cuts the k range of a tile where the tiles alone would leave SMs idle, and adds its
@@ -27,7 +28,7 @@
 // multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
 // again through shared memory (redo_plain): 333 rows of NaN by 12,288 x 2,048 weights 1.26 ms, where gemm_simt.cu takes 0.89.
 // Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 118 us (142 TFLOP/s), by 2,048 x 6,144
-// 799 -> 78 us; 9 rows 306 -> 51 us; 256 x 256 weights, the smallest that come here, 20 -> 5.5 us.
+// 799 -> 78 us; 9 rows 306 -> 51 us; 200 rows by 1,024 x 320 weights, the shortest k that comes here, 26 -> 17 us.
 #include "sm100_ptx.cuh"
 #include <algorithm>
 #include <array>

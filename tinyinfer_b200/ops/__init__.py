@@ -274,12 +274,14 @@ def _tensor_core_ok(x: torch.Tensor, w: torch.Tensor, *others) -> bool:
 
 F32_FEW_ROWS = 8          # up to so many rows a float32 product streams its weights past the rows of x held in registers
 F32_MIN_K = 256           # below, the general kernel's few steps are as quick, and its sums have one order for any number of rows
+F32_SPLIT_MIN_K = 320     # and with more rows: the split products' error is 2.2 to 3.2e-7 whatever K is, the general kernel's grows with
+                          # it: 2.3 to 2.9e-7 at 256, 2.5 to 3.2e-7 at 320 (200 x 1,024 outputs there: 17 us for 26)
 
 
 def _float32_product(out, x, w, bias, residual, m, n, k, gated) -> bool:
     """Runs a float32 product on the kernel made for its size, if there is one; False: the general kernel is to run it.
     The weights are read 16 bytes at a time: whole rows of them, on 16-byte boundaries."""
-    if x.dtype != torch.float32 or k % 4 or k < F32_MIN_K or m < 1 or (x.data_ptr() | w.data_ptr()) % 16:
+    if x.dtype != torch.float32 or k % 4 or k < (F32_MIN_K if m <= F32_FEW_ROWS else F32_SPLIT_MIN_K) or m < 1 or (x.data_ptr() | w.data_ptr()) % 16:
         return False
     if m <= F32_FEW_ROWS:
         _run("f32", "ti_gemm_f32_few", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), m, n, k, gated,
@@ -1152,7 +1154,7 @@ class _StackCall(ctypes.Structure):
                 + [(n, c_int) for n in ("layers", "tokens", "hidden", "heads", "kv_heads", "head_dim", "inter", "act", "page_size",
                                         "dtype", "num_decode", "num_tiles", "num_pairs", "max_context", "table_positions",
                                         "interleaved", "rotary_dim", "num_counters", "link_max_tokens", "pair_min_ctas",
-                                        "split_max_ctas", "few_rows", "min_k", "tile_rows")]
+                                        "split_max_ctas", "few_rows", "min_k", "split_min_k", "tile_rows")]
                 + [(n, c_float) for n in ("eps1", "eps2", "qk_eps", "scale")] + [("failed", c_int)])
 
 
@@ -1194,7 +1196,7 @@ def dense_stack(x: torch.Tensor, layers: list, step, *, heads: int, kv_heads: in
         call.table_positions = rotation.cos_sin.shape[0] if rotation.cos_sin is not None else 0
         call.interleaved, call.rotary_dim = int(rotation.interleaved), rotation.rotary_dim
     call.link_max_tokens, call.pair_min_ctas, call.split_max_ctas = NORM_LINK_MAX_TOKENS, PAIR_MIN_CTAS, KEY_SPLIT_MAX_CTAS
-    call.few_rows, call.min_k, call.tile_rows = F32_FEW_ROWS, F32_MIN_K, PREFILL_TILE
+    call.few_rows, call.min_k, call.split_min_k, call.tile_rows = F32_FEW_ROWS, F32_MIN_K, F32_SPLIT_MIN_K, PREFILL_TILE
     call.eps1, call.eps2, call.qk_eps = eps
     call.scale = scale
     if code == 1:
