@@ -42,30 +42,45 @@ class DenseStack:
         if not blocks or any(shape(b) != shape(blocks[0]) for b in blocks[1:]):
             return None
         turn = shape(blocks[0])[6]
-        return cls(blocks, execution) if turn is None or turn[2] == 1.0 else None
+        return cls(blocks, execution) if turn is None or (turn[2] == 1.0 and turn[0] <= blocks[0].mixer.spec.head_dim) else None
 
     def run(self, x: torch.Tensor, step) -> Optional[torch.Tensor]:
         """The last block's output, or None where the parts have to run themselves (shapes that take other kernels)."""
         first = self.blocks[0]
         s, ff = first.mixer.spec, first.feed_forward.spec
-        if not x.is_cuda or x.dim() != 2 or x.shape[0] == 0 or not x.is_contiguous() or x.data_ptr() % 16:
+        if x.dim() != 2 or x.shape[0] == 0 or not _lies(x, x.dtype, (x.shape[0], s.hidden_size)) or x.data_ptr() % 16:
             return None
         if s.hidden_size % 8 or s.q_size % 8 or ff.intermediate_size % 8:
             return None
+        if not all(_lies(t, torch.int32, (t.numel(),)) for t in (step.positions, step.token_seq)):
+            return None
+        # what the parts' own calls look at: an operand that is not as the kernels read it is left to them to refuse
+        kind, real = x.dtype, torch.float32
+        hidden, inter, packed = s.hidden_size, ff.intermediate_size, s.q_size + 2 * s.kv_size
+        of_qkv, of_o, of_gate_up, of_down = (packed, hidden), (hidden, s.q_size), (2 * inter, hidden), (hidden, inter)
         rows, page = [], 0
         for entry in self.execution:
             block, view = self.blocks[entry.layer], step.cache_view(entry)
-            m, f, kv = block.mixer, block.feed_forward, view.kv
-            if kv is None or kv.dtype != x.dtype or kv.shape[0] != 2 or kv.shape[2] != s.num_kv_heads or kv.shape[4] != s.head_dim:
+            m, f, kv, table, r = block.mixer, block.feed_forward, view.kv, view.block_table, block.mixer._rotation
+            if kv is None or kv.dim() != 5 or table is None or table.dim() != 2:
                 return None
-            if page and kv.shape[3] != page:
+            page = page or kv.shape[3]
+            if not (_lies(m.w_qkv, kind, of_qkv) and _lies(m.w_o, kind, of_o) and _lies(f.w_gate_up, kind, of_gate_up)
+                    and _lies(f.w_down, kind, of_down) and _lies(block.mixer_norm.weight, real, (hidden,))
+                    and _lies(block.feed_forward_norm.weight, real, (hidden,)) and _lies(table, torch.int32, table.shape)
+                    and _lies(kv, kind, (2, kv.shape[1], s.num_kv_heads, page, s.head_dim))
+                    and (m.b_qkv is None or _lies(m.b_qkv, real, (packed,))) and (m.b_o is None or _lies(m.b_o, real, (hidden,)))
+                    and (m.q_norm is None or _lies(m.q_norm, real, (s.head_dim,)))
+                    and (m.k_norm is None or _lies(m.k_norm, real, (s.head_dim,)))):
                 return None
-            page = kv.shape[3]
-            r = m._rotation
+            if r is not None:
+                t = r.inv_freq if r.inv_freq is not None else r.cos_sin
+                if not _lies(t, real, t.shape):
+                    return None
             row = (m.w_qkv.data_ptr(), _at(m.b_qkv), m.w_o.data_ptr(), _at(m.b_o), _at(m.q_norm), _at(m.k_norm),
                    _at(r.inv_freq) if r is not None else 0, _at(r.cos_sin) if r is not None else 0, block.mixer_norm.weight.data_ptr(),
                    block.feed_forward_norm.weight.data_ptr(), f.w_gate_up.data_ptr(), f.w_down.data_ptr(), kv.data_ptr(),
-                   view.block_table.data_ptr(), view.block_table.shape[1], kv.shape[1], int(m.spec.window or 0), int(view.writes))
+                   table.data_ptr(), table.shape[1], kv.shape[1], int(m.spec.window or 0), int(view.writes))
             if (row[0] | row[2] | row[8] | row[9] | row[10] | row[11] | row[12]) % 16:
                 return None
             rows.append(row)
@@ -75,6 +90,11 @@ class DenseStack:
             x, rows, step, heads=s.num_heads, kv_heads=s.num_kv_heads, head_dim=s.head_dim, inter=ff.intermediate_size,
             activation=ff.activation, page_size=page, scale=s.scale, rotation=first.mixer._rotation,
             eps=(first.mixer_norm.spec.eps, first.feed_forward_norm.spec.eps, s.qk_norm.eps if s.qk_norm is not None else 0.0))
+
+
+def _lies(t: torch.Tensor, kind: torch.dtype, shape) -> bool:
+    """Whether the kernels can read ``t`` as it lies: on the GPU, of this type and shape, without gaps."""
+    return t.is_cuda and t.dtype is kind and t.is_contiguous() and t.shape == shape
 
 
 def _at(t: Optional[torch.Tensor]) -> int:
