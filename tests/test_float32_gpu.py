@@ -156,6 +156,29 @@ def test_attention(ops, hq, hkv, d, page, window, work):
         row += n
 
 
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_attention_multiplies_every_value_that_a_row_sees(ops, value):
+    """A seen key whose probability underflows still brings 0 x its value, as in the general kernel: in a tile that all rows see
+    whole, in one that some do not, and for single tokens."""
+    hq, hkv, d, page = 4, 2, 64, 16
+    work = [(200, 200), (170, 1)]
+    bt, kv = paged_setup(torch.float32, [c for c, _ in work], hq, hkv, d, page, seed=1)
+    fill_cache(kv, bt, [c for c, _ in work], hkv, d, page, torch.float32)
+    rows, tiles, pairs = ops.plan_attention([n for _, n in work], [c - n for c, n in work])
+    step = SimpleNamespace(decode_rows=torch.tensor(rows, dtype=torch.int32, device=dev()), num_decode=1,
+                           prefill_tiles=torch.tensor(tiles, dtype=torch.int32, device=dev()), num_prefill_tiles=len(tiles) // 4,
+                           num_pair_tiles=pairs, max_context=200)
+    q = rnd(201, hq, d, dtype=torch.float32, seed=3).abs() + 0.1
+    args = dict(positions=torch.tensor(list(range(200)) + [169], dtype=torch.int32, device=dev()),
+                token_seq=torch.tensor([0] * 200 + [1], dtype=torch.int32, device=dev()), block_table=bt, scale=0.125)
+    for request, key in ((0, 3), (0, 150), (1, 20)):
+        at = (0, int(bt[request, key // page]), slice(None), key % page)
+        kv[at] = -1e4                                   # a score far below every other
+        kv[(1,) + at[1:]] = value
+    got, want = ops.paged_attention(q, kv, step=step, **args), ops.paged_attention(q, kv, **args)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.isnan(got[160]).all() and not torch.isnan(got[2]).any()
+
+
 def test_attention_reports_a_key_without_a_page_and_keeps_rows_apart(ops):
     """A missing page is reported and its keys are left out; infinities of a later token of the portion do not reach the
     tokens before it."""

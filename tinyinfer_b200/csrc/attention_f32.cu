@@ -282,13 +282,18 @@ __global__ void __launch_bounds__(PR_ROWS * 8) portion_f32_kernel(const AfArgs a
                 }
             }
         }
+        // A key that a row does not see must not reach it even as 0 x infinity: its probability says so by its sign. Only tiles with
+        // such keys pay for the test.
+        const bool all_see = key0 + PR_KEYS - 1 <= pos0 && key0 >= ti_first_key(last, a.window);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             float top = m[r];
+            bool seen[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int j = key0 + tx + 16 * i;
-                s[r][i] = j >= lo[r] && j <= pos[r] && off[tx + 16 * i] >= 0 ? s[r][i] * a.scale : -INFINITY;
+                seen[i] = j >= lo[r] && j <= pos[r] && off[tx + 16 * i] >= 0;
+                s[r][i] = seen[i] ? s[r][i] * a.scale : -INFINITY;
                 top = fmaxf(top, s[r][i]);
             }
 #pragma unroll
@@ -299,7 +304,7 @@ __global__ void __launch_bounds__(PR_ROWS * 8) portion_f32_kernel(const AfArgs a
             for (int i = 0; i < 4; ++i) {
                 const float p = s[r][i] == -INFINITY ? 0.f : expf(s[r][i] - top);
                 sum += p;
-                ps[(ty * 2 + r) * (PR_KEYS + 4) + tx + 16 * i] = p;
+                ps[(ty * 2 + r) * (PR_KEYS + 4) + tx + 16 * i] = seen[i] || all_see ? p : -1.f;
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -310,8 +315,6 @@ __global__ void __launch_bounds__(PR_ROWS * 8) portion_f32_kernel(const AfArgs a
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                     // the values and everyone's probabilities are there
-        // A key that a row does not see must not reach it even as 0 x infinity; only tiles with such keys pay for the test.
-        const bool all_see = key0 + PR_KEYS - 1 <= pos0 && key0 >= ti_first_key(last, a.window);
         auto add = [&](auto guarded) {
 #pragma unroll 2
             for (int j = 0; j < PR_KEYS; j += 4) {
@@ -326,7 +329,7 @@ __global__ void __launch_bounds__(PR_ROWS * 8) portion_f32_kernel(const AfArgs a
                         const float4 vv = *reinterpret_cast<const float4*>(vs + (j + jj) * D + tx * 4 + 64 * i);
 #pragma unroll
                         for (int r = 0; r < 2; ++r) {
-                            if constexpr (decltype(guarded)::value) { if (pr[r][jj] == 0.f) continue; }
+                            if constexpr (decltype(guarded)::value) { if (pr[r][jj] < 0.f) continue; }
                             acc[r][4 * i] = fmaf(pr[r][jj], vv.x, acc[r][4 * i]);
                             acc[r][4 * i + 1] = fmaf(pr[r][jj], vv.y, acc[r][4 * i + 1]);
                             acc[r][4 * i + 2] = fmaf(pr[r][jj], vv.z, acc[r][4 * i + 2]);
