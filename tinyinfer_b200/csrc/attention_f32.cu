@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(PR_ROWS * 8) portion_f32_kernel(const AfArgs a
 
 template <int D, int PR_ROWS>
 int launch_portions(const AfArgs& a, int tiles, int tile_rows, cudaStream_t stream) {
-    static const cudaError_t set = cudaFuncSetAttribute(portion_f32_kernel<D, PR_ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, portion_smem<D, PR_ROWS>());
+    const cudaError_t set = ti_allow_shared<portion_f32_kernel<D, PR_ROWS>>(portion_smem<D, PR_ROWS>());
     TI_REQUIRE(set == cudaSuccess, "attention_f32: %s", cudaGetErrorString(set));
     const int per = PR_ROWS / (a.hq / a.hkv);
     ti_launch(portion_f32_kernel<D, PR_ROWS>, dim3(a.hkv, (tile_rows + per - 1) / per, tiles), PR_ROWS * 8, portion_smem<D, PR_ROWS>(), stream, a);

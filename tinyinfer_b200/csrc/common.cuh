@@ -71,6 +71,21 @@ cudaError_t ti_launch_alone(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
 }
 
+// Lets KERNEL have `bytes` of dynamic shared memory on the current device. The attribute belongs to a device, and so does the
+// record of having set it (beyond 64 devices it is set on every call).
+template <auto KERNEL>
+cudaError_t ti_allow_shared(int bytes) {
+    constexpr int DEVICES = 64;
+    static int allowed[DEVICES] = {};
+    int dev = -1;
+    const cudaError_t got = cudaGetDevice(&dev);
+    if (got != cudaSuccess) return got;
+    if (dev < DEVICES && allowed[dev] >= bytes) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < DEVICES) allowed[dev] = bytes;
+    return e;
+}
+
 template <typename T> __device__ __forceinline__ float to_f32(T v);
 template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }

@@ -191,9 +191,9 @@ TI_API int ti_moe_gemm_tcgen05(void* out, const void* x, const void* w, const in
     const int bn = wide ? 256 : 128;
     if (!ti_get_bf16_map(x, slots, K, GT_BM, &map_x)) return -1;
     if (!ti_get_bf16_map(w, (long long)experts * N, K, bn, &map_w)) return -1;
-    static const cudaError_t narrow_set = cudaFuncSetAttribute(moe_gemm_tcgen05_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtShape<128>::SMEM);
-    static const cudaError_t wide_set = cudaFuncSetAttribute(moe_gemm_tcgen05_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, GtShape<256>::SMEM);
-    TI_REQUIRE(narrow_set == cudaSuccess && wide_set == cudaSuccess, "moe_gemm_tcgen05: shared memory: %s", cudaGetErrorString(wide ? wide_set : narrow_set));
+    const cudaError_t set = wide ? ti_allow_shared<moe_gemm_tcgen05_kernel<256>>(GtShape<256>::SMEM)
+                                 : ti_allow_shared<moe_gemm_tcgen05_kernel<128>>(GtShape<128>::SMEM);
+    TI_REQUIRE(set == cudaSuccess, "moe_gemm_tcgen05: shared memory: %s", cudaGetErrorString(set));
     GtParams p;
     p.out = out; p.tiles = tiles; p.num_tiles = num_tiles; p.N = N; p.K = K; p.col_tiles = (N + bn - 1) / bn; p.up = up;
     p.status = status;

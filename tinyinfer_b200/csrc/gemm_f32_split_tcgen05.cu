@@ -514,7 +514,7 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     TI_REQUIRE(r == CUDA_SUCCESS && rw == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed (%d, %d) for M=%d N=%d K=%d", (int)r, (int)rw, M, N, K);
-    static const cudaError_t set = cudaFuncSetAttribute(gemm_f32_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    const cudaError_t set = ti_allow_shared<gemm_f32_split_kernel>(SMEM_BYTES);
     TI_REQUIRE(set == cudaSuccess, "gemm_f32_split: %s", cudaGetErrorString(set));
     const int splits = choose_splits(row_tiles * col_tiles, (K + BK - 1) / BK);
     const long long quads = (long long)M * Kp / 4;
