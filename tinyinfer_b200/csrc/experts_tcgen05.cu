@@ -178,6 +178,12 @@ TI_API int ti_moe_gemm_tcgen05_ok(int slots, int experts, int N, int K) {
 }
 TI_API int ti_moe_tcgen05_tile_rows() { return GT_BM; }
 
+// The output features of a unit: 256 where every SM keeps two units, else 128. The real number of row tiles is on the device; it
+// is at least slots / 128.
+TI_API int ti_moe_tcgen05_unit_features(int slots, int N) {
+    return N >= 256 && (long long)(slots / GT_BM) * ((N + 255) / 256) >= 2 * ti_sm_count() ? 256 : 128;
+}
+
 // x: sorted rows [slots, K] bfloat16; w [experts, N, K] bfloat16; tiles/num_tiles: the plan with row tiles of 128.
 // up == 1: out [slots, N] bfloat16 after max(v, 0)^2; up == 2: bfloat16 as it is; else out [slots, N] float32.
 TI_API int ti_moe_gemm_tcgen05(void* out, const void* x, const void* w, const int* tiles, const int* num_tiles, int slots,
@@ -186,9 +192,8 @@ TI_API int ti_moe_gemm_tcgen05(void* out, const void* x, const void* w, const in
     TI_REQUIRE(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0 && ((uintptr_t)out & 15) == 0, "moe_gemm_tcgen05: operands must be 16-byte aligned");
     if (max_tiles <= 0) return 0;
     CUtensorMap map_x, map_w;
-    // the real number of row tiles is on the device; at least slots / 128
-    const bool wide = N >= 256 && (long long)(slots / GT_BM) * ((N + 255) / 256) >= 2 * ti_sm_count();
-    const int bn = wide ? 256 : 128;
+    const int bn = ti_moe_tcgen05_unit_features(slots, N);
+    const bool wide = bn == 256;
     if (!ti_get_bf16_map(x, slots, K, GT_BM, &map_x)) return -1;
     if (!ti_get_bf16_map(w, (long long)experts * N, K, bn, &map_w)) return -1;
     const cudaError_t set = wide ? ti_allow_shared<moe_gemm_tcgen05_kernel<256>>(GtShape<256>::SMEM)

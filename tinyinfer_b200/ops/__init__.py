@@ -147,6 +147,7 @@ _SIGNATURES["sm100"] = {
 }
 _SIGNATURES["sm100"]["ti_gemm_set_pair_form"] = [c_int]
 _SIGNATURES["sm100"]["ti_moe_gemm_tcgen05_ok"] = [c_int, c_int, c_int, c_int]
+_SIGNATURES["sm100"]["ti_moe_tcgen05_unit_features"] = [c_int, c_int]
 _SIGNATURES["sm100"]["ti_moe_tcgen05_tile_rows"] = []
 _SIGNATURES["sm100"]["ti_moe_gemm_tcgen05"] = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                                c_int, c_void_p, c_void_p]
