@@ -9,12 +9,16 @@ def make(dtype, heads, kv_heads, dim, hidden, inter, layers, page, tied=True):
     from tinyinfer_b200.config import Qwen3Config
     from tinyinfer_b200 import models  # noqa: F401
     from tinyinfer_b200.config import lookup_architecture
-    from tinyinfer_b200.engine.runner import ModelRunner
     cfg = dict(architectures=["Qwen3ForCausalLM"], vocab_size=515, hidden_size=hidden, num_hidden_layers=layers, num_attention_heads=heads,
                num_key_value_heads=kv_heads, head_dim=dim, intermediate_size=inter, rms_norm_eps=1e-6, rope_theta=1e6,
                tie_word_embeddings=tied, max_position_embeddings=4096)
     arch = lookup_architecture("Qwen3ForCausalLM")
-    model = arch.model_factory(Qwen3Config.from_dict(cfg), dtype, torch.device("cuda:0"))
+    return fill(arch.model_factory(Qwen3Config.from_dict(cfg), dtype, torch.device("cuda:0")), dtype, page)
+
+
+def fill(model, dtype, page):
+    """The model with random weights, and what makes runners of it."""
+    from tinyinfer_b200.engine.runner import ModelRunner
     gen = torch.Generator(device="cuda:0").manual_seed(3)
     tensors = {}
     for name, ts in model.expected_tensors().items():
@@ -82,4 +86,53 @@ def test_portions_beside_decoded_tokens_behind_a_long_prefix(heads, kv_heads, di
     model._stack = None
     want = run(runner(), steps)
     assert all(torch.equal(g, w) and torch.isfinite(g).all() for g, w in zip(got, want))
+    ops.check_kernel_status()
+
+
+def make_mixed(dtype, table, page=16):
+    """Layers with and without a window, one that runs twice, an entry that only reads what another cached; with ``table``
+    also biases, norms of q and k, gelu, and a rotation of neighbouring features by a table, else positions are not used."""
+    from tinyinfer_b200 import ops
+    from tinyinfer_b200.config import AttentionSpec, ExecStep, GatedMLPSpec, LayerSpec, ModelSpec, NormSpec, PositionSpec
+    from tinyinfer_b200.models import DecoderModel
+    norm = NormSpec(256, 1e-5)
+
+    def layer(window):
+        mixer = AttentionSpec(hidden_size=256, num_heads=6, num_kv_heads=2, head_dim=64, scale=0.11, position=PositionSpec(kind="none"),
+                              qk_norm=NormSpec(64, 1e-4) if table else None, bias=table, window=window)
+        return LayerSpec(mixer=mixer, feed_forward=GatedMLPSpec(256, 384, activation="gelu_tanh" if table else "silu"),
+                         mixer_norm=norm, feed_forward_norm=norm)
+    spec = ModelSpec(architecture="Mixed", vocab_size=515, hidden_size=256, layers=(layer(40), layer(None), layer(300)),
+                     execution=(ExecStep(0, 0), ExecStep(1, 1), ExecStep(1, 2), ExecStep(2, 3), ExecStep(2, 3, writes_cache=False),
+                                ExecStep(0, 4)),
+                     final_norm=norm, tie_embeddings=True, max_positions=4096)
+    model = DecoderModel(spec, dtype, "cuda:0")
+    if table:
+        angle = torch.log1p(torch.arange(4096.0))[:, None] * 100.0 ** (-torch.arange(24.0) / 24)
+        turn = ops.Rotation(48, cos_sin=torch.cat([angle.cos(), angle.sin()], dim=1).contiguous().cuda(), interleaved=True)
+        for b in model.blocks:
+            b.mixer._rotation = turn
+    return fill(model, dtype, page)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("table", [False, True])
+def test_stack_of_windows_biases_tables_and_shared_entries(dtype, table):
+    """Everything that a layer can hand to the native call, bit for bit as the parts run it, and the same bits every time."""
+    from tinyinfer_b200 import ops
+    model, runner = make_mixed(dtype, table)
+    stack = model._stack
+    assert stack is not None
+    taken = []
+    run_stack = stack.run
+    stack.run = lambda x, step: taken.append(run_stack(x, step)) or taken[-1]
+    for graphs in (False, True):
+        model._stack = None
+        want = run(runner(graphs), STEPS)
+        model._stack = stack
+        for _ in range(3):
+            got = run(runner(graphs), STEPS)
+            for g, w, step in zip(got, want, STEPS):
+                assert torch.isfinite(g).all() and torch.equal(g, w), (step, ((g - w).norm() / w.norm()).item())
+    assert taken and all(t is not None for t in taken)
     ops.check_kernel_status()
