@@ -48,3 +48,24 @@ def test_scratch_of_portions_beside_decoded_tokens_is_aligned(calls, monkeypatch
             assert call.side == 1 and call.decode_floats >= need[-1]
             assert (call.attn_scratch + 4 * call.decode_floats) % 16 == 0
             assert call.attn_floats >= call.decode_floats + 4096
+
+
+@pytest.mark.parametrize("heads,dim", [(1, 64), (7, 64), (16, 128), (40, 128)])
+def test_the_native_call_shares_keys_out_as_the_part_does(heads, dim):
+    """The scratch that the native call asks for is what ``key_split``'s shares need, whatever tiles and contexts there are."""
+    floats = ops._fn("stack", "ti_dense_stack_portion_floats")
+    floats.restype = ops.c_ll
+    call = ops._StackCall()
+    call.dtype, call.heads, call.head_dim = 1, heads, dim
+    call.pair_min_ctas, call.split_max_ctas = ops.PAIR_MIN_CTAS, ops.KEY_SPLIT_MAX_CTAS
+    for pairs in (0, 1, 2, 5, 37, 148):
+        for singles in (0, 1, 3, 30, 75):
+            for context in (1, 1000, 2047, 2048, 2049, 3000, 4096, 9999, 32768, 40960):
+                call.num_pairs, call.num_tiles, call.max_context = pairs, pairs + singles, context
+                need = [0]
+                for count, halves in ((pairs if pairs * heads < ops.PAIR_MIN_CTAS else 0, 2), (singles, 1)):
+                    if count:
+                        splits, keys = ops.key_split(count * halves * heads, context)
+                        assert splits == 1 or (keys % 128 == 0 and splits * keys >= context)
+                        need.append(count * halves * splits * heads * 128 * (dim + 2) if splits > 1 else 0)
+                assert floats(ops.ctypes.addressof(call)) == max(need), (pairs, singles, context)

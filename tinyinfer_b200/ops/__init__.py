@@ -275,7 +275,7 @@ def _tensor_core_ok(x: torch.Tensor, w: torch.Tensor, *others) -> bool:
 
 F32_FEW_ROWS = 8          # up to so many rows a float32 product streams its weights past the rows of x held in registers
 F32_MIN_K = 256           # below, the general kernel's few steps are as quick, and its sums have one order for any number of rows
-F32_SPLIT_MIN_K = 320     # and with more rows: the split products' error is 2.2 to 3.2e-7 whatever K is, the general kernel's grows with
+F32_SPLIT_MIN_K = 320     # and with more rows: the split products' error is 1.3 to 3.3e-7 whatever K is, the general kernel's grows with
                           # it: 2.3 to 2.9e-7 at 256, 2.5 to 3.2e-7 at 320 (200 x 1,024 outputs there: 17 us for 26)
 
 
@@ -684,29 +684,24 @@ def plan_attention(q_lens, starts):
     return decode_rows, [x for t in pairs + singles for x in t], len(pairs)
 
 
-def attention_shape_ok(dtype: torch.dtype, hq: int, hkv: int, d: int, page: int) -> bool:
-    """Whether these sizes have attention kernels of their own: bfloat16 on the tensor cores, or the float32 ones."""
+def attention_shape_ok(dtype: torch.dtype, hq: int, hkv: int, d: int, page: int, maps: int = 1) -> bool:
+    """Whether these sizes have attention kernels of their own. Head sizes 64 and 128 both; float32: up to 32 query heads per kv
+    head; bfloat16 (tensor cores): up to 16 (with two maps a head, 8) and pages of 16, 32 or a multiple of 64 tokens."""
     if d not in (64, 128) or hq % hkv:
         return False
     if dtype == torch.float32:
-        return hq // hkv <= 32
-    return dtype == torch.bfloat16 and hq // hkv <= 16 and (page in (16, 32) or page % 64 == 0)
+        return maps == 1 and hq // hkv <= 32
+    return dtype == torch.bfloat16 and hq // hkv * maps <= 16 and (page in (16, 32) or page % 64 == 0)
 
 
 def attention_tensor_cores_ok(q: torch.Tensor, kv_cache: torch.Tensor, maps: int = 1) -> bool:
-    """The tensor-core attention kernels take bfloat16, head sizes 64 and 128, up to 16 query heads (or, with two maps a
-    head, 8) per kv head, and pages of 16, 32 or a multiple of 64 tokens."""
-    _, hq, d = q.shape
-    hkv, page = kv_cache.shape[2], kv_cache.shape[3]
-    return (q.dtype == torch.bfloat16 and d in (64, 128) and hq % hkv == 0 and hq // hkv * maps <= 16
-            and (page in (16, 32) or page % 64 == 0))
+    """Whether the tensor-core attention kernels take these operands."""
+    return q.dtype == torch.bfloat16 and attention_shape_ok(q.dtype, q.shape[1], kv_cache.shape[2], q.shape[2], kv_cache.shape[3], maps)
 
 
 def attention_float32_ok(q: torch.Tensor, kv_cache: torch.Tensor) -> bool:
-    """The float32 attention kernels take head sizes 64 and 128 and up to 32 query heads per kv head."""
-    _, hq, d = q.shape
-    hkv = kv_cache.shape[2]
-    return (q.dtype == torch.float32 and d in (64, 128) and hq % hkv == 0 and hq // hkv <= 32
+    """Whether the float32 attention kernels take these operands."""
+    return (q.dtype == torch.float32 and attention_shape_ok(q.dtype, q.shape[1], kv_cache.shape[2], q.shape[2], kv_cache.shape[3])
             and (q.data_ptr() | kv_cache.data_ptr()) % 16 == 0)
 
 
@@ -782,6 +777,16 @@ def _keep_first(keep_first: int, window: Optional[int]) -> int:
     if keep_first < 0 or (keep_first and not window):
         raise KernelError("attention: first positions are kept beside a window")
     return int(keep_first)
+
+
+def key_split(ctas: int, max_context: int):
+    """(shares, keys a share) of the one-tile attention of prompt portions. Few query tiles behind a long prefix: the keys are
+    shared out over CTAs too (at least 1,024 to a CTA), so that most SMs have a CTA; their partial results meet in a merge kernel.
+    ``csrc/dense_stack.cu`` has the same rule for the launches it makes."""
+    splits = 1
+    if ctas * 2 <= KEY_SPLIT_MAX_CTAS and max_context >= 2048:
+        splits = max(1, min(KEY_SPLIT_MAX_CTAS // ctas, max_context // 1024))
+    return splits, -(-(-(-max_context // splits)) // 128) * 128 if splits > 1 else 0
 
 
 def paged_attention(q: torch.Tensor, kv_cache: torch.Tensor, *, positions: torch.Tensor,
@@ -880,13 +885,7 @@ def paged_attention(q: torch.Tensor, kv_cache: torch.Tensor, *, positions: torch
              num_pages, float(scale), mask, keep, int(max_context), has_sink, sink_v, float(out_scale), *extras, *two_maps,
              kstatus, _stream())
     def one_tile_kernel(first: int, count: int, halves: int) -> None:
-        # Few query tiles behind a long prefix: the keys are shared out over CTAs too (at least 1,024 to a CTA),
-        # so that most SMs have a CTA; their partial results meet in a merge kernel.
-        ctas = count * (2 if halves else 1) * hq
-        splits = 1
-        if ctas * 2 <= KEY_SPLIT_MAX_CTAS and max_context >= 2048:
-            splits = max(1, min(KEY_SPLIT_MAX_CTAS // ctas, int(max_context) // 1024))
-        split_keys = -(-(-(-int(max_context) // splits)) // 128) * 128 if splits > 1 else 0
+        splits, split_keys = key_split(count * (2 if halves else 1) * hq, int(max_context))
         scratch_ptr, scratch_floats = None, 0
         if splits > 1:
             scratch = _decode_scratch(q.device, count * (2 if halves else 1) * splits * hq * 128 * (d + 2))
