@@ -1,10 +1,11 @@
 // The blocks of a dense pre-norm decoder (grouped-query attention, gated feed-forward) from ONE call: every launch of a step's
 // layers is made here, through the launchers of the other libraries, on buffers that one workspace holds.
 //
-// Bound by the host in steps of few or some hundred tokens: a launch through Python cost 16 to 21 us (three output tensors,
+// Bound by the host in steps of some hundred tokens: a launch through Python cost 16 to 21 us (three output tensors,
 // 20 arguments, checks), 172 of them a step of 37 tokens over 28 layers, whose kernels need 0.9 ms; from here it costs what
-// the launch costs. What is launched, on what and in which order is what the layers' parts would launch.
-// 37 tokens, 28 layers of hidden size 1024: 3.66 -> 1.30 ms a step, the outputs the same bit for bit.
+// the launch costs. The kernels and their operands are what the layers' parts would launch, in their order, and the outputs the
+// same bit for bit; only the two attention kernels of a step that brings portions and decoded tokens run on two streams.
+// 37 tokens, 28 layers of hidden size 1024: 3.66 -> 1.31 ms a step.
 #include "common.cuh"
 #include <algorithm>
 

@@ -3,7 +3,9 @@
 Part by part, every kernel of a step is checked, given its output and launched from Python, which costs several times what a
 kernel of a short step runs for. A model whose blocks are all pre-norm blocks of plain attention and a gated feed-forward, of
 the same sizes, is recognised here once; its steps then hand the native side their layers' addresses and make the launches of
-all layers in one call. What is launched, on what and in which order is what the parts would launch."""
+all layers in one call. The kernels are the parts' own, on the same operands in the same order, but for the two attention kernels of a
+step that brings portions and decoded tokens: these run beside each other, on two streams. Operands that the parts' calls would
+refuse are left to them."""
 from __future__ import annotations
 
 from typing import Optional
