@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(EX_ROUTE_THREADS) moe_route_kernel(
 // clears the counts beforehand.
 constexpr int EX_PLACE_THREADS = 256;
 constexpr int EX_ALONE_MAX = 1024;                 // (token, choice) pairs of a step that one block places
+constexpr int EX_MANY_TOKENS = 8 * 148;            // tokens of a step whose router takes eight a block
+static_assert(EX_MANY_TOKENS > EX_ALONE_MAX, "eight tokens a block: the choices are placed by many, so they draw ranks");
 
 template <bool ALONE>
 __global__ void __launch_bounds__(EX_PLACE_THREADS) moe_place_kernel(
@@ -318,7 +320,7 @@ TI_API int ti_moe_route(int* chosen, float* weight, int* rank, int* counts, int*
     const bool on16 = ((uintptr_t)w_router & 15) == 0 && ((uintptr_t)x & 15) == 0;
     const bool vec = on16 && x_dtype == TI_F32 && hidden % (16 / esize) == 0;
     // eight tokens a block once that still leaves a block for every SM (and their rows fit beside another block's)
-    const bool many = on16 && hidden % 8 == 0 && num_tokens >= 8 * 148 && hidden <= 3072;
+    const bool many = on16 && hidden % 8 == 0 && num_tokens >= EX_MANY_TOKENS && hidden <= 3072;
     typedef __nv_bfloat16 B;
 #define EX_ROUTE(T, XT, TOK, L, RANKED)                                                                                            \
     do {                                                                                                                           \
@@ -340,8 +342,8 @@ TI_API int ti_moe_route(int* chosen, float* weight, int* rank, int* counts, int*
 #define EX_ROUTE_SIZED(T, XT)                                                      \
     do {                                                                           \
         constexpr int WIDE = sizeof(XT) == 4 ? 16 / sizeof(T) : 1;                 \
-        if (many && vec) EX_ROUTE_RANKED(T, XT, 8, WIDE);                          \
-        else if (many) EX_ROUTE_RANKED(T, XT, 8, 1);                               \
+        if (many && vec) EX_ROUTE(T, XT, 8, WIDE, true);                           \
+        else if (many) EX_ROUTE(T, XT, 8, 1, true);                                \
         else if (vec) EX_ROUTE_RANKED(T, XT, 1, WIDE);                             \
         else EX_ROUTE_RANKED(T, XT, 1, 1);                                         \
     } while (0)
