@@ -59,6 +59,20 @@ def test_product_on_the_tensor_cores(ops, m, n, k):
     check_product(ops, m, n, k, k / 16 + 8)
 
 
+@pytest.mark.parametrize("m", [1, 5, 8, 9, 200])
+def test_product_by_what_the_kernel_before_makes(ops, m):
+    """The second operand of a product may be the output of a kernel that has just been launched, in memory that held another."""
+    x, a = rnd(m, 2048, dtype=torch.float32, seed=1), rnd(3000, 2048, dtype=torch.float32, seed=2)
+    bs = [rnd(2048, 2048, dtype=torch.float32, seed=3 + i) for i in range(4)]
+    for i in range(8):
+        w = ops.linear(a, bs[i % 4])                          # long
+        y = ops.linear(x, w)
+        z = ops.gated_linear(x, w)
+        torch.cuda.synchronize()
+        assert torch.equal(ops.linear(x, w), y) and torch.equal(ops.gated_linear(x, w), z)
+        del w
+
+
 def test_split_products_back_to_back(ops):
     """Products that start while the one before still runs (their weights are on their way long before x is there)."""
     x, w = rnd(333, 6144, dtype=torch.float32, seed=1), rnd(2048, 6144, dtype=torch.float32, seed=2)

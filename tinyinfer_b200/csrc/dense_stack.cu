@@ -29,8 +29,8 @@ typedef int (*OneTileFn)(void*, const void*, const void*, const int*, int, int, 
 typedef int (*TwoTileFn)(void*, const void*, const void*, const int*, int, int, const int*, int, int, int, int, int, int, float, int,
                          int*, cudaStream_t);
 typedef int (*SimtFn)(void*, const void*, const void*, const float*, const void*, int, int, int, int, int, int, cudaStream_t);
-typedef int (*FewFn)(float*, const float*, const float*, const float*, const float*, int, int, int, int, cudaStream_t);
-typedef int (*SplitFn)(float*, const float*, const float*, const float*, const float*, void*, int, int, int, int, int*, cudaStream_t);
+typedef int (*FewFn)(float*, const float*, const float*, const float*, const float*, int, int, int, int, int, cudaStream_t);
+typedef int (*SplitFn)(float*, const float*, const float*, const float*, const float*, void*, int, int, int, int, int, int*, cudaStream_t);
 typedef int (*Attention32Fn)(float*, const float*, const float*, const int*, const int*, const int*, int, const int*, int, int,
                              const int*, int, int, int, int, int, int, float, int, int*, cudaStream_t);
 
@@ -152,12 +152,13 @@ TI_API int ti_dense_stack(TiStackCall* call) {
                        bool scaled, float eps, const float* emit) -> int {
         if (f32) {
             const bool fits = k % 4 == 0 && k >= (T <= c.few_rows ? c.min_k : c.split_min_k) && ((uintptr_t)x | (uintptr_t)w) % 16 == 0;
+            const int early = 1;                    // the weights are the model's: no kernel of a step writes them
             if (!fits) STACK_RUN(0, c.simt(out, x, w, bias, residual, T, n, k, gated, 0, c.dtype, c.stream));
             else if (T <= c.few_rows)
-                STACK_RUN(2, c.few((float*)out, (const float*)x, (const float*)w, bias, (const float*)residual, T, n, k, gated, c.stream));
+                STACK_RUN(2, c.few((float*)out, (const float*)x, (const float*)w, bias, (const float*)residual, T, n, k, gated, early, c.stream));
             else
                 STACK_RUN(2, c.split((float*)out, (const float*)x, (const float*)w, bias, (const float*)residual, b.planes, T, n, k, gated,
-                                     c.wait_status, c.stream));
+                                     early, c.wait_status, c.stream));
             return 0;
         }
         if (scaled || emit) {

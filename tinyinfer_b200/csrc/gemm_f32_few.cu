@@ -5,7 +5,8 @@
 // interleaved pieces of 128 (4 floats a lane), so that a block asks for 8 x ROWS x 512 contiguous bytes at a time, and add
 // their sums up through shared memory. ROWS x M accumulators a lane: 4 rows of w up to M = 4 (64 bytes a lane in flight an
 // unrolled step, twice), 8 rows for M = 5..8, where the x that a lane reads from L1/L2 would otherwise cost more than the
-// weights. The first weights are asked for before the wait for the kernels ahead in the stream.
+// weights. With `early` the first weights are asked for before the wait for the kernels ahead in the stream, which none of those
+// may write then.
 // The order of the sums does not depend on M: a lane's k pieces in rising order, a tree over the lanes, the warps in order.
 // In place of the 64 x 64 tiles of gemm_simt.cu, which used 4 of their 64 rows and 16 to 96 blocks: a decode step of 4
 // requests over a 1.7B model (28 layers, hidden size 2048), 69.0 -> 2.1 ms together with attention_f32.cu. Alone, 12,288 x 2,048 weights: 15.8 us
@@ -53,7 +54,7 @@ template <int V, int OFF> __device__ __forceinline__ void fold(float* v, int lan
 // same outputs.
 template <int MT, int ROWS, int GATED>
 __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(
-    float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K) {
+    float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K, bool early) {
     constexpr int V = MT * ROWS;                 // sums a block makes
     constexpr int OUTS = GATED ? ROWS / 2 : ROWS;
     constexpr int U = ROWS <= 4 ? 2 : 1;         // steps whose weights are asked for together
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(
         wrow[r] = w + (size_t)(r < OUTS ? o : N + o) * K;
     }
     float acc[V] = {};
+    if (!early) ti_grid_wait();
     bool waited = false;
     for (int k0 = warp * PIECE; k0 < K || !waited; k0 += U * WARPS * PIECE) {
         float4 wv[U][ROWS];
@@ -135,26 +137,27 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_f32_few_kernel(
 
 template <int MT, int ROWS>
 void launch_few(float* out, const float* x, const float* w, const float* bias, const float* residual, int M, int N, int K,
-                int gated, cudaStream_t stream) {
+                int gated, bool early, cudaStream_t stream) {
     const int outs = gated ? ROWS / 2 : ROWS;
     const dim3 grid((N + outs - 1) / outs);
-    if (gated == 2) ti_launch(gemm_f32_few_kernel<MT, ROWS, 2>, grid, WARPS * 32, 0, stream, out, x, w, bias, residual, M, N, K);
-    else if (gated) ti_launch(gemm_f32_few_kernel<MT, ROWS, 1>, grid, WARPS * 32, 0, stream, out, x, w, bias, residual, M, N, K);
-    else ti_launch(gemm_f32_few_kernel<MT, ROWS, 0>, grid, WARPS * 32, 0, stream, out, x, w, bias, residual, M, N, K);
+    if (gated == 2) ti_launch(gemm_f32_few_kernel<MT, ROWS, 2>, grid, WARPS * 32, 0, stream, out, x, w, bias, residual, M, N, K, early);
+    else if (gated) ti_launch(gemm_f32_few_kernel<MT, ROWS, 1>, grid, WARPS * 32, 0, stream, out, x, w, bias, residual, M, N, K, early);
+    else ti_launch(gemm_f32_few_kernel<MT, ROWS, 0>, grid, WARPS * 32, 0, stream, out, x, w, bias, residual, M, N, K, early);
 }
 
 }  // namespace
 
-// As ti_gemm_simt for float32 operands with 1 <= M <= 8, K a multiple of 4 and x and w on 16-byte boundaries.
+// As ti_gemm_simt for float32 operands with 1 <= M <= 8, K a multiple of 4 and x and w on 16-byte boundaries. early: no kernel that
+// may still run writes w (a model's weights).
 TI_API int ti_gemm_f32_few(float* out, const float* x, const float* w, const float* bias, const float* residual,
-                           int M, int N, int K, int gated, cudaStream_t stream) {
+                           int M, int N, int K, int gated, int early, cudaStream_t stream) {
     TI_REQUIRE(M >= 1 && M <= 8 && N > 0 && K > 0 && K % 4 == 0, "gemm_f32_few: bad sizes M=%d N=%d K=%d", M, N, K);
     TI_REQUIRE(((uintptr_t)x | (uintptr_t)w) % 16 == 0, "gemm_f32_few: operands must lie on 16-byte boundaries");
     TI_REQUIRE(!(gated && residual), "gemm: the gated form takes no residual");
-    if (M == 1) launch_few<1, 4>(out, x, w, bias, residual, M, N, K, gated, stream);
-    else if (M == 2) launch_few<2, 4>(out, x, w, bias, residual, M, N, K, gated, stream);
-    else if (M <= 4) launch_few<4, 4>(out, x, w, bias, residual, M, N, K, gated, stream);
-    else launch_few<8, 8>(out, x, w, bias, residual, M, N, K, gated, stream);
+    if (M == 1) launch_few<1, 4>(out, x, w, bias, residual, M, N, K, gated, early, stream);
+    else if (M == 2) launch_few<2, 4>(out, x, w, bias, residual, M, N, K, gated, early, stream);
+    else if (M <= 4) launch_few<4, 4>(out, x, w, bias, residual, M, N, K, gated, early, stream);
+    else launch_few<8, 8>(out, x, w, bias, residual, M, N, K, gated, early, stream);
     TI_CHECK_LAUNCH("gemm_f32_few");
     return 0;
 }

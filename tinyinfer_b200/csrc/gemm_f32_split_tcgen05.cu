@@ -54,7 +54,7 @@ struct SplitParams {
     float* out;
     const float *x, *w, *bias, *residual;
     int M, N, K, gated;                          // gated: 0 no, 1 silu, 2 the tanh form of gelu; then w has 2N rows
-    int bn, b_stages, slots;
+    int bn, b_stages, slots, early;
     int* status;
 };
 
@@ -306,8 +306,9 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             }
         }
     } else if (warp == W_WARP) {
-        // ------------------------------------------------------------ TMA: the weights, which no earlier kernel writes
+        // ------------------------------------------------------------ TMA: the weights; `early`: no earlier kernel writes them
         if (lane == 0) {
+            if (!p.early) ti_grid_wait();
             int slot = 0;
             uint32_t phase = 0;
             bool ok = true;
@@ -481,14 +482,14 @@ int choose_splits(int tiles, int num_kb) {
 }  // namespace
 
 // As ti_gemm_simt for float32 operands with K a multiple of 4 and x and w on 16-byte boundaries. ``planes``: room for
-// 3 * M * Kp bfloat16 on a 16-byte boundary, Kp = K rounded up to a multiple of 64.
+// 3 * M * Kp bfloat16 on a 16-byte boundary, Kp = K rounded up to a multiple of 64. early: no kernel that may still run writes w.
 TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const float* bias, const float* residual, void* planes,
-                             int M, int N, int K, int gated, int* status, cudaStream_t stream) {
+                             int M, int N, int K, int gated, int early, int* status, cudaStream_t stream) {
     TI_REQUIRE(M >= 1 && N > 0 && K > 0 && K % 4 == 0, "gemm_f32_split: bad sizes M=%d N=%d K=%d", M, N, K);
     TI_REQUIRE(((uintptr_t)x | (uintptr_t)w | (uintptr_t)planes) % 16 == 0, "gemm_f32_split: operands must lie on 16-byte boundaries");
     TI_REQUIRE(!(gated && residual), "gemm: the gated form takes no residual");
     const int Kp = (K + 63) / 64 * 64;
-    SplitParams p{out, x, w, bias, residual, M, N, K, gated, 0, 0, 0, status};
+    SplitParams p{out, x, w, bias, residual, M, N, K, gated, 0, 0, 0, early, status};
     const int row_tiles = (M + MAX_BN - 1) / MAX_BN;
     p.bn = ((M + row_tiles - 1) / row_tiles + 15) / 16 * 16;
     const int outs = gated ? 64 : 128, col_tiles = (N + outs - 1) / outs;

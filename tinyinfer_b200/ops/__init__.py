@@ -189,8 +189,8 @@ _SIGNATURES["stack"] = {
     "ti_dense_stack_bytes": [c_int, c_int, c_int, c_int, c_int, c_int],
 }
 _SIGNATURES["f32"] = {
-    "ti_gemm_f32_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
-    "ti_gemm_f32_split": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    "ti_gemm_f32_few": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "ti_gemm_f32_split": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "ti_attention_f32": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p,
                          c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
 }
@@ -281,16 +281,17 @@ F32_SPLIT_MIN_K = 320     # and with more rows: the split products' error is 1.3
 
 def _float32_product(out, x, w, bias, residual, m, n, k, gated) -> bool:
     """Runs a float32 product on the kernel made for its size, if there is one; False: the general kernel is to run it.
-    The weights are read 16 bytes at a time: whole rows of them, on 16-byte boundaries."""
+    The weights are read 16 bytes at a time: whole rows of them, on 16-byte boundaries; not before the kernels ahead have ended,
+    which may have made them."""
     if x.dtype != torch.float32 or k % 4 or k < (F32_MIN_K if m <= F32_FEW_ROWS else F32_SPLIT_MIN_K) or m < 1 or (x.data_ptr() | w.data_ptr()) % 16:
         return False
     if m <= F32_FEW_ROWS:
         _run("f32", "ti_gemm_f32_few", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), m, n, k, gated,
-             _stream())
+             0, _stream())
     else:
         planes = torch.empty((3, m, -(-k // 64) * 64), dtype=torch.bfloat16, device=x.device)
         _run("f32", "ti_gemm_f32_split", out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias), _ptr(residual), planes.data_ptr(),
-             m, n, k, gated, kernel_status(x.device).data_ptr(), _stream())
+             m, n, k, gated, 0, kernel_status(x.device).data_ptr(), _stream())
     return True
 
 
