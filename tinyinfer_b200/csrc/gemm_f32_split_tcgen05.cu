@@ -23,6 +23,8 @@
 //   warp 14       TMA: the three planes of x, which a small kernel has laid out before ([3][M][Kp])
 //   warp 15       one thread issues the MMAs, 12 of 128 x BN x 16 a k block
 //   warps 0..7    drain finished chunks into their registers, at the end into shared memory
+// Bound by the chain of a k block (copy, split, products, drain): 333 x 12,288 x 2,048 keeps the tensor pipe active 39 % of the time,
+// shared memory 28 %, L2 at 23 % and HBM at 12 %.
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
 // multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
