@@ -6,7 +6,7 @@
 // part of a number below 2^-109 would lose bits (rows of 1e-36 came out 2.6e-5 off, now 3.2e-7); times 2^24 every part of every float32 number,
 // subnormal ones included, is a normal bfloat16 number. What grows past float32's range by it (operands from 2^104,
 // sums from 2^80 on) comes out infinite and is computed again as below. In packed arithmetic the split costs no more with the
-// factor than it did without: 333 x 12,288 x 2,048 120.9 -> 121.0 us, 1,000 x 4,096 x 2,048 122.1 -> 118.2.
+// factor than it did without: 333 rows by 2 x 6,144 x 2,048 121.0 -> 119.7 us, 30 rows 53.5 -> 53.4, 9 rows by 12,288 x 2,048 52.0 -> 51.4.
 //
 // The sums decide the precision. The tensor core cuts bits off when it adds to its accumulator, always towards zero, so a
 // long run in one accumulator would drift. Here a run is CHUNK = 2 k blocks of 32, the small parts of a block before the
@@ -28,7 +28,7 @@
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
 // multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
-// again through shared memory (redo_plain): 333 rows of NaN by 12,288 x 2,048 weights 1.26 ms, where gemm_simt.cu takes 0.89.
+// again through shared memory (finish_odd): 333 rows of NaN by 12,288 x 2,048 weights 1.24 ms, where gemm_simt.cu takes 0.89.
 // Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 118 us (142 TFLOP/s), by 2,048 x 6,144
 // 799 -> 78 us; 9 rows 306 -> 51 us; 200 rows by 1,024 x 320 weights, the shortest k that comes here, 26 -> 17 us.
 #include "sm100_ptx.cuh"
@@ -168,13 +168,60 @@ __device__ __forceinline__ void redo_plain(float* out, float* pieces, const Spli
     __syncthreads();
 }
 
+// Bias, activation or residual, and the store of four neighbouring outputs of token m (gated: of the gates and the ups).
+__device__ __forceinline__ void store_quad(const SplitParams& p, int m, int n, const float (&total)[2][4]) {
+    float res[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (n + e >= p.N) { res[e] = 0.f; continue; }
+        float v = total[0][e];
+        if (p.bias) v += p.bias[n + e];
+        if (p.gated) {
+            float up = total[1][e];
+            if (p.bias) up += p.bias[p.N + n + e];
+            if (p.gated == 1) v = v / (1.f + expf(-v));
+            else v = 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
+            v *= up;
+        } else if (p.residual) {
+            v += p.residual[(size_t)m * p.N + n + e];
+        }
+        res[e] = v;
+    }
+    float* dst = p.out + (size_t)m * p.N + n;
+    if (p.N % 4 == 0 && ((uintptr_t)p.out & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(res[0], res[1], res[2], res[3]);
+    else
+        for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = res[e];
+}
+
+// The kernel's last act where sums were not finite: `odd` names the calling thread's quads that have some, which are stored from
+// what is made again. A function of its own, so that the kernel holds nothing for it: what it would hold goes to local memory, and a
+// few spilled registers cost the products 2 %.
+__device__ __noinline__ void finish_odd(const SplitParams& p, float* sums, uint32_t odd) {
+    const int splits = (int)gridDim.x, part = (int)blockIdx.x, outs = p.gated ? 64 : 128, shift = p.gated ? 4 : 5;
+    const int c0 = p.bn * part / splits, c1 = p.bn * (part + 1) / splits;
+    const int m = (int)blockIdx.y * p.bn + c0, n0 = (int)blockIdx.z * outs;
+    redo_plain(sums, sums + MAX_BN * 128, p, m, c1 - c0, n0, outs);
+    for (int i = threadIdx.x; odd; i += NUM_THREADS, odd >>= 1) {
+        if (!(odd & 1)) continue;
+        const int col = i >> shift, o = (i & ((1 << shift) - 1)) * 4;
+        float total[2][4] = {};
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            if (g && !p.gated) break;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) total[g][e] = sums[col * 128 + o + 64 * g + e];
+        }
+        store_quad(p, m + col, n0 + o, total);
+    }
+}
+
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ SplitParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ uint64_t bars[2 * (A_STAGES + MAX_B_STAGES + MAX_SLOTS) + 4];
     __shared__ uint32_t tmem_base_sh;
-    __shared__ int abort_sh;
+    __shared__ int abort_sh, odd_sh;                         // a wait ran out; an output that is not finite
     volatile int* abort_flag = &abort_sh;
     const uint32_t bar0 = smem_u32(bars);
     auto acc_full_bar = [&](int a) { return bar0 + 8u * a; };
@@ -199,7 +246,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     uint8_t* slot_ring = b_ring + p.b_stages * 3 * plane_b;
 
     if (threadIdx.x == 0) {
-        abort_sh = 0;
+        abort_sh = odd_sh = 0;
         for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full_bar(s), PAIR); mbar_init(a_empty_bar(s), 1); }
         for (int s = 0; s < MAX_SLOTS; ++s) { mbar_init(w_full_bar(s), 1); mbar_init(w_empty_bar(s), PAIR); }
         for (int s = 0; s < MAX_B_STAGES; ++s) { mbar_init(b_full_bar(s), 1); mbar_init(b_empty_bar(s), 1); }
@@ -376,73 +423,48 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     __syncwarp();
     if (splits > 1) cluster.sync();
     else __syncthreads();
-    const int c0 = p.bn * part / splits, c1 = p.bn * (part + 1) / splits;
+    uint32_t odd = 0;                                        // this thread's quads that are not finite
     if (!*abort_flag) {
         ti_grid_wait();                                      // out and residual belong to the kernels ahead until now
-        const int quads = outs / 4, kinds = p.gated ? 2 : 1; // four neighbouring outputs a thread
-        float* again = sums + MAX_BN * 128;                  // [c1 - c0][128]: outputs made again, behind the sums
-        // first the outputs whose sums are finite; if there are others, these once they have been made again
-        for (bool redone = false;; redone = true) {
-            bool odd = false;
-            for (int i = threadIdx.x; i < (c1 - c0) * quads; i += NUM_THREADS) {
-                const int col = c0 + i / quads, o = i % quads * 4, m = m0 + col, n = n0 + o;
-                if (m >= p.M || n >= p.N) continue;
-                float total[2][4] = {};
-                bool finite = true;
-                for (int g = 0; g < kinds; ++g) {
-                    float4 f[8];
+        const int c0 = p.bn * part / splits, c1 = p.bn * (part + 1) / splits;
+        const int shift = p.gated ? 4 : 5, kinds = p.gated ? 2 : 1;
+        for (int i = threadIdx.x, q = 0; i < (c1 - c0) << shift; i += NUM_THREADS, ++q) {       // four neighbouring outputs a thread
+            const int col = c0 + (i >> shift), o = (i & ((1 << shift) - 1)) * 4, m = m0 + col, n = n0 + o;
+            if (m >= p.M || n >= p.N) continue;
+            float total[2][4] = {};
+            bool finite = true;
+            for (int g = 0; g < kinds; ++g) {
 #pragma unroll
-                    for (int r = 0; r < 8; ++r)
-                        if (r < splits) f[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums + col * 128 + o + 64 * g, r));
+                for (int r0 = 0; r0 < 8; r0 += 4) {          // four at a time: the registers of eight would spill
+                    float4 f[4];
 #pragma unroll
-                    for (int r = 0; r < 8; ++r)
-                        if (r < splits) {
+                    for (int r = 0; r < 4; ++r)
+                        if (r0 + r < splits) f[r] = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums + col * 128 + o + 64 * g, r0 + r));
+#pragma unroll
+                    for (int r = 0; r < 4; ++r)
+                        if (r0 + r < splits) {
                             total[g][0] += f[r].x; total[g][1] += f[r].y; total[g][2] += f[r].z; total[g][3] += f[r].w;
                         }
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        if (isfinite(total[g][e])) total[g][e] *= RESULT_SCALE;
-                        else if (n + e < p.N) {
-                            finite = false;
-                            total[g][e] = again[(col - c0) * 128 + o + 64 * g + e];
-                        }
-                    }
                 }
-                odd |= !finite;
-                if (finite == redone) continue;
-                float res[4];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    if (n + e >= p.N) { res[e] = 0.f; continue; }
-                    float v = total[0][e];
-                    if (p.bias) v += p.bias[n + e];
-                    if (p.gated) {
-                        float up = total[1][e];
-                        if (p.bias) up += p.bias[p.N + n + e];
-                        if (p.gated == 1) v = v / (1.f + expf(-v));
-                        else v = 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)));
-                        v *= up;
-                    } else if (p.residual) {
-                        v += p.residual[(size_t)m * p.N + n + e];
-                    }
-                    res[e] = v;
+                    finite = finite && (n + e >= p.N || isfinite(total[g][e]));
+                    total[g][e] *= RESULT_SCALE;
                 }
-                float* dst = p.out + (size_t)m * p.N + n;
-                if (p.N % 4 == 0 && ((uintptr_t)p.out & 15) == 0) *reinterpret_cast<float4*>(dst) = make_float4(res[0], res[1], res[2], res[3]);
-                else
-                    for (int e = 0; e < 4 && n + e < p.N; ++e) dst[e] = res[e];
             }
-            if (redone || !__syncthreads_or(odd)) break;
-            redo_plain(again, again + MAX_BN * 128, p, m0 + c0, c1 - c0, n0, outs);
+            if (finite) store_quad(p, m, n, total);
+            else odd |= 1u << q;
         }
+        if (odd) odd_sh = 1;
     }
     tmem_fence_before();
-    if (splits > 1) cluster.sync();                          // nobody leaves while its sums may be read
+    if (splits > 1) cluster.sync();                          // nobody leaves, or writes over its sums, while they may be read
     else __syncthreads();
     if (warp == MMA_WARP) {
         tmem_fence_after();
         tmem_dealloc(tmem_base, 2 * MAX_BN);
     }
+    if (odd_sh) finish_odd(p, sums, odd);
 }
 
 // How many clusters of s CTAs the device holds at a time (a cluster lies within one GPC, so some sizes leave SMs unused).
@@ -501,7 +523,8 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
     const int b_bytes = 3 * p.bn * BK * 2, room = SMEM_BYTES - 1024 - A_STAGES * 3 * PLANE_A;
     p.b_stages = std::min(MAX_B_STAGES, (room - 3 * SLOT) / b_bytes);       // at least three
     p.slots = std::min(MAX_SLOTS, (room - p.b_stages * b_bytes) / SLOT / A_STAGES * A_STAGES);
-    static_assert(4 * (2 * MAX_BN * 128 + 2 * REDO_PIECE) <= SMEM_BYTES - 1024, "the sums, the outputs made again and their operands");
+    static_assert(4 * (MAX_BN * 128 + 2 * REDO_PIECE) <= SMEM_BYTES - 1024, "the outputs made again and their operands");
+    static_assert(MAX_BN * 32 <= 32 * NUM_THREADS, "a thread's quads have a bit each");
     static_assert(A_STAGES * 3 * PLANE_A + 3 * 3 * MAX_BN * BK * 2 + 3 * SLOT <= SMEM_BYTES - 1024, "128 columns: three copies, three slots");
     static_assert(MAX_SLOTS % A_STAGES == 0 && A_STAGES == 3, "three slots at least, a whole number a pair");
     TiEncodeTiledFn encode = ti_encode_tiled_fn();
