@@ -1,0 +1,55 @@
+"""The attention over cached latent rows on tcgen05 (prompt portions) against 64 bits, and against the warp-level form, whose
+probabilities it rounds alike: edges of its tiles of 32 keys and of its row tiles, pages of 16 keys, rows past a chunk of 64
+features, sinks, shared-out keys, portions beside decoded tokens, pages that hold NaN behind the last key."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,rank,rot,page,sink,work", [
+    (16, 512, 64, 64, True, [(75, 75), (900, 1), (300, 9)]),         # two CTAs a row tile; a decoded token among portions
+    (16, 512, 64, 16, False, [(33, 33), (64, 31), (65, 2)]),
+    (16, 512, 64, 64, True, [(1500, 16)]),                           # keys shared out over CTAs
+    (5, 256, 32, 32, False, [(130, 130), (31, 31), (32, 32)]),       # heads that do not divide the 128 rows
+    (3, 64, 8, 48, True, [(700, 600)]),                              # features past a chunk; pages of 48
+    (130, 128, 0, 128, False, [(40, 3)]),                            # more heads than rows
+])
+def test_portions_on_tcgen05(monkeypatch, heads, rank, rot, page, sink, work):
+    from tinyinfer_b200 import ops
+    from tinyinfer_b200.engine.batch import BatchBuffers, StepEntry
+    gen = torch.Generator().manual_seed(heads * rank)
+    dk, lens = rank + rot, [c for c, _ in work]
+    pages_of = [-(-n // page) for n in lens]
+    perm = torch.randperm(sum(pages_of) + 2, generator=gen).tolist()
+    tables = [[perm.pop() for _ in range(nb)] for nb in pages_of]
+    cache = torch.full((1, sum(pages_of) + 2, 1, page, dk), float("nan"), dtype=torch.bfloat16)
+    rows = [torch.randn(n, dk, generator=gen).to(torch.bfloat16) for n in lens]
+    for i, n in enumerate(lens):
+        for p in range(n):
+            cache[0, tables[i][p // page], 0, p % page] = rows[i][p]
+    buffers = BatchBuffers(torch.device("cuda"), sum(n for _, n in work), len(work), max(pages_of), 1)
+    step = buffers.build([StepEntry(i, [0] * n, []) for i, (_, n) in enumerate(work)], [c - n for c, n in work], [0] * len(work), [tables])
+    T = step.num_tokens
+    q = 2.0 * torch.randn(T, heads * dk, generator=gen)
+    scale = dk ** -0.5
+    sinks = torch.randn(heads, generator=gen) if sink else None
+    args = dict(heads=heads, rank=rank, rot=rot, scale=scale, sink=sinks.cuda() if sink else None, positions=step.positions,
+                token_seq=step.token_seq, block_table=step.block_tables[0], max_context=max(lens), step=step)
+    assert ops._fn("latent", "ti_latent_attend_tc_ctas")(T, len(work), heads, rank, rot, page) > 0
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    new = ops.latent_attention(q.cuda(), cache.cuda(), status=status, **args).cpu().double()
+    monkeypatch.setattr(ops, "LATENT_TCGEN05", False)
+    old = ops.latent_attention(q.cuda(), cache.cuda(), status=status, **args).cpu().double()
+    ops.check_kernel_status()
+    pos, seq = step.positions.cpu().tolist(), step.token_seq.cpu().tolist()
+    want = torch.empty_like(new)
+    for t in range(T):
+        keys = rows[seq[t]][:pos[t] + 1].double()
+        z = (q[t].view(heads, dk).to(torch.bfloat16).double() @ keys.T) * scale
+        if sink:
+            z = torch.cat([z, sinks.double()[:, None]], dim=1)
+        want[t] = (torch.softmax(z, dim=1)[:, :pos[t] + 1] @ keys[:, :rank]).reshape(-1)
+    # two roundings to 8 bits, of the probabilities and of the result: at most 2^-9 of the result's norm each
+    err, err_old = ((x - want).norm() / want.norm() for x in (new, old))
+    assert err <= 2.0 ** -8 and err <= 1.02 * err_old + 1e-5, (err, err_old)

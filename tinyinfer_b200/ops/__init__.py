@@ -67,6 +67,9 @@ _SIGNATURES = {
         "ti_latent_attend_mma": [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int,
                                  c_void_p, c_void_p],
+        "ti_latent_attend_tc_ctas": [c_int, c_int, c_int, c_int, c_int, c_int],
+        "ti_latent_attend_tc": [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+                                c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
         "ti_causal_conv": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                            c_int, c_int, c_int, c_int, c_void_p],
         "ti_gated_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
@@ -1071,6 +1074,9 @@ def latent_query_rotate(rows: torch.Tensor, q: torch.Tensor, *, heads: int, plai
 
 LATENT_SPLIT_MIN_KEYS = 128     # a split of the keys over blocks gets at least this many
 LATENT_TARGET_BLOCKS = 296      # enough blocks to have two on every SM
+LATENT_TCGEN05 = True           # prompt portions on tcgen05 where its sizes allow
+LATENT_TC_CTAS = 148            # a CTA of that form has an SM to itself
+LATENT_TC_SPLIT_MIN_KEYS = 256
 
 
 def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, rank: int, rot: int, scale: float,
@@ -1116,6 +1122,21 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
     if (step is not None and cache.dtype == torch.bfloat16
             and int(_fn("latent", "ti_latent_attend_mma_ok")(rank, rot))):
         decode = step.max_q_len == 1
+        page_size = cache.shape[3]
+        ctas = 0 if decode or window else int(_fn("latent", "ti_latent_attend_tc_ctas")(t, step.num_seqs, heads, rank, rot, page_size))
+        if ctas and LATENT_TCGEN05 and (q_rows.data_ptr() | cache.data_ptr()) % 16 == 0:
+            splits = 1
+            if ctas < LATENT_TC_CTAS and reach >= 2 * LATENT_TC_SPLIT_MIN_KEYS:
+                splits = max(1, min(LATENT_TC_CTAS // ctas, reach // LATENT_TC_SPLIT_MIN_KEYS, 64))
+            parts, parts_floats = scratch(splits)
+            _run("latent", "ti_latent_attend_tc", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), cache.data_ptr(),
+                 _ptr(sink), positions.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(), block_table.shape[1],
+                 step.num_seqs, t, heads, rank, rot, page_size, cache.shape[1], float(scale), splits,
+                 status_words(cache.device).data_ptr(), _stream())
+            if splits > 1:
+                _run("latent", "ti_latent_merge", out.data_ptr(), parts.data_ptr(), _ptr(sink), t, heads, rank, splits,
+                     _dtype_code(cache), _stream())
+            return out
         rows = 16 if decode else 32
         per_block = min(heads, rows)
         tokens_per_block = 1 if decode else max(1, rows // per_block)
