@@ -422,13 +422,19 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     }
 }
 
-// Merges the partial results of a split of the keys: one block per (query row of a tile, head), one thread
-// per feature, the shares in key order. A share the tile has no keys in was not computed and is not read.
+// Merges the partial results of a split of the keys: a warp per (query row of a tile, head), D / 32 neighbouring features a
+// lane, the shares in key order, four shares' loads on their way at a time. A share the tile has no keys in was not computed and
+// is not read. (A block per row and head with a feature a thread waited for its loads share by share.)
+constexpr int MERGE_WARPS = 8;
 template <int D>
-__global__ void prefill_merge_kernel(const PrefillParams p) {
+__global__ void __launch_bounds__(MERGE_WARPS * 32) prefill_merge_kernel(const PrefillParams p, int items) {
+    constexpr int VEC = D / 32, Z = 4;
+    struct alignas(4 * VEC) Pack { float e[VEC]; };
     ti_grid_launch_dependents();
     ti_grid_wait();
-    const int slot = blockIdx.x / QM, r = blockIdx.x % QM, head = blockIdx.y, d = threadIdx.x;
+    const int item = blockIdx.x * MERGE_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (item >= items) return;
+    const int head = item % p.hq, row = item / p.hq, slot = row / QM, r = row % QM;
     const int4 td = reinterpret_cast<const int4*>(p.tiles)[p.halves ? slot >> 1 : slot];
     const int half_off = p.halves ? (slot & 1) * QM : 0;
     const int row0 = td.y + half_off, pos0 = td.w + half_off;
@@ -436,23 +442,43 @@ __global__ void prefill_merge_kernel(const PrefillParams p) {
     if (r >= nrows) return;
     const int hi = pos0 + nrows;
     const int lo = ti_first_key(pos0, p.window);
-    float m_run = -INFINITY, acc = 0.f, l_all = 0.f;
-    for (int z = 0; z < p.splits; ++z) {
-        if (KeyTiles(p, lo, hi, z).count() <= 0) continue;
-        const size_t part = (((size_t)slot * p.splits + z) * p.hq + head) * QM + r;
-        const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.part_ml + part * 2));
-        const float ov = __ldcg(p.part_o + part * D + d);
-        const float m_new = fmaxf(m_run, ml.x);
-        const float m_use = m_new == -INFINITY ? 0.f : m_new;
-        const float keep = ex2(m_run - m_use), f = ex2(ml.x - m_use);      // 0 while nothing has been merged yet
-        acc = acc * keep + f * ov;
-        l_all = l_all * keep + f * ml.y;
-        m_run = m_new;
+    float m_run = -INFINITY, l_all = 0.f, acc[VEC] = {};
+    for (int z0 = 0; z0 < p.splits; z0 += Z) {
+        bool has[Z];
+        float2 ml[Z];
+        Pack ov[Z];
+#pragma unroll
+        for (int i = 0; i < Z; ++i) {
+            has[i] = z0 + i < p.splits && KeyTiles(p, lo, hi, z0 + i).count() > 0;
+            if (!has[i]) continue;
+            const size_t part = (((size_t)slot * p.splits + z0 + i) * p.hq + head) * QM + r;
+            ml[i] = __ldcg(reinterpret_cast<const float2*>(p.part_ml + part * 2));
+            if constexpr (VEC == 4) *reinterpret_cast<float4*>(&ov[i]) = __ldcg(reinterpret_cast<const float4*>(p.part_o + part * D) + lane);
+            else *reinterpret_cast<float2*>(&ov[i]) = __ldcg(reinterpret_cast<const float2*>(p.part_o + part * D) + lane);
+        }
+#pragma unroll
+        for (int i = 0; i < Z; ++i) {
+            if (!has[i]) continue;
+            const float m_new = fmaxf(m_run, ml[i].x);
+            const float m_use = m_new == -INFINITY ? 0.f : m_new;
+            const float keep = ex2(m_run - m_use), f = ex2(ml[i].x - m_use);      // 0 while nothing has been merged yet
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] = acc[e] * keep + f * ov[i].e[e];
+            l_all = l_all * keep + f * ml[i].y;
+            m_run = m_new;
+        }
     }
     if (p.has_sink) l_all += ex2(ti_sink_log2(p, head) - m_run);
-    float res = l_all > 0.f ? acc * ti_head_out_scale(p, (size_t)(row0 + r), head) / l_all : 0.f;
-    ti_gate_features<1>(p, (size_t)(row0 + r), head, D, d, &res);
-    p.out[((size_t)(row0 + r) * p.hq + head) * D + d] = __float2bfloat16_rn(res);
+    alignas(8) __nv_bfloat16 out[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+        float res = l_all > 0.f ? acc[e] * ti_head_out_scale(p, (size_t)(row0 + r), head) / l_all : 0.f;
+        ti_gate_features<1>(p, (size_t)(row0 + r), head, D, lane * VEC + e, &res);
+        out[e] = __float2bfloat16_rn(res);
+    }
+    __nv_bfloat16* dst = p.out + ((size_t)(row0 + r) * p.hq + head) * D + lane * VEC;
+    if constexpr (VEC == 4) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(out);
+    else *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(out);
 }
 
 }  // namespace
@@ -531,8 +557,11 @@ TI_API int ti_attention_prefill_tc_sink_bf16(void* out, const void* q, const voi
 #undef PF_GO
     TI_CHECK_LAUNCH("attention_prefill_tc");
     if (splits > 1) {
-        if (d == 128) ti_launch(prefill_merge_kernel<128>, dim3(slots * QM, hq), 128, 0, stream, p);
-        else ti_launch(prefill_merge_kernel<64>, dim3(slots * QM, hq), 64, 0, stream, p);
+        const long long items = (long long)slots * QM * hq;
+        TI_REQUIRE(items < (1ll << 31), "attention_prefill_tc: too many rows to merge");
+        const unsigned blocks = (unsigned)((items + MERGE_WARPS - 1) / MERGE_WARPS);
+        if (d == 128) ti_launch(prefill_merge_kernel<128>, blocks, MERGE_WARPS * 32, 0, stream, p, (int)items);
+        else ti_launch(prefill_merge_kernel<64>, blocks, MERGE_WARPS * 32, 0, stream, p, (int)items);
         TI_CHECK_LAUNCH("attention_prefill_merge");
     }
     return 0;
