@@ -32,6 +32,14 @@
 //                      `group` features divided by its root mean square (float32), act silu or sigmoid, one rounding
 #include "common.cuh"
 
+// linear_chunk.cu: long portions with one decay per head and token
+bool lc_takes(const void* q, int ld_q, int q_off, const void* k, int ld_k, int k_off, const void* v, int ld_v, int v_off, const float* scratch,
+              int dk, int dv, int esize);
+int lc_launch(int part, float* y, const void* q, int ld_q, int q_off, const void* k, int ld_k, int k_off, const void* v, int ld_v, int v_off,
+              const float* decay, int ld_decay, int decay_off, const float* kscale, const float* skip, float q_scale, const int* cu_seqlens,
+              int num_seqs, int heads, int groups, int dk, int dv, int chunks, float* part_b, float* part_a, int* status, int dtype,
+              cudaStream_t stream);
+
 enum { LS_GATE_RAW = 0, LS_GATE_SIGMOID_POW = 1, LS_GATE_STEP = 2 };
 constexpr int LS_WARPS = 4;
 
@@ -325,6 +333,13 @@ TI_API long long ti_linear_scan_scratch_floats(int num_seqs, int num_tokens, int
     return stretches > 1 ? (long long)num_seqs * stretches * heads * dk * (dv + 1) + (long long)num_tokens * heads * dk : 0;
 }
 
+// Whether ti_linear_scan takes these operands `chunked` (scratch on a 16-byte boundary).
+TI_API int ti_linear_scan_chunks_ok(const void* q, int ld_q, int q_off, const void* k, int ld_k, int k_off, const void* v, int ld_v, int v_off,
+                                    int dk, int dv, int dtype) {
+    return lc_takes(q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, nullptr, dk, dv, dtype == TI_F32 ? 4 : 2) ? 1 : 0;
+}
+
+// chunked: `stretches` chunks of 64 tokens hold every request's tokens (a request with more sets *status), gate per head.
 // gate_mode 0: `gate` holds the decays themselves. Otherwise they are made first, into `gate_out` (float32, as many
 // entries as the gate has per step: num_tokens x heads (x dk if per channel); gate mode 2 needs as many again behind
 // them for the keys' factors).
@@ -333,7 +348,7 @@ TI_API int ti_linear_scan(float* y, float* state, long long slot_stride, const v
                           int gate_off, int gate_mode, int gate_per_channel, float tau, const float* a_log,
                           const float* dt_bias, const float* skip, float q_scale, const int* cu_seqlens,
                           const int* state_slots, int num_seqs, int num_tokens, int heads, int groups, int dk, int dv,
-                          int stretches, float* scratch, long long scratch_floats, float* gate_out, int dtype,
+                          int stretches, float* scratch, long long scratch_floats, float* gate_out, int chunked, int* status, int dtype,
                           cudaStream_t stream) {
     TI_REQUIRE(num_seqs >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dk > 0 && dv > 0, "linear_scan: bad sizes");
     TI_REQUIRE(dk <= 1024, "linear_scan: %d key channels a head (at most 1024)", dk);
@@ -361,6 +376,22 @@ TI_API int ti_linear_scan(float* y, float* state, long long slot_stride, const v
         ld_decay = heads * per_head;
         decay_off = 0;
         if (gate_mode == LS_GATE_STEP) kscale = gate_out + n;
+    }
+    if (chunked) {
+        TI_REQUIRE(!gate_per_channel && stretches > 1 && lc_takes(q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, scratch, dk, dv, dtype == TI_F32 ? 4 : 2),
+                   "linear_scan: operands that the chunked form does not take");
+        float* part_a = scratch + (long long)num_seqs * stretches * heads * dk * dv;
+        const int fold = heads * dv * dk;
+        for (int part = 0; part < 2; ++part) {
+            const int rc = lc_launch(part, y, q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, decay, ld_decay, decay_off, kscale, skip, q_scale,
+                                     cu_seqlens, num_seqs, heads, groups, dk, dv, stretches, scratch, part_a, status, dtype, stream);
+            if (rc) return rc;
+            if (part) break;
+            ti_launch(linear_scan_fold_kernel, dim3((fold + 255) / 256, num_seqs), 256, 0, stream, state, slot_stride, scratch,
+                      (const float*)part_a, state_slots, stretches, heads, dk, dv);
+            TI_CHECK_LAUNCH("linear_scan (fold)");
+        }
+        return 0;
     }
     // rows of a column over KP lanes, KPT rows a lane: the fewest lanes that keep a lane's share at 16 rows or fewer
     int kp = 1;
