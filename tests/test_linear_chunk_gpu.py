@@ -60,3 +60,29 @@ def test_chunks_against_plain(monkeypatch, heads, groups, dk, dv, gate, lens, dt
         err, err_walk = ((u - z).norm() / z.norm() for u in (x, y))
         assert torch.isfinite(x).all() and err <= 2e-6 and err <= 1.5 * err_walk + 1e-7, (err, err_walk)
     assert torch.equal(state[0], start[0].double())
+
+
+def test_chunks_hold_any_division_and_look_at_no_later_token():
+    """``max_q_len`` is a hint: one too small gives the same outputs. And a value that is no number reaches no token before its own."""
+    from tinyinfer_b200 import ops
+    lens, heads, dk = [3, 700, 1, 66], 2, 64
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32).cuda()
+    gen = torch.Generator().manual_seed(7)
+    row = torch.randn(sum(lens), 3 * heads * dk, generator=gen).cuda()
+    decay = ops.ScanGate("constant", torch.tensor([[0.9, 0.99]]).cuda(), per_channel=False)
+
+    def run(rows, longest):
+        state = torch.zeros(len(lens), heads, dk, dk, device="cuda")
+        out = ops.linear_scan(rows, rows, rows, decay, state=state, heads=heads, groups=heads, key_dim=dk, value_dim=dk, k_offset=heads * dk,
+                              v_offset=2 * heads * dk, cu_seqlens=cu, state_slots=torch.arange(len(lens), dtype=torch.int32).cuda(),
+                              num_seqs=len(lens), max_q_len=longest)
+        return out, state
+
+    out, state = run(row, 700)
+    again, state_again = run(row, 128)
+    assert torch.equal(out, again) and torch.equal(state, state_again)
+    for at in (3 + 77, 3 + 64, 3 + 127):
+        spoiled = row.clone()
+        spoiled[at, 2 * heads * dk:] = float("nan")
+        got, _ = run(spoiled, 700)
+        assert torch.equal(got[:at], out[:at]) and got[at:703].isnan().all() and torch.equal(got[703:], out[703:])

@@ -37,7 +37,7 @@ bool lc_takes(const void* q, int ld_q, int q_off, const void* k, int ld_k, int k
               int dk, int dv, int esize);
 int lc_launch(int part, float* y, const void* q, int ld_q, int q_off, const void* k, int ld_k, int k_off, const void* v, int ld_v, int v_off,
               const float* decay, int ld_decay, int decay_off, const float* kscale, const float* skip, float q_scale, const int* cu_seqlens,
-              int num_seqs, int heads, int groups, int dk, int dv, int chunks, float* part_b, float* part_a, int* status, int dtype,
+              int num_seqs, int heads, int groups, int dk, int dv, int chunks, float* part_b, float* part_a, int dtype,
               cudaStream_t stream);
 
 enum { LS_GATE_RAW = 0, LS_GATE_SIGMOID_POW = 1, LS_GATE_STEP = 2 };
@@ -278,30 +278,36 @@ __global__ void __launch_bounds__(LS_WARPS * 32, KPT <= 16 ? 7 : 1) linear_scan_
 }
 
 // A request's stretches in order: S <- A S + B. Each stretch's B becomes the state it starts from; the slot gets
-// the state after the last. One thread per element of a request's states.
+// the state after the last. One thread per element of a request's states. cu_seqlens null: `stretches` a request; else
+// chunks of 64 tokens, laid out as linear_chunk.cu says.
 __global__ void linear_scan_fold_kernel(float* __restrict__ state, long long slot_stride, float* __restrict__ part_b,
                                         const float* __restrict__ part_a, const int* __restrict__ state_slots,
-                                        int stretches, int heads, int dk, int dv) {
+                                        const int* __restrict__ cu_seqlens, int stretches, int heads, int dk, int dv) {
     ti_grid_launch_dependents();
     ti_grid_wait();
     const int per = heads * dv * dk;
     const int e = blockIdx.x * blockDim.x + threadIdx.x, seq = blockIdx.y;
     if (e >= per) return;
     const int idx = e % dk, h = e / (dv * dk);
+    size_t first = (size_t)seq * stretches;
+    if (cu_seqlens) {
+        first = cu_seqlens[seq] / 64 + seq;
+        stretches = (cu_seqlens[seq + 1] - cu_seqlens[seq] + 63) / 64;
+    }
     float* slot = state + (size_t)state_slots[seq] * slot_stride;
     float S = slot[e];
     for (int k0 = 0; k0 < stretches; k0 += 8) {          // eight stretches' loads in flight at once
         float b[8], a[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            const size_t part = (size_t)seq * stretches + min(k0 + j, stretches - 1);
+            const size_t part = first + min(k0 + j, stretches - 1);
             b[j] = part_b[part * per + e];
             a[j] = part_a[(part * heads + h) * dk + idx];
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             if (k0 + j < stretches) {
-                part_b[((size_t)seq * stretches + k0 + j) * per + e] = S;
+                part_b[(first + k0 + j) * per + e] = S;
                 S = fmaf(a[j], S, b[j]);
             }
         }
@@ -339,7 +345,8 @@ TI_API int ti_linear_scan_chunks_ok(const void* q, int ld_q, int q_off, const vo
     return lc_takes(q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, nullptr, dk, dv, dtype == TI_F32 ? 4 : 2) ? 1 : 0;
 }
 
-// chunked: `stretches` chunks of 64 tokens hold every request's tokens (a request with more sets *status), gate per head.
+// chunks (gate per head): 0, or num_tokens / 64 + num_seqs: the form of linear_chunk.cu, whose scratch holds dk * (dv + 1) floats
+// a chunk and head on a 16-byte boundary; `stretches` is not used then.
 // gate_mode 0: `gate` holds the decays themselves. Otherwise they are made first, into `gate_out` (float32, as many
 // entries as the gate has per step: num_tokens x heads (x dk if per channel); gate mode 2 needs as many again behind
 // them for the keys' factors).
@@ -348,7 +355,7 @@ TI_API int ti_linear_scan(float* y, float* state, long long slot_stride, const v
                           int gate_off, int gate_mode, int gate_per_channel, float tau, const float* a_log,
                           const float* dt_bias, const float* skip, float q_scale, const int* cu_seqlens,
                           const int* state_slots, int num_seqs, int num_tokens, int heads, int groups, int dk, int dv,
-                          int stretches, float* scratch, long long scratch_floats, float* gate_out, int chunked, int* status, int dtype,
+                          int stretches, float* scratch, long long scratch_floats, float* gate_out, int chunks, int dtype,
                           cudaStream_t stream) {
     TI_REQUIRE(num_seqs >= 0 && heads > 0 && groups > 0 && heads % groups == 0 && dk > 0 && dv > 0, "linear_scan: bad sizes");
     TI_REQUIRE(dk <= 1024, "linear_scan: %d key channels a head (at most 1024)", dk);
@@ -357,15 +364,15 @@ TI_API int ti_linear_scan(float* y, float* state, long long slot_stride, const v
     TI_REQUIRE(gate_mode != LS_GATE_SIGMOID_POW || tau > 0.f, "linear_scan: tau must be positive");
     TI_REQUIRE(num_seqs <= 65535, "linear_scan: too many requests");
     TI_REQUIRE(stretches >= 1 && stretches <= 1024, "linear_scan: %d stretches", stretches);
-    TI_REQUIRE(stretches == 1 || (scratch && scratch_floats >= ti_linear_scan_scratch_floats(num_seqs, num_tokens, heads, dk, dv, stretches)),
+    TI_REQUIRE(chunks || stretches == 1 || (scratch && scratch_floats >= ti_linear_scan_scratch_floats(num_seqs, num_tokens, heads, dk, dv, stretches)),
                "linear_scan: %d stretches need %lld floats of scratch", stretches,
                ti_linear_scan_scratch_floats(num_seqs, num_tokens, heads, dk, dv, stretches));
-    TI_REQUIRE(gate_mode == LS_GATE_RAW || stretches == 1 || gate_out, "linear_scan: the decays need a place to be made in");
+    TI_REQUIRE(gate_mode == LS_GATE_RAW || (!chunks && stretches == 1) || gate_out, "linear_scan: the decays need a place to be made in");
     if (num_seqs == 0 || num_tokens == 0) return 0;
     const float* decay = gate;
     const float* kscale = nullptr;
     int ld_decay = ld_gate, decay_off = gate_off;
-    const bool gate_apart = gate_mode != LS_GATE_RAW && stretches > 1;      // long portions: the decays are made once
+    const bool gate_apart = gate_mode != LS_GATE_RAW && (chunks || stretches > 1);      // long portions: the decays are made once
     if (gate_apart) {
         const int per_head = gate_per_channel ? dk : 1;
         const size_t n = (size_t)num_tokens * heads * per_head;
@@ -377,18 +384,20 @@ TI_API int ti_linear_scan(float* y, float* state, long long slot_stride, const v
         decay_off = 0;
         if (gate_mode == LS_GATE_STEP) kscale = gate_out + n;
     }
-    if (chunked) {
-        TI_REQUIRE(!gate_per_channel && stretches > 1 && lc_takes(q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, scratch, dk, dv, dtype == TI_F32 ? 4 : 2),
+    if (chunks) {
+        TI_REQUIRE(!gate_per_channel && chunks == num_tokens / 64 + num_seqs && chunks <= 65535, "linear_scan: %d chunks", chunks);
+        TI_REQUIRE(scratch && scratch_floats >= (long long)chunks * heads * dk * (dv + 1), "linear_scan: scratch of %d chunks", chunks);
+        TI_REQUIRE(lc_takes(q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, scratch, dk, dv, dtype == TI_F32 ? 4 : 2),
                    "linear_scan: operands that the chunked form does not take");
-        float* part_a = scratch + (long long)num_seqs * stretches * heads * dk * dv;
+        float* part_a = scratch + (long long)chunks * heads * dk * dv;
         const int fold = heads * dv * dk;
         for (int part = 0; part < 2; ++part) {
             const int rc = lc_launch(part, y, q, ld_q, q_off, k, ld_k, k_off, v, ld_v, v_off, decay, ld_decay, decay_off, kscale, skip, q_scale,
-                                     cu_seqlens, num_seqs, heads, groups, dk, dv, stretches, scratch, part_a, status, dtype, stream);
+                                     cu_seqlens, num_seqs, heads, groups, dk, dv, chunks, scratch, part_a, dtype, stream);
             if (rc) return rc;
             if (part) break;
             ti_launch(linear_scan_fold_kernel, dim3((fold + 255) / 256, num_seqs), 256, 0, stream, state, slot_stride, scratch,
-                      (const float*)part_a, state_slots, stretches, heads, dk, dv);
+                      (const float*)part_a, state_slots, cu_seqlens, 0, heads, dk, dv);
             TI_CHECK_LAUNCH("linear_scan (fold)");
         }
         return 0;
@@ -433,7 +442,7 @@ TI_API int ti_linear_scan(float* y, float* state, long long slot_stride, const v
     TI_CHECK_LAUNCH("linear_scan (stretches from zero)");
     const int per = heads * dv * dk;
     ti_launch(linear_scan_fold_kernel, dim3((per + 255) / 256, num_seqs), 256, 0, stream, state, slot_stride, a.part_b,
-              (const float*)a.part_a, state_slots, stretches, heads, dk, dv);
+              (const float*)a.part_a, state_slots, (const int*)nullptr, stretches, heads, dk, dv);
     TI_CHECK_LAUNCH("linear_scan (fold)");
     TI_SCAN_PASS(2);
     TI_CHECK_LAUNCH("linear_scan (what the stretches' starts give)");

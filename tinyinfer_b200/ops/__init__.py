@@ -135,7 +135,7 @@ _SIGNATURES = {
                               c_int, c_float, c_float, c_int, c_float, c_float, c_void_p, c_int, c_void_p],
         "ti_linear_scan": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                            c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
-                           c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_int, c_void_p],
+                           c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p],
         "ti_linear_scan_chunks_ok": [c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int],
         "ti_linear_scan_scratch_floats": [c_int, c_int, c_int, c_int, c_int, c_int],
         "ti_gated_group_norm": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float,
@@ -1879,7 +1879,7 @@ class ScanGate:
 SCAN_MIN_STRETCH = 32        # tokens a stretch of a long portion has at least
 SCAN_CHUNK = 64              # tokens of a chunk where a head has one decay
 LINEAR_CHUNKS = True
-SCAN_CHUNK_MIN_TOKENS = 128
+SCAN_CHUNK_MIN_TOKENS = 128  # 16 heads of 128 x 128, host included: 75 us in stretches, 48 in chunks; 64 tokens 64 in stretches, where chunks were not tried
 SCAN_CHUNK_MAX_FLOATS = 64 * 1024 * 1024     # states of the chunks: 256 MB
 SCAN_TARGET_BLOCKS = 148 * 7  # what runs side by side at 72 registers a thread: more blocks would wait for a second round
 
@@ -1904,9 +1904,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: ScanGat
     (+ skip[h] * v), from and back into ``state`` float32 [slots, heads, value_dim, key_dim] (S transposed).
     q and k: columns [offset, + groups * key_dim) of their tensors (head h reads group h // (heads / groups));
     v: columns [offset, + heads * value_dim). Returns o float32 [T, heads * value_dim]. ``max_q_len`` (a host
-    number: the most tokens a request brings, 0: unknown) decides into how many stretches long portions are cut
-    to run side by side, or, with one decay a head, how many chunks of 64 tokens hold a request (a request with more
-    sets the status word)."""
+    number: the most tokens a request brings, 0: unknown) only decides into how many stretches long portions are cut
+    to run side by side, and whether they run in chunks of 64 tokens as matrix products (one decay a head)."""
     for name, ten in (("q", q), ("k", k), ("v", v)):
         _check(ten, name, q.dtype, 2)
     _check(gate.values, "gate", torch.float32, 2)
@@ -1929,20 +1928,20 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: ScanGat
         return out
     longest = t if num_seqs == 1 else max_q_len
     stretches, scratch = scan_stretches(max_q_len or t, num_seqs, heads, key_dim, value_dim), None
-    chunks = -(-longest // SCAN_CHUNK)
+    chunks = t // SCAN_CHUNK + num_seqs
     chunked = (LINEAR_CHUNKS and not gate.per_channel and longest >= SCAN_CHUNK_MIN_TOKENS
-               and num_seqs * chunks * heads * key_dim * value_dim <= SCAN_CHUNK_MAX_FLOATS and chunks <= 1024
+               and chunks * heads * key_dim * value_dim <= SCAN_CHUNK_MAX_FLOATS and chunks <= 65535
                and int(_fn("hybrid", "ti_linear_scan_chunks_ok")(
                    q.data_ptr(), q.shape[1], q_offset, k.data_ptr(), k.shape[1], k_offset, v.data_ptr(), v.shape[1], v_offset,
                    key_dim, value_dim, _dtype_code(q))))
     if chunked:
-        stretches = chunks
-    if stretches > 1:
+        scratch = torch.empty(chunks * heads * key_dim * (value_dim + 1), dtype=torch.float32, device=q.device)
+    elif stretches > 1:
         fn = _fn("hybrid", "ti_linear_scan_scratch_floats")
         fn.restype = ctypes.c_longlong
         scratch = torch.empty(int(fn(num_seqs, t, heads, key_dim, value_dim, stretches)), dtype=torch.float32, device=q.device)
     made = None          # the decays (and the keys' factors) as the scan reads them, unless the gate holds them already
-    if gate.kind not in ("raw", "constant") and stretches > 1:
+    if gate.kind not in ("raw", "constant") and (chunked or stretches > 1):
         made = torch.empty(t * heads * (key_dim if gate.per_channel else 1) * (2 if gate.kind == "step_size" else 1),
                            dtype=torch.float32, device=q.device)
     _run("hybrid", "ti_linear_scan", out.data_ptr(), state.data_ptr(), stride, q.data_ptr(), q.shape[1], q_offset,
@@ -1950,7 +1949,7 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: ScanGat
          0 if constant else gate.values.shape[1], gate.offset, ScanGate.KINDS[gate.kind], int(gate.per_channel), float(gate.tau),
          _ptr(gate.a_log), _ptr(gate.dt_bias), _ptr(skip), float(q_scale), cu_seqlens.data_ptr(), state_slots.data_ptr(),
          num_seqs, t, heads, groups, key_dim, value_dim, stretches, _ptr(scratch),
-         scratch.numel() if scratch is not None else 0, _ptr(made), int(chunked), page_status(q.device).data_ptr(), _dtype_code(q), _stream())
+         scratch.numel() if scratch is not None else 0, _ptr(made), chunks if chunked else 0, _dtype_code(q), _stream())
     return out
 
 
