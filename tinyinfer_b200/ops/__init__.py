@@ -106,6 +106,10 @@ _SIGNATURES = {
         "ti_delta_scan": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
                           c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p,
                           c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_int, c_void_p],
+        "ti_delta_quads": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_int,
+                          c_void_p, c_int, c_int, c_void_p, c_int, c_int, c_void_p, c_void_p, c_float, c_float, c_void_p,
+                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_ll, c_void_p, c_int, c_void_p],
+        "ti_delta_quads_floats": [c_int, c_int, c_int, c_int, c_int],
         "ti_streams_step": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_int,
                             c_int, c_int, c_int, c_int, c_int, c_void_p, c_float, c_void_p],
         "ti_stream_enter": [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p,
@@ -2009,6 +2013,9 @@ def head_rotation(rows: torch.Tensor, *, num_heads: int, num_kv_heads: int, head
     return out if to_row else out.view(t, num_heads, maps * head_dim)
 
 
+DELTA_QUADS = True           # long portions four tokens at a time
+
+
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logits: torch.Tensor, beta_logits: torch.Tensor,
                *, a_log: torch.Tensor, dt_bias: Optional[torch.Tensor], state: torch.Tensor, heads: int, groups: int,
                key_dim: int, value_dim: int, q_offset: int = 0, k_offset: int = 0, v_offset: int = 0,
@@ -2038,14 +2045,21 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logits: 
     stride = _slot_stride(state, heads * value_dim * key_dim, "state")
     out = torch.empty((t, heads * value_dim), dtype=torch.float32, device=q.device)
     if t:
-        # what the recurrence reads of every token, made once: unit q and k, the decays, v, beta and k.q, float32
-        work = torch.empty(t * (2 * groups * key_dim + heads * (key_dim + value_dim + 1) + groups) + 24,
+        # what the recurrence reads of every token, made once, float32: unit q and k, the decays, v, beta and k.q
+        fn = _fn("hybrid", "ti_delta_quads_floats")
+        fn.restype = ctypes.c_longlong
+        quads = int(fn(int(num_seqs), t, heads, key_dim, value_dim)) if DELTA_QUADS else 0
+        work = torch.empty(quads or t * (2 * groups * key_dim + heads * (key_dim + value_dim + 1) + groups) + 24,
                            dtype=torch.float32, device=q.device)
-        _run("hybrid", "ti_delta_scan", out.data_ptr(), state.data_ptr(), stride, q.data_ptr(), q.shape[1], int(q_offset),
-             k.data_ptr(), k.shape[1], int(k_offset), v.data_ptr(), v.shape[1], int(v_offset), decay_logits.data_ptr(),
-             decay_logits.shape[1], int(decay_offset), beta_logits.data_ptr(), beta_logits.shape[1], int(beta_offset),
-             a_log.data_ptr(), _ptr(dt_bias), float(q_scale), float(unit_eps), cu_seqlens.data_ptr(), state_slots.data_ptr(),
-             int(num_seqs), t, heads, groups, key_dim, value_dim, work.data_ptr(), work.numel(), _dtype_code(q), _stream())
+        args = [out.data_ptr(), state.data_ptr(), stride, q.data_ptr(), q.shape[1], int(q_offset),
+                k.data_ptr(), k.shape[1], int(k_offset), v.data_ptr(), v.shape[1], int(v_offset), decay_logits.data_ptr(),
+                decay_logits.shape[1], int(decay_offset), beta_logits.data_ptr(), beta_logits.shape[1], int(beta_offset),
+                a_log.data_ptr(), _ptr(dt_bias), float(q_scale), float(unit_eps), cu_seqlens.data_ptr(), state_slots.data_ptr(),
+                int(num_seqs), t, heads, groups, key_dim, value_dim, work.data_ptr(), work.numel()]
+        if quads:
+            _run("hybrid", "ti_delta_quads", *args, kernel_status(q.device).data_ptr(), _dtype_code(q), _stream())
+        else:
+            _run("hybrid", "ti_delta_scan", *args, _dtype_code(q), _stream())
     return out
 
 
