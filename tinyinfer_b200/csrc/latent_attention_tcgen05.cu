@@ -2,12 +2,16 @@
 // cores, bfloat16. The 128 accumulator lanes are (token, head) rows (8 tokens of 16 heads): every head reads the same cached
 // rows [c | k_rot], so one tile of cached rows serves as keys (all features) and as values (the first `rank`).
 //
-//   warp 0      TMA: tiles of 32 cached rows through the block table, 64 features a copy, into a ring of two
-//   warp 1      one thread issues S = Q K^T (128 x 32, two buffers in tensor memory) and O += P V, P from tensor memory, V the
+//   warp 0      TMA: tiles of 32 cached rows through the block table, 64 features a copy, into a ring of four
+//   warp 1      issues S = Q K^T (128 x 32, two buffers in tensor memory) and O += P V, P from tensor memory, V the
 //               first features of the same shared-memory tile read as an MN-major operand
-//   warps 2..9  the rows, rounded to bfloat16, into shared memory; then the softmax: two threads a row, each 16 of a tile's keys and
+//   warps 2..9  the rows, rounded to bfloat16, into shared and tensor memory; then the softmax: two threads a row, each 16 of a tile's keys and
 //               half of O's columns. O stays in tensor memory and is multiplied there when a row of the warp has a new maximum.
 //
+// The rows' last features, up to 320 of them, are read by the MMAs from tensor memory: with all 576 in shared memory it would hold a
+// ring of two tiles alone, each refilled only when its products with P are through. 2,048 tokens over 16 heads of rank 512, a
+// layer: 420 us with a ring of two, 354 with four, 285 with the MMAs issued from uniform registers as well (see elect_one); of
+// these 110 are the CTAs' beginnings and ends, mostly the rows' way from float32 in memory, the rest the softmax's chain of a tile.
 // O of 512 value features would fill tensor memory and leave no room for scores: above 256 a row tile goes to two CTAs, which
 // both make the scores and take half of the value features each.
 // The products, their operands' roundings and the softmax's steps of 32 keys are those of the warp-level form
@@ -15,10 +19,12 @@
 // running maximum after its own 32 keys. So the two forms differ by the order of float32 sums alone; larger tiles would round
 // every probability anew, and a model with routers turns that into other choices of experts near a tie.
 #include "sm100_ptx.cuh"
+#include <algorithm>
 
 namespace lt {
-constexpr int QM = 128, KT = 32, STAGES = 2, THREADS = 320;
-constexpr int S_COL = 256, P_COL = S_COL + 2 * KT, TMEM_COLS = 512;
+constexpr int QM = 128, KT = 32, STAGES = 4, THREADS = 320, SOFTMAX_THREADS = 256;
+constexpr int S_COL = 256, P_COL = S_COL + 2 * KT, Q_COL = P_COL + KT, TMEM_COLS = 512;
+constexpr int MAX_TMEM_CHUNKS = (TMEM_COLS - Q_COL) / 32;             // 64 features: 32 columns
 
 struct Args {
     __nv_bfloat16* out;
@@ -29,6 +35,7 @@ struct Args {
     int max_blocks, num_seqs, heads, rank, rot, page_size, num_pages, piece_rows;
     float scale;
     int splits, tpb, hpb, chunks, value_halves;
+    int smem_chunks;                                              // of the rows' features in shared memory, the others in tensor memory
     int* status;                                                  // [0] a wait that ran out, [1] a key without a page
 };
 
@@ -57,7 +64,9 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
-int smem_bytes(int chunks) { return 1024 + chunks * (QM * 128) + STAGES * chunks * (KT * 128) + 128; }
+// The rows' chunks on their way to tensor memory wait in the ring behind its first tile.
+int tmem_chunks(int chunks) { return std::min(MAX_TMEM_CHUNKS, (STAGES - 1) * chunks * KT / QM); }
+int smem_bytes(int chunks) { return 1024 + (chunks - tmem_chunks(chunks)) * (QM * 128) + STAGES * chunks * (KT * 128) + 128; }
 
 // NV: value features of a CTA.
 template <int NV>
@@ -65,14 +74,14 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_tile = smem;                                       // [chunk of 64 features][row][128 bytes, swizzled]
-    uint8_t* ring = smem + a.chunks * (QM * 128);                 // [stage][chunk][key][128 bytes, swizzled]
+    uint8_t* ring = smem + a.smem_chunks * (QM * 128);            // [stage][chunk][key][128 bytes, swizzled]
     const int stage_bytes = a.chunks * (KT * 128);
     const uint32_t bar0 = smem_u32(ring + STAGES * stage_bytes);
-    const uint32_t q_full = bar0, p_full = bar0 + 8u * 9, o_full = bar0 + 8u * 10;
-    auto kv_full = [&](int s) { return bar0 + 8u * (1 + s); };
-    auto kv_empty = [&](int s) { return bar0 + 8u * (3 + s); };
-    auto s_full = [&](int b) { return bar0 + 8u * (5 + b); };
-    auto s_empty = [&](int b) { return bar0 + 8u * (7 + b); };
+    const uint32_t q_full = bar0, p_full = bar0 + 8u, o_full = bar0 + 16u;
+    auto s_full = [&](int b) { return bar0 + 8u * (3 + b); };
+    auto s_empty = [&](int b) { return bar0 + 8u * (5 + b); };
+    auto kv_full = [&](int s) { return bar0 + 8u * (7 + s); };
+    auto kv_empty = [&](int s) { return bar0 + 8u * (7 + STAGES + s); };
     __shared__ uint32_t tmem_base_sh;
     __shared__ float sum_xch[2][QM];
     __shared__ int abort_sh, tile_sh[3];
@@ -83,12 +92,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     if (threadIdx.x == 0) {
         abort_sh = 0;
         mbar_init(q_full, 8);
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(kv_full(s), 1);
-            mbar_init(kv_empty(s), 1);
-            mbar_init(s_full(s), 1);
-            mbar_init(s_empty(s), 8);
-        }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(s_full(b), 1); mbar_init(s_empty(b), 8); }
         mbar_init(p_full, 8);
         mbar_init(o_full, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -149,6 +154,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             int go = 1;
             if (lane == 0) {
                 go = mbar_wait(kv_empty(s), ((j / STAGES) & 1u) ^ 1u, abort_flag, a.status, 81) ? 1 : 0;
+                if (j == 1 && go) go = mbar_wait(q_full, 0, abort_flag, a.status, 82) ? 1 : 0;      // the rows' chunks have left the ring
                 if (go) mbar_expect_tx(kv_full(s), (uint32_t)stage_bytes);
             }
             if (!__shfl_sync(0xffffffffu, go, 0)) break;
@@ -164,42 +170,44 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0 && num_tiles > 0) {
+        if (num_tiles > 0) {
+            const bool leader = elect_one();
             constexpr uint32_t idesc_s = make_idesc(QM, KT), idesc_o = make_idesc(QM, NV, true);
             const uint64_t q_desc = make_sw128_desc(smem_u32(q_tile));
-            uint64_t k_desc[STAGES], v_desc[STAGES];
-#pragma unroll
-            for (int st = 0; st < STAGES; ++st) {
-                const uint32_t at = smem_u32(ring + st * stage_bytes);
-                k_desc[st] = make_sw128_desc(at);
-                v_desc[st] = make_sw128_desc_mn(at + vhalf * (NV / 64) * (KT * 128), KT * 128, 1024);
-            }
-            const int ksteps = a.chunks * 4;
-            bool go = mbar_wait(q_full, 0, abort_flag, a.status, 82);
+            const uint64_t k_desc = make_sw128_desc(smem_u32(ring));
+            const uint64_t v_desc = make_sw128_desc_mn(smem_u32(ring) + vhalf * (NV / 64) * (KT * 128), KT * 128, 1024);
+            bool go = mbar_wait_warp(q_full, 0, abort_flag, a.status, 82);
+            tmem_fence_after();
             auto issue_s = [&](int j) {                            // scores of tile j into buffer j % 2
                 const int s = j % STAGES, b = j & 1;
-                if (!mbar_wait(kv_full(s), (j / STAGES) & 1u, abort_flag, a.status, 83)) return false;
-                if (!mbar_wait(s_empty(b), ((j >> 1) & 1u) ^ 1u, abort_flag, a.status, 84)) return false;
+                if (!mbar_wait_warp(kv_full(s), (j / STAGES) & 1u, abort_flag, a.status, 83)) return false;
+                if (!mbar_wait_warp(s_empty(b), ((j >> 1) & 1u) ^ 1u, abort_flag, a.status, 84)) return false;
                 tmem_fence_after();
-                const uint64_t kd = s == 0 ? k_desc[0] : k_desc[1];
-#pragma unroll 4
-                for (int ks = 0; ks < ksteps; ++ks)
-                    umma_bf16(tmem_base + S_COL + b * KT, q_desc + (uint64_t)(((ks >> 2) * (QM * 128) + (ks & 3) * 32) >> 4),
-                              kd + (uint64_t)(((ks >> 2) * (KT * 128) + (ks & 3) * 32) >> 4), idesc_s, ks > 0 ? 1u : 0u);
-                umma_commit(s_full(b));
+                const uint64_t kd = k_desc + (uint64_t)((s * stage_bytes) >> 4);
+                const uint32_t d = tmem_base + S_COL + b * KT;
+                uint64_t qd = q_desc, kk = kd;
+                for (int c = 0; c < a.smem_chunks; ++c, qd += (QM * 128) >> 4, kk += (KT * 128) >> 4)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (leader) umma_bf16(d, qd + 2 * k, kk + 2 * k, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
+                uint32_t qt = tmem_base + Q_COL;
+                for (int c = a.smem_chunks; c < a.chunks; ++c, qt += 32, kk += (KT * 128) >> 4)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (leader) umma_ts(d, qt + 8 * k, kk + 2 * k, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
+                if (leader) umma_commit(s_full(b));
                 return true;
             };
             if (go) go = issue_s(0);
             for (int j = 0; j < num_tiles && go; ++j) {
                 if (j + 1 < num_tiles) go = issue_s(j + 1);
-                if (!go || !mbar_wait(p_full, j & 1u, abort_flag, a.status, 85)) break;
+                if (!go || !mbar_wait_warp(p_full, j & 1u, abort_flag, a.status, 85)) break;
                 tmem_fence_after();
-                const uint64_t vd = (j & 1) == 0 ? v_desc[0] : v_desc[1];
+                const uint64_t vd = v_desc + (uint64_t)(((j % STAGES) * stage_bytes) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < KT / 16; ++ks)
-                    umma_ts(tmem_base, tmem_base + P_COL + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
-                umma_commit(o_full);
-                umma_commit(kv_empty(j % STAGES));
+                    if (leader) umma_ts(tmem_base, tmem_base + P_COL + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+                if (leader) { umma_commit(o_full); umma_commit(kv_empty(j % STAGES)); }
             }
         }
     } else {
@@ -207,7 +215,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
         const int etid = threadIdx.x - 64;
         {
             const int chunks8 = a.chunks * 8, total = QM * chunks8;
-#pragma unroll 6
+#pragma unroll 12
             for (int i = etid; i < total; i += 256) {              // 8 features: two 16-byte loads, one store
                 const int row = i / chunks8, c = i % chunks8, rt = row / a.hpb, hl = row % a.hpb;
                 uint4 w = make_uint4(0, 0, 0, 0);
@@ -216,8 +224,23 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
                     const float4 u = src[0], v = src[1];
                     w = make_uint4(pack2(u.x, u.y), pack2(u.z, u.w), pack2(v.x, v.y), pack2(v.z, v.w));
                 }
-                *reinterpret_cast<uint4*>(q_tile + (c >> 3) * (QM * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = w;
+                const int chunk = c >> 3, behind = chunk - a.smem_chunks;
+                uint8_t* dst = behind < 0 ? q_tile + chunk * (QM * 128) : ring + stage_bytes + behind * (QM * 128);
+                *reinterpret_cast<uint4*>(dst + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = w;
             }
+            asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory");
+            for (int t = 0; t < a.chunks - a.smem_chunks; ++t) {   // a thread's half of its row's chunk: 32 features, 16 columns
+                const uint8_t* src = ring + stage_bytes + t * (QM * 128) + r * 128;
+#pragma unroll
+                for (int i = 0; i < 4; i += 2) {
+                    const uint4 u = *reinterpret_cast<const uint4*>(src + (((half * 4 + i) ^ (r & 7)) << 4));
+                    const uint4 w = *reinterpret_cast<const uint4*>(src + (((half * 4 + i + 1) ^ (r & 7)) << 4));
+                    const uint32_t words[8] = {u.x, u.y, u.z, u.w, w.x, w.y, w.z, w.w};
+                    tmem_st8(lane_addr + Q_COL + t * 32 + half * 16 + i * 4, words);
+                }
+            }
+            tmem_wait_st();
+            tmem_fence_before();
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(q_full);
@@ -374,6 +397,7 @@ TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, 
     a.hpb = heads < lt::QM ? heads : lt::QM;
     a.tpb = lt::QM / a.hpb;
     a.chunks = (rank + rot + 63) / 64;
+    a.smem_chunks = a.chunks - lt::tmem_chunks(a.chunks);
     a.value_halves = rank > 256 ? 2 : 1;
     a.piece_rows = page_size % 32 == 0 ? 32 : 16;
     CUtensorMap map;

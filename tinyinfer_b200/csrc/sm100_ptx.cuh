@@ -87,6 +87,19 @@ __device__ __forceinline__ uint64_t make_sw128_desc_mn(uint32_t smem_addr, uint3
     d |= (uint64_t)2 << 61;
     return d;
 }
+// One lane of a converged warp. A warp whose lanes all walk the loop that issues MMAs, this one alone issuing, keeps addresses and
+// descriptors in uniform registers, and an MMA takes some 20 cycles to issue; under `if (lane == 0)` they are moved there for each, and
+// it takes 60 to 75 (128 x 32 x 16, from products left out one by one): as long as 128 x 256 x 16 multiply-adds.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(one));
+    return one != 0;
+}
+// Bounded wait of a converged warp, which stays together: all its lanes get the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
+__device__ __forceinline__ bool mbar_test_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)); }
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}"
