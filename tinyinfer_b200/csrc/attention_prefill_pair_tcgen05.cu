@@ -248,10 +248,11 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             constexpr uint32_t idesc_s = make_idesc(QM, KT);               // S = Q K^T: both operands K-major
             constexpr uint32_t idesc_o = make_idesc(QM, D, true);          // O = P V: V is MN-major (features contiguous)
-            bool ok = mbar_wait(q_full, 0, abort_flag, p.status, 42);
+            bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.status, 42);
             int js[2] = {0, 0}, jp[2] = {0, 0};                            // next S and next P V to issue: query tile X's js[X]-th, jp[X]-th
             uint32_t spins = 0;
             unsigned long long idle_since = 0;
@@ -264,8 +265,8 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                 const int a = place_of(0, v), b = place_of(1, v);
                 return (a < 0 || next[0] > a) && (b < 0 || next[1] > b);
             };
-            // This one thread's instructions are what the tensor cores wait for between products (a descriptor made
-            // from an address costs it as much as the MMA it describes costs the tensor pipe), so the descriptors
+            // The issuing warp's instructions are what the tensor cores wait for between products (a descriptor made
+            // from an address costs as much as the MMA it describes costs the tensor pipe), so the descriptors
             // of the two query tiles and of the four key/value buffers are made once: a k step then is an addition.
             const uint64_t q_desc[2] = {make_sw128_desc(smem_u32(q_tiles)), make_sw128_desc(smem_u32(q_tiles) + S::Q_BYTES)};
             uint64_t k_desc[NBUF], v_desc[NBUF];
@@ -282,19 +283,19 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                     const uint32_t s_tmem = tmem_base + x * KT, o_tmem = tmem_base + 2 * KT + x * D;
                     if (jp[x] < js[x]) {                                   // P V of tile jp: P written, V landed
                         const int v = number_of(x, jp[x]), li = 2 * v + 1, b = li % NBUF;
-                        if (mbar_test_wait(p_full(x), jp[x] & 1u) && mbar_test_wait(kv_full(b), (li / NBUF) & 1u)) {
+                        if (mbar_test_wait_warp(p_full(x), jp[x] & 1u) && mbar_test_wait_warp(kv_full(b), (li / NBUF) & 1u)) {
                             tmem_fence_after();
                             const uint64_t vd = pick(v_desc, b);
                             // A: 16 keys = 8 columns of packed bfloat16 pairs (P lies over the first 64 of the
                             // tile's 128 score columns); B: 16 key rows of V = 2048 bytes further on (128 in the
                             // descriptor's 16-byte units)
-                            umma_bf16_tmem_a(o_tmem, s_tmem, vd, idesc_o, jp[x] > 0 ? 1u : 0u);
+                            if (leader) umma_bf16_tmem_a(o_tmem, s_tmem, vd, idesc_o, jp[x] > 0 ? 1u : 0u);
 #pragma unroll
                             for (int ks = 1; ks < KT / 16; ++ks)
-                                umma_bf16_tmem_a(o_tmem, s_tmem + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, 1u);
-                            umma_commit(o_full(x));
+                                if (leader) umma_bf16_tmem_a(o_tmem, s_tmem + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, 1u);
+                            if (leader) umma_commit(o_full(x));
                             ++jp[x];
-                            if (all_issued(jp, v)) umma_commit(kv_empty(b));   // both tiles have read these values
+                            if (all_issued(jp, v) && leader) umma_commit(kv_empty(b));   // both tiles have read these values
                             moved = true;
                         }
                     }
@@ -305,7 +306,7 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                     if (js[x] < count[x] && js[x] == jp[x] &&
                         (x == 0 || js[1] >= (FORM != 0 && js[1] < own_kept[1] ? 2 : own_kept[1] + 2) || jp[0] + 1 >= number_of(1, js[1]))) {
                         const int v = number_of(x, js[x]), li = 2 * v, b = li % NBUF;
-                        if (mbar_test_wait(kv_full(b), (li / NBUF) & 1u)) {
+                        if (mbar_test_wait_warp(kv_full(b), (li / NBUF) & 1u)) {
                             tmem_fence_after();
                             const uint64_t kd = pick(k_desc, b), qd = q_desc[FORM == 2 ? 0 : x];
 #pragma unroll
@@ -313,11 +314,11 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                                 // half of the head, then 32 bytes a step: in the descriptor's 16-byte units
                                 const int kstep = FORM == 2 ? x * (D / 32) + ks : ks;      // map x's share of the features
                                 const uint64_t off = (uint64_t)(((kstep >> 2) * (QM * 128) + (kstep & 3) * 32) >> 4);
-                                umma_bf16(s_tmem, qd + off, kd + off, idesc_s, ks > 0 ? 1u : 0u);
+                                if (leader) umma_bf16(s_tmem, qd + off, kd + off, idesc_s, ks > 0 ? 1u : 0u);
                             }
-                            umma_commit(s_full(x));
+                            if (leader) umma_commit(s_full(x));
                             ++js[x];
-                            if (all_issued(js, v)) umma_commit(kv_empty(b));   // both tiles have read these keys
+                            if (all_issued(js, v) && leader) umma_commit(kv_empty(b));   // both tiles have read these keys
                             moved = true;
                         }
                     }
@@ -325,12 +326,12 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                 if (moved) { spins = 0; idle_since = 0; continue; }
                 if ((++spins & 1023u) == 0u) {
                     if (idle_since == 0) idle_since = global_ns();
-                    if (*abort_flag) ok = false;
-                    else if (global_ns() - idle_since > TI_WAIT_NS) {
+                    const bool late = global_ns() - idle_since > TI_WAIT_NS;
+                    if (late && !*abort_flag) {
                         *abort_flag = 1;
                         if (p.status) atomicExch(p.status, 43);
-                        ok = false;
                     }
+                    ok = !__any_sync(0xffffffffu, late || *abort_flag);
                 }
             }
         }

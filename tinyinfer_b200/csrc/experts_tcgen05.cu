@@ -123,29 +123,30 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             constexpr uint32_t idesc = make_idesc(GT_BM, GT_BN);
             uint32_t it = 0, unit_i = 0;
             bool ok = true;
             for (int unit = blockIdx.x; ok && unit < num_units; unit += gridDim.x, ++unit_i) {
                 const uint32_t as = unit_i & 1u, aph = (unit_i >> 1) & 1u;
-                if (!mbar_wait(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
+                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
                 tmem_fence_after();
                 const uint32_t d_tmem = tmem_base + as * GT_BN;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % GT_STAGES;
                     const uint32_t ph = (it / GT_STAGES) & 1u;
-                    if (!mbar_wait(full_bar(s), ph, abort_flag, p.status, 33)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), ph, abort_flag, p.status, 33)) { ok = false; break; }
                     tmem_fence_after();
                     const uint32_t a_addr = smem_u32(stages + s * GT_STAGE_BYTES);
                     const uint64_t adesc = make_sw128_desc(a_addr);
                     const uint64_t bdesc = make_sw128_desc(a_addr + GT_BM * GT_BK * 2);
 #pragma unroll
                     for (int k = 0; k < GT_BK / GT_UMMA_K; ++k)
-                        umma_bf16(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(empty_bar(s));
+                        if (leader) umma_bf16(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    if (leader) umma_commit(empty_bar(s));
                 }
-                if (ok) umma_commit(acc_full_bar(as));
+                if (ok && leader) umma_commit(acc_full_bar(as));
             }
         }
     } else {
@@ -242,26 +243,27 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const bool leader = elect_one();
             constexpr uint32_t idesc = make_idesc(2 * GT_BM, GP_BN);
             uint32_t it = 0, unit_i = 0;
             bool ok = true;
             for (int unit = first; ok && unit < num_units; unit += step, ++unit_i) {
                 const uint32_t as = unit_i & 1u, aph = (unit_i >> 1) & 1u;
-                if (!mbar_wait(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 36)) { ok = false; break; }
+                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 36)) { ok = false; break; }
                 tmem_fence_after();
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % GP_STAGES;
-                    if (!mbar_wait(full_bar(s), (it / GP_STAGES) & 1u, abort_flag, p.status, 37)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), (it / GP_STAGES) & 1u, abort_flag, p.status, 37)) { ok = false; break; }
                     tmem_fence_after();
                     const uint32_t a_addr = smem_u32(stages + s * GP_STAGE_BYTES);
                     const uint64_t adesc = make_sw128_desc(a_addr), bdesc = make_sw128_desc(a_addr + GT_BM * GT_BK * 2);
 #pragma unroll
                     for (int k = 0; k < GT_BK / GT_UMMA_K; ++k)
-                        umma_bf16_pair(tmem_base + as * GP_BN, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    umma_commit_pair(empty_bar(s));
+                        if (leader) umma_bf16_pair(tmem_base + as * GP_BN, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    if (leader) umma_commit_pair(empty_bar(s));
                 }
-                if (ok) umma_commit_pair(acc_full_bar(as));
+                if (ok && leader) umma_commit_pair(acc_full_bar(as));
             }
         }
     } else {

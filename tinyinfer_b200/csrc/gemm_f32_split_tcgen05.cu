@@ -23,8 +23,9 @@
 //   warp 14       TMA: the three planes of x, which a small kernel has laid out before ([3][M][Kp])
 //   warp 15       one thread issues the MMAs, 12 of 128 x BN x 16 a k block
 //   warps 0..7    drain finished chunks into their registers, at the end into shared memory
-// Bound by the chain of a k block (copy, split, products, drain): 333 x 12,288 x 2,048 keeps the tensor pipe active 39 % of the time,
-// shared memory 28 %, L2 at 23 % and HBM at 12 %.
+// Bound by the chain of a k block (copy, split, products, drain): 333 x 12,288 x 2,048 kept the tensor pipe active 39 % of the time,
+// shared memory 28 %, L2 at 23 % and HBM at 12 %, at 113.6 us. The issue of the MMAs was a link of it: from uniform registers (see
+// elect_one) 103.6 us, 64 rows 55.7 -> 46.0, 16 rows 53.6 -> 40.7.
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
 // multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
@@ -375,21 +376,22 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 while (global_ns() - t0 < 1000000ull) {}
             }
         }
-    } else if (lane == 0) {
+    } else {
         // ------------------------------------------------------------ MMA issuer
+        const bool leader = elect_one();
         const uint32_t idesc = make_idesc(128, p.bn);
         int sa = 0, sb = 0, kb = 0;
         uint32_t phase_a = 0, phase_b = 0;
         bool ok = true;
         for (int c = 0; c < chunks && ok; ++c) {
             const int a = c & 1;
-            if (!mbar_wait(acc_empty_bar(a), ((c >> 1) & 1u) ^ 1u, abort_flag, p.status, 84)) { ok = false; break; }
+            if (!mbar_wait_warp(acc_empty_bar(a), ((c >> 1) & 1u) ^ 1u, abort_flag, p.status, 84)) { ok = false; break; }
             tmem_fence_after();
             const uint32_t d = tmem_base + a * MAX_BN;
             uint32_t accumulate = 0;
             for (int j = 0; j < CHUNK && kb < blocks; ++j, ++kb) {
-                if (!mbar_wait(b_full_bar(sb), phase_b, abort_flag, p.status, 85) ||
-                    !mbar_wait(a_full_bar(sa), phase_a, abort_flag, p.status, 86)) { ok = false; break; }
+                if (!mbar_wait_warp(b_full_bar(sb), phase_b, abort_flag, p.status, 85) ||
+                    !mbar_wait_warp(a_full_bar(sa), phase_a, abort_flag, p.status, 86)) { ok = false; break; }
                 tmem_fence_after();
                 const uint32_t addr = smem_u32(smem) + sa * (3 * PLANE_A), addr_b = smem_u32(b_ring) + sb * 3 * plane_b;
                 uint64_t A[3], B[3];
@@ -401,19 +403,21 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 auto products = [&](int qa, int qb) {
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
-                        umma_bf16(d, A[qa] + 2u * k, B[qb] + 2u * k, idesc, accumulate);
+                        if (leader) umma_bf16(d, A[qa] + 2u * k, B[qb] + 2u * k, idesc, accumulate);
                         accumulate = 1;
                     }
                 };
                 products(1, 1); products(0, 2); products(2, 0);          // the small ones first
                 products(0, 1); products(1, 0);
                 products(0, 0);
-                umma_commit(a_empty_bar(sa));
-                umma_commit(b_empty_bar(sb));
+                if (leader) {
+                    umma_commit(a_empty_bar(sa));
+                    umma_commit(b_empty_bar(sb));
+                }
                 if (++sa == A_STAGES) { sa = 0; phase_a ^= 1u; }
                 if (++sb == p.b_stages) { sb = 0; phase_b ^= 1u; }
             }
-            if (ok) umma_commit(acc_full_bar(a));
+            if (ok && leader) umma_commit(acc_full_bar(a));
         }
     }
 

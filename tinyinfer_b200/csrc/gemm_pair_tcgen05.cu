@@ -146,28 +146,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (even CTA)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
+            const bool leader = elect_one();
             constexpr uint32_t idesc = make_idesc(2 * BM, BN);
             uint32_t it = 0, tile_i = 0;
             bool ok = true;
             for (int tile = first_tile; tile < num_tiles && ok; tile += tile_step, ++tile_i) {
                 const uint32_t as = tile_i & 1u, aph = (tile_i >> 1) & 1u;
-                if (!mbar_wait(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 62)) { ok = false; break; }
+                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 62)) { ok = false; break; }
                 tmem_fence_after();
                 const uint32_t d_tmem = tmem_base + as * BN;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % STAGES;
-                    if (!mbar_wait(full_bar(s), (it / STAGES) & 1u, abort_flag, p.status, 63)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), (it / STAGES) & 1u, abort_flag, p.status, 63)) { ok = false; break; }
                     tmem_fence_after();
                     const uint32_t a_addr = smem_u32(stages + s * STAGE_BYTES);
                     const uint64_t adesc = make_sw128_desc(a_addr);
                     const uint64_t bdesc = make_sw128_desc(a_addr + BM * BK * 2);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k)
-                        umma_bf16_pair(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    umma_commit_pair(empty_bar(s));          // the stage is free, in both CTAs, once these MMAs have read it
+                        if (leader) umma_bf16_pair(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    if (leader) umma_commit_pair(empty_bar(s));          // the stage is free, in both CTAs, once these MMAs have read it
                 }
-                if (ok) umma_commit_pair(acc_full_bar(as));  // the accumulator is complete, in both CTAs
+                if (ok && leader) umma_commit_pair(acc_full_bar(as));  // the accumulator is complete, in both CTAs
             }
         }
     } else {

@@ -222,7 +222,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const bool leader = elect_one();
             constexpr uint32_t idesc = make_idesc(BM, BN);
             uint32_t it = 0, tile_i = 0;
             bool ok = true;
@@ -231,13 +232,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
                 const int kb0 = wk.kb0, kb1 = wk.kb1;
                 // tall tiles own all of tensor memory: one accumulator buffer, a phase per tile
                 const uint32_t as = TM == 2 ? 0u : (tile_i & 1u), aph = TM == 2 ? (tile_i & 1u) : ((tile_i >> 1) & 1u);
-                if (!mbar_wait(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 12)) { ok = false; break; }
+                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 12)) { ok = false; break; }
                 tmem_fence_after();
                 const uint32_t d_tmem = tmem_base + as * BN;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % C::STAGES;
                     const uint32_t ph = (it / C::STAGES) & 1u;
-                    if (!mbar_wait(full_bar(s), ph, abort_flag, p.status, 13)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), ph, abort_flag, p.status, 13)) { ok = false; break; }
                     tmem_fence_after();
                     const uint32_t a_addr = smem_u32(stages + s * C::STAGE_BYTES);
                     const uint64_t adesc = make_sw128_desc(a_addr);
@@ -245,14 +246,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 #pragma unroll
                     for (int k = 0; k < BK / UMMA_K; ++k) {
                         // 16 bf16 = 32 bytes along K inside the 128-byte swizzled row: +2 in 16-byte units
-                        umma_bf16(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        if (leader) umma_bf16(d_tmem, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                         if constexpr (TM == 2)      // rows 128..255 of the tile: 16 KB further in the stage, next 256 columns
-                            umma_bf16(d_tmem + BN, make_sw128_desc(a_addr + BM * BK * 2) + 2u * k, bdesc + 2u * k, idesc,
+                            if (leader) umma_bf16(d_tmem + BN, make_sw128_desc(a_addr + BM * BK * 2) + 2u * k, bdesc + 2u * k, idesc,
                                       (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    umma_commit(empty_bar(s));           // the stage is free once these MMAs have read it
+                    if (leader) umma_commit(empty_bar(s));           // the stage is free once these MMAs have read it
                 }
-                if (ok) umma_commit(acc_full_bar(as));   // the accumulator is complete
+                if (ok && leader) umma_commit(acc_full_bar(as));   // the accumulator is complete
             }
         }
     } else {
