@@ -39,6 +39,8 @@ def test_portions_on_tcgen05(monkeypatch, heads, rank, rot, page, sink, work):
     assert ops._fn("latent", "ti_latent_attend_tc_ctas")(T, len(work), heads, rank, rot, page) > 0
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     new = ops.latent_attention(q.cuda(), cache.cuda(), status=status, **args).cpu().double()
+    assert ops.latent_rows_dtype(T, cache.cuda(), heads=heads, rank=rank, rot=rot, step=step) == torch.bfloat16
+    assert torch.equal(new, ops.latent_attention(q.cuda().bfloat16(), cache.cuda(), status=status, **args).cpu().double())    # rounded before
     monkeypatch.setattr(ops, "LATENT_TCGEN05", False)
     old = ops.latent_attention(q.cuda(), cache.cuda(), status=status, **args).cpu().double()
     ops.check_kernel_status()

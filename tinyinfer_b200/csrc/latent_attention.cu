@@ -118,8 +118,8 @@ TI_API int ti_latent_prepare(void* q_latent, void* cache, const float* down, int
 // ------------------------------------------------------------------ query rotation
 // q [T, H, plain + rot] (rows of ld_q elements) in the compute dtype -> rows[t][h][rank .. rank + rot) float32 (the first `rank` features
 // of a row are written by the batched product with the key maps).
-template <typename T>
-__global__ void latent_query_kernel(float* __restrict__ rows, const T* __restrict__ q, int ld_q, int heads, int plain, int rot, int rank,
+template <typename T, typename R>
+__global__ void latent_query_kernel(R* __restrict__ rows, const T* __restrict__ q, int ld_q, int heads, int plain, int rot, int rank,
                                     LaRotation rotation, const int* __restrict__ positions) {
     extern __shared__ float part[];
     ti_grid_launch_dependents();
@@ -135,11 +135,12 @@ __global__ void latent_query_kernel(float* __restrict__ rows, const T* __restric
     const bool in_table = rotation.table == nullptr || (pos >= 0 && pos < rotation.table_positions);
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int h = i / rot, f = i % rot;
-        rows[((size_t)t * heads + h) * (rank + rot) + rank + f] = in_table ? la_rotated(part + h * rot, f, pos, rotation) : 0.f;
+        rows[((size_t)t * heads + h) * (rank + rot) + rank + f] = from_f32<R>(in_table ? la_rotated(part + h * rot, f, pos, rotation) : 0.f);
     }
 }
 
-TI_API int ti_latent_query(float* rows, const void* q, int ld_q, int num_tokens, int heads, int plain, int rot, int rank,
+// rows: float32, or with rows_bf16 and a bfloat16 q bfloat16.
+TI_API int ti_latent_query(void* rows, int rows_bf16, const void* q, int ld_q, int num_tokens, int heads, int plain, int rot, int rank,
                            const float* inv_freq, const float* table, int table_positions, int interleaved, int rotary_dim,
                            float rot_factor, const int* positions, int dtype, cudaStream_t stream) {
     TI_REQUIRE(num_tokens >= 0 && heads > 0 && plain >= 0 && rot >= 0 && rank > 0 && ld_q >= heads * (plain + rot), "latent_query: bad sizes");
@@ -148,11 +149,11 @@ TI_API int ti_latent_query(float* rows, const void* q, int ld_q, int num_tokens,
     if (num_tokens == 0 || rot == 0) return 0;
     LaRotation r{inv_freq, table, table_positions, interleaved, rotary_dim, rot_factor};
     const size_t smem = (size_t)heads * rot * 4;
-    if (dtype == TI_F32)
-        ti_launch(latent_query_kernel<float>, num_tokens, 128, smem, stream, rows, (const float*)q, ld_q, heads, plain, rot, rank, r, positions);
-    else if (dtype == TI_BF16)
-        ti_launch(latent_query_kernel<__nv_bfloat16>, num_tokens, 128, smem, stream, rows, (const __nv_bfloat16*)q, ld_q, heads, plain, rot, rank, r, positions);
-    else TI_REQUIRE(false, "latent_query: unknown dtype %d", dtype);
+    typedef __nv_bfloat16 B;
+    TI_REQUIRE(dtype == TI_BF16 || (dtype == TI_F32 && !rows_bf16), "latent_query: unknown dtype %d", dtype);
+    if (dtype == TI_F32) ti_launch(latent_query_kernel<float, float>, num_tokens, 128, smem, stream, (float*)rows, (const float*)q, ld_q, heads, plain, rot, rank, r, positions);
+    else if (rows_bf16) ti_launch(latent_query_kernel<B, B>, num_tokens, 128, smem, stream, (B*)rows, (const B*)q, ld_q, heads, plain, rot, rank, r, positions);
+    else ti_launch(latent_query_kernel<B, float>, num_tokens, 128, smem, stream, (float*)rows, (const B*)q, ld_q, heads, plain, rot, rank, r, positions);
     TI_CHECK_LAUNCH("latent_query");
     return 0;
 }

@@ -5,13 +5,14 @@
 //   warp 0      TMA: tiles of 32 cached rows through the block table, 64 features a copy, into a ring of four
 //   warp 1      issues S = Q K^T (128 x 32, two buffers in tensor memory) and O += P V, P from tensor memory, V the
 //               first features of the same shared-memory tile read as an MN-major operand
-//   warps 2..9  the rows, rounded to bfloat16, into shared and tensor memory; then the softmax: two threads a row, each 16 of a tile's keys and
+//   warps 2..9  the rows, rounded to bfloat16 (or brought so, by TMA), into shared and tensor memory; then the softmax: two threads a row, each 16 of a tile's keys and
 //               half of O's columns. O stays in tensor memory and is multiplied there when a row of the warp has a new maximum.
 //
 // The rows' last features, up to 320 of them, are read by the MMAs from tensor memory: with all 576 in shared memory it would hold a
 // ring of two tiles alone, each refilled only when its products with P are through. 2,048 tokens over 16 heads of rank 512, a
-// layer: 420 us with a ring of two, 354 with four, 285 with the MMAs issued from uniform registers as well (see elect_one); of
-// these 110 are the CTAs' beginnings and ends, mostly the rows' way from float32 in memory, the rest the softmax's chain of a tile.
+// layer: 420 us with a ring of two, 354 with four, 285 with the MMAs issued from uniform registers as well (see elect_one), 218 with
+// rows that the kernels before leave as bfloat16: TMA brings these, where 110 us were the CTAs' beginnings, rounding rows of float32.
+// What is left is the softmax's chain of a tile.
 // O of 512 value features would fill tensor memory and leave no room for scores: above 256 a row tile goes to two CTAs, which
 // both make the scores and take half of the value features each.
 // The products, their operands' roundings and the softmax's steps of 32 keys are those of the warp-level form
@@ -29,7 +30,7 @@ constexpr int MAX_TMEM_CHUNKS = (TMEM_COLS - Q_COL) / 32;             // 64 feat
 struct Args {
     __nv_bfloat16* out;
     float* parts;
-    const float* q;
+    const float* q;                                               // null: the rows come as bfloat16, by TMA
     const float* sink;
     const int *positions, *cu_seqlens, *block_table;
     int max_blocks, num_seqs, heads, rank, rot, page_size, num_pages, piece_rows;
@@ -70,7 +71,7 @@ int smem_bytes(int chunks) { return 1024 + (chunks - tmem_chunks(chunks)) * (QM 
 
 // NV: value features of a CTA.
 template <int NV>
-__global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __grid_constant__ CUtensorMap map, const Args a) {
+__global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __grid_constant__ CUtensorMap map, const __grid_constant__ CUtensorMap map_q, const Args a) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* q_tile = smem;                                       // [chunk of 64 features][row][128 bytes, swizzled]
@@ -80,6 +81,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     const uint32_t q_full = bar0, p_full = bar0 + 8u, o_full = bar0 + 16u;
     auto s_full = [&](int b) { return bar0 + 8u * (3 + b); };
     auto s_empty = [&](int b) { return bar0 + 8u * (5 + b); };
+    const uint32_t q_landed = bar0 + 8u * (7 + 2 * STAGES);
     auto kv_full = [&](int s) { return bar0 + 8u * (7 + s); };
     auto kv_empty = [&](int s) { return bar0 + 8u * (7 + STAGES + s); };
     __shared__ uint32_t tmem_base_sh;
@@ -92,6 +94,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     if (threadIdx.x == 0) {
         abort_sh = 0;
         mbar_init(q_full, 8);
+        mbar_init(q_landed, 1);
         for (int s = 0; s < STAGES; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(s_full(b), 1); mbar_init(s_empty(b), 8); }
         mbar_init(p_full, 8);
@@ -149,6 +152,15 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
         // ------------------------------------------------------------ TMA producer: a lane a copy
         const int* table = a.block_table + (size_t)seq * a.max_blocks;
         const int pieces = KT / a.piece_rows, copies = pieces * a.chunks;
+        if (a.q == nullptr) {                                      // rows of (token, head) lie one behind the other
+            if (lane == 0) mbar_expect_tx(q_landed, (uint32_t)a.chunks * (QM * 128));
+            __syncwarp();
+            if (lane < a.chunks) {
+                const int behind = lane - a.smem_chunks;
+                uint8_t* dst = behind < 0 ? q_tile + lane * (QM * 128) : ring + stage_bytes + behind * (QM * 128);
+                tma_load_2d(smem_u32(dst), &map_q, q_landed, lane * 64, tok0 * a.heads + h0);
+            }
+        }
         for (int j = 0; j < num_tiles; ++j) {
             const int s = j % STAGES;
             int go = 1;
@@ -213,7 +225,9 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     } else {
         // ------------------------------------------------------------ rows and softmax (warps 2..9)
         const int etid = threadIdx.x - 64;
-        {
+        if (a.q == nullptr) {
+            ok = mbar_wait_warp(q_landed, 0, abort_flag, a.status, 89);
+        } else {
             const int chunks8 = a.chunks * 8, total = QM * chunks8;
 #pragma unroll 12
             for (int i = etid; i < total; i += 256) {              // 8 features: two 16-byte loads, one store
@@ -229,6 +243,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
                 *reinterpret_cast<uint4*>(dst + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = w;
             }
             asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_THREADS) : "memory");
+        }
+        if (ok) {
             for (int t = 0; t < a.chunks - a.smem_chunks; ++t) {   // a thread's half of its row's chunk: 32 features, 16 columns
                 const uint8_t* src = ring + stage_bytes + t * (QM * 128) + r * 128;
 #pragma unroll
@@ -246,7 +262,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             if (lane == 0) mbar_arrive(q_full);
         }
         const int pos = live ? a.positions[tok0 + tl] : -1;
-        for (int j = 0; j < num_tiles; ++j) {
+        for (int j = 0; j < num_tiles && ok; ++j) {
             const int b = j & 1, key0 = first_key + j * KT;
             // a warp's threads stay together: tensor memory is read and written by whole warps
             ok = __all_sync(0xffffffffu, mbar_wait(s_full(b), (j >> 1) & 1u, abort_flag, a.status, 86));
@@ -359,9 +375,9 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     }
 }
 
-template <int NV> static cudaError_t launch(const CUtensorMap& map, const Args& a, dim3 grid, int smem, cudaStream_t stream) {
+template <int NV> static cudaError_t launch(const CUtensorMap& map, const CUtensorMap& map_q, const Args& a, dim3 grid, int smem, cudaStream_t stream) {
     const cudaError_t e = ti_allow_shared<latent_attend_tc_kernel<NV>>(smem);
-    return e != cudaSuccess ? e : ti_launch(latent_attend_tc_kernel<NV>, grid, THREADS, smem, stream, map, a);
+    return e != cudaSuccess ? e : ti_launch(latent_attend_tc_kernel<NV>, grid, THREADS, smem, stream, map, map_q, a);
 }
 }  // namespace lt
 
@@ -375,9 +391,9 @@ TI_API int ti_latent_attend_tc_ctas(int num_tokens, int num_seqs, int heads, int
     return ((num_tokens + tpb - 1) / tpb + num_seqs - 1) * ((heads + hpb - 1) / hpb) * (rank > 256 ? 2 : 1);
 }
 
-// Every token's keys 0 .. its position (no window). q float32 [T, heads, rank + rot]; out bfloat16 [T, heads, rank]; splits > 1:
+// Every token's keys 0 .. its position (no window). q [T, heads, rank + rot] float32 or, q_bf16, bfloat16; out bfloat16 [T, heads, rank]; splits > 1:
 // the keys are shared out over grid z and the parts are left for ti_latent_merge. status: two words, or null.
-TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, const float* q, const void* cache, const float* sink,
+TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, const void* q, int q_bf16, const void* cache, const float* sink,
                                const int* positions, const int* cu_seqlens, const int* block_table, int max_blocks, int num_seqs,
                                int num_tokens, int heads, int rank, int rot, int page_size, int num_pages, float scale, int splits,
                                int* status, cudaStream_t stream) {
@@ -391,7 +407,7 @@ TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, 
                "latent_attend_tc: scratch too small for %d splits", splits);
     TI_REQUIRE((long long)num_pages * page_size < (1ll << 31) - 65536, "latent_attend_tc: too many cached rows");
     lt::Args a;
-    a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q; a.sink = sink; a.positions = positions; a.cu_seqlens = cu_seqlens;
+    a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q_bf16 ? nullptr : (const float*)q; a.sink = sink; a.positions = positions; a.cu_seqlens = cu_seqlens;
     a.block_table = block_table; a.max_blocks = max_blocks; a.num_seqs = num_seqs; a.heads = heads; a.rank = rank; a.rot = rot;
     a.page_size = page_size; a.num_pages = num_pages; a.scale = scale; a.splits = splits; a.status = status;
     a.hpb = heads < lt::QM ? heads : lt::QM;
@@ -400,14 +416,17 @@ TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, 
     a.smem_chunks = a.chunks - lt::tmem_chunks(a.chunks);
     a.value_halves = rank > 256 ? 2 : 1;
     a.piece_rows = page_size % 32 == 0 ? 32 : 16;
-    CUtensorMap map;
+    TI_REQUIRE((long long)num_tokens * heads < (1ll << 31) - 65536, "latent_attend_tc: too many query rows");
+    CUtensorMap map, map_q;
     if (!ti_get_bf16_map(cache, (long long)num_pages * page_size, rank + rot, a.piece_rows, &map)) return -1;
+    map_q = map;
+    if (q_bf16 && !ti_get_bf16_map(q, (long long)num_tokens * heads, rank + rot, lt::QM, &map_q)) return -1;
     const int groups = (heads + a.hpb - 1) / a.hpb, smem = lt::smem_bytes(a.chunks);
     TI_REQUIRE(groups <= 65535, "latent_attend_tc: too many heads");
     const dim3 grid(ctas / groups, groups, splits);
     const int nv = rank / a.value_halves;
-    const cudaError_t e = nv == 64 ? lt::launch<64>(map, a, grid, smem, stream) : nv == 128 ? lt::launch<128>(map, a, grid, smem, stream)
-                                                                                         : lt::launch<256>(map, a, grid, smem, stream);
+    const cudaError_t e = nv == 64 ? lt::launch<64>(map, map_q, a, grid, smem, stream) : nv == 128 ? lt::launch<128>(map, map_q, a, grid, smem, stream)
+                                                                                         : lt::launch<256>(map, map_q, a, grid, smem, stream);
     TI_REQUIRE(e == cudaSuccess, "latent_attend_tc: %s", cudaGetErrorString(e));
     TI_CHECK_LAUNCH("latent_attend_tc");
     return 0;

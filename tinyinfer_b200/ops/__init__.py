@@ -58,7 +58,7 @@ _SIGNATURES = {
         "ti_latent_prepare": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_int, c_int, c_int,
                               c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                               c_int, c_void_p, c_int, c_void_p],
-        "ti_latent_query": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
+        "ti_latent_query": [c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int,
                             c_float, c_void_p, c_int, c_void_p],
         "ti_latent_attend": [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_int, c_void_p],
@@ -68,7 +68,7 @@ _SIGNATURES = {
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int,
                                  c_void_p, c_void_p],
         "ti_latent_attend_tc_ctas": [c_int, c_int, c_int, c_int, c_int, c_int],
-        "ti_latent_attend_tc": [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
+        "ti_latent_attend_tc": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
                                 c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
         "ti_causal_conv": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                            c_int, c_int, c_int, c_int, c_void_p],
@@ -1067,13 +1067,15 @@ def latent_prepare(down: torch.Tensor, *, q_rank: int, rank: int, rot: int, q_no
 def latent_query_rotate(rows: torch.Tensor, q: torch.Tensor, *, heads: int, plain: int, rot: int, rank: int,
                         rotation: Optional[Rotation], positions: torch.Tensor) -> None:
     """Writes the rotated last ``rot`` features of every head of ``q`` [T, heads * (plain + rot) (+ columns not read)] into
-    ``rows`` float32 [T, heads * (rank + rot)], behind each head's first ``rank`` features."""
-    _check(rows, "rows", torch.float32, 2)
+    ``rows`` [T, heads * (rank + rot)], float32 or q's dtype, behind each head's first ``rank`` features."""
+    _check(rows, "rows", None, 2)
+    if rows.dtype not in (torch.float32, q.dtype):
+        raise KernelError(f"latent_query_rotate: rows must be float32 or {q.dtype}, got {rows.dtype}")
     _check(q, "q", None, 2)
     _check(positions, "positions", torch.int32, 1)
     if q.shape[1] < heads * (plain + rot) or rows.shape[1] != heads * (rank + rot) or rows.shape[0] != q.shape[0]:
         raise KernelError("latent_query_rotate: widths do not match the head sizes")
-    _run("latent", "ti_latent_query", rows.data_ptr(), q.data_ptr(), q.shape[1], q.shape[0], heads, plain, rot, rank,
+    _run("latent", "ti_latent_query", rows.data_ptr(), int(rows.dtype == torch.bfloat16), q.data_ptr(), q.shape[1], q.shape[0], heads, plain, rot, rank,
          *_rotation_args(rotation), positions.data_ptr(), _dtype_code(q), _stream())
 
 
@@ -1084,19 +1086,36 @@ LATENT_TC_CTAS = 148            # a CTA of that form has an SM to itself
 LATENT_TC_SPLIT_MIN_KEYS = 256
 
 
+def _latent_tc_ctas(t: int, cache: torch.Tensor, heads: int, rank: int, rot: int, window: Optional[int], step) -> int:
+    """CTAs of the tcgen05 form for a step, 0 where the other forms run."""
+    if (not LATENT_TCGEN05 or step is None or cache.dtype != torch.bfloat16 or window or step.max_q_len == 1 or cache.data_ptr() % 16
+            or not int(_fn("latent", "ti_latent_attend_mma_ok")(rank, rot))):
+        return 0
+    return int(_fn("latent", "ti_latent_attend_tc_ctas")(t, step.num_seqs, heads, rank, rot, cache.shape[3]))
+
+
+def latent_rows_dtype(tokens: int, cache: torch.Tensor, *, heads: int, rank: int, rot: int, window: Optional[int] = None, step=None) -> torch.dtype:
+    """The dtype that ``latent_attention``'s query rows are best made in: that of the cache where the tensor cores take them as they
+    are (every form rounds them to it once), else float32."""
+    return cache.dtype if _latent_tc_ctas(tokens, cache, heads, rank, rot, window, step) else torch.float32
+
+
 def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, rank: int, rot: int, scale: float,
                      sink: Optional[torch.Tensor], positions: torch.Tensor, token_seq: torch.Tensor,
                      block_table: torch.Tensor, max_context: int, window: Optional[int] = None, step=None,
                      status: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Causal attention of query rows float32 [T, heads * (rank + rot)] over each token's own request's cached
+    """Causal attention of query rows float32 (or as ``latent_rows_dtype`` says) [T, heads * (rank + rot)] over each token's own request's cached
     rows [c | k_rot] (``cache`` [1, pages, 1, page, rank + rot]); returns sum_j p_j c_j per head, [T, heads * rank]
     in the cache's dtype. ``sink`` float32 [heads]: exp(sink) joins every softmax denominator. ``max_context``
     (a host number, the longest context of the step) only decides over how many blocks the keys are shared.
     ``step`` (the StepContext): with it a bfloat16 cache whose rows are a multiple of 8 features runs on the
     tensor cores, prompt portions and decoded tokens in their own forms; without it, or in float32, the
     float32-arithmetic kernel runs. ``window``: a query sees only the last so many keys, itself included."""
-    _check(q_rows, "q_rows", torch.float32, 2)
+    _check(q_rows, "q_rows", None, 2)
     _check(cache, "cache", None, 5)
+    ctas = _latent_tc_ctas(q_rows.shape[0], cache, heads, rank, rot, window, step) if q_rows.data_ptr() % 16 == 0 else 0
+    if q_rows.dtype != torch.float32 and not (ctas and q_rows.dtype == cache.dtype):
+        raise KernelError(f"latent_attention: q_rows must be float32 here, got {q_rows.dtype}")
     _check(positions, "positions", torch.int32, 1)
     _check(token_seq, "token_seq", torch.int32, 1)
     _check(block_table, "block_table", torch.int32, 2)
@@ -1128,14 +1147,13 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
             and int(_fn("latent", "ti_latent_attend_mma_ok")(rank, rot))):
         decode = step.max_q_len == 1
         page_size = cache.shape[3]
-        ctas = 0 if decode or window else int(_fn("latent", "ti_latent_attend_tc_ctas")(t, step.num_seqs, heads, rank, rot, page_size))
-        if ctas and LATENT_TCGEN05 and (q_rows.data_ptr() | cache.data_ptr()) % 16 == 0:
+        if ctas:
             splits = 1
             if ctas < LATENT_TC_CTAS and reach >= 2 * LATENT_TC_SPLIT_MIN_KEYS:
                 splits = max(1, min(LATENT_TC_CTAS // ctas, reach // LATENT_TC_SPLIT_MIN_KEYS, 64))
             parts, parts_floats = scratch(splits)
-            _run("latent", "ti_latent_attend_tc", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), cache.data_ptr(),
-                 _ptr(sink), positions.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(), block_table.shape[1],
+            _run("latent", "ti_latent_attend_tc", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), int(q_rows.dtype == torch.bfloat16),
+                 cache.data_ptr(), _ptr(sink), positions.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(), block_table.shape[1],
                  step.num_seqs, t, heads, rank, rot, page_size, cache.shape[1], float(scale), splits,
                  status_words(cache.device).data_ptr(), _stream())
             if splits > 1:

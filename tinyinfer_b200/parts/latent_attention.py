@@ -104,7 +104,9 @@ class LatentAttention(Mixer):
             q = ops.linear(x, self.w_q)                           # [T, H * (head_dim + rot_dim) (+ H * v_dim gate logits)]
             if s.output_gate:
                 gate, gate_at = q, q_width
-        rows = torch.empty((q.shape[0], s.num_heads * (s.kv_rank + s.rot_dim)), dtype=torch.float32, device=q.device)
+        rows = torch.empty((q.shape[0], s.num_heads * (s.kv_rank + s.rot_dim)), device=q.device,
+                           dtype=ops.latent_rows_dtype(q.shape[0], cache.kv, heads=s.num_heads, rank=s.kv_rank, rot=s.rot_dim,
+                                                       window=s.window, step=step))
         ops.batched_linear(q, self.w_uk_t, x_batch_stride=s.head_dim + s.rot_dim, k=s.head_dim, out=rows,
                            out_batch_stride=s.kv_rank + s.rot_dim)
         ops.latent_query_rotate(rows, q, heads=s.num_heads, plain=s.head_dim, rot=s.rot_dim, rank=s.kv_rank,
