@@ -18,20 +18,20 @@
 //   on the columns; a cluster of S CTAs cuts the k range of a tile where the tiles alone would leave SMs idle, and adds its
 //   parts up in a fixed order through distributed shared memory, each CTA finishing a share of the tokens.
 //   warp 16       TMA: the float32 weights, several k blocks ahead
-//   warps 8..13   in pairs, a k block each: take it into registers, split it, write three swizzled bfloat16 planes. (All
-//                 on one block at a time waited for one another's latencies: 0.9 us a block whatever the number of tokens.)
-//   warp 14       TMA: the three planes of x, which a small kernel has laid out before ([3][M][Kp])
-//   warp 15       one thread issues the MMAs, 12 of 128 x BN x 16 a k block
+//   warps 8..15   in two groups, a k block each: a thread takes a row of it into registers, splits it and writes three bfloat16 planes
+//                 to tensor memory, where the MMAs read them as their A operand
+//   warp 17       TMA: the three planes of x, which a small kernel has laid out before ([3][M][Kp])
+//   warp 18       issues the MMAs, 12 of 128 x BN x 16 a k block
 //   warps 0..7    drain finished chunks into their registers, at the end into shared memory
-// Bound by the chain of a k block (copy, split, products, drain): 333 x 12,288 x 2,048 kept the tensor pipe active 39 % of the time,
-// shared memory 28 %, L2 at 23 % and HBM at 12 %, at 113.6 us. The issue of the MMAs was a link of it: from uniform registers (see
-// elect_one) 103.6 us, 64 rows 55.7 -> 46.0, 16 rows 53.6 -> 40.7.
+// Bound by the chain of a k block (copy, split, products, drain). With the weights' planes in shared memory and the MMAs issued by one
+// lane of a diverged warp 333 x 12,288 x 2,048 took 113.6 us; from uniform registers (see elect_one) 103.2, with the planes in tensor
+// memory as well 97.4; 64 rows 55.7, 46.1, 41.2; 16 rows 53.6, 40.7, 32.0; 333 x 2,048 x 6,144 77.1, 70.7, 65.3.
 // A weight is read from HBM once per 128 tokens and never stored in another form, so the 32-bit model stays as large as it is.
 // An output that comes out infinite or NaN (an infinite operand has no finite parts) is computed again by plain
 // multiply-adds in k order, so that such operands give what they give in float32: the CTA that finds one makes all its outputs
 // again through shared memory (finish_odd): 333 rows of NaN by 12,288 x 2,048 weights 1.24 ms, where gemm_simt.cu takes 0.89.
-// Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 118 us (142 TFLOP/s), by 2,048 x 6,144
-// 799 -> 78 us; 9 rows 306 -> 51 us; 200 rows by 1,024 x 320 weights, the shortest k that comes here, 26 -> 17 us.
+// Against the 64 x 64 tiles of gemm_simt.cu: 333 rows by 12,288 x 2,048 weights 882 -> 97 us (172 TFLOP/s), by 2,048 x 6,144
+// 799 -> 65 us; 9 to 16 rows 306 -> 32 us; 200 rows by 1,024 x 320 weights, the shortest k that comes here, 26 -> 17 us.
 #include "sm100_ptx.cuh"
 #include <algorithm>
 #include <array>
@@ -42,15 +42,16 @@ namespace {
 constexpr int BK = 32;                           // bf16 elements of a 64-byte swizzled row
 constexpr int CHUNK = 2;                         // k blocks a run of the accumulator
 constexpr int MAX_BN = 128;
-constexpr int PLANE_A = 128 * BK * 2;            // 8 KB
+constexpr int PLANE_A = BK / 2;                  // columns of tensor memory: two bf16 each
 constexpr int SLOT = 128 * BK * 4;               // float32 weights of a k block
-constexpr int A_STAGES = 3;                      // planes of the weights: stage s belongs to the splitting pair s
+constexpr int A_STAGES = 4;                      // planes of the weights
+constexpr int A_COL = 2 * MAX_BN, TMEM_COLS = 512;
 constexpr int MAX_B_STAGES = 6;                  // planes of x: a copy takes about a microsecond to come
-constexpr int MAX_SLOTS = 6;                     // fetched weights; a multiple of A_STAGES, so that a slot too is one pair's: it
-                                                 // sees every phase of the barriers it waits on
-constexpr int DRAIN_WARPS = 8, SPLIT_WARPS = 6, PAIR = SPLIT_WARPS / A_STAGES;
-constexpr int X_WARP = DRAIN_WARPS + SPLIT_WARPS, MMA_WARP = X_WARP + 1, W_WARP = X_WARP + 2;
-constexpr int NUM_THREADS = (W_WARP + 1) * 32;
+constexpr int DRAIN_WARPS = 8, SPLIT_WARPS = 8, GROUPS = SPLIT_WARPS / 4;       // a group: a warp for each 32 lanes
+constexpr int MAX_SLOTS = 6;                     // fetched weights; like A_STAGES a multiple of GROUPS, so that a slot and a stage are
+                                                 // one group's: it sees every phase of the barriers it waits on
+constexpr int W_WARP = DRAIN_WARPS + SPLIT_WARPS, X_WARP = W_WARP + 1, MMA_WARP = W_WARP + 2;
+constexpr int NUM_THREADS = (MMA_WARP + 1) * 32;
 constexpr int SMEM_BYTES = 226 * 1024;           // beside the barriers, of 227 KB
 
 struct SplitParams {
@@ -110,6 +111,17 @@ __global__ void __launch_bounds__(256) split_rows_kernel(__nv_bfloat16* planes, 
 // Shared-memory operand descriptor: K-major tile of rows x 32 bf16, 64-byte swizzle; groups of 8 rows 512 bytes apart.
 __device__ __forceinline__ uint64_t make_sw64_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
+
+// A from tensor memory, a row a lane.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 
 // The CTA's share of the outputs by multiply-adds in k order, one accumulator an output: out[col][row] for `cols` tokens from
@@ -243,18 +255,18 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     const int kb0 = num_kb * part / splits, kb1 = num_kb * (part + 1) / splits;      // at least one each: splits <= num_kb
     const int blocks = kb1 - kb0, chunks = (blocks + CHUNK - 1) / CHUNK;
     const int plane_b = p.bn * BK * 2;
-    uint8_t* b_ring = smem + A_STAGES * 3 * PLANE_A;
+    uint8_t* b_ring = smem;
     uint8_t* slot_ring = b_ring + p.b_stages * 3 * plane_b;
 
     if (threadIdx.x == 0) {
         abort_sh = odd_sh = 0;
-        for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full_bar(s), PAIR); mbar_init(a_empty_bar(s), 1); }
-        for (int s = 0; s < MAX_SLOTS; ++s) { mbar_init(w_full_bar(s), 1); mbar_init(w_empty_bar(s), PAIR); }
+        for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full_bar(s), 4); mbar_init(a_empty_bar(s), 1); }
+        for (int s = 0; s < MAX_SLOTS; ++s) { mbar_init(w_full_bar(s), 1); mbar_init(w_empty_bar(s), 4); }
         for (int s = 0; s < MAX_B_STAGES; ++s) { mbar_init(b_full_bar(s), 1); mbar_init(b_empty_bar(s), 1); }
         for (int a = 0; a < 2; ++a) { mbar_init(acc_full_bar(a), 1); mbar_init(acc_empty_bar(a), DRAIN_WARPS); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == MMA_WARP) tmem_alloc(&tmem_base_sh, 2 * MAX_BN);
+    if (warp == MMA_WARP) tmem_alloc(&tmem_base_sh, TMEM_COLS);
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
@@ -293,47 +305,42 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 for (int i = 0; i < 16; ++i) sums[((unit0 + u) * 16 + i) * 128 + group * 32 + lane] = acc[u][i];
             }
         }
-    } else if (warp < X_WARP) {
+    } else if (warp < W_WARP) {
         // ------------------------------------------------------------ weights: float32 -> three planes
-        const int s = (warp - DRAIN_WARPS) / PAIR;           // this pair's stage; it takes k blocks s, s + A_STAGES, ...
-        const int t = ((int)threadIdx.x - DRAIN_WARPS * 32) % (PAIR * 32);
-        constexpr int ROWS = PAIR * 8, STEPS = 128 / ROWS;   // 4 lanes a row of 32 floats
-        const int c = t & 3, row0 = t >> 2;
-        uint8_t* a = smem + s * (3 * PLANE_A);
-        int slot = s;
+        const int group = (warp - DRAIN_WARPS) >> 2;         // this group takes k blocks group, group + GROUPS, ...
+        const int row = (warp & 3) * 32 + lane;              // the thread's row of the tile = lane of tensor memory
+        int slot = group, stage = group;
         uint32_t slot_phase = 0, phase = 0;
-        for (int i = s; i < blocks; i += A_STAGES, phase ^= 1u) {
+        for (int i = group; i < blocks; i += GROUPS) {
             if (!__all_sync(0xffffffffu, mbar_wait(w_full_bar(slot), slot_phase, abort_flag, p.status, 87))) break;
-            const uint8_t* d = slot_ring + slot * SLOT;      // rows of 128 bytes, 128-byte swizzle
-            float4 v[STEPS][2];
+            const uint8_t* d = slot_ring + slot * SLOT + row * 128;      // rows of 128 bytes, 128-byte swizzle
+            float4 v[BK / 4];
 #pragma unroll
-            for (int j = 0; j < STEPS; ++j)
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const int r = row0 + ROWS * j;
-                    v[j][h] = *reinterpret_cast<const float4*>(d + r * 128 + (((2 * c + h) ^ (r & 7)) << 4));
-                }
+            for (int c = 0; c < BK / 4; ++c) v[c] = *reinterpret_cast<const float4*>(d + ((c ^ (row & 7)) << 4));
             // the copy that refills the slot is the async proxy's: without this fence the loads above may be put off past it
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(w_empty_bar(slot));
-            if ((slot += A_STAGES) >= p.slots) { slot = s; slot_phase ^= 1u; }
-            if (!__all_sync(0xffffffffu, mbar_wait(a_empty_bar(s), phase ^ 1u, abort_flag, p.status, 82))) break;
+            if ((slot += GROUPS) >= p.slots) { slot = group; slot_phase ^= 1u; }
+            if (!__all_sync(0xffffffffu, mbar_wait(a_empty_bar(stage), phase ^ 1u, abort_flag, p.status, 82))) break;
+            tmem_fence_after();
+            const uint32_t to = tmem_base + A_COL + stage * (3 * PLANE_A) + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll
-            for (int j = 0; j < STEPS; ++j) {
-                const int r = row0 + ROWS * j;
-                uint4 q[3];
-                split2(v[j][0].x, v[j][0].y, q[0].x, q[1].x, q[2].x);
-                split2(v[j][0].z, v[j][0].w, q[0].y, q[1].y, q[2].y);
-                split2(v[j][1].x, v[j][1].y, q[0].z, q[1].z, q[2].z);
-                split2(v[j][1].z, v[j][1].w, q[0].w, q[1].w, q[2].w);
+            for (int h = 0; h < 2; ++h) {                    // 16 k: 8 columns of each plane
+                uint32_t q[3][8];
 #pragma unroll
-                for (int plane = 0; plane < 3; ++plane)
-                    *reinterpret_cast<uint4*>(a + plane * PLANE_A + r * 64 + ((c ^ ((r >> 1) & 3)) << 4)) = q[plane];
+                for (int c = 0; c < 4; ++c) {
+                    split2(v[4 * h + c].x, v[4 * h + c].y, q[0][2 * c], q[1][2 * c], q[2][2 * c]);
+                    split2(v[4 * h + c].z, v[4 * h + c].w, q[0][2 * c + 1], q[1][2 * c + 1], q[2][2 * c + 1]);
+                }
+#pragma unroll
+                for (int plane = 0; plane < 3; ++plane) tmem_st8(to + plane * PLANE_A + 8 * h, q[plane]);
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");     // the MMAs read what was written
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tmem_fence_before();                             // the MMAs read what was written
             __syncwarp();
-            if (lane == 0) mbar_arrive(a_full_bar(s));
+            if (lane == 0) mbar_arrive(a_full_bar(stage));
+            if ((stage += GROUPS) >= A_STAGES) { stage = group; phase ^= 1u; }
         }
     } else if (warp == X_WARP) {
         // ------------------------------------------------------------ TMA: the planes of x
@@ -393,17 +400,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 if (!mbar_wait_warp(b_full_bar(sb), phase_b, abort_flag, p.status, 85) ||
                     !mbar_wait_warp(a_full_bar(sa), phase_a, abort_flag, p.status, 86)) { ok = false; break; }
                 tmem_fence_after();
-                const uint32_t addr = smem_u32(smem) + sa * (3 * PLANE_A), addr_b = smem_u32(b_ring) + sb * 3 * plane_b;
-                uint64_t A[3], B[3];
+                const uint32_t A = tmem_base + A_COL + sa * (3 * PLANE_A), addr_b = smem_u32(b_ring) + sb * 3 * plane_b;
+                uint64_t B[3];
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    A[q] = make_sw64_desc(addr + q * PLANE_A);
-                    B[q] = make_sw64_desc(addr_b + q * plane_b);
-                }
+                for (int q = 0; q < 3; ++q) B[q] = make_sw64_desc(addr_b + q * plane_b);
                 auto products = [&](int qa, int qb) {
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k) {
-                        if (leader) umma_bf16(d, A[qa] + 2u * k, B[qb] + 2u * k, idesc, accumulate);
+                        if (leader) umma_bf16_ts(d, A + qa * PLANE_A + 8 * k, B[qb] + 2u * k, idesc, accumulate);
                         accumulate = 1;
                     }
                 };
@@ -466,7 +470,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     else __syncthreads();
     if (warp == MMA_WARP) {
         tmem_fence_after();
-        tmem_dealloc(tmem_base, 2 * MAX_BN);
+        tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (odd_sh) finish_odd(p, sums, odd);
 }
@@ -522,15 +526,14 @@ TI_API int ti_gemm_f32_split(float* out, const float* x, const float* w, const f
     p.bn = ((M + row_tiles - 1) / row_tiles + 15) / 16 * 16;
     const int outs = gated ? 64 : 128, col_tiles = (N + outs - 1) / outs;
     TI_REQUIRE(row_tiles <= 65535 && col_tiles <= 65535, "gemm_f32_split: too many tiles");
-    // shared memory: the weights' planes, then for many columns as many copies of x as leave room for three slots, for few
-    // columns (where the weights' way from HBM is what a step waits for) as many slots as there are
-    const int b_bytes = 3 * p.bn * BK * 2, room = SMEM_BYTES - 1024 - A_STAGES * 3 * PLANE_A;
-    p.b_stages = std::min(MAX_B_STAGES, (room - 3 * SLOT) / b_bytes);       // at least three
-    p.slots = std::min(MAX_SLOTS, (room - p.b_stages * b_bytes) / SLOT / A_STAGES * A_STAGES);
+    // shared memory: the slots, and as many copies of x as leave room for them
+    const int b_bytes = 3 * p.bn * BK * 2, room = SMEM_BYTES - 1024;
+    p.b_stages = std::min(MAX_B_STAGES, (room - MAX_SLOTS * SLOT) / b_bytes);       // at least five
+    p.slots = MAX_SLOTS;
     static_assert(4 * (MAX_BN * 128 + 2 * REDO_PIECE) <= SMEM_BYTES - 1024, "the outputs made again and their operands");
     static_assert(MAX_BN * 32 <= 32 * NUM_THREADS, "a thread's quads have a bit each");
-    static_assert(A_STAGES * 3 * PLANE_A + 3 * 3 * MAX_BN * BK * 2 + 3 * SLOT <= SMEM_BYTES - 1024, "128 columns: three copies, three slots");
-    static_assert(MAX_SLOTS % A_STAGES == 0 && A_STAGES == 3, "three slots at least, a whole number a pair");
+    static_assert(5 * 3 * MAX_BN * BK * 2 + MAX_SLOTS * SLOT <= SMEM_BYTES - 1024, "128 columns: five copies of x");
+    static_assert(MAX_SLOTS % GROUPS == 0 && A_STAGES % GROUPS == 0 && A_COL + A_STAGES * 3 * PLANE_A <= TMEM_COLS, "stages and slots");
     TiEncodeTiledFn encode = ti_encode_tiled_fn();
     TI_REQUIRE(encode, "cuTensorMapEncodeTiled is not available from this driver");
     CUtensorMap map, map_w;
