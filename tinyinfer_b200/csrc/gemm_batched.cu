@@ -8,6 +8,12 @@
 #include "common.cuh"
 #include "mma_tile.cuh"
 
+// gemm_batched_tcgen05.cu: many rows
+bool gbt_takes(const void* out, const void* x, const void* w, int batch, int M, int N, int K, long long ldx, long long sx, long long ldw,
+               long long sw, long long ldo, long long so, int out_f32);
+int gbt_launch(void* out, const void* x, const void* w, int batch, int M, int N, int K, long long ldx, long long sx, long long ldo, long long so,
+               int out_f32, int* status, cudaStream_t stream);
+
 constexpr int GB_BM = 64, GB_BN = 64, GB_BK = 16, GB_THREADS = 256;
 
 struct GbShape {
@@ -106,14 +112,17 @@ __global__ void __launch_bounds__(mt::THREADS) gemm_batched_mma_kernel(
     });
 }
 
+// status (may be null): set if a wait of the tcgen05 form runs out. form: 0 whichever takes it, 1 not the tcgen05 form.
 TI_API int ti_gemm_batched(void* out, const void* x, const void* w, const float* bias, int batch, int M, int N, int K,
                            long long ldx, long long sx, long long ldw, long long sw, long long ldo, long long so,
                            long long sbias, int act, int out_f32, const void* gate, long long ldg, long long sg, int dtype,
-                           cudaStream_t stream) {
+                           int form, int* status, cudaStream_t stream) {
     TI_REQUIRE(batch > 0 && M >= 0 && N > 0 && K > 0, "gemm_batched: bad sizes");
     TI_REQUIRE(act == 0 || act == 1, "gemm_batched: unknown activation %d", act);
     TI_REQUIRE(batch <= 65535, "gemm_batched: too many batches");
     if (M == 0) return 0;
+    if (dtype == TI_BF16 && form == 0 && !bias && !act && !gate && gbt_takes(out, x, w, batch, M, N, K, ldx, sx, ldw, sw, ldo, so, out_f32))
+        return gbt_launch(out, x, w, batch, M, N, K, ldx, sx, ldo, so, out_f32, status, stream);
     dim3 grid((N + GB_BN - 1) / GB_BN, (M + GB_BM - 1) / GB_BM, batch);
     TI_REQUIRE(grid.y <= 65535, "gemm_batched: too many rows");
     GbShape s{M, N, K, ldx, sx, ldw, sw, ldo, so, sbias, gate, ldg, sg};

@@ -54,7 +54,7 @@ _SIGNATURES = {
         "ti_rmsnorm_rows32": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_float, c_int, c_void_p],
         "ti_relu_squared": [c_void_p, c_void_p, c_ll, c_int, c_void_p],
         "ti_gemm_batched": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_ll,
-                            c_ll, c_ll, c_ll, c_int, c_int, c_void_p, c_ll, c_ll, c_int, c_void_p],
+                            c_ll, c_ll, c_ll, c_int, c_int, c_void_p, c_ll, c_ll, c_int, c_int, c_void_p, c_void_p],
         "ti_latent_prepare": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_int, c_int, c_int,
                               c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                               c_int, c_void_p, c_int, c_void_p],
@@ -977,6 +977,9 @@ def relu_squared(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
+BATCHED_TCGEN05 = True          # many rows on tcgen05 where the sizes allow
+
+
 def batched_linear(x: torch.Tensor, w: torch.Tensor, *, x_offset: int = 0, x_batch_stride: int, k: int,
                    out: Optional[torch.Tensor] = None, out_offset: int = 0, out_batch_stride: Optional[int] = None,
                    bias: Optional[torch.Tensor] = None, sigmoid: bool = False, out_float32: bool = False,
@@ -1017,7 +1020,7 @@ def batched_linear(x: torch.Tensor, w: torch.Tensor, *, x_offset: int = 0, x_bat
          _ptr(bias), batch, m, n, k, x.shape[1], x_batch_stride, k, n * k, out.shape[1], out_batch_stride, n,
          int(sigmoid), int(out.dtype == torch.float32 and x.dtype != torch.float32),
          gate.data_ptr() + gate_offset * isz_x if gate is not None else None, gate.shape[1] if gate is not None else 0, n,
-         _dtype_code(x), _stream())
+         _dtype_code(x), 0 if BATCHED_TCGEN05 else 1, kernel_status(x.device).data_ptr(), _stream())
     return out
 
 

@@ -42,7 +42,7 @@ LIBRARIES: Dict[str, dict] = {
     "f32": dict(sources=["runtime.cu", "sm100_host.cu", "gemm_f32_few.cu", "gemm_f32_split_tcgen05.cu", "attention_f32.cu"],
                 headers=["common.cuh", "sm100_ptx.cuh"], link=[]),
     # parts of designs with a cached latent, gated recurrences and routed experts around a float32 stream
-    "latent": dict(sources=["runtime.cu", "sm100_host.cu", "stream.cu", "gemm_batched.cu", "latent_attention.cu",
+    "latent": dict(sources=["runtime.cu", "sm100_host.cu", "stream.cu", "gemm_batched.cu", "gemm_batched_tcgen05.cu", "latent_attention.cu",
                             "latent_attention_mma.cu", "latent_attention_tcgen05.cu", "recurrent.cu"],
                    headers=["common.cuh", "mma_tile.cuh", "sm100_ptx.cuh"], link=[]),
     # routed experts: router, plan, grouped products, activations, combine
