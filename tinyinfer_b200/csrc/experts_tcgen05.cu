@@ -12,7 +12,7 @@
 // the up form, and store. Rows of a tile beyond the expert's (the next expert's rows, or nothing) and features
 // beyond N (the next expert's weights) are computed and not stored. Every wait is bounded and reports through the
 // status word; tensor memory is freed on the common exit.
-#include "sm100_pair.cuh"
+#include "sm100_ptx.cuh"
 
 namespace {
 constexpr int GT_BM = 128, GT_BK = 64, GT_UMMA_K = 16, GT_THREADS = 192;
@@ -29,43 +29,6 @@ struct GtParams {
     int N, K, col_tiles, up;
     int* status;
 };
-
-// The epilogue of a thread's row: BN columns of its accumulator lane, from feature n0 on, to sorted row `row`.
-template <int BN> __device__ __forceinline__ void store_rows(const GtParams& p, uint32_t t_addr, bool live, int row, int n0) {
-    for (int c = 0; c < BN; c += 32) {
-        float v[32];
-        tmem_ld32(t_addr + c, v);
-        if (!live || n0 + c >= p.N) continue;
-        const size_t at = (size_t)row * p.N + n0 + c;
-        if (p.up) {
-            if (p.up == 1) {                          // up == 2: stored as it is, the activation is a kernel of its own
-#pragma unroll
-                for (int i = 0; i < 32; ++i) { v[i] = fmaxf(v[i], 0.f); v[i] *= v[i]; }
-            }
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + at;
-            if (n0 + c + 32 <= p.N && (p.N & 7) == 0) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) {
-                    uint4 q;
-                    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
-                    *reinterpret_cast<uint4*>(dst + i) = q;
-                }
-            } else {
-                for (int i = 0; i < 32 && n0 + c + i < p.N; ++i) dst[i] = __float2bfloat16_rn(v[i]);
-            }
-        } else {
-            float* dst = reinterpret_cast<float*>(p.out) + at;
-            if (n0 + c + 32 <= p.N && (p.N & 3) == 0) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-            } else {
-                for (int i = 0; i < 32 && n0 + c + i < p.N; ++i) dst[i] = v[i];
-            }
-        }
-    }
-}
 
 template <int GT_BN>
 __global__ void __launch_bounds__(GT_THREADS, 1)
@@ -161,7 +124,41 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             if (!mbar_wait(acc_full_bar(as), aph, abort_flag, p.status, 34)) { ok = false; break; }
             tmem_fence_after();
             const uint32_t t_addr = tmem_base + as * GT_BN + ((uint32_t)(lane_group * 32) << 16);
-            store_rows<GT_BN>(p, t_addr, r < rows, row0 + r, ct * GT_BN);
+            const bool live = r < rows;
+            const int n0 = ct * GT_BN;
+            for (int c = 0; c < GT_BN; c += 32) {
+                float v[32];
+                tmem_ld32(t_addr + c, v);
+                if (!live || n0 + c >= p.N) continue;
+                const size_t at = (size_t)(row0 + r) * p.N + n0 + c;
+                if (p.up) {
+                    if (p.up == 1) {                          // up == 2: stored as it is, the activation is a kernel of its own
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) { v[i] = fmaxf(v[i], 0.f); v[i] *= v[i]; }
+                    }
+                    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.out) + at;
+                    if (n0 + c + 32 <= p.N && (p.N & 7) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 8) {
+                            uint4 q;
+                            __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) h[j] = __floats2bfloat162_rn(v[i + 2 * j], v[i + 2 * j + 1]);
+                            *reinterpret_cast<uint4*>(dst + i) = q;
+                        }
+                    } else {
+                        for (int i = 0; i < 32 && n0 + c + i < p.N; ++i) dst[i] = __float2bfloat16_rn(v[i]);
+                    }
+                } else {
+                    float* dst = reinterpret_cast<float*>(p.out) + at;
+                    if (n0 + c + 32 <= p.N && (p.N & 3) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                    } else {
+                        for (int i = 0; i < 32 && n0 + c + i < p.N; ++i) dst[i] = v[i];
+                    }
+                }
+            }
             tmem_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty_bar(as));  // this accumulator may be overwritten
@@ -175,122 +172,6 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
         tmem_dealloc(tmem_base, 2 * GT_BN);
     }
 }
-
-// ---------------------------------------------------------------------- the pair form
-// Row tiles of 256 rows of one expert (two CTAs of a cluster, 128 each) by 256 features: a CTA loads its own rows and half of
-// the weights, 32 KB a k block for the 512 cycles of MMAs for which a lone CTA takes 48 KB (see gemm_pair_tcgen05.cu, whose roles
-// and barriers these are).
-constexpr int GP_STAGES = 6, GP_BN = 256, GP_STAGE_BYTES = (GT_BM + GP_BN / 2) * GT_BK * 2;
-constexpr int GP_SMEM = 1024 + GP_STAGES * GP_STAGE_BYTES + 256;
-
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GT_THREADS, 1)
-moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const GtParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(stages + GP_STAGES * GP_STAGE_BYTES);
-    const uint32_t bar0 = smem_u32(bars);                 // full[STAGES] (the even CTA's), empty[STAGES], acc_full[2], acc_empty[2] (the even CTA's)
-    auto full_bar = [&](int s) { return bar0 + 8u * s; };
-    auto empty_bar = [&](int s) { return bar0 + 8u * (GP_STAGES + s); };
-    auto acc_full_bar = [&](int a) { return bar0 + 8u * (2 * GP_STAGES + a); };
-    auto acc_empty_bar = [&](int a) { return bar0 + 8u * (2 * GP_STAGES + 2 + a); };
-    __shared__ uint32_t tmem_base_sh;
-    __shared__ int abort_sh;
-    volatile int* abort_flag = &abort_sh;
-
-    ti_grid_launch_dependents();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int rank = (int)cluster_rank(), first = (int)cluster_id_x(), step = (int)num_clusters_x();
-    if (threadIdx.x == 0) {
-        abort_sh = 0;
-        for (int s = 0; s < GP_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(acc_full_bar(a), 1); mbar_init(acc_empty_bar(a), 8); }   // four warps of each CTA
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 1) {        // one warp of EACH CTA of the pair takes part in the allocation
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_base_sh)), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    tmem_fence_before();
-    __syncthreads();
-    cluster_sync_all();
-    tmem_fence_after();
-    const uint32_t tmem_base = tmem_base_sh;
-    ti_grid_wait();                                        // the plan, the sorted rows and `out` belong to earlier kernels until now
-    const int num_units = p.num_tiles[0] * p.col_tiles, num_kb = (p.K + GT_BK - 1) / GT_BK;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            const uint32_t full0 = map_to_cta(bar0, 0);
-            uint32_t it = 0;
-            bool ok = true;
-            for (int unit = first; ok && unit < num_units; unit += step) {
-                const int tile = unit / p.col_tiles, ct = unit % p.col_tiles;
-                const int x_row = p.tiles[3 * tile + 1] + rank * GT_BM;      // past the expert's rows: computed and not stored
-                const int w_row = p.tiles[3 * tile] * p.N + ct * GP_BN + rank * (GP_BN / 2);
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % GP_STAGES;
-                    if (!mbar_wait(empty_bar(s), ((it / GP_STAGES) & 1u) ^ 1u, abort_flag, p.status, 35)) { ok = false; break; }
-                    if (rank == 0) mbar_expect_tx(full_bar(s), 2 * GP_STAGE_BYTES);
-                    const uint32_t dst = smem_u32(stages + s * GP_STAGE_BYTES);
-                    tma_load_2d_pair(dst, &map_x, full0 + 8u * s, kb * GT_BK, x_row);
-                    tma_load_2d_pair(dst + GT_BM * GT_BK * 2, &map_w, full0 + 8u * s, kb * GT_BK, w_row);
-                }
-            }
-            if (!ok) {                                     // let the copies in flight land before shared memory is given up
-                const unsigned long long t0 = global_ns();
-                while (global_ns() - t0 < 1000000ull) {}
-            }
-        }
-    } else if (warp == 1) {
-        if (rank == 0) {
-            const bool leader = elect_one();
-            constexpr uint32_t idesc = make_idesc(2 * GT_BM, GP_BN);
-            uint32_t it = 0, unit_i = 0;
-            bool ok = true;
-            for (int unit = first; ok && unit < num_units; unit += step, ++unit_i) {
-                const uint32_t as = unit_i & 1u, aph = (unit_i >> 1) & 1u;
-                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 36)) { ok = false; break; }
-                tmem_fence_after();
-                for (int kb = 0; kb < num_kb; ++kb, ++it) {
-                    const int s = it % GP_STAGES;
-                    if (!mbar_wait_warp(full_bar(s), (it / GP_STAGES) & 1u, abort_flag, p.status, 37)) { ok = false; break; }
-                    tmem_fence_after();
-                    const uint32_t a_addr = smem_u32(stages + s * GP_STAGE_BYTES);
-                    const uint64_t adesc = make_sw128_desc(a_addr), bdesc = make_sw128_desc(a_addr + GT_BM * GT_BK * 2);
-#pragma unroll
-                    for (int k = 0; k < GT_BK / GT_UMMA_K; ++k)
-                        if (leader) umma_bf16_pair(tmem_base + as * GP_BN, adesc + 2u * k, bdesc + 2u * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    if (leader) umma_commit_pair(empty_bar(s));
-                }
-                if (ok && leader) umma_commit_pair(acc_full_bar(as));
-            }
-        }
-    } else {
-        const int lane_group = warp & 3, r = rank * GT_BM + lane_group * 32 + lane;
-        const uint32_t acc_empty0 = map_to_cta(acc_empty_bar(0), 0);
-        uint32_t unit_i = 0;
-        for (int unit = first; unit < num_units; unit += step, ++unit_i) {
-            const int tile = unit / p.col_tiles, ct = unit % p.col_tiles;
-            const int row0 = p.tiles[3 * tile + 1], rows = p.tiles[3 * tile + 2];
-            const uint32_t as = unit_i & 1u, aph = (unit_i >> 1) & 1u;
-            if (!__all_sync(0xffffffffu, mbar_wait(acc_full_bar(as), aph, abort_flag, p.status, 38))) break;
-            tmem_fence_after();
-            store_rows<GP_BN>(p, tmem_base + as * GP_BN + ((uint32_t)(lane_group * 32) << 16), r < rows, row0 + r, ct * GP_BN);
-            tmem_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(acc_empty0 + 8u * as);   // this half of tensor memory may be overwritten
-        }
-    }
-    // ---------------------------------------------------------------- common exit
-    tmem_fence_before();
-    __syncthreads();
-    cluster_sync_all();                  // nobody leaves while the other CTA's MMAs still read its shared memory or write its tensor memory
-    if (warp == 1) {
-        tmem_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
-    }
-}
 }  // namespace
 
 // 1 if the tcgen05 form takes these operands: whole k blocks, rows on 16-byte boundaries, operands at least a box tall.
@@ -298,26 +179,6 @@ TI_API int ti_moe_gemm_tcgen05_ok(int slots, int experts, int N, int K) {
     return (K % GT_BK == 0 && slots >= GT_BM && (long long)experts * N >= 128 && N > 0) ? 1 : 0;
 }
 TI_API int ti_moe_tcgen05_tile_rows() { return GT_BM; }
-
-// As ti_moe_gemm_tcgen05 with a plan of row tiles of 256, in the pair form.
-TI_API int ti_moe_gemm_pair(void* out, const void* x, const void* w, const int* tiles, const int* num_tiles, int slots,
-                            int experts, int N, int K, int max_tiles, int up, int* status, cudaStream_t stream) {
-    TI_REQUIRE(ti_moe_gemm_tcgen05_ok(slots, experts, N, K) && N >= GP_BN, "moe_gemm_pair: operands [%d, %d] x [%d, %d, %d] are not taken", slots, K, experts, N, K);
-    TI_REQUIRE((((uintptr_t)x | (uintptr_t)w | (uintptr_t)out) & 15) == 0, "moe_gemm_pair: operands must be 16-byte aligned");
-    if (max_tiles <= 0) return 0;
-    CUtensorMap map_x, map_w;
-    if (!ti_get_bf16_map(x, slots, K, GT_BM, &map_x)) return -1;
-    if (!ti_get_bf16_map(w, (long long)experts * N, K, GP_BN / 2, &map_w)) return -1;
-    const cudaError_t set = ti_allow_shared<moe_gemm_pair_kernel>(GP_SMEM);
-    TI_REQUIRE(set == cudaSuccess, "moe_gemm_pair: shared memory: %s", cudaGetErrorString(set));
-    GtParams p;
-    p.out = out; p.tiles = tiles; p.num_tiles = num_tiles; p.N = N; p.K = K; p.col_tiles = (N + GP_BN - 1) / GP_BN; p.up = up;
-    p.status = status;
-    const long long units = (long long)max_tiles * p.col_tiles, pairs = ti_sm_count() / 2;
-    ti_launch(moe_gemm_pair_kernel, (unsigned)(2 * (units < pairs ? units : pairs)), GT_THREADS, GP_SMEM, stream, map_x, map_w, p);
-    TI_CHECK_LAUNCH("moe_gemm_pair");
-    return 0;
-}
 
 // The output features of a unit: 256 where every SM keeps two units, else 128. The real number of row tiles is on the device; it
 // is at least slots / 128.

@@ -157,7 +157,7 @@ _SIGNATURES["sm100"]["ti_gemm_set_pair_form"] = [c_int]
 _SIGNATURES["sm100"]["ti_moe_gemm_tcgen05_ok"] = [c_int, c_int, c_int, c_int]
 _SIGNATURES["sm100"]["ti_moe_tcgen05_unit_features"] = [c_int, c_int]
 _SIGNATURES["sm100"]["ti_moe_tcgen05_tile_rows"] = []
-_SIGNATURES["sm100"]["ti_moe_gemm_pair"] = _SIGNATURES["sm100"]["ti_moe_gemm_tcgen05"] = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+_SIGNATURES["sm100"]["ti_moe_gemm_tcgen05"] = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                                c_int, c_void_p, c_void_p]
 _SIGNATURES["sm100"]["ti_gemm_pair_bf16"] = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                              c_int, c_void_p, c_void_p]
@@ -1418,12 +1418,11 @@ def expert_tiles_may_be_wide(x: torch.Tensor, *inner_sizes: int) -> bool:
     return all(int(_fn("experts", "ti_moe_wide_tiles_ok")(k, _dtype_code(x))) for k in (x.shape[1],) + inner_sizes)
 
 
-EXPERT_PAIR_MIN_ROWS = 160       # and from which two CTAs take row tiles of 256
 EXPERT_TCGEN05_MIN_ROWS = 96     # rows an expert gets on average from which the tcgen05 grouped product is used
 
 
 def expert_tile_rows(x: torch.Tensor, num_experts: int, top: int, *inner_sizes: int) -> int:
-    """The height of the row tiles that the grouped products of a step should be planned with: 256 or 128 (tcgen05: many
+    """The height of the row tiles that the grouped products of a step should be planned with: 128 (tcgen05: many
     rows an expert, bfloat16, whole k blocks of 64), 64 or 32 (the warp-level tensor-core tiles; 32 also float32)."""
     return expert_tile_rows_of(x.shape[0], x.shape[1], x.dtype, num_experts, top, *inner_sizes)
 
@@ -1434,8 +1433,6 @@ def expert_tile_rows_of(t: int, hidden: int, dtype: torch.dtype, num_experts: in
     if bf16 and t * top >= EXPERT_TCGEN05_MIN_ROWS * num_experts:
         ok = _fn("sm100", "ti_moe_gemm_tcgen05_ok")
         if all(int(ok(t * top, num_experts, n, k)) for n, k in ((inner_sizes[0], hidden), (hidden, inner_sizes[0]))):
-            if t * top >= EXPERT_PAIR_MIN_ROWS * num_experts and min(inner_sizes[0], hidden) >= 256:
-                return 256
             return int(_fn("sm100", "ti_moe_tcgen05_tile_rows")())
     if t * top >= 48 * num_experts and all(int(_fn("experts", "ti_moe_wide_tiles_ok")(k, int(bf16))) for k in (hidden,) + inner_sizes):
         return 64
@@ -1455,13 +1452,13 @@ def expert_linear(x: torch.Tensor, w: torch.Tensor, routing: ExpertRouting, *, u
     slots = routing.token_of.shape[0]
     out = torch.empty((slots, n), dtype=x.dtype if up else torch.float32, device=x.device)
     form = (1 if activation else 2) if up else 0
-    if routing.tile_rows in (128, 256):          # tcgen05, one CTA a tile or two: tiled operand copies want the rows in expert order
+    if routing.tile_rows == 128:                 # tcgen05: tiled operand copies want the rows in expert order
         rows = x
         if up:
             rows = torch.empty((slots, k), dtype=x.dtype, device=x.device)
             _run("experts", "ti_moe_gather", rows.data_ptr(), x.data_ptr(), routing.token_of.data_ptr(), slots, k,
                  _dtype_code(x), _stream())
-        _run("sm100", "ti_moe_gemm_tcgen05" if routing.tile_rows == 128 else "ti_moe_gemm_pair", out.data_ptr(), rows.data_ptr(), w.data_ptr(), routing.tiles.data_ptr(),
+        _run("sm100", "ti_moe_gemm_tcgen05", out.data_ptr(), rows.data_ptr(), w.data_ptr(), routing.tiles.data_ptr(),
              routing.num_tiles.data_ptr(), slots, w.shape[0], n, k, routing.max_tiles, form,
              kernel_status(x.device).data_ptr(), _stream())
         return out

@@ -57,7 +57,7 @@ LIBRARIES: Dict[str, dict] = {
     "sm100": dict(sources=["runtime.cu", "sm100_host.cu", "gemm_tcgen05.cu", "attention_mma.cu",
                            "attention_prefill_tcgen05.cu", "attention_prefill_pair_tcgen05.cu", "gemm_pair_tcgen05.cu",
                            "experts_tcgen05.cu"],
-                  headers=["common.cuh", "sm100_ptx.cuh", "sm100_pair.cuh"], link=[]),
+                  headers=["common.cuh", "sm100_ptx.cuh"], link=[]),
 }
 
 _loaded: Dict[str, ctypes.CDLL] = {}
