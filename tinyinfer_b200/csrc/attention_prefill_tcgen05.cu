@@ -114,7 +114,6 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     __shared__ int abort_sh;
     volatile int* abort_flag = &abort_sh;
 
-    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_sh = 0;
@@ -133,6 +132,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
+    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     ti_grid_wait();                                     // q, the pages and the tables come from earlier kernels
 

@@ -246,7 +246,6 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     auto w_full_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + 2 * MAX_B_STAGES + s); };
     auto w_empty_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + 2 * MAX_B_STAGES + MAX_SLOTS + s); };
 
-    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int splits = (int)gridDim.x, part = (int)blockIdx.x;           // the cluster spans gridDim.x
     const int outs = p.gated ? 64 : 128;
@@ -270,6 +269,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
+    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     float* sums = reinterpret_cast<float*>(smem);            // [bn][128], once the stages are done with
 

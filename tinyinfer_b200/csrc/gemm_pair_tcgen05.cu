@@ -122,7 +122,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __shared__ int abort_sh;
     volatile int* abort_flag = &abort_sh;
 
-    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const bool gelu = p.gated == 2;
@@ -148,6 +147,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncthreads();
     cluster_sync_all();                                  // the other CTA's barriers and tensor memory are there too
     tmem_fence_after();
+    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
 
     // tile -> first token row of the PAIR's tile, first output column

@@ -89,7 +89,6 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     __shared__ int abort_sh, tile_sh[3];
     volatile int* abort_flag = &abort_sh;
 
-    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_sh = 0;
@@ -123,6 +122,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
+    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     const int seq = tile_sh[0], tok0 = tile_sh[1], ntok = tile_sh[2];
     const int vhalf = place % a.value_halves;

@@ -135,7 +135,9 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
-// Tensor-memory allocation by one whole warp; the base address lands in *slot (shared memory).
+// Tensor-memory allocation by one whole warp; the base address lands in *slot (shared memory). It waits, without a limit, for columns
+// that other blocks of the SM hold. A block of the next grid holds its own until this grid has ended (ti_grid_wait), so a kernel calls
+// ti_grid_launch_dependents only behind the barrier after its allocation: none of its blocks can be left waiting for such columns then.
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
