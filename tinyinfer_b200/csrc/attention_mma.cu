@@ -310,6 +310,7 @@ __global__ void __launch_bounds__(THREADS) decode_attention_kernel(const __grid_
                     load_tile<D>(&kv_map, p, table, it.kvh, t, smem_u32(smem + s * S::STAGE_BYTES), bar0 + 8u * s);
                 }
             }
+            if (!ok) land_copies(abort_flag);
         }
         return;
     }
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(THREADS) decode_attention_kernel(const __grid_
         for (int v = item.tile0; v < item.tile1; ++v, ++n) {
             const int t = KEEP ? ti_nth_tile(v, item.kept, item.lo_tile) : item.lo_tile + v;
             const int s = n % STAGES;
-            if (!mbar_wait(bar0 + 8u * s, (n / STAGES) & 1u, abort_flag, p.status, 22)) return;
+            if (!mbar_wait(bar0 + 8u * s, (n / STAGES) & 1u, abort_flag, p.status, 22)) { land_copies(abort_flag); return; }
             uint8_t* k_tile = smem + s * S::STAGE_BYTES;
             uint8_t* v_tile = k_tile + S::TILE_BYTES;
             const int w0 = warp * 16;                         // this warp's 16 keys of the tile

@@ -419,6 +419,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
+        land_copies(abort_flag);
         tmem_dealloc(tmem_base, S::TMEM_COLS);
     }
 }

@@ -195,11 +195,7 @@ __global__ void __launch_bounds__((MAX_WARPS + 1) * 32) walk_kernel(Args a) {
         if (lane == 0) {
             for (int j = 0; j < nq; ++j) {
                 const int s = j % STAGES;
-                if (!mbar_wait(empty(s), ((j / STAGES) & 1u) ^ 1u, abort_flag, a.status, 91)) {
-                    const unsigned long long since = global_ns();        // the copies in flight land before shared memory is given up
-                    while (global_ns() - since < 1000000ull) {}
-                    break;
-                }
+                if (!mbar_wait(empty(s), ((j / STAGES) & 1u) ^ 1u, abort_flag, a.status, 91)) break;
                 const size_t item = (size_t)(first + j) * a.heads + h;
                 const uint32_t dst = smem_u32(smem + (size_t)s * stage_floats);
                 mbar_expect_tx(full(s), (uint32_t)stage_floats * 4u);
@@ -334,6 +330,7 @@ __global__ void __launch_bounds__((MAX_WARPS + 1) * 32) walk_kernel(Args a) {
                 }
     }
     __syncthreads();
+    if (warp == warps) land_copies(abort_flag);
     ti_grid_launch_dependents();                         // only now (a block's first thread speaks for it): the walk is long, and the next
 }                                                        // kernel's blocks would sit on the SMs through it
 

@@ -80,10 +80,6 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                     tma_load_2d(a_dst + GT_BM * GT_BK * 2, &map_w, full_bar(s), kb * GT_BK, w_row);
                 }
             }
-            if (!ok) {                                     // let the copies in flight land before shared memory is given up
-                const unsigned long long t0 = global_ns();
-                while (global_ns() - t0 < 1000000ull) {}
-            }
         }
     } else if (warp == 1) {
         {
@@ -169,6 +165,7 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
+        land_copies(abort_flag);
         tmem_dealloc(tmem_base, 2 * GT_BN);
     }
 }

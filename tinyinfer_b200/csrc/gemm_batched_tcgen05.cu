@@ -50,11 +50,7 @@ kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtens
         if (lane == 0) {
             for (int kb = 0; kb < blocks; ++kb) {
                 const int s = kb % STAGES;
-                if (!mbar_wait(empty(s), ((kb / STAGES) & 1u) ^ 1u, abort_flag, p.status, 94)) {
-                    const unsigned long long t0 = global_ns();           // the copies in flight land before shared memory is given up
-                    while (global_ns() - t0 < 1000000ull) {}
-                    break;
-                }
+                if (!mbar_wait(empty(s), ((kb / STAGES) & 1u) ^ 1u, abort_flag, p.status, 94)) break;
                 mbar_expect_tx(full(s), STAGE_BYTES);
                 const uint32_t dst = smem_u32(stages + s * STAGE_BYTES);
                 tma_load_2d(dst, &map_x, full(s), b * p.sx + kb * BK, m0);
@@ -107,6 +103,7 @@ kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtens
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
+        land_copies(abort_flag);
         tmem_dealloc(tmem_base, BN);
     }
 }

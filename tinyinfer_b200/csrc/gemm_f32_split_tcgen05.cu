@@ -348,18 +348,13 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             ti_grid_wait();
             int s = 0;
             uint32_t phase = 0;
-            bool ok = true;
             for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(b_empty_bar(s), phase ^ 1u, abort_flag, p.status, 83)) { ok = false; break; }
+                if (!mbar_wait(b_empty_bar(s), phase ^ 1u, abort_flag, p.status, 83)) break;
                 mbar_expect_tx(b_full_bar(s), 3 * plane_b);
                 const uint32_t b = smem_u32(b_ring) + s * 3 * plane_b;
                 // rows past M of a plane are the next plane's, or zeros: columns that nothing reads
                 for (int q = 0; q < 3; ++q) tma_load_2d(b + q * plane_b, &map_x, b_full_bar(s), kb * BK, q * p.M + m0);
                 if (++s == p.b_stages) { s = 0; phase ^= 1u; }
-            }
-            if (!ok) {       // give the copies still in flight time to land before shared memory is given up
-                const unsigned long long t0 = global_ns();
-                while (global_ns() - t0 < 1000000ull) {}
             }
         }
     } else if (warp == W_WARP) {
@@ -368,19 +363,14 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             if (!p.early) ti_grid_wait();
             int slot = 0;
             uint32_t phase = 0;
-            bool ok = true;
             for (int kb = kb0; kb < kb1; ++kb) {
-                if (!mbar_wait(w_empty_bar(slot), phase ^ 1u, abort_flag, p.status, 88)) { ok = false; break; }
+                if (!mbar_wait(w_empty_bar(slot), phase ^ 1u, abort_flag, p.status, 88)) break;
                 mbar_expect_tx(w_full_bar(slot), SLOT);
                 const uint32_t d = smem_u32(slot_ring) + slot * SLOT;
                 // rows past N are the other half's, or zeros: outputs that nothing stores
                 tma_load_2d(d, &map_w, w_full_bar(slot), kb * BK, n0);
                 tma_load_2d(d + SLOT / 2, &map_w, w_full_bar(slot), kb * BK, p.gated ? p.N + n0 : n0 + 64);
                 if (++slot == p.slots) { slot = 0; phase ^= 1u; }
-            }
-            if (!ok) {
-                const unsigned long long t0 = global_ns();
-                while (global_ns() - t0 < 1000000ull) {}
             }
         }
     } else {
@@ -470,6 +460,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     else __syncthreads();
     if (warp == MMA_WARP) {
         tmem_fence_after();
+        land_copies(abort_flag);
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (odd_sh) finish_odd(p, sums, odd);

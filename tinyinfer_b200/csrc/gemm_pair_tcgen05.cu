@@ -195,10 +195,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                     issue_w(c0, kb, s);
                 }
             }
-            if (!ok) {       // give the copies still in flight time to land before shared memory is given up
-                const unsigned long long t0 = global_ns();
-                while (global_ns() - t0 < 1000000ull) {}
-            }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer (even CTA)
@@ -377,6 +373,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     cluster_sync_all();                  // nobody leaves while the other CTA's MMAs still read its shared memory or write its tensor memory
     if (warp == 1) {
         tmem_fence_after();
+        land_copies(abort_flag);
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }

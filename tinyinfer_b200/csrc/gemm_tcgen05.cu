@@ -213,12 +213,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
                     issue(r0, c0, kb, s, true, true);
                 }
             }
-            // After an abort, give the copies this CTA still has in flight time to land (they take
-            // microseconds) before shared memory is given up: a bounded wait of one millisecond.
-            if (!ok) {
-                const unsigned long long t0 = global_ns();
-                while (global_ns() - t0 < 1000000ull) {}
-            }
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -750,6 +744,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
+        land_copies(abort_flag);
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::TMEM_COLS) : "memory");
     }
 }

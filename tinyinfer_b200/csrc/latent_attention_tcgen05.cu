@@ -327,10 +327,6 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
         if (ok && num_tiles > 0) ok = __all_sync(0xffffffffu, mbar_wait(o_full, (num_tiles - 1) & 1u, abort_flag, a.status, 88));
         sum_xch[half][r] = l_run;
     }
-    if (warp == 0 && *abort_flag) {                                // let the copies in flight land before shared memory is given up
-        const unsigned long long t0 = global_ns();
-        while (global_ns() - t0 < 1000000ull) {}
-    }
     __syncthreads();                                               // every role has ended, well or not
     if (ok) {                                                      // the same for a whole warp
         tmem_fence_after();
@@ -371,6 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
+        land_copies(abort_flag);
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
 }

@@ -52,6 +52,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         }
     }
 }
+// After the barrier that ends a block's roles, by the warp that frees its tensor memory or leaves last (without such a barrier: by every
+// role that a wait ends): whichever wait ran out, copies and products may be in flight, and get a millisecond to land (they take
+// microseconds) before shared and tensor memory are given up.
+__device__ __forceinline__ void land_copies(volatile int* abort_flag) {
+    if (*abort_flag) {
+        const unsigned long long t0 = global_ns();
+        while (global_ns() - t0 < 1000000ull) {}
+    }
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
