@@ -12,15 +12,16 @@ def holders():
 
 
 @pytest.mark.parametrize("name", holders())
-def test_next_grid_begins_when_this_one_has_its_tensor_memory(name):
-    """A block of the next grid keeps the columns that it takes until this grid has ended: let go earlier, it could take those that a
-    block of this one still waits for."""
-    text = (CSRC / name).read_text()
-    alloc = re.search(r"tmem_alloc\(&|tcgen05\.alloc", text).start()
-    kernel = text.rindex("__global__", 0, alloc)
-    barrier = text.index("__syncthreads();", alloc)
-    assert "ti_grid_launch_dependents" not in text[kernel:barrier]
-    assert "ti_grid_launch_dependents();" in text[barrier:text.index("\n}\n", barrier)]
+def test_blocks_that_may_share_an_sm_find_their_tensor_memory(name):
+    """Every kernel's columns and shared memory are held to the rule that keeps an allocation from waiting for a later grid's block, and
+    the rule itself leaves no such meeting: an SM has 228 KB, a block 1 KB more than it asks for, and 512 columns."""
+    assert "static_assert(tmem_shares_sm(" in (CSRC / name).read_text()
+    header = (CSRC / "sm100_ptx.cuh").read_text()
+    least = int(re.search(r"TMEM_SHARED_LEAST = (\d+) \* 1024", header).group(1))
+    assert "TMEM_SHARED_ALONE = 228 * 1024 - TMEM_SHARED_LEAST;" in header
+    assert "shared >= TMEM_SHARED_ALONE || (columns <= 128 && shared >= TMEM_SHARED_LEAST)" in header
+    alone = 228 - least
+    assert 3 * (least + 1) > 228 and (alone + 1) + (least + 1) > 228 and 2 * 128 <= 512
 
 
 @pytest.mark.parametrize("name", sorted(p.name for p in CSRC.glob("*.cu") if re.search(r"tma_load_2d(_pair)?\(|bulk_load\(dst", p.read_text())))

@@ -84,9 +84,10 @@ struct PpSmem {
     static constexpr int HALVES = D / 64;
     static constexpr int Q_BYTES = HALVES * QM * 128;          // one query tile
     static constexpr int KV_TILE = HALVES * KT * 128;          // keys OR values of a tile
-    static constexpr int BYTES = 1024 + 2 * Q_BYTES + NBUF * KV_TILE + 256;
+    static constexpr int USED = 1024 + 2 * Q_BYTES + NBUF * KV_TILE + 256, BYTES = USED < TMEM_SHARED_ALONE ? TMEM_SHARED_ALONE : USED;
     // tensor memory: S_A at 0, S_B at 128 (P_X over columns 0..31 and 64..95 of S_X), O_A at 256, O_B at 256 + D
     static constexpr int TMEM_COLS = 512;
+    static_assert(tmem_shares_sm(TMEM_COLS, BYTES), "heads of 64 use less: see TMEM_SHARED_ALONE");
 };
 
 __device__ __forceinline__ float ex2(float x) {          // 2^x, flushing; inputs are finite or -inf
@@ -155,6 +156,7 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
     __shared__ float inv_sh[FORM == 2 ? 2 : 1][FORM == 2 ? QM : 1], ss_sh[FORM == 2 ? 2 : 1][FORM == 2 ? QM : 1];
     volatile int* abort_flag = &abort_sh;
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_sh = 0;
@@ -167,7 +169,6 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     ti_grid_wait();                                     // q, the pages and the tables come from earlier kernels
 

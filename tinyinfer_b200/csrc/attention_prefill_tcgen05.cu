@@ -53,8 +53,9 @@ struct PfSmem {
     static constexpr int KV_TILE = HALVES * KT * 128;         // keys OR values of a tile
     static constexpr int STAGE = 2 * KV_TILE;
     static constexpr int P_BYTES = (KT / 64) * QM * 128;
-    static constexpr int BYTES = 1024 + Q_BYTES + KV_STAGES * STAGE + P_BYTES + 256;
+    static constexpr int USED = 1024 + Q_BYTES + KV_STAGES * STAGE + P_BYTES + 256, BYTES = USED < TMEM_SHARED_ALONE ? TMEM_SHARED_ALONE : USED;
     static constexpr int TMEM_COLS = 512;                     // S0 at 0, S1 at 128, O_j at 256
+    static_assert(tmem_shares_sm(TMEM_COLS, BYTES), "heads of 64 use less: see TMEM_SHARED_ALONE");
 };
 
 __device__ __forceinline__ float ex2(float x) {          // 2^x, flushing; inputs are <= 0 or -inf
@@ -114,6 +115,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     __shared__ int abort_sh;
     volatile int* abort_flag = &abort_sh;
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_sh = 0;
@@ -132,7 +134,6 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     ti_grid_wait();                                     // q, the pages and the tables come from earlier kernels
 

@@ -20,6 +20,7 @@ template <int BN> struct GtShape {
     static constexpr int STAGES = BN == 128 ? 5 : 4;
     static constexpr int STAGE_BYTES = (GT_BM + BN) * GT_BK * 2;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+    static_assert(tmem_shares_sm(2 * BN, SMEM), "two accumulators");
 };
 
 struct GtParams {
@@ -46,6 +47,7 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     __shared__ int abort_sh;
     volatile int* abort_flag = &abort_sh;
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) abort_sh = 0;
     if (threadIdx.x < 2 * GT_STAGES + 4) {
@@ -56,7 +58,6 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     ti_grid_wait();                                        // the plan, the sorted rows and `out` belong to earlier kernels until now
     const int num_units = p.num_tiles[0] * p.col_tiles;   // a unit: row tile (unit / col_tiles), column tile (unit % col_tiles)

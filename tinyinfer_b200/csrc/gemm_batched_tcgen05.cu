@@ -11,6 +11,7 @@
 namespace gbt {
 constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3, THREADS = 192;
 constexpr int STAGE_BYTES = (BM + BN) * BK * 2, SMEM = 1024 + STAGES * STAGE_BYTES;
+static_assert(tmem_shares_sm(BN, SMEM), "one accumulator");
 
 struct Args {
     void* out;
@@ -31,6 +32,7 @@ kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtens
     const uint32_t bar0 = smem_u32(bars), done = bar0 + 16u * STAGES;
     auto full = [&](int s) { return bar0 + 8u * s; };
     auto empty = [&](int s) { return bar0 + 8u * (STAGES + s); };
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_sh = 0;
@@ -42,7 +44,6 @@ kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtens
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM, b = blockIdx.z, blocks = p.K / BK;
     ti_grid_wait();

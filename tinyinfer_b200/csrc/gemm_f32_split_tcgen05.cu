@@ -53,6 +53,7 @@ constexpr int MAX_SLOTS = 6;                     // fetched weights; like A_STAG
 constexpr int W_WARP = DRAIN_WARPS + SPLIT_WARPS, X_WARP = W_WARP + 1, MMA_WARP = W_WARP + 2;
 constexpr int NUM_THREADS = (MMA_WARP + 1) * 32;
 constexpr int SMEM_BYTES = 226 * 1024;           // beside the barriers, of 227 KB
+static_assert(tmem_shares_sm(TMEM_COLS, SMEM_BYTES), "all of tensor memory");
 
 struct SplitParams {
     float* out;
@@ -246,6 +247,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     auto w_full_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + 2 * MAX_B_STAGES + s); };
     auto w_empty_bar = [&](int s) { return bar0 + 8u * (4 + 2 * A_STAGES + 2 * MAX_B_STAGES + MAX_SLOTS + s); };
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int splits = (int)gridDim.x, part = (int)blockIdx.x;           // the cluster spans gridDim.x
     const int outs = p.gated ? 64 : 128;
@@ -269,7 +271,6 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     float* sums = reinterpret_cast<float*>(smem);            // [bn][128], once the stages are done with
 

@@ -34,6 +34,7 @@ constexpr int STAGES = 6;
 constexpr int STAGE_BYTES = (BM + BN / 2) * BK * 2;          // 32 KB: 128 rows of x, 128 rows of w
 constexpr int NUM_THREADS = 192;
 constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + 256;
+static_assert(tmem_shares_sm(512, SMEM_BYTES), "all of tensor memory");
 
 struct PairGemmParams {
     void* out;
@@ -122,6 +123,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __shared__ int abort_sh;
     volatile int* abort_flag = &abort_sh;
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const bool gelu = p.gated == 2;
@@ -147,7 +149,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     __syncthreads();
     cluster_sync_all();                                  // the other CTA's barriers and tensor memory are there too
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
 
     // tile -> first token row of the PAIR's tile, first output column

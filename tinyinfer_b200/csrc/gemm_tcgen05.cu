@@ -89,6 +89,7 @@ struct Cfg {
     static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + EXCH_FLOATS * 4 + 256;
     static_assert(STAGES >= 2, "too little shared memory for a pipeline");
     static_assert(CTAS_PER_SM * (SMEM_BYTES + 1024) <= 227 * 1024, "the CTAs of an SM do not fit its shared memory");
+    static_assert(tmem_shares_sm(TMEM_COLS, SMEM_BYTES), "the columns of the kernels that an SM may hold");
 };
 
 // SWAP: weights on the lanes (a compile-time choice, so that a decode step's kernels carry none of the code for many tokens).
@@ -113,6 +114,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     __shared__ float row_scale_sh[128];     // scale_*: 1 / rms of every token of the tile (1 if no scale)
     volatile int* abort_flag = &abort_sh;
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // tiles: gated normal tiles hold BN/2 gate and BN/2 up columns; gated swapped tiles 64 + 64 rows
     const bool gelu = p.gated == 2;
@@ -151,7 +153,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
 
     if (warp == 0) {

@@ -67,7 +67,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 }
 // The rows' chunks on their way to tensor memory wait in the ring behind its first tile.
 int tmem_chunks(int chunks) { return std::min(MAX_TMEM_CHUNKS, (STAGES - 1) * chunks * KT / QM); }
-int smem_bytes(int chunks) { return 1024 + (chunks - tmem_chunks(chunks)) * (QM * 128) + STAGES * chunks * (KT * 128) + 128; }
+int smem_bytes(int chunks) {                                          // small ranks use less than all of tensor memory asks for
+    return std::max(TMEM_SHARED_ALONE, 1024 + (chunks - tmem_chunks(chunks)) * (QM * 128) + STAGES * chunks * (KT * 128) + 128);
+}
+static_assert(tmem_shares_sm(TMEM_COLS, TMEM_SHARED_ALONE), "smem_bytes");
 
 // NV: value features of a CTA.
 template <int NV>
@@ -89,6 +92,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     __shared__ int abort_sh, tile_sh[3];
     volatile int* abort_flag = &abort_sh;
 
+    ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         abort_sh = 0;
@@ -122,7 +126,6 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
-    ti_grid_launch_dependents();                         // not before this grid has its tensor memory
     const uint32_t tmem_base = tmem_base_sh;
     const int seq = tile_sh[0], tok0 = tile_sh[1], ntok = tile_sh[2];
     const int vhalf = place % a.value_halves;

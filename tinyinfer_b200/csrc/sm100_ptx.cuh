@@ -144,9 +144,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 #pragma unroll
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
-// Tensor-memory allocation by one whole warp; the base address lands in *slot (shared memory). It waits, without a limit, for columns
-// that other blocks of the SM hold. A block of the next grid holds its own until this grid has ended (ti_grid_wait), so a kernel calls
-// ti_grid_launch_dependents only behind the barrier after its allocation: none of its blocks can be left waiting for such columns then.
+// An allocation of tensor memory waits, without a limit, for columns that other blocks of the SM hold, and a block of the next grid, let
+// in early, holds its own until this grid has ended (ti_grid_wait): a block of this grid that such a one overtook would wait for ever. So
+// what may meet on an SM never needs more than its 512 columns. Every kernel with tensor memory has at least LEAST bytes of dynamic shared
+// memory, so that no three share an SM's 228 KB (two of them 256 columns at most), and one with more than 128 columns has ALONE, which
+// leaves less than LEAST beside it. (Letting the next grid in only behind the allocation would do too, but made a decoded token of the
+// 0.6B model 1,016 -> 1,029 us, its prompt of 37 tokens 1,300 -> 1,311.)
+constexpr int TMEM_SHARED_LEAST = 95 * 1024, TMEM_SHARED_ALONE = 228 * 1024 - TMEM_SHARED_LEAST;
+constexpr bool tmem_shares_sm(int columns, int shared) { return shared >= TMEM_SHARED_ALONE || (columns <= 128 && shared >= TMEM_SHARED_LEAST); }
+// Tensor-memory allocation by one whole warp; the base address lands in *slot (shared memory).
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
