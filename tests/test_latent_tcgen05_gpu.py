@@ -55,3 +55,37 @@ def test_portions_on_tcgen05(monkeypatch, heads, rank, rot, page, sink, work):
     # two roundings to 8 bits, of the probabilities and of the result: at most 2^-9 of the result's norm each
     err, err_old = ((x - want).norm() / want.norm() for x in (new, old))
     assert err <= 2.0 ** -8 and err <= 1.02 * err_old + 1e-5, (err, err_old)
+
+
+@pytest.mark.parametrize("heads,rank,rot,page,work,at", [
+    (16, 512, 64, 64, [(75, 75), (33, 9)], 42),                      # 8 tokens a row tile, two CTAs
+    (16, 512, 64, 64, [(1500, 16)], 1491),                           # keys shared out over CTAs
+    (3, 64, 8, 48, [(300, 100), (64, 1)], 231),                      # 42 tokens a row tile, whose keys lie in three tiles
+    (1, 128, 0, 16, [(160, 160)], 64),
+])
+@pytest.mark.parametrize("value,feature", [(float("nan"), 3), (float("inf"), 40), (float("-inf"), 63), (float("inf"), -1)])
+def test_a_value_that_is_no_number_reaches_no_token_before_its_own(monkeypatch, heads, rank, rot, page, work, at, value, feature):
+    from tinyinfer_b200 import ops
+    from tinyinfer_b200.engine.batch import BatchBuffers, StepEntry
+    gen = torch.Generator().manual_seed(heads + at)
+    dk, pages = rank + rot, [-(-c // page) for c, _ in work]
+    tables = [list(range(sum(pages[:i]), sum(pages[:i + 1]))) for i in range(len(work))]
+    cache = torch.randn(1, sum(pages), 1, page, dk, generator=gen).bfloat16()
+    buffers = BatchBuffers(torch.device("cuda"), sum(n for _, n in work), len(work), max(pages), 1)
+    step = buffers.build([StepEntry(i, [0] * n, []) for i, (_, n) in enumerate(work)], [c - n for c, n in work], [0] * len(work), [tables])
+    q = torch.randn(step.num_tokens, heads * dk, generator=gen).bfloat16()
+
+    def run(rows):
+        return ops.latent_attention(q.cuda() if ops.LATENT_TCGEN05 else q.float().cuda(), rows.cuda(), heads=heads, rank=rank, rot=rot,
+                                    scale=dk ** -0.5, sink=None, positions=step.positions, token_seq=step.token_seq,
+                                    block_table=step.block_tables[0], max_context=max(c for c, _ in work), step=step).cpu()
+
+    spoiled = cache.clone()
+    spoiled[0, at // page, 0, at % page, feature] = value             # of the first request's token at position `at`
+    clean, got = run(cache), run(spoiled)
+    monkeypatch.setattr(ops, "LATENT_TCGEN05", False)
+    warp_level = run(spoiled)
+    ops.check_kernel_status()
+    row, end = at - (work[0][0] - work[0][1]), work[0][1]             # the token's place in the step
+    assert torch.equal(got[:row], clean[:row]) and torch.equal(got[end:], clean[end:])
+    assert torch.equal(got[row:end].isnan(), warp_level[row:end].isnan()) and got[row:end].isnan().any()

@@ -31,6 +31,7 @@ struct Args {
     __nv_bfloat16* out;
     float* parts;
     const float* q;                                               // null: the rows come as bfloat16, by TMA
+    const __nv_bfloat16* cache;
     const float* sink;
     const int *positions, *cu_seqlens, *block_table;
     int max_blocks, num_seqs, heads, rank, rot, page_size, num_pages, piece_rows;
@@ -65,6 +66,32 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
+// 8 bfloat16 without those that are infinite or NaN; says whether there were any.
+__device__ __forceinline__ bool drop_odd(uint4& u) {
+    uint32_t* w = &u.x;
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool lo = (w[i] & 0x7f80u) == 0x7f80u, hi = (w[i] & 0x7f800000u) == 0x7f800000u;
+        w[i] &= (lo ? 0xffff0000u : ~0u) & (hi ? 0xffffu : ~0u);
+        odd |= lo || hi;
+    }
+    return odd;
+}
+// Which of 32 value features, the first of them at `values` of a row of dk, are infinite or NaN in any of the keys key0 .. key1 - 1 of the
+// request whose pages `table` holds.
+__device__ __noinline__ uint32_t odd_features(const __nv_bfloat16* values, int dk, const int* table, int max_blocks, int page_size, int num_pages,
+                                              int key0, int key1) {
+    uint32_t odd = 0;
+    for (int key = key0; key < key1; ++key) {
+        const int logical = key / page_size, page = logical < max_blocks ? table[logical] : -1;
+        if (page < 0 || page >= num_pages) continue;
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(values + ((size_t)page * page_size + key % page_size) * dk);
+        for (int i = 0; i < 16; ++i)
+            odd |= ((row[i] & 0x7f80u) == 0x7f80u ? 1u : 0u) << (2 * i) | ((row[i] & 0x7f800000u) == 0x7f800000u ? 2u : 0u) << (2 * i);
+    }
+    return odd;
+}
 // The rows' chunks on their way to tensor memory wait in the ring behind its first tile.
 int tmem_chunks(int chunks) { return std::min(MAX_TMEM_CHUNKS, (STAGES - 1) * chunks * KT / QM); }
 int smem_bytes(int chunks) {                                          // small ranks use less than all of tensor memory asks for
@@ -89,13 +116,13 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     auto kv_empty = [&](int s) { return bar0 + 8u * (7 + STAGES + s); };
     __shared__ uint32_t tmem_base_sh;
     __shared__ float sum_xch[2][QM];
-    __shared__ int abort_sh, tile_sh[3];
+    __shared__ int abort_sh, odd_sh, tile_sh[3];
     volatile int* abort_flag = &abort_sh;
 
     ti_grid_launch_dependents();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        abort_sh = 0;
+        abort_sh = odd_sh = 0;
         mbar_init(q_full, 8);
         mbar_init(q_landed, 1);
         for (int s = 0; s < STAGES; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
@@ -130,8 +157,9 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     const int seq = tile_sh[0], tok0 = tile_sh[1], ntok = tile_sh[2];
     const int vhalf = place % a.value_halves;
     const int dk = a.rank + a.rot, h0 = blockIdx.y * a.hpb;
-    int first_key = 0, last_key = 0;
+    int first_key = 0, last_key = 0, common = 0;                  // keys below `common` are seen by every row
     if (seq >= 0) {
+        common = a.positions[tok0] + 1;
         last_key = a.positions[tok0 + ntok - 1] + 1;
         if (a.splits > 1) {
             const int per = ((last_key + a.splits - 1) / a.splits + KT - 1) / KT * KT;
@@ -145,6 +173,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     const uint32_t lane_addr = tmem_base + ((uint32_t)(lane_group * 32) << 16);
     const int tl = r / a.hpb, head = h0 + r % a.hpb;
     const bool live = warp >= 2 && tl < ntok && head < a.heads;
+    const int pos = live ? a.positions[tok0 + tl] : -1;
     constexpr int KH = KT / 2, VH = NV / 2;
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = warp >= 2 && seq >= 0;
@@ -264,7 +293,6 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             __syncwarp();
             if (lane == 0) mbar_arrive(q_full);
         }
-        const int pos = live ? a.positions[tok0 + tl] : -1;
         for (int j = 0; j < num_tiles && ok; ++j) {
             const int b = j & 1, key0 = first_key + j * KT;
             // a warp's threads stay together: tensor memory is read and written by whole warps
@@ -312,13 +340,20 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
                 }
             }
             tmem_st8(lane_addr + P_COL + half * 8, pk);
-            // value rows past the last key: whatever the page holds there must not meet a probability of zero
-            if (key0 + KT > last_key) {
+            // Values that not every row sees must not meet a probability of zero: those past the last key, whatever the page holds
+            // there, become zero, and so do infinities and NaN among those that only some rows see. These rows get them at the end.
+            if (key0 + KT > common) {
                 uint8_t* v_tile = ring + (j % STAGES) * stage_bytes + vhalf * (NV / 64) * (KT * 128);
                 for (int i = etid; i < KT * (NV / 8); i += 256) {
                     const int row = i / (NV / 8), c = i % (NV / 8);
-                    if (row >= last_key - key0)
-                        *reinterpret_cast<uint4*>(v_tile + (c >> 3) * (KT * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
+                    if (row < common - key0) continue;
+                    uint4* at = reinterpret_cast<uint4*>(v_tile + (c >> 3) * (KT * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4));
+                    if (row >= last_key - key0) {
+                        *at = make_uint4(0, 0, 0, 0);
+                    } else {
+                        uint4 u = *at;
+                        if (drop_odd(u)) { *at = u; odd_sh = 1; }
+                    }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
@@ -352,6 +387,14 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             } else {
 #pragma unroll
                 for (int i = 0; i < 32; ++i) o[i] = 0.f;
+            }
+            if (odd_sh && live) {
+                // a seen value of infinity makes its sum NaN whatever its probability: its key's score is infinite or NaN, so that
+                // is 0 or NaN
+                const uint32_t odd = odd_features(a.cache + col0 + cc, dk, a.block_table + (size_t)seq * a.max_blocks, a.max_blocks, a.page_size,
+                                                  a.num_pages, max(first_key, common), min(pos + 1, last_key));
+#pragma unroll
+                for (int i = 0; i < 32; ++i) if (odd >> i & 1u) o[i] = NAN;
             }
             if (live && part) {
 #pragma unroll
@@ -407,7 +450,7 @@ TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, 
                "latent_attend_tc: scratch too small for %d splits", splits);
     TI_REQUIRE((long long)num_pages * page_size < (1ll << 31) - 65536, "latent_attend_tc: too many cached rows");
     lt::Args a;
-    a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q_bf16 ? nullptr : (const float*)q; a.sink = sink; a.positions = positions; a.cu_seqlens = cu_seqlens;
+    a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q_bf16 ? nullptr : (const float*)q; a.cache = (const __nv_bfloat16*)cache; a.sink = sink; a.positions = positions; a.cu_seqlens = cu_seqlens;
     a.block_table = block_table; a.max_blocks = max_blocks; a.num_seqs = num_seqs; a.heads = heads; a.rank = rank; a.rot = rot;
     a.page_size = page_size; a.num_pages = num_pages; a.scale = scale; a.splits = splits; a.status = status;
     a.hpb = heads < lt::QM ? heads : lt::QM;
