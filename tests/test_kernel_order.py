@@ -30,12 +30,17 @@ def test_copies_land_whichever_wait_ran_out(name):
     last barrier, and shared and tensor memory are given up only then."""
     text = (CSRC / name).read_text()
     assert "1000000ull" not in text
-    if name == "attention_mma.cu":                       # no such barrier: every role that a wait ends stays for them itself
+    if name == "attention_mma.cu":                       # no barrier ends the roles: every one that a wait ends stays itself
         waits = re.findall(r"if \(!mbar_wait\(.*\)\) (.*)", text)
         assert waits == ["{ ok = false; break; }", "{ land_copies(abort_flag); return; }"] and "if (!ok) land_copies(abort_flag);" in text
         return
     assert text.count("land_copies(abort_flag);") == 1
     land = text.index("land_copies(abort_flag);")
+    if "if (!ok) land_copies(abort_flag);" in text:      # the warp that issues the MMAs, which waits for every copy
+        role = text[text.rindex("elect_one()", 0, land):land]
+        assert "mbar_wait_warp(" in role and not re.search(r"\bmbar_wait\(", role)
+        assert role.count("if (!mbar_wait_warp(") == role.count("{ ok = false; break; }")      # no wait that does not end it
+        return
     assert text.rindex("mbar_wait", 0, land) < text.rindex("sync", 0, land)             # every role's waits, the barrier, the look
     freed = re.search(r"tmem_dealloc\(|tcgen05\.dealloc", text)
     assert freed is None or land < freed.start()

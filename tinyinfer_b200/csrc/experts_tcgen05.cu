@@ -108,6 +108,7 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                 }
                 if (ok && leader) umma_commit(acc_full_bar(as));
             }
+            if (!ok) land_copies(abort_flag);
         }
     } else {
         const int lane_group = warp & 3;                   // the 32 accumulator lanes this warp may read
@@ -166,7 +167,6 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
-        land_copies(abort_flag);
         tmem_dealloc(tmem_base, 2 * GT_BN);
     }
 }

@@ -74,6 +74,7 @@ kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtens
             if (leader) umma_commit(empty(s));
         }
         if (ok && leader) umma_commit(done);
+        if (!ok) land_copies(abort_flag);
     } else if (mbar_wait_warp(done, 0, abort_flag, p.status, 96)) {
         tmem_fence_after();
         const int lane_group = warp & 3, m = m0 + lane_group * 32 + lane;
@@ -104,7 +105,6 @@ kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtens
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
-        land_copies(abort_flag);
         tmem_dealloc(tmem_base, BN);
     }
 }

@@ -414,6 +414,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             }
             if (ok && leader) umma_commit(acc_full_bar(a));
         }
+        if (!ok) land_copies(abort_flag);
     }
 
     // ---------------------------------------------------------------- the cluster's parts meet; epilogue and store
@@ -461,7 +462,6 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     else __syncthreads();
     if (warp == MMA_WARP) {
         tmem_fence_after();
-        land_copies(abort_flag);
         tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (odd_sh) finish_odd(p, sums, odd);

@@ -223,6 +223,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
                 if (ok && leader) umma_commit_pair(acc_full_bar(as));  // the accumulator is complete, in both CTAs
             }
+            if (!ok) land_copies(abort_flag);                // the other CTA waits for this one at the exit
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
@@ -374,7 +375,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     cluster_sync_all();                  // nobody leaves while the other CTA's MMAs still read its shared memory or write its tensor memory
     if (warp == 1) {
         tmem_fence_after();
-        land_copies(abort_flag);
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
     }
 }

@@ -250,6 +250,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
                 }
                 if (ok && leader) umma_commit(acc_full_bar(as));   // the accumulator is complete
             }
+            if (!ok) land_copies(abort_flag);
         }
     } else {
         // ------------------------------------------------------------ epilogue (warps 2..5)
@@ -745,7 +746,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     __syncthreads();
     if (warp == 1) {
         tmem_fence_after();
-        land_copies(abort_flag);
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)C::TMEM_COLS) : "memory");
     }
 }

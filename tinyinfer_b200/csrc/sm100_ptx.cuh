@@ -52,9 +52,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         }
     }
 }
-// After the barrier that ends a block's roles, by the warp that frees its tensor memory or leaves last (without such a barrier: by every
-// role that a wait ends): whichever wait ran out, copies and products may be in flight, and get a millisecond to land (they take
-// microseconds) before shared and tensor memory are given up.
+// Whichever wait of a block ran out, copies may be in flight, and get a millisecond to land (they take microseconds) before shared and
+// tensor memory are given up. Where one warp waits for every copy, as the warp that issues a product's MMAs does, it alone knows whether
+// they have landed, and stays when a wait ended it; elsewhere the warp that frees tensor memory looks behind the barrier that ends the
+// roles, or, without such a barrier, every role that a wait ended stays. (That look in the products of few tokens: the 0.6B model's prompt
+// of 37 tokens 1,303 -> 1,310 us, with 112 of them.)
 __device__ __forceinline__ void land_copies(volatile int* abort_flag) {
     if (*abort_flag) {
         const unsigned long long t0 = global_ns();
