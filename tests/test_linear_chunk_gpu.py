@@ -37,6 +37,9 @@ def test_chunks_against_plain(monkeypatch, heads, groups, dk, dv, gate, lens, dt
                               state_slots=torch.arange(n, 0, -1, dtype=torch.int32).cuda(), num_seqs=n, max_q_len=max(lens))
         return out.cpu().double().view(T, heads, dv), state.cpu().double()
 
+    from tinyinfer_b200.ops import _dtype_code, _fn
+    at = [x for offset in (pad, pad + groups * dk, pad + 2 * groups * dk) for x in (0, row.shape[1], offset)]       # address (any on 16 bytes), row, offset
+    assert ops.linear_chunks(T, n, max(lens), heads, dk, dv) and _fn("hybrid", "ti_linear_scan_chunks_ok")(*at, dk, dv, _dtype_code(row))
     got, state = run(True)
     walk, walk_state = run(False)
     ops.check_kernel_status()
@@ -78,6 +81,7 @@ def test_chunks_hold_any_division_and_look_at_no_later_token():
                               num_seqs=len(lens), max_q_len=longest)
         return out, state
 
+    assert all(ops.linear_chunks(sum(lens), len(lens), longest, heads, dk, dk) for longest in (128, 700))
     out, state = run(row, 700)
     again, state_again = run(row, 128)
     assert torch.equal(out, again) and torch.equal(state, state_again)

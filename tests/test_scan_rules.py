@@ -1,0 +1,28 @@
+"""Which form the recurrences' steps take, from host numbers alone: on each side of the lines, with what both forms were measured to take."""
+import pytest
+
+from tinyinfer_b200 import ops
+
+ONE = [1]
+
+
+@pytest.mark.parametrize("lens,heads,dim,chunked", [
+    ([128], 16, 128, True),                   # us in stretches and in chunks: 86, 64
+    ([127], 16, 128, False),
+    (ONE * 8 + [128], 16, 128, True),         # 152, 92
+    (ONE * 27 + [128], 16, 128, False),       # 162, 197
+    (ONE * 27 + [512], 16, 128, True),        # 547, 199
+    (ONE * 64 + [128], 16, 128, False),       # 182, 412
+    (ONE * 128 + [128], 16, 128, False),      # 221, 784
+    (ONE * 128 + [512], 16, 128, False),      # 610, 795
+    (ONE * 128 + [512], 4, 64, True),         # 392, 111
+    ([8] * 32 + [128], 32, 64, False),        # 131, 201
+    ([128] * 16, 16, 128, True),              # 371, 195
+    ([128] * 16, 32, 64, False),              # 158, 223
+    ([512] * 8, 32, 64, True),
+    (ONE * 250 + [256], 32, 64, False),       # 285, 1,278
+    ([4096] * 2, 64, 128, False),             # the chunks' states would take more than their share of memory
+])
+def test_linear_attention_in_chunks(lens, heads, dim, chunked):
+    tokens, n = sum(lens), len(lens)
+    assert ops.linear_chunks(tokens, n, max(lens), heads, dim, dim) == (tokens // 64 + n if chunked else 0)

@@ -1901,7 +1901,8 @@ class ScanGate:
 SCAN_MIN_STRETCH = 32        # tokens a stretch of a long portion has at least
 SCAN_CHUNK = 64              # tokens of a chunk where a head has one decay
 LINEAR_CHUNKS = True
-SCAN_CHUNK_MIN_TOKENS = 128  # 16 heads of 128 x 128, host included: 75 us in stretches, 48 in chunks; 64 tokens 64 in stretches, where chunks were not tried
+SCAN_CHUNK_MIN_TOKENS = 128  # 16 heads of 128 x 128: 86 us in stretches, 64 in chunks (8 heads of 64: 47, 49)
+SCAN_CHUNK_LIMIT = 820       # chunks x heads x (key + value channels) a token of the longest portion: see linear_chunks
 SCAN_CHUNK_MAX_FLOATS = 64 * 1024 * 1024     # states of the chunks: 256 MB
 SCAN_TARGET_BLOCKS = 148 * 7  # what runs side by side at 72 registers a thread: more blocks would wait for a second round
 
@@ -1916,6 +1917,24 @@ def scan_stretches(max_q_len: int, num_seqs: int, heads: int, key_dim: int, valu
         lanes *= 2
     blocks = num_seqs * heads * -(-value_dim // (4 * (32 // lanes)))
     return max(1, min(SCAN_TARGET_BLOCKS // blocks, max_q_len // SCAN_MIN_STRETCH, 64))
+
+
+def linear_chunks(tokens: int, num_seqs: int, longest: int, heads: int, key_dim: int, value_dim: int) -> int:
+    """The chunks of 64 tokens in which ``linear_scan`` runs a step with one decay a head, or 0: in stretches, token by token.
+
+    A chunk costs the same whatever it holds, and every request has one of its own, a decoded token too. The stretches take as long as
+    the longest portion, which many requests leave in few pieces; portions of 64 tokens and more on average fill their chunks, which
+    then win by their work, unless heads of up to 64 leave half of a tile empty. Measured, stretches and chunks in us (and what is held
+    against the limit of 820): 16 heads of 128, 512 tokens beside 27 decoded 547, 199 (288), 128 beside 8 152, 92 (352), 256 beside 48
+    299, 324 (848), 128 beside 27 162, 197 (960), 128 beside 128 221, 784 (4,256), 16 portions of 128 371, 195 (they fill theirs);
+    32 heads of 64, 512 beside 27 414, 187 (288), 8 of 512 488, 342 (576), 8 of 128 154, 119 (768), 256 beside 48 221, 277 (848),
+    128 beside 27 117, 176 (960), 16 of 128 158, 223 (1,536)."""
+    chunks = tokens // SCAN_CHUNK + num_seqs
+    if longest < SCAN_CHUNK_MIN_TOKENS or chunks > 65535 or chunks * heads * key_dim * value_dim > SCAN_CHUNK_MAX_FLOATS:
+        return 0
+    width = key_dim + value_dim
+    pays = chunks * heads * width <= SCAN_CHUNK_LIMIT * longest or (tokens >= SCAN_CHUNK * num_seqs and width > 128)
+    return chunks if pays else 0
 
 
 def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: ScanGate, *, state: torch.Tensor, heads: int,
@@ -1950,9 +1969,8 @@ def linear_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: ScanGat
         return out
     longest = t if num_seqs == 1 else max_q_len
     stretches, scratch = scan_stretches(max_q_len or t, num_seqs, heads, key_dim, value_dim), None
-    chunks = t // SCAN_CHUNK + num_seqs
-    chunked = (LINEAR_CHUNKS and not gate.per_channel and longest >= SCAN_CHUNK_MIN_TOKENS
-               and chunks * heads * key_dim * value_dim <= SCAN_CHUNK_MAX_FLOATS and chunks <= 65535
+    chunks = linear_chunks(t, num_seqs, longest, heads, key_dim, value_dim) if LINEAR_CHUNKS and not gate.per_channel else 0
+    chunked = (chunks > 0
                and int(_fn("hybrid", "ti_linear_scan_chunks_ok")(
                    q.data_ptr(), q.shape[1], q_offset, k.data_ptr(), k.shape[1], k_offset, v.data_ptr(), v.shape[1], v_offset,
                    key_dim, value_dim, _dtype_code(q))))
