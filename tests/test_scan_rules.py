@@ -26,3 +26,27 @@ ONE = [1]
 def test_linear_attention_in_chunks(lens, heads, dim, chunked):
     tokens, n = sum(lens), len(lens)
     assert ops.linear_chunks(tokens, n, max(lens), heads, dim, dim) == (tokens // 64 + n if chunked else 0)
+
+
+@pytest.mark.parametrize("lens,heads,dim,quads", [
+    ([68], 16, 128, True),
+    ([67], 16, 128, False),
+    ([1000], 16, 128, True),                  # us token by token and by quads: 289, 213
+    ([1000, 200, 200, 200], 16, 128, True),   # 391, 301
+    ([512] * 2, 16, 128, False),              # 205, 219
+    ([256] * 3, 16, 128, False),              # 141, 172
+    ([16] * 64, 16, 128, False),              # 238, 270
+    ([5] * 80, 16, 128, False),               # 176, 217
+    ([64] * 4, 16, 128, False),               # 65, 70
+    (ONE * 128 + [600], 16, 128, True),       # 424, 383
+    ([1000], 32, 128, False),                 # 391, 408
+    ([512] * 2, 32, 64, True),                # 164, 119
+    ([512] * 8, 32, 64, False),               # 389, 434
+    ([512] * 8, 4, 64, True),                 # 143, 102
+    ([128], 8, 256, False),                   # 70, 76
+    ([1000], 8, 256, True),                   # 431, 395
+    ([512] * 2, 8, 256, True),                # 500, 406
+    ([256] * 3, 8, 256, False),               # 299, 314
+])
+def test_delta_rule_by_quads(lens, heads, dim, quads):
+    assert ops.delta_quads_pay(lens, heads, dim, dim) is quads

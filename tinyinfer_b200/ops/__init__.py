@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import array
 import ctypes
-from typing import Optional
+from typing import Optional, Sequence
 
 import torch
 
@@ -2049,20 +2049,41 @@ def head_rotation(rows: torch.Tensor, *, num_heads: int, num_kv_heads: int, head
     return out if to_row else out.view(t, num_heads, maps * head_dim)
 
 
-DELTA_QUADS = True           # long portions four tokens at a time
+DELTA_QUADS: Optional[bool] = None     # four tokens at a time wherever that is taken (True), nowhere (False), where it was measured to be faster
+
+
+def delta_quads_pay(q_lens: Sequence[int], heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether the gated delta rule is faster four tokens at a time than token by token, for requests of these many tokens.
+
+    A quad shortens the chain of the longest portion and costs a little more work, so it pays while the blocks of the portions that last
+    (half of the longest at least) all run at a time and wait for themselves. Us token by token and by quads: 16 heads of 128, one portion of
+    1,000 tokens 289, 213 (128 blocks), beside three of 200 391, 301 (128), two of 512 205, 219 (256), three of 256 141, 172 (384), 64 of 16
+    238, 270; 32 heads of 128, 1,000 391, 408 (256); 32 heads of 64, 1,000 268, 188 (64), three of 256 119, 119 (192), eight of 512 389,
+    434 (512); 80 requests of 5 tokens 176, 217. Heads beyond 128 run half as many columns a block: 8 heads of 256, 1,000 tokens 431, 395 (256
+    blocks), two of 512 500, 406 (512), three of 256 299, 314 (768); alone up to 255 tokens they are slower (128: 70, 76)."""
+    longest = max(q_lens)
+    if longest < 68:                                 # what one request must bring: ti_delta_quads_floats
+        return False
+    lasting = sum(2 * n >= longest for n in q_lens)
+    blocks = lasting * heads * -(-value_dim // (32 if key_dim <= 64 else 16 if key_dim <= 128 else 8))
+    if key_dim > 128:
+        return blocks <= 512 and (longest >= 256 or len(q_lens) > 1)
+    return blocks <= 210
 
 
 def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logits: torch.Tensor, beta_logits: torch.Tensor,
                *, a_log: torch.Tensor, dt_bias: Optional[torch.Tensor], state: torch.Tensor, heads: int, groups: int,
                key_dim: int, value_dim: int, q_offset: int = 0, k_offset: int = 0, v_offset: int = 0,
                decay_offset: int = 0, beta_offset: int = 0, q_scale: float = 1.0, unit_eps: float = 1e-6,
-               cu_seqlens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int) -> torch.Tensor:
+               cu_seqlens: torch.Tensor, state_slots: torch.Tensor, num_seqs: int,
+               q_lens: Optional[Sequence[int]] = None) -> torch.Tensor:
     """The gated delta rule with a decay per head and key channel. Per request and head, over the step's tokens in
     order: S <- diag(g) S, u = beta (v - S^T k), S <- S + k u^T, o = S^T q, from and back into ``state`` float32
     [slots, heads, value_dim, key_dim] (S transposed). q and k (columns [offset, + groups * key_dim) of their tensors,
     head h reads group h // (heads / groups)) are made unit vectors, x / sqrt(sum x^2 + unit_eps), q also times
     ``q_scale``; g = exp(-exp(a_log[h]) * softplus(decay_logits[t, h, c] + dt_bias[h, c])) and
-    beta = sigmoid(beta_logits[t, h]) from float32 rows. Returns o float32 [T, heads * value_dim]."""
+    beta = sigmoid(beta_logits[t, h]) from float32 rows. Returns o float32 [T, heads * value_dim]. ``q_lens`` (host numbers: the
+    tokens of each request, known for one request without it) only decides whether long portions go four tokens at a time."""
     for name, ten in (("q", q), ("k", k), ("v", v)):
         _check(ten, name, q.dtype, 2)
     _check(decay_logits, "decay_logits", torch.float32, 2)
@@ -2084,7 +2105,9 @@ def delta_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_logits: 
         # what the recurrence reads of every token, made once, float32: unit q and k, the decays, v, beta and k.q
         fn = _fn("hybrid", "ti_delta_quads_floats")
         fn.restype = ctypes.c_longlong
-        quads = int(fn(int(num_seqs), t, heads, key_dim, value_dim)) if DELTA_QUADS else 0
+        lens = q_lens or ([t] if num_seqs == 1 else [1])
+        wanted = delta_quads_pay(lens, heads, key_dim, value_dim) if DELTA_QUADS is None else DELTA_QUADS
+        quads = int(fn(int(num_seqs), t, heads, key_dim, value_dim)) if wanted else 0
         work = torch.empty(quads or t * (2 * groups * key_dim + heads * (key_dim + value_dim + 1) + groups) + 24,
                            dtype=torch.float32, device=q.device)
         args = [out.data_ptr(), state.data_ptr(), stride, q.data_ptr(), q.shape[1], int(q_offset),

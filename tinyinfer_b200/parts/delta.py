@@ -92,7 +92,8 @@ class ChannelDelta(Mixer):
         o = ops.delta_scan(conv, conv, conv, decay, beta, a_log=self.a_log, dt_bias=self.dt_bias, state=state,
                            heads=s.num_heads, groups=s.num_kv_heads, key_dim=s.key_dim, value_dim=s.value_dim,
                            q_offset=0, k_offset=nq, v_offset=nq + nk, q_scale=s.key_dim ** -0.5, unit_eps=s.unit_eps,
-                           cu_seqlens=step.cu_seqlens, state_slots=step.state_slots, num_seqs=step.num_seqs)
+                           cu_seqlens=step.cu_seqlens, state_slots=step.state_slots, num_seqs=step.num_seqs,
+                           q_lens=step.q_lens)
         return ops.gated_group_norm(o, gate, self.norm_w, group=s.value_dim, eps=s.norm_eps, gate_first=False,
                                     out_dtype=self.dtype, gate_activation="sigmoid")
 
