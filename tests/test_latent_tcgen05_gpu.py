@@ -89,3 +89,21 @@ def test_a_value_that_is_no_number_reaches_no_token_before_its_own(monkeypatch, 
     row, end = at - (work[0][0] - work[0][1]), work[0][1]             # the token's place in the step
     assert torch.equal(got[:row], clean[:row]) and torch.equal(got[end:], clean[end:])
     assert torch.equal(got[row:end].isnan(), warp_level[row:end].isnan()) and got[row:end].isnan().any()
+
+
+@pytest.mark.parametrize("tc", [True, False])
+def test_a_key_without_a_page_is_reported_to_the_caller_s_word_alone(monkeypatch, tc):
+    from tinyinfer_b200 import ops
+    from tinyinfer_b200.engine.batch import BatchBuffers, StepEntry
+    monkeypatch.setattr(ops, "LATENT_TCGEN05", tc)
+    heads, rank, rot, page = 16, 512, 64, 64
+    buffers = BatchBuffers(torch.device("cuda"), 100, 1, 4, 1)
+    step = buffers.build([StepEntry(0, [0] * 100, [])], [100], [0], [[[0, 1, -1, 3]]])     # keys 128 .. 191 have no page
+    cache = torch.zeros(1, 4, 1, page, rank + rot, dtype=torch.bfloat16, device="cuda")
+    q = torch.zeros(100, heads * (rank + rot), device="cuda")
+    word = torch.zeros(2, dtype=torch.int32, device="cuda")
+    for status in (word[:1], None):
+        ops.latent_attention(q, cache, heads=heads, rank=rank, rot=rot, scale=0.1, sink=None, positions=step.positions,
+                             token_seq=step.token_seq, block_table=step.block_tables[0], max_context=200, step=step, status=status)
+    assert word.tolist() == [2, 0]
+    ops.check_kernel_status()                            # nothing in the device's own words

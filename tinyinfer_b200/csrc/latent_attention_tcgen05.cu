@@ -38,7 +38,7 @@ struct Args {
     float scale;
     int splits, tpb, hpb, chunks, value_halves;
     int smem_chunks;                                              // of the rows' features in shared memory, the others in tensor memory
-    int* status;                                                  // [0] a wait that ran out, [1] a key without a page
+    int *status, *page_status;                                    // a wait that ran out, a key without a page; either may be null
 };
 
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
                 const int page = logical < a.max_blocks ? table[logical] : -1;
                 int row = a.num_pages * a.page_size;               // outside the map: zeros
                 if (page >= 0 && page < a.num_pages) row = page * a.page_size + key % a.page_size;
-                else if (key < last_key && a.status) atomicExch(a.status + 1, 2);     // a visible key without a page
+                else if (key < last_key && a.page_status) atomicExch(a.page_status, 2);     // a visible key without a page
                 tma_load_2d(smem_u32(ring + s * stage_bytes + chunk * (KT * 128) + piece * a.piece_rows * 128), &map, kv_full(s), chunk * 64, row);
             }
         }
@@ -435,11 +435,11 @@ TI_API int ti_latent_attend_tc_ctas(int num_tokens, int num_seqs, int heads, int
 }
 
 // Every token's keys 0 .. its position (no window). q [T, heads, rank + rot] float32 or, q_bf16, bfloat16; out bfloat16 [T, heads, rank]; splits > 1:
-// the keys are shared out over grid z and the parts are left for ti_latent_merge. status: two words, or null.
+// the keys are shared out over grid z and the parts are left for ti_latent_merge. status (may be null): set if a wait runs out; page_status (may be null): if a visible key has no page.
 TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, const void* q, int q_bf16, const void* cache, const float* sink,
                                const int* positions, const int* cu_seqlens, const int* block_table, int max_blocks, int num_seqs,
                                int num_tokens, int heads, int rank, int rot, int page_size, int num_pages, float scale, int splits,
-                               int* status, cudaStream_t stream) {
+                               int* status, int* page_status, cudaStream_t stream) {
     TI_REQUIRE(num_tokens >= 0 && num_seqs > 0 && num_pages > 0, "latent_attend_tc: bad sizes");
     if (num_tokens == 0) return 0;
     const int ctas = ti_latent_attend_tc_ctas(num_tokens, num_seqs, heads, rank, rot, page_size);
@@ -452,7 +452,7 @@ TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, 
     lt::Args a;
     a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q_bf16 ? nullptr : (const float*)q; a.cache = (const __nv_bfloat16*)cache; a.sink = sink; a.positions = positions; a.cu_seqlens = cu_seqlens;
     a.block_table = block_table; a.max_blocks = max_blocks; a.num_seqs = num_seqs; a.heads = heads; a.rank = rank; a.rot = rot;
-    a.page_size = page_size; a.num_pages = num_pages; a.scale = scale; a.splits = splits; a.status = status;
+    a.page_size = page_size; a.num_pages = num_pages; a.scale = scale; a.splits = splits; a.status = status; a.page_status = page_status;
     a.hpb = heads < lt::QM ? heads : lt::QM;
     a.tpb = lt::QM / a.hpb;
     a.chunks = (rank + rot + 63) / 64;

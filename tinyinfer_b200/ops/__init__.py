@@ -69,7 +69,7 @@ _SIGNATURES = {
                                  c_void_p, c_void_p],
         "ti_latent_attend_tc_ctas": [c_int, c_int, c_int, c_int, c_int, c_int],
         "ti_latent_attend_tc": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,
-                                c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
+                                c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p],
         "ti_causal_conv": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                            c_int, c_int, c_int, c_int, c_void_p],
         "ti_gated_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
@@ -1113,7 +1113,8 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
     (a host number, the longest context of the step) only decides over how many blocks the keys are shared.
     ``step`` (the StepContext): with it a bfloat16 cache whose rows are a multiple of 8 features runs on the
     tensor cores, prompt portions and decoded tokens in their own forms; without it, or in float32, the
-    float32-arithmetic kernel runs. ``window``: a query sees only the last so many keys, itself included."""
+    float32-arithmetic kernel runs. ``window``: a query sees only the last so many keys, itself included. ``status``: an int32
+    word that a visible key without a page sets to 2."""
     _check(q_rows, "q_rows", None, 2)
     _check(cache, "cache", None, 5)
     ctas = _latent_tc_ctas(q_rows.shape[0], cache, heads, rank, rot, window, step) if q_rows.data_ptr() % 16 == 0 else 0
@@ -1158,7 +1159,7 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
             _run("latent", "ti_latent_attend_tc", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), int(q_rows.dtype == torch.bfloat16),
                  cache.data_ptr(), _ptr(sink), positions.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(), block_table.shape[1],
                  step.num_seqs, t, heads, rank, rot, page_size, cache.shape[1], float(scale), splits,
-                 status_words(cache.device).data_ptr(), _stream())
+                 kernel_status(cache.device).data_ptr(), _ptr(status), _stream())
             if splits > 1:
                 _run("latent", "ti_latent_merge", out.data_ptr(), parts.data_ptr(), _ptr(sink), t, heads, rank, splits,
                      _dtype_code(cache), _stream())
