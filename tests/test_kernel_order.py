@@ -44,3 +44,12 @@ def test_copies_land_whichever_wait_ran_out(name):
     assert text.rindex("mbar_wait", 0, land) < text.rindex("sync", 0, land)             # every role's waits, the barrier, the look
     freed = re.search(r"tmem_dealloc\(|tcgen05\.dealloc", text)
     assert freed is None or land < freed.start()
+
+
+def test_a_wait_s_number_names_its_kernel():
+    """What a status word tells of a wait that ran out is its number alone."""
+    whose = {}
+    for path in sorted(CSRC.glob("*.cu")):
+        for code in re.findall(r"(?:abort_flag, [pa]\.status|atomicExch\(p\.status), (\d\d)\)", path.read_text()):
+            whose.setdefault(code, set()).add(path.name)
+    assert len(whose) > 40 and all(len(files) == 1 for files in whose.values()), whose

@@ -74,7 +74,7 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % GT_STAGES;
                     const uint32_t ph = (it / GT_STAGES) & 1u;
-                    if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, 31)) { ok = false; break; }
+                    if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, p.status, 51)) { ok = false; break; }
                     mbar_expect_tx(full_bar(s), GT_STAGE_BYTES);
                     const uint32_t a_dst = smem_u32(stages + s * GT_STAGE_BYTES);
                     tma_load_2d(a_dst, &map_x, full_bar(s), kb * GT_BK, row0);
@@ -90,13 +90,13 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             bool ok = true;
             for (int unit = blockIdx.x; ok && unit < num_units; unit += gridDim.x, ++unit_i) {
                 const uint32_t as = unit_i & 1u, aph = (unit_i >> 1) & 1u;
-                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 32)) { ok = false; break; }
+                if (!mbar_wait_warp(acc_empty_bar(as), aph ^ 1u, abort_flag, p.status, 52)) { ok = false; break; }
                 tmem_fence_after();
                 const uint32_t d_tmem = tmem_base + as * GT_BN;
                 for (int kb = 0; kb < num_kb; ++kb, ++it) {
                     const int s = it % GT_STAGES;
                     const uint32_t ph = (it / GT_STAGES) & 1u;
-                    if (!mbar_wait_warp(full_bar(s), ph, abort_flag, p.status, 33)) { ok = false; break; }
+                    if (!mbar_wait_warp(full_bar(s), ph, abort_flag, p.status, 53)) { ok = false; break; }
                     tmem_fence_after();
                     const uint32_t a_addr = smem_u32(stages + s * GT_STAGE_BYTES);
                     const uint64_t adesc = make_sw128_desc(a_addr);
@@ -119,7 +119,7 @@ moe_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_
             const int tile = unit / p.col_tiles, ct = unit % p.col_tiles;
             const int row0 = p.tiles[3 * tile + 1], rows = p.tiles[3 * tile + 2];
             const uint32_t as = unit_i & 1u, aph = (unit_i >> 1) & 1u;
-            if (!mbar_wait(acc_full_bar(as), aph, abort_flag, p.status, 34)) { ok = false; break; }
+            if (!mbar_wait(acc_full_bar(as), aph, abort_flag, p.status, 54)) { ok = false; break; }
             tmem_fence_after();
             const uint32_t t_addr = tmem_base + as * GT_BN + ((uint32_t)(lane_group * 32) << 16);
             const bool live = r < rows;

@@ -197,8 +197,8 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             const int s = j % STAGES;
             int go = 1;
             if (lane == 0) {
-                go = mbar_wait(kv_empty(s), ((j / STAGES) & 1u) ^ 1u, abort_flag, a.status, 81) ? 1 : 0;
-                if (j == 1 && go) go = mbar_wait(q_full, 0, abort_flag, a.status, 82) ? 1 : 0;      // the rows' chunks have left the ring
+                go = mbar_wait(kv_empty(s), ((j / STAGES) & 1u) ^ 1u, abort_flag, a.status, 71) ? 1 : 0;
+                if (j == 1 && go) go = mbar_wait(q_full, 0, abort_flag, a.status, 72) ? 1 : 0;      // the rows' chunks have left the ring
                 if (go) mbar_expect_tx(kv_full(s), (uint32_t)stage_bytes);
             }
             if (!__shfl_sync(0xffffffffu, go, 0)) break;
@@ -220,12 +220,12 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             const uint64_t q_desc = make_sw128_desc(smem_u32(q_tile));
             const uint64_t k_desc = make_sw128_desc(smem_u32(ring));
             const uint64_t v_desc = make_sw128_desc_mn(smem_u32(ring) + vhalf * (NV / 64) * (KT * 128), KT * 128, 1024);
-            bool go = mbar_wait_warp(q_full, 0, abort_flag, a.status, 82);
+            bool go = mbar_wait_warp(q_full, 0, abort_flag, a.status, 72);
             tmem_fence_after();
             auto issue_s = [&](int j) {                            // scores of tile j into buffer j % 2
                 const int s = j % STAGES, b = j & 1;
-                if (!mbar_wait_warp(kv_full(s), (j / STAGES) & 1u, abort_flag, a.status, 83)) return false;
-                if (!mbar_wait_warp(s_empty(b), ((j >> 1) & 1u) ^ 1u, abort_flag, a.status, 84)) return false;
+                if (!mbar_wait_warp(kv_full(s), (j / STAGES) & 1u, abort_flag, a.status, 73)) return false;
+                if (!mbar_wait_warp(s_empty(b), ((j >> 1) & 1u) ^ 1u, abort_flag, a.status, 74)) return false;
                 tmem_fence_after();
                 const uint64_t kd = k_desc + (uint64_t)((s * stage_bytes) >> 4);
                 const uint32_t d = tmem_base + S_COL + b * KT;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             if (go) go = issue_s(0);
             for (int j = 0; j < num_tiles && go; ++j) {
                 if (j + 1 < num_tiles) go = issue_s(j + 1);
-                if (!go || !mbar_wait_warp(p_full, j & 1u, abort_flag, a.status, 85)) break;
+                if (!go || !mbar_wait_warp(p_full, j & 1u, abort_flag, a.status, 75)) break;
                 tmem_fence_after();
                 const uint64_t vd = v_desc + (uint64_t)(((j % STAGES) * stage_bytes) >> 4);
 #pragma unroll
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
         // ------------------------------------------------------------ rows and softmax (warps 2..9)
         const int etid = threadIdx.x - 64;
         if (a.q == nullptr) {
-            ok = mbar_wait_warp(q_landed, 0, abort_flag, a.status, 89);
+            ok = mbar_wait_warp(q_landed, 0, abort_flag, a.status, 79);
         } else {
             const int chunks8 = a.chunks * 8, total = QM * chunks8;
 #pragma unroll 12
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
         for (int j = 0; j < num_tiles && ok; ++j) {
             const int b = j & 1, key0 = first_key + j * KT;
             // a warp's threads stay together: tensor memory is read and written by whole warps
-            ok = __all_sync(0xffffffffu, mbar_wait(s_full(b), (j >> 1) & 1u, abort_flag, a.status, 86));
+            ok = __all_sync(0xffffffffu, mbar_wait(s_full(b), (j >> 1) & 1u, abort_flag, a.status, 76));
             if (!ok) break;
             tmem_fence_after();
             float v[KT], e[KH];
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
 #pragma unroll
             for (int i = 0; i < 8; ++i) pk[i] = pack2(e[2 * i], e[2 * i + 1]);
             if (j > 0) {                                           // O and P are free when the product before has ended
-                ok = __all_sync(0xffffffffu, mbar_wait(o_full, (j - 1) & 1u, abort_flag, a.status, 87));
+                ok = __all_sync(0xffffffffu, mbar_wait(o_full, (j - 1) & 1u, abort_flag, a.status, 77));
                 if (!ok) break;
                 tmem_fence_after();
                 if (__any_sync(0xffffffffu, corr != 1.f)) {
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full);
         }
-        if (ok && num_tiles > 0) ok = __all_sync(0xffffffffu, mbar_wait(o_full, (num_tiles - 1) & 1u, abort_flag, a.status, 88));
+        if (ok && num_tiles > 0) ok = __all_sync(0xffffffffu, mbar_wait(o_full, (num_tiles - 1) & 1u, abort_flag, a.status, 78));
         sum_xch[half][r] = l_run;
     }
     __syncthreads();                                               // every role has ended, well or not
