@@ -1086,7 +1086,7 @@ LATENT_SPLIT_MIN_KEYS = 128     # a split of the keys over blocks gets at least 
 LATENT_TARGET_BLOCKS = 296      # enough blocks to have two on every SM
 LATENT_TCGEN05 = True           # prompt portions on tcgen05 where its sizes allow
 LATENT_TC_CTAS = 148            # a CTA of that form has an SM to itself
-LATENT_TC_SPLIT_MIN_KEYS = 256
+LATENT_TC_SPLIT_MIN_KEYS = 128  # 8 tokens behind 1,024: 31 us, with 256 keys a share 37; one head of 64, 8 behind 1,024: 23 and 27
 
 
 def _latent_tc_ctas(t: int, cache: torch.Tensor, heads: int, rank: int, rot: int, window: Optional[int], step) -> int:
