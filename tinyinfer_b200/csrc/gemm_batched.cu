@@ -112,6 +112,12 @@ __global__ void __launch_bounds__(mt::THREADS) gemm_batched_mma_kernel(
     });
 }
 
+// Whether ti_gemm_batched runs a bfloat16 product without bias, activation or gate in the tcgen05 form.
+TI_API int ti_gemm_batched_tc_ok(const void* out, const void* x, const void* w, int batch, int M, int N, int K, long long ldx, long long sx,
+                                 long long ldo, long long so, int out_f32) {
+    return gbt_takes(out, x, w, batch, M, N, K, ldx, sx, K, (long long)N * K, ldo, so, out_f32) ? 1 : 0;
+}
+
 // status (may be null): set if a wait of the tcgen05 form runs out. form: 0 whichever takes it, 1 not the tcgen05 form.
 TI_API int ti_gemm_batched(void* out, const void* x, const void* w, const float* bias, int batch, int M, int N, int K,
                            long long ldx, long long sx, long long ldw, long long sw, long long ldo, long long so,

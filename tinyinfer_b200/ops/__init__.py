@@ -55,6 +55,7 @@ _SIGNATURES = {
         "ti_relu_squared": [c_void_p, c_void_p, c_ll, c_int, c_void_p],
         "ti_gemm_batched": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_ll,
                             c_ll, c_ll, c_ll, c_int, c_int, c_void_p, c_ll, c_ll, c_int, c_int, c_void_p, c_void_p],
+        "ti_gemm_batched_tc_ok": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_ll, c_ll, c_ll, c_ll, c_int],
         "ti_latent_prepare": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_float, c_int, c_int, c_int,
                               c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                               c_int, c_void_p, c_int, c_void_p],
