@@ -107,3 +107,34 @@ def test_a_key_without_a_page_is_reported_to_the_caller_s_word_alone(monkeypatch
                              token_seq=step.token_seq, block_table=step.block_tables[0], max_context=200, step=step, status=status)
     assert word.tolist() == [2, 0]
     ops.check_kernel_status()                            # nothing in the device's own words
+
+
+@pytest.mark.parametrize("heads,rank,rot,decoded,portion", [(16, 512, 64, [4200] + [70] * 8, (70, 70)), (4, 128, 32, [33, 5000], (300, 100))])
+def test_decoded_tokens_behind_many_keys_take_their_own_form(heads, rank, rot, decoded, portion):
+    """Beside a portion they come out as in a step of their own, and so does the portion."""
+    from tinyinfer_b200 import ops
+    from tinyinfer_b200.engine.batch import BatchBuffers, StepEntry
+    gen = torch.Generator().manual_seed(heads)
+    dk, page, work = rank + rot, 64, [(c, 1) for c in decoded] + [portion]
+    pages = [-(-c // page) for c, _ in work]
+    tables = [list(range(sum(pages[:i]), sum(pages[:i + 1]))) for i in range(len(work))]
+    cache = torch.randn(1, sum(pages), 1, page, dk, generator=gen).bfloat16().cuda()
+    q = torch.randn(sum(n for _, n in work), heads * dk, generator=gen).bfloat16().cuda()
+
+    def run(some):
+        mine = work[some]
+        buffers = BatchBuffers(torch.device("cuda"), 400, len(mine), max(pages), 1)
+        step = buffers.build([StepEntry(i, [0] * n, []) for i, (_, n) in enumerate(mine)], [c - n for c, n in mine], [0] * len(mine), [tables[some]])
+        first = sum(n for _, n in work[:some.start or 0])
+        rows = q[first:first + step.num_tokens]
+        kind = ops.latent_rows_dtype(step.num_tokens, cache, heads=heads, rank=rank, rot=rot, step=step)
+        out = ops.latent_attention(rows.to(kind), cache, heads=heads, rank=rank, rot=rot, scale=dk ** -0.5, sink=None, positions=step.positions,
+                                   token_seq=step.token_seq, block_table=step.block_tables[0], max_context=max(c for c, _ in mine), step=step)
+        return out, ops.latent_decoded_apart(step.q_lens, step.starts)
+
+    n = len(decoded)
+    both, apart = run(slice(0, n + 1))
+    alone, portion_alone = run(slice(0, n)), run(slice(n, n + 1))
+    ops.check_kernel_status()
+    assert apart == n and alone[1] == portion_alone[1] == 0
+    assert torch.equal(both[:n], alone[0]) and torch.equal(both[n:], portion_alone[0])

@@ -50,3 +50,21 @@ def test_linear_attention_in_chunks(lens, heads, dim, chunked):
 ])
 def test_delta_rule_by_quads(lens, heads, dim, quads):
     assert ops.delta_quads_pay(lens, heads, dim, dim) is quads
+
+
+@pytest.mark.parametrize("decoded,keys,portion,apart", [
+    (1, 1024, [512], False),                  # us together and apart: 66, 68
+    (1, 2048, [512], True),                   # 117, 72
+    (1, 8192, [64], True),                    # 86, 61
+    (1, 2048, [64], False),                   # 43, 49
+    (8, 4096, [8], False),                    # 55, 66
+    (16, 2048, [8], True),                    # 62, 57
+    (27, 4096, [60, 4], True),                # 221, 107
+    (27, 4096, [], False),                    # decoded tokens alone
+    (0, 0, [64, 300], False),
+])
+def test_decoded_tokens_beside_a_portion_of_latent_attention(decoded, keys, portion, apart):
+    lens = [1] * decoded + portion
+    starts = [keys - 1] * decoded + [0] * len(portion)
+    assert ops.latent_decoded_apart(lens, starts) == (decoded if apart else 0)
+    assert ops.latent_decoded_apart(portion + [1] * decoded, [0] * len(portion) + [keys - 1] * decoded) == 0     # not ahead of the portions

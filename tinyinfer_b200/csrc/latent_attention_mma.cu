@@ -1,5 +1,6 @@
 // The attention over a cached latent (see latent_attention.cu for the mechanism) on the warp-level tensor cores,
-// bfloat16: the prompt-portion and the decode form of the same kernel.
+// bfloat16: the decode form, and a form for the prompt portions that latent_attention_tcgen05.cu does not take: windows, ranks other
+// than 64, 128, 256 and 512, rows of more than 576 features, pages that are not of whole 16 keys, a cache that TMA cannot start at.
 //
 // The rows of a block's query tile are (token, head) pairs: every head of a token reads the same cached rows
 // [c | k_rot], so the heads fill the 16-row tiles of mma.sync that a single token's head could not. A block of
@@ -35,7 +36,8 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
 struct Args {
     __nv_bfloat16* out;
     float* parts;
-    const float* q;
+    const void* q;                 // float32, or with q_bf16 bfloat16
+    int q_bf16;
     const __nv_bfloat16* cache;
     const float* sink;
     const int *positions, *token_seq, *cu_seqlens, *block_table;
@@ -108,10 +110,17 @@ __global__ void __launch_bounds__(128 * MW, PER_SM) latent_attend_mma_kernel(Arg
 #pragma unroll 4
         for (int i = tid; i < ROWS * quads; i += THREADS) {
             const int r = i / quads, c = (i % quads) * 4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (row_tok[r] >= 0 && c < dk)
-                v = *reinterpret_cast<const float4*>(a.q + ((size_t)row_tok[r] * a.heads + row_head[r]) * dk + c);
-            *reinterpret_cast<uint2*>(Qs + r * lds + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+            uint2 w = make_uint2(0u, 0u);
+            if (row_tok[r] >= 0 && c < dk) {
+                const size_t at = ((size_t)row_tok[r] * a.heads + row_head[r]) * dk + c;
+                if (a.q_bf16) {
+                    w = *reinterpret_cast<const uint2*>((const __nv_bfloat16*)a.q + at);
+                } else {
+                    const float4 v = *reinterpret_cast<const float4*>((const float*)a.q + at);
+                    w = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+                }
+            }
+            *reinterpret_cast<uint2*>(Qs + r * lds + c) = w;
         }
     }
     const int hi = a.positions[tok0 + ntok - 1];              // the block's last token sees the most keys,
@@ -317,8 +326,8 @@ static cudaError_t launch(const Args& a, dim3 grid, size_t smem, cudaStream_t st
 TI_API int ti_latent_attend_mma_ok(int rank, int rot) { return (rank + rot) % 8 == 0 && rank <= 512 && rank > 0 ? 1 : 0; }
 
 // decode != 0: every token is a block of its own (its heads are the rows); else blocks of 32 rows are dealt to the
-// requests' consecutive tokens, two blocks an SM. q float32 [T, heads, rank + rot]; out bfloat16 [T, heads, rank].
-TI_API int ti_latent_attend_mma(void* out, float* parts, long long parts_floats, const float* q, const void* cache,
+// requests' consecutive tokens, two blocks an SM. q float32 or, q_bf16, bfloat16 [T, heads, rank + rot]; out bfloat16 [T, heads, rank].
+TI_API int ti_latent_attend_mma(void* out, float* parts, long long parts_floats, const void* q, int q_bf16, const void* cache,
                                 const float* sink, const int* positions, const int* token_seq, const int* cu_seqlens,
                                 const int* block_table, int max_blocks, int num_seqs, int num_tokens, int heads, int rank,
                                 int rot, int page_size, int num_pages, float scale, int window, int splits, int decode,
@@ -332,7 +341,7 @@ TI_API int ti_latent_attend_mma(void* out, float* parts, long long parts_floats,
     const int mw = decode ? 1 : 2, kbuf = decode ? 2 : 1;
     const int rows = 16 * mw;
     lm::Args a;
-    a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q; a.cache = (const __nv_bfloat16*)cache; a.sink = sink;
+    a.out = (__nv_bfloat16*)out; a.parts = parts; a.q = q; a.q_bf16 = q_bf16; a.cache = (const __nv_bfloat16*)cache; a.sink = sink;
     a.positions = positions; a.token_seq = token_seq; a.cu_seqlens = cu_seqlens; a.block_table = block_table;
     a.max_blocks = max_blocks; a.num_seqs = num_seqs; a.num_tokens = num_tokens; a.heads = heads; a.rank = rank; a.rot = rot;
     a.page_size = page_size; a.num_pages = num_pages; a.scale = scale; a.window = window; a.splits = splits; a.status = status;

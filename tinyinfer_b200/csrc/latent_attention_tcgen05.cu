@@ -5,8 +5,10 @@
 //   warp 0      TMA: tiles of 32 cached rows through the block table, 64 features a copy, into a ring of four
 //   warp 1      issues S = Q K^T (128 x 32, two buffers in tensor memory) and O += P V, P from tensor memory, V the
 //               first features of the same shared-memory tile read as an MN-major operand
-//   warps 2..9  the rows, rounded to bfloat16 (or brought so, by TMA), into shared and tensor memory; then the softmax: two threads a row, each 16 of a tile's keys and
-//               half of O's columns. O stays in tensor memory and is multiplied there when a row of the warp has a new maximum.
+//   warps 2..9  the rows, brought as bfloat16 by TMA, their last features into tensor memory; then the softmax: two threads a row, each
+//               16 of a tile's keys and half of O's columns. O stays in tensor memory and is multiplied there when a row of the warp has
+//               a new maximum. (Rows of float32, which a caller with rows of its own may have, these warps fetch and round; the model's
+//               kernels leave bfloat16.)
 //
 // The rows' last features, up to 320 of them, are read by the MMAs from tensor memory: with all 576 in shared memory it would hold a
 // ring of two tiles alone, each refilled only when its products with P are through. 2,048 tokens over 16 heads of rank 512, a
@@ -133,13 +135,15 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
     }
     if (warp == 1) tmem_alloc(&tmem_base_sh, TMEM_COLS);
     ti_grid_wait();
-    // the tokens of this CTA: row tiles are dealt request by request, the last (the longest key ranges) to the first CTAs
+    // the tokens of this CTA: row tiles are dealt request by request, the last to the first CTAs (a prompt's longest key ranges; decoded
+    // tokens, which a step has before its portions and whose ranges may be longer still, start last, and have a form of their own then)
     const int place = (int)gridDim.x - 1 - (int)blockIdx.x;
     if (threadIdx.x == 64) {
         const int tile = place / a.value_halves;
         int at = 0, seq = -1, first = 0, n = 0;
+        const int base = a.cu_seqlens[0];                          // requests before these may lie ahead of the rows
         for (int s = 0; s < a.num_seqs; ++s) {
-            const int r0 = a.cu_seqlens[s], len = a.cu_seqlens[s + 1] - r0, nb = (len + a.tpb - 1) / a.tpb;
+            const int r0 = a.cu_seqlens[s] - base, len = a.cu_seqlens[s + 1] - base - r0, nb = (len + a.tpb - 1) / a.tpb;
             if (tile < at + nb) {
                 seq = s;
                 first = r0 + (tile - at) * a.tpb;
@@ -444,7 +448,7 @@ TI_API int ti_latent_attend_tc_ctas(int num_tokens, int num_seqs, int heads, int
     return ((num_tokens + tpb - 1) / tpb + num_seqs - 1) * ((heads + hpb - 1) / hpb) * (rank > 256 ? 2 : 1);
 }
 
-// Every token's keys 0 .. its position (no window). q [T, heads, rank + rot] float32 or, q_bf16, bfloat16; out bfloat16 [T, heads, rank]; splits > 1:
+// Every token's keys 0 .. its position (no window). cu_seqlens counts from its first entry on. q [T, heads, rank + rot] float32 or, q_bf16, bfloat16; out bfloat16 [T, heads, rank]; splits > 1:
 // the keys are shared out over grid z and the parts are left for ti_latent_merge. status (may be null): set if a wait runs out; page_status (may be null): if a visible key has no page.
 TI_API int ti_latent_attend_tc(void* out, float* parts, long long parts_floats, const void* q, int q_bf16, const void* cache, const float* sink,
                                const int* positions, const int* cu_seqlens, const int* block_table, int max_blocks, int num_seqs,

@@ -65,7 +65,7 @@ _SIGNATURES = {
                              c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_void_p, c_int, c_void_p],
         "ti_latent_merge": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "ti_latent_attend_mma_ok": [c_int, c_int],
-        "ti_latent_attend_mma": [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+        "ti_latent_attend_mma": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int, c_int,
                                  c_void_p, c_void_p],
         "ti_latent_attend_tc_ctas": [c_int, c_int, c_int, c_int, c_int, c_int],
@@ -1104,6 +1104,25 @@ def latent_rows_dtype(tokens: int, cache: torch.Tensor, *, heads: int, rank: int
     return cache.dtype if _latent_tc_ctas(tokens, cache, heads, rank, rot, window, step) else torch.float32
 
 
+def latent_decoded_apart(q_lens: Sequence[int], starts: Sequence[int]) -> int:
+    """How many decoded tokens, which a step has before its portions, take the decode form in a launch of their own: all, or none.
+
+    Together with a portion a token has a CTA of the portions' form to itself, 16 of 128 rows, which walks through all of its keys; the
+    decode form shares them out, at the price of two launches. Us for 16 heads of rank 512, together and apart: 512 tokens beside one
+    token at 1,024 keys 66, 68, at 2,048 117, 72, at 8,192 410, 82; 64 beside one at 2,048 43, 49, at 8,192 86, 61; beside 8 at 2,048
+    53, 53, beside 16 80, 57, beside 27 at 1,024 70, 60, at 4,096 221, 107; 8 beside 8 at 4,096 55, 66, beside 16 at 2,048 62, 57, at 8,192
+    164, 98, beside 64 at 2,048 129, 138, at 8,192 424, 385. (All at warp level 8 beside 27 at 1,024 took 47, here 53, and 8 beside 64 at
+    8,192 363.)"""
+    alone = 0
+    while alone < len(q_lens) and q_lens[alone] == 1:
+        alone += 1
+    if not alone or alone == len(q_lens):
+        return 0
+    keys, rest = max(starts[:alone]) + 1, sum(q_lens[alone:])
+    pays = keys >= 2048 and (rest >= 256 or alone >= 16) or keys >= 4096 and rest >= 64
+    return alone if pays else 0
+
+
 def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, rank: int, rot: int, scale: float,
                      sink: Optional[torch.Tensor], positions: torch.Tensor, token_seq: torch.Tensor,
                      block_table: torch.Tensor, max_context: int, window: Optional[int] = None, step=None,
@@ -1137,49 +1156,61 @@ def latent_attention(q_rows: torch.Tensor, cache: torch.Tensor, *, heads: int, r
 
     reach = min(int(max_context), int(window)) if window else int(max_context)     # keys a query can see at most
 
-    def share_out(blocks: int, least: int = LATENT_SPLIT_MIN_KEYS) -> int:
+    def share_out(blocks: int, reach: int, least: int = LATENT_SPLIT_MIN_KEYS) -> int:
         if blocks < LATENT_TARGET_BLOCKS and reach >= 2 * least:
             return max(1, min(-(-LATENT_TARGET_BLOCKS // blocks), reach // least, 64))
         return 1
 
-    def scratch(splits: int):
+    def scratch(rows: int, splits: int):
         if splits == 1:
             return None, 0
-        parts = _decode_scratch(cache.device, t * heads * splits * (rank + 2))
+        parts = _decode_scratch(cache.device, rows * heads * splits * (rank + 2))
         return parts, parts.numel()
+
+    def merge(out: torch.Tensor, parts: torch.Tensor, splits: int) -> None:
+        _run("latent", "ti_latent_merge", out.data_ptr(), parts.data_ptr(), _ptr(sink), out.shape[0], heads, rank, splits,
+             _dtype_code(cache), _stream())
+
+    def portions(first: int, ctas: int, reach: int) -> None:          # the requests from `first` on, one token each before it
+        q, o = q_rows[first:], out[first:]
+        splits = 1
+        if ctas < LATENT_TC_CTAS and reach >= 2 * LATENT_TC_SPLIT_MIN_KEYS:
+            splits = max(1, min(LATENT_TC_CTAS // ctas, reach // LATENT_TC_SPLIT_MIN_KEYS, 64))
+        parts, parts_floats = scratch(t - first, splits)
+        _run("latent", "ti_latent_attend_tc", o.data_ptr(), _ptr(parts), parts_floats, q.data_ptr(), int(q.dtype == torch.bfloat16),
+             cache.data_ptr(), _ptr(sink), positions[first:].data_ptr(), step.cu_seqlens[first:].data_ptr(), block_table[first:].data_ptr(),
+             block_table.shape[1], step.num_seqs - first, t - first, heads, rank, rot, cache.shape[3], cache.shape[1], float(scale), splits,
+             kernel_status(cache.device).data_ptr(), _ptr(status), _stream())
+        if splits > 1:
+            merge(o, parts, splits)
+
+    def warp_level(rows: int, decode: bool, reach: int) -> None:      # the first `rows` tokens
+        lanes = 16 if decode else 32
+        per_block = min(heads, lanes)
+        tokens_per_block = 1 if decode else max(1, lanes // per_block)
+        splits = share_out(-(-rows // tokens_per_block) * -(-heads // per_block), reach, 64 if decode else LATENT_SPLIT_MIN_KEYS)
+        parts, parts_floats = scratch(rows, splits)
+        _run("latent", "ti_latent_attend_mma", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), int(q_rows.dtype == torch.bfloat16),
+             cache.data_ptr(), _ptr(sink), positions.data_ptr(), token_seq.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(),
+             block_table.shape[1], step.num_seqs, rows, heads, rank, rot, cache.shape[3], cache.shape[1], float(scale),
+             int(window or 0), splits, int(decode), _ptr(status), _stream())
+        if splits > 1:
+            merge(out[:rows], parts, splits)
 
     if (step is not None and cache.dtype == torch.bfloat16
             and int(_fn("latent", "ti_latent_attend_mma_ok")(rank, rot))):
-        decode = step.max_q_len == 1
-        page_size = cache.shape[3]
         if ctas:
-            splits = 1
-            if ctas < LATENT_TC_CTAS and reach >= 2 * LATENT_TC_SPLIT_MIN_KEYS:
-                splits = max(1, min(LATENT_TC_CTAS // ctas, reach // LATENT_TC_SPLIT_MIN_KEYS, 64))
-            parts, parts_floats = scratch(splits)
-            _run("latent", "ti_latent_attend_tc", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), int(q_rows.dtype == torch.bfloat16),
-                 cache.data_ptr(), _ptr(sink), positions.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(), block_table.shape[1],
-                 step.num_seqs, t, heads, rank, rot, page_size, cache.shape[1], float(scale), splits,
-                 kernel_status(cache.device).data_ptr(), _ptr(status), _stream())
-            if splits > 1:
-                _run("latent", "ti_latent_merge", out.data_ptr(), parts.data_ptr(), _ptr(sink), t, heads, rank, splits,
-                     _dtype_code(cache), _stream())
-            return out
-        rows = 16 if decode else 32
-        per_block = min(heads, rows)
-        tokens_per_block = 1 if decode else max(1, rows // per_block)
-        splits = share_out(-(-t // tokens_per_block) * -(-heads // per_block), 64 if decode else LATENT_SPLIT_MIN_KEYS)
-        parts, parts_floats = scratch(splits)
-        _run("latent", "ti_latent_attend_mma", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), cache.data_ptr(),
-             _ptr(sink), positions.data_ptr(), token_seq.data_ptr(), step.cu_seqlens.data_ptr(), block_table.data_ptr(),
-             block_table.shape[1], step.num_seqs, t, heads, rank, rot, cache.shape[3], cache.shape[1], float(scale),
-             int(window or 0), splits, int(decode), _ptr(status), _stream())
-        if splits > 1:
-            _run("latent", "ti_latent_merge", out.data_ptr(), parts.data_ptr(), _ptr(sink), t, heads, rank, splits,
-                 _dtype_code(cache), _stream())
+            alone = latent_decoded_apart(step.q_lens, step.starts)
+            if alone:
+                warp_level(alone, True, max(step.starts[:alone]) + 1)
+                ctas = int(_fn("latent", "ti_latent_attend_tc_ctas")(t - alone, step.num_seqs - alone, heads, rank, rot, cache.shape[3]))
+                reach = max(n + start for n, start in zip(step.q_lens[alone:], step.starts[alone:]))
+            portions(alone, ctas, reach)
+        else:
+            warp_level(t, step.max_q_len == 1, reach)
         return out
-    splits = share_out(t * ((heads + 7) // 8))
-    parts, parts_floats = scratch(splits)
+    splits = share_out(t * ((heads + 7) // 8), reach)
+    parts, parts_floats = scratch(t, splits)
     _run("latent", "ti_latent_attend", out.data_ptr(), _ptr(parts), parts_floats, q_rows.data_ptr(), cache.data_ptr(),
          _ptr(sink), positions.data_ptr(), token_seq.data_ptr(), block_table.data_ptr(), block_table.shape[1], t, heads,
          rank, rot, cache.shape[3], cache.shape[1], float(scale), int(window or 0), splits, _ptr(status),
