@@ -13,7 +13,8 @@
 //   them; all lanes fetch the s_i and solve for their two columns' u.
 // Bound by the chain of a quad, 0.72 us of it (sums, five rounds of shuffles, the solve, the update) on one warp a scheduler, beside 26
 // reads of 16 bytes a lane from shared memory. Measured with the prepare kernel, 16 heads of 128 x 128, against the walk: 2,000 tokens
-// 572 -> 405 us, 1,000 285 -> 205, 333 102 -> 76, 128 46 -> 37, 64 30 -> 31, 16 36 -> 41 (host included); 1 to 4 % closer to 64 bits.
+// 572 -> 405 us, 1,000 285 -> 205, 333 102 -> 76, 128 46 -> 37, 64 30 -> 31, 16 36 -> 41 (host included); 1 to 4 % closer to 64 bits. More
+// blocks than run at a time lose: ops.delta_quads_pay.
 // Quads lie at cu_seqlens[i] / 4 + i and behind for request i, so num_tokens / 4 + num_seqs of them hold any division of the tokens
 // among the requests. A request's last quad may be short: rows of zeros, and u_i = 0 by choice, not by product.
 #include "sm100_ptx.cuh"

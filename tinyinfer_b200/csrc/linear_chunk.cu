@@ -10,9 +10,11 @@
 // the requests; those that no request reaches end at once.
 // Products of decays are made in 64 bits and rounded once, and sums over 128 channels in pieces of 32: without, 2,000 tokens of decays
 // of 0.999 came out 1.0e-6 from 64 bits, where the walk has 6.1e-7.
-// Bound by the multiply-adds: 2,000 tokens of 16 heads of 128 x 128 need 2.5 G of them a layer, 70 us of the chip's float32 rate.
+// 2,000 tokens of 16 heads of 128 x 128 are 1.4 G multiply-adds a layer, 39 us of the chip's float32 rate, of 130. The rest is the fold, a
+// third of the time (its threads wait for loads), and operands on their way: the state and out kernels fill the FMA pipe to 46 and 33 %.
 // Measured, three kernels, against the walk in stretches: 2,000 tokens 552 -> 130 us (out 1.7e-7 to 2.8e-7 from 64 bits, the walk
-// 2.0e-7 to 6.1e-7), 1,000 284 -> 68, 333 108 -> 58, 128 75 -> 48.
+// 2.0e-7 to 6.1e-7), 1,000 284 -> 68, 333 108 -> 58, 128 75 -> 48. Decoded tokens and many short portions stay with the walk: see
+// ops.linear_chunks.
 #include "common.cuh"
 
 namespace lc {
