@@ -55,8 +55,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // Whichever wait of a block ran out, copies may be in flight, and get a millisecond to land (they take microseconds) before shared and
 // tensor memory are given up. Where one warp waits for every copy, as the warp that issues a product's MMAs does, it alone knows whether
 // they have landed, and stays when a wait ended it; elsewhere the warp that frees tensor memory looks behind the barrier that ends the
-// roles, or, without such a barrier, every role that a wait ended stays. (That look in the products of few tokens: the 0.6B model's prompt
-// of 37 tokens 1,303 -> 1,310 us, with 112 of them.)
+// roles, or, without such a barrier, every role that a wait ended stays.
 __device__ __forceinline__ void land_copies(volatile int* abort_flag) {
     if (*abort_flag) {
         const unsigned long long t0 = global_ns();
@@ -151,7 +150,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 // what may meet on an SM never needs more than its 512 columns. Every kernel with tensor memory has at least LEAST bytes of dynamic shared
 // memory, so that no three share an SM's 228 KB (two of them 256 columns at most), and one with more than 128 columns has ALONE, which
 // leaves less than LEAST beside it. (Letting the next grid in only behind the allocation would do too, but made a decoded token of the
-// 0.6B model 1,016 -> 1,029 us, its prompt of 37 tokens 1,300 -> 1,311.)
+// 0.6B model 1,012 -> 1,024 us.)
 constexpr int TMEM_SHARED_LEAST = 95 * 1024, TMEM_SHARED_ALONE = 228 * 1024 - TMEM_SHARED_LEAST;
 constexpr bool tmem_shares_sm(int columns, int shared) { return shared >= TMEM_SHARED_ALONE || (columns <= 128 && shared >= TMEM_SHARED_LEAST); }
 // Tensor-memory allocation by one whole warp; the base address lands in *slot (shared memory).
