@@ -104,12 +104,6 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
-// D += A B with A in tensor memory (rows on the lanes, two bfloat16 of k a column), B from shared memory.
-__device__ __forceinline__ void umma_bf16_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t* r) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -131,7 +125,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 template <int D, bool CAP, int FORM>
 __global__ void __launch_bounds__(PP_THREADS, 1)
@@ -290,10 +283,10 @@ prefill_attention_pair_kernel(const __grid_constant__ CUtensorMap q_map, const _
                             // A: 16 keys = 8 columns of packed bfloat16 pairs (P lies over the first 64 of the
                             // tile's 128 score columns); B: 16 key rows of V = 2048 bytes further on (128 in the
                             // descriptor's 16-byte units)
-                            if (leader) umma_bf16_tmem_a(o_tmem, s_tmem, vd, idesc_o, jp[x] > 0 ? 1u : 0u);
+                            if (leader) umma_bf16_ts(o_tmem, s_tmem, vd, idesc_o, jp[x] > 0 ? 1u : 0u);
 #pragma unroll
                             for (int ks = 1; ks < KT / 16; ++ks)
-                                if (leader) umma_bf16_tmem_a(o_tmem, s_tmem + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, 1u);
+                                if (leader) umma_bf16_ts(o_tmem, s_tmem + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, 1u);
                             if (leader) umma_commit(o_full(x));
                             ++jp[x];
                             if (all_issued(jp, v) && leader) umma_commit(kv_empty(b));   // both tiles have read these values

@@ -114,16 +114,6 @@ __device__ __forceinline__ uint64_t make_sw64_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
 }
 
-// A from tensor memory, a row a lane.
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
-}
 
 // The CTA's share of the outputs by multiply-adds in k order, one accumulator an output: out[col][row] for `cols` tokens from
 // m on and the 128 rows of w that the tile has on its lanes. A thread has one row and every fourth token; operands come 32 k at a
@@ -337,7 +327,7 @@ gemm_f32_split_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
 #pragma unroll
                 for (int plane = 0; plane < 3; ++plane) tmem_st8(to + plane * PLANE_A + 8 * h, q[plane]);
             }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tmem_wait_st();
             tmem_fence_before();                             // the MMAs read what was written
             __syncwarp();
             if (lane == 0) mbar_arrive(a_full_bar(stage));

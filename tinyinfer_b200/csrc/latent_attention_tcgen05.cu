@@ -43,12 +43,6 @@ struct Args {
     int *status, *page_status;                                    // a wait that ran out, a key without a page; either may be null
 };
 
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
     const uint32_t* r = reinterpret_cast<const uint32_t*>(v);
     asm volatile(
@@ -59,10 +53,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
           "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
           "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
         : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
 }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -242,7 +232,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
                 for (int c = a.smem_chunks; c < a.chunks; ++c, qt += 32, kk += (KT * 128) >> 4)
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        if (leader) umma_ts(d, qt + 8 * k, kk + 2 * k, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
+                        if (leader) umma_bf16_ts(d, qt + 8 * k, kk + 2 * k, idesc_s, (c > 0 || k > 0) ? 1u : 0u);
                 if (leader) umma_commit(s_full(b));
                 return true;
             };
@@ -254,7 +244,7 @@ __global__ void __launch_bounds__(THREADS, 1) latent_attend_tc_kernel(const __gr
                 const uint64_t vd = v_desc + (uint64_t)(((j % STAGES) * stage_bytes) >> 4);
 #pragma unroll
                 for (int ks = 0; ks < KT / 16; ++ks)
-                    if (leader) umma_ts(tmem_base, tmem_base + P_COL + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+                    if (leader) umma_bf16_ts(tmem_base, tmem_base + P_COL + ks * 8, vd + (uint64_t)(ks * 128), idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
                 if (leader) { umma_commit(o_full); umma_commit(kv_empty(j % STAGES)); }
             }
         }
